@@ -20,7 +20,7 @@
 // (64 bf16 or 32 fp32 columns), writes a chunk into a 128B-swizzled 4 KiB staging buffer of its own (two per
 // warp) and one lane hands it to TMA: a tiled store for bf16 / fp32 outputs, a tiled reduce-add for the
 // "accumulate into an fp32 destination" mode, so the weight-gradient GEMMs never read their destination into
-// the SM. TMA clips rows and columns beyond M and N. The older epilogue (each thread storing its own row with
+// the SM and a tile's K can be split over several CTA pairs (split_k_blocks). TMA clips rows and columns beyond M and N. The older epilogue (each thread storing its own row with
 // 16-byte stores, read-modify-write for the accumulate mode) is kept as a template variant.
 //
 // Fused epilogues (forward GEMMs X W^T with bf16 output only):
@@ -79,6 +79,7 @@ struct EpiArgs {
   int seq;                // RoPE: row r is at position r % seq
   int rot_cols;           // RoPE: columns [0, rot_cols) are rotated (rotated heads x d)
   int group_m;            // tile numbering: rows of tiles per group (all epilogues)
+  int kb_per_split;       // k-blocks per work unit; a tile is one unit unless its K is split (OUT_F32_ACC only, split_k_blocks)
   // cross-entropy statistics (EPI_CE): per row and per 256-column tile the maximum and the sum of exp(logit - maximum)
   // of the ROUNDED logits go to ce_part[row * ce_tiles + n_blk]; the logit of the row's target column goes to ce_tgt[row]
   float2* ce_part;
@@ -148,8 +149,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   const int num_clusters = gridDim.x >> 1;
   const int num_m = (M + 2 * BM - 1) / (2 * BM);
   const int num_n = (EPI == EPI_SWIGLU) ? (N + BN_HALF - 1) / BN_HALF : (N + BN - 1) / BN;
-  const int num_tiles = num_m * num_n;
   const int num_kb = (K + BK - 1) / BK;
+  // Work units: every output tile, once per K split (outermost, so that concurrently running units share operand panels as
+  // before). Several units of a tile add to the same destination with TMA reduce-adds.
+  const int tiles = num_m * num_n;
+  const int kbs = (OUT_MODE == OUT_F32_ACC) ? ea.kb_per_split : num_kb;
+  const int num_tiles = (OUT_MODE == OUT_F32_ACC) ? tiles * ((num_kb + kbs - 1) / kbs) : tiles;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -190,11 +195,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       bool ok = true;
       for (int t = cluster_id; t < num_tiles && ok; t += num_clusters) {
         int m_blk, n_blk;
-        tile_coords(t, num_m, num_n, ea.group_m, m_blk, n_blk);
+        const int split = (OUT_MODE == OUT_F32_ACC) ? t / tiles : 0;
+        tile_coords(t - split * tiles, num_m, num_n, ea.group_m, m_blk, n_blk);
         const int row0 = m_blk * 2 * BM + (int)rank * BM;          // this CTA's rows of A
         // this CTA's columns of B (SwiGLU: gate rows for the leader, the up rows of the same units for its partner)
         const int col0 = (EPI == EPI_SWIGLU) ? n_blk * BN_HALF + (int)rank * ea.inter : n_blk * BN + (int)rank * BN_HALF;
-        for (int kb = 0; kb < num_kb; ++kb) {
+        const int kb_end = min(num_kb, (split + 1) * kbs);
+        for (int kb = split * kbs; kb < kb_end; ++kb) {
           if (!mbar_wait(&bars.empty[stage], phase ^ 1, abort_flag)) {
             report_error(status, KERNEL_ID, 1);
             ok = false;
@@ -243,7 +250,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         }
         tcgen05_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = 0; kb < num_kb; ++kb) {
+        const int split = (OUT_MODE == OUT_F32_ACC) ? t / tiles : 0;
+        const int num_here = min(num_kb - split * kbs, kbs);
+        for (int kb = 0; kb < num_here; ++kb) {
           if (!mbar_wait(&bars.full[stage], phase, abort_flag)) {
             report_error(status, KERNEL_ID, 3);
             ok = false;
@@ -531,7 +540,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       int buf = 0;
       for (int t = cluster_id; t < num_tiles && ok; t += num_clusters, ++local) {
         int m_blk, n_blk;
-        tile_coords(t, num_m, num_n, ea.group_m, m_blk, n_blk);
+        tile_coords(t % tiles, num_m, num_n, ea.group_m, m_blk, n_blk);
         const int acc = local & 1;
         const uint32_t acc_phase = (local >> 1) & 1;
         if (!mbar_wait(&bars.tmem_full[acc], acc_phase, abort_flag)) {
@@ -681,6 +690,28 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
 
 static int g_group_m = 8;   // rows of 256-row tiles per group; measured on the model's shapes: 8 and 16 beat 4 by ~1 %, 1 is worst
 
+// k-blocks per work unit of a GEMM that accumulates into fp32 (weight gradients: K is the number of tokens). With few output
+// tiles a unit per tile leaves most CTA pairs idle behind a long K loop, so K is split over the idle pairs. A unit costs its
+// k-blocks plus about 12 k-blocks' time for its epilogue and the reduce-add traffic of its tile (fitted to a sweep of 1..16
+// splits over the shapes of 20M to 1.7B models); the S with the least waves * unit time wins, S = 1 whenever the tiles alone
+// fill the pairs. Measured (us per launch): 576x576, 8192 tokens: 45.6 -> 12.4 (S = 8); 3072x576, 1803 tokens: 15.5 -> 11.9
+// (S = 2); 6144x2048, 4096 tokens: 82 with S = 1 (chosen), 89 with S = 2.
+static int split_k_blocks(int tiles, int num_kb, int clusters) {
+  constexpr int EPI_KB = 12, MIN_KB = 4;
+  int best = num_kb;
+  long long best_cost = -1;
+  for (int S = 1; S <= 32 && (S == 1 || num_kb / S >= MIN_KB); ++S) {
+    const int kbs = (num_kb + S - 1) / S;
+    const int units = tiles * ((num_kb + kbs - 1) / kbs);
+    const long long cost = (long long)((units + clusters - 1) / clusters) * (kbs + EPI_KB);
+    if (best_cost < 0 || cost < best_cost) {
+      best = kbs;
+      best_cost = cost;
+    }
+  }
+  return best;
+}
+
 template <bool A_MN, bool B_MN, int OUT_MODE, bool EPI_TMA, int EPI = EPI_NONE>
 static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& md, void* D, int M, int N, int K,
                   long long ldd, KernelStatus* status, cudaStream_t stream, const CUtensorMap* mh = nullptr,
@@ -709,8 +740,11 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMa
   }
   const int n_tiles = (EPI == EPI_SWIGLU) ? (N + BN_HALF - 1) / BN_HALF : (N + BN - 1) / BN;
   const int tiles = ((M + 2 * BM - 1) / (2 * BM)) * n_tiles;
-  const int clusters = tiles < max_clusters ? tiles : max_clusters;
+  const int num_kb = (K + BK - 1) / BK;
   ea.group_m = g_group_m;
+  ea.kb_per_split = (OUT_MODE == OUT_F32_ACC && EPI_TMA) ? split_k_blocks(tiles, num_kb, max_clusters) : num_kb;
+  const int units = tiles * ((num_kb + ea.kb_per_split - 1) / ea.kb_per_split);
+  const int clusters = units < max_clusters ? units : max_clusters;
   const cudaError_t err = launch_pdl(kern, dim3(2 * clusters), dim3(NUM_THREADS), smem_bytes_of(EPI), stream, ma, mb, md,
                                      mh ? *mh : md, D, M, N, K, ldd, status, ea);
   pt_count_launches(1);

@@ -77,6 +77,22 @@ def test_gemm_wgrad_layout_and_fp32_accumulate(C, M, N, K):
     assert _rel(acc - 0.5, 2 * want) < 1e-4                   # fp32 accumulation: only the bf16 inputs round
 
 
+@pytest.mark.parametrize("M,N,K", [(256, 256, 512), (256, 256, 511), (264, 520, 449), (576, 576, 8192), (8, 8, 16384), (1024, 512, 577)])
+def test_gemm_fp32_accumulation_with_k_split_over_cta_pairs(M, N, K):
+    """Few output tiles and a long reduction: several CTA pairs add their part of K to one tile (remainders of the split,
+    a last k-block of one row, tiles that stick out of the matrix)."""
+    from picotron_b200.ops import _ext
+    C = _ext.load()
+    C.set_gemm_pair(True)
+    C.set_gemm_tma_epilogue(True)
+    a, b = bf(K, M, seed=71), bf(K, N, seed=72)
+    acc = torch.full((M, N), 0.5, device="cuda", dtype=torch.float32)
+    C.gemm(a, b, True, True, acc, True)
+    _status_ok(C)
+    # fp32 sums of K products in another order: error of order sqrt(K) * 2^-24 of the sum's size sqrt(K)
+    assert _rel(acc - 0.5, a.double().t() @ b.double()) < 1e-5
+
+
 @pytest.mark.parametrize("T,I,K", [(256, 128, 64), (300, 384, 320), (1024, 2048, 512), (4096, 1024, 2048)])
 def test_gemm_with_swiglu_epilogue(T, I, K):
     """gate/up GEMM whose epilogue also writes silu(gate) * up, against the two separate kernels and fp32 math."""
