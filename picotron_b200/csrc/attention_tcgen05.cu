@@ -17,14 +17,16 @@
 //             as bf16 into 128B-swizzled shared memory for the second MMA, the running output kept in
 //             registers:  acc = (acc + O_{j-1}) * alpha_j.
 //
-// Backward, one CTA per (128-key block, kv head, batch) looping over the query heads of the group and the
-// query blocks that see this key block:
-//   S = Q K^T and dP = dO V^T into TMEM; threads form P = exp2(S*c - lse) and dS = P*(dP - delta)*scale and
-//   store both (bf16, swizzled) to shared memory; then dV += P^T dO, dK += dS^T Q (TMEM accumulators that live
-//   for the whole CTA) and dQ = dS K, which the threads add to an fp32 workspace with vector reductions.
+// Backward, one CTA per (128-key block, kv head, batch) looping over the query heads of the group and the query blocks that see
+// this key block, pipelined over the steps (attn_bwd_kernel):
+//   S^T = K Q^T and dP^T = V dO^T into TMEM; threads (one key each) form P^T = exp2(S^T*c - lse), stored as bf16 into TMEM, and
+//   dS^T = P^T*(dP^T - delta)*scale, stored as bf16 into swizzled shared memory; then dV += P^T dO, dK += dS^T Q (TMEM
+//   accumulators that live for the whole CTA) and dQ = dS K, which four warps add to an fp32 workspace with TMA reduce-adds.
 //   A small kernel computes delta = rowsum(dO*O) beforehand and another converts the fp32 dQ to bf16.
 #include "common.cuh"
 #include "tensormap.cuh"
+
+#include <type_traits>
 
 extern "C" void pt_count_launches(int n);
 extern "C" void* pt_status_word();
@@ -92,9 +94,9 @@ struct AttnParams {
   unsigned long long* prof;   // optional phase counters (see pt_attention_set_profile); nullptr = not measured
 };
 
-// Phase counters of the kernels' consumer threads, in SM clock cycles, summed over all CTAs (thread 0 of each CTA measures):
-//   [0] bwd: waiting for S and dP    [1] bwd: TMEM read, exponentials, P/dS stores    [2] bwd: waiting for dQ
-//   [3] bwd: dQ drain                [4] bwd: steps          [5] bwd: lifetime of the compute loop    [6] bwd: CTAs
+// Phase counters of the kernels' consumer threads, in SM clock cycles, summed over all CTAs (one thread of each CTA measures):
+//   [0] bwd: waiting for S and dP    [1] bwd: TMEM read, exponentials, P/dS stores    [2] bwd, drain warps: waiting for dQ
+//   [3] bwd, drain warps: dQ drain   [4] bwd: steps          [5] bwd: lifetime of the compute loop    [6] bwd: CTAs
 //   [8] fwd: S read + row maximum    [9] fwd: wait for O / rescale   [10] fwd: exponentials + P stores   [11] fwd: blocks
 //   [12] fwd: lifetime of the softmax loop   [13] fwd: CTAs   [14] fwd: waiting for S
 // Measured only by the PROF instantiations of the kernels, which are launched while a counter buffer is set; the regular
@@ -455,10 +457,6 @@ __global__ void convert_dq_rope_kernel(const float* __restrict__ ws, bf16* __res
   *reinterpret_cast<uint2*>(dst + half) = o2;
 }
 
-__device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float c, float d) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
-
 // ---------------------------------------------------------------------------------------------------------
 // backward main kernel
 // ---------------------------------------------------------------------------------------------------------
@@ -468,26 +466,34 @@ struct BwdCfg {
   static constexpr int BN = 128;   // keys per CTA
   static constexpr int DCH = D / 64;
   static constexpr int TILE_BYTES = 128 * D * 2;         // Q, dO, K, V tiles
-  static constexpr int PS_BYTES = BM * BN * 2;           // P and dS tiles
-  static constexpr int QSTAGES = (D == 64) ? 3 : 1;      // Q/dO ring: a tile is loaded two steps before its MMAs (d = 64)
-  // The dQ tile of a step is staged in shared memory, 128 rows x 32 fp32 columns per buffer, and added to the fp32
-  // workspace by one TMA reduce per buffer instead of 8 vector atomics per thread and 32 columns (per-thread atomics
-  // were ~half of the step time for d = 128 and saturated L2 for d = 64). Two buffers: d = 64 needs one round, d = 128 two.
-  static constexpr bool DQ_TMA = true;
-  static constexpr int DQ_BYTES = 2 * BM * 32 * 4;
-  static constexpr int SMEM = 2 * TILE_BYTES + QSTAGES * 2 * TILE_BYTES + 2 * PS_BYTES + DQ_BYTES + 1024;
+  static constexpr int DS_BYTES = BM * BN * 2;           // dS^T tile (P^T never leaves tensor memory)
+  static constexpr int QSTAGES = (D == 64) ? 3 : 2;      // S of step i+1 is computed while dK of step i still reads Q_i
+  static constexpr int OSTAGES = (D == 64) ? 3 : 1;      // dO ring; d = 128: dO_i is free after dV_i, half a step before its next use
+  // The dQ tile of a step is staged in shared memory, 32 rows x 32 fp32 columns at a time (two buffers per drain warp), and
+  // added to the fp32 workspace by TMA reduces (per-thread vector atomics saturate L2).
+  static constexpr int DQ_BYTES = 4 * 2 * 32 * 32 * 4;
+  static constexpr int STAT_BYTES = 2 * 2 * BM * 4;      // two stages of (lse, delta) of 128 query rows
+  static constexpr int TILES = 2 * TILE_BYTES + (QSTAGES + OSTAGES) * TILE_BYTES + DS_BYTES + DQ_BYTES + STAT_BYTES;
+  static constexpr int SMEM = TILES + 256;               // + barriers; the block starts 1024-byte aligned
   static constexpr int TMEM_COLS = 512;
-  static constexpr bool SHARE_S_DQ = (D == 128);
+  // d = 64: everything has columns of its own. d = 128: P^T reuses the columns S^T was read from (each half of a row its own
+  // half of them) and dQ those of dP^T, so S and dP of the next step wait for dV and for the dQ drain.
+  static constexpr bool SHARE = (D == 128);
   static constexpr int S_COL = 0, DP_COL = 128, DV_COL = 256, DK_COL = 256 + D;
-  static constexpr int DQ_COL = SHARE_S_DQ ? 0 : 256 + 2 * D;
-  static_assert(DQ_COL + D <= 512 && DK_COL + D <= 512, "TMEM budget");
+  static constexpr int DQ_COL = SHARE ? DP_COL : 256 + 2 * D;
+  static constexpr int P_COL = SHARE ? S_COL : 256 + 3 * D;
+  static constexpr int P_HALF = SHARE ? 64 : 32;         // columns between the two 64-query halves of P^T
+  static_assert(DQ_COL + D <= 512 && DK_COL + D <= 512 && P_COL + P_HALF + 32 <= 512, "TMEM budget");
+  static_assert(SMEM <= 232448, "shared memory budget");
 };
 
 struct BwdBars {
-  uint64_t kv_full, q_full[3], q_empty[3], s_full, dp_full, pds_ready, dq_full, dq_read, acc_full;
+  uint64_t kv_full, q_full[3], q_empty[3], do_full[3], do_empty[3], st_full[2], st_empty[2];
+  uint64_t s_full, s_read, p_ready, p_free, dp_full, dp_read, ds_ready, ds_free, dq_full, dq_read, acc_full;
   uint32_t tmem_base;
   int abort_flag;
 };
+static_assert(sizeof(BwdBars) <= 256, "barrier block");
 
 struct BwdParams {
   int B, Sq, Sk, hq, hkv;
@@ -504,26 +510,39 @@ struct BwdParams {
   unsigned long long* prof;      // optional phase counters, as AttnParams::prof
 };
 
-constexpr int BWD_THREADS = 320;   // warps 0-7 compute (two per TMEM lane quarter), warp 8 TMA producer, warp 9 MMA issuer
+// warps 0-7 compute (two per TMEM lane quarter), 8-11 drain dQ, 12 TMA producer, 13 MMA issuer, 14 row statistics (15 idle)
+constexpr int BWD_THREADS = 512;
+// registers per thread: 128 at launch, then redistributed between the warpgroups (2 x compute + drain + the rest = 4 x 128)
+constexpr int BWD_REGS = 128, BWD_REGS_COMPUTE = 160, BWD_REGS_DRAIN = 96, BWD_REGS_REST = 96;
+static_assert(2 * BWD_REGS_COMPUTE + BWD_REGS_DRAIN + BWD_REGS_REST <= 4 * BWD_REGS, "setmaxnreg must not ask for more than the launch gave");
+template <int N> __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
+// What bounds it: a step (128 keys x 128 queries) is a chain S -> exp -> dP -> dS -> dQ -> drain of hand-offs between the
+// tensor core and the compute warps, each of a few hundred cycles; run one after the other they cost 5,400 (d = 64) and
+// 7,900 (d = 128) cycles per step against ~1,300 / 2,600 of MMA and ~1,100 of special-function work. So the chain is pipelined
+// over steps: S_{i+1} and dP_{i+1} run under the arithmetic of step i, dQ_i / dK_i under the exponentials of step i+1, and
+// dQ_i is drained by warps of their own. The scores are computed TRANSPOSED (lane = key): then P^T is written straight back to
+// tensor memory as the A operand of dV += P^T dO, and only dS^T goes through shared memory (which the MMAs read all the time).
+// Measured (us; 1 x 32768, 32 / 8 heads, d = 64; 1 x 8192, 32 / 8 heads, d = 128): 21,500 -> 16,200 and 2,160 -> 1,410.
 template <int D, bool OUT_F32, bool PROF>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ KVSegs segs,
                 const __grid_constant__ CUtensorMap tm_do, const __grid_constant__ CUtensorMap tm_dq,
-                const float* __restrict__ LSE,
-                const float* __restrict__ DELTA, float* __restrict__ dq_ws, void* __restrict__ dK_, void* __restrict__ dV_,
-                BwdParams p, KernelStatus* status) {
+                const float* __restrict__ LSE, const float* __restrict__ DELTA, void* __restrict__ dK_,
+                void* __restrict__ dV_, BwdParams p, KernelStatus* status) {
   using Cfg = BwdCfg<D>;
   pdl_launch_dependents();
-  extern __shared__ uint8_t smem_raw[];
-  __shared__ BwdBars bars;
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  // no static shared memory in this kernel: the dynamic block starts at the (1024-byte aligned) window base
+  extern __shared__ __align__(1024) uint8_t smem[];
+  BwdBars& bars = *reinterpret_cast<BwdBars*>(smem + Cfg::TILES);
   uint8_t* sK = smem;
   uint8_t* sV = sK + Cfg::TILE_BYTES;
-  uint8_t* sQ = sV + Cfg::TILE_BYTES;                                 // QSTAGES x (Q tile, dO tile)
-  uint8_t* sP = sQ + Cfg::QSTAGES * 2 * Cfg::TILE_BYTES;
-  uint8_t* sdS = sP + Cfg::PS_BYTES;
-  uint8_t* sDQ = sdS + Cfg::PS_BYTES;                                 // [D/32][128 rows][32 fp32], 128B swizzle (d = 64 only)
+  uint8_t* sQ = sV + Cfg::TILE_BYTES;
+  uint8_t* sdO = sQ + Cfg::QSTAGES * Cfg::TILE_BYTES;
+  uint8_t* sdS = sdO + Cfg::OSTAGES * Cfg::TILE_BYTES;                // dS^T: two chunks of [128 keys][64 queries], 128B swizzle
+  uint8_t* sDQ = sdS + Cfg::DS_BYTES;                                 // per drain warp two of [32 rows][32 fp32], 128B swizzle
+  float* sStat = reinterpret_cast<float*>(sDQ + Cfg::DQ_BYTES);       // [stage][lse * log2(e) | delta * scale][128]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int bps = (p.Sk + Cfg::BN - 1) / Cfg::BN;         // key blocks per segment
@@ -549,12 +568,23 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     for (int s = 0; s < 3; ++s) {
       mbar_init(&bars.q_full[s], 1);
       mbar_init(&bars.q_empty[s], 1);
+      mbar_init(&bars.do_full[s], 1);
+      mbar_init(&bars.do_empty[s], 1);
+    }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&bars.st_full[s], 32);
+      mbar_init(&bars.st_empty[s], 8);
     }
     mbar_init(&bars.s_full, 1);
+    mbar_init(&bars.s_read, 8);        // compute -> MMA: one arrival per warp
+    mbar_init(&bars.p_ready, 8);
+    mbar_init(&bars.p_free, 1);
     mbar_init(&bars.dp_full, 1);
-    mbar_init(&bars.pds_ready, 256);
+    mbar_init(&bars.dp_read, 8);
+    mbar_init(&bars.ds_ready, 8);
+    mbar_init(&bars.ds_free, 1);
     mbar_init(&bars.dq_full, 1);
-    mbar_init(&bars.dq_read, 256);
+    mbar_init(&bars.dq_read, 4);
     mbar_init(&bars.acc_full, 1);
     bars.abort_flag = 0;
     fence_barrier_init();
@@ -563,8 +593,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     tma_prefetch_desc(&segs.k[seg]);
     tma_prefetch_desc(&segs.v[seg]);
     tma_prefetch_desc(&tm_do);
+    tma_prefetch_desc(&tm_dq);
   }
-  if (warp == 9) {
+  if (warp == 13) {
     tmem_alloc(&bars.tmem_base, Cfg::TMEM_COLS);
     tmem_relinquish();
   }
@@ -575,7 +606,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const uint32_t tmem_base = bars.tmem_base;
   volatile int* abort_flag = &bars.abort_flag;
 
-  if (warp == 8) {
+  if (warp >= 12) regs_dec<BWD_REGS_REST>();
+  if (warp == 12) {
     // ------------------------------------------------------------------------------ TMA producer
     if (lane == 0 && total_steps > 0) {
       mbar_expect_tx(&bars.kv_full, 2 * Cfg::TILE_BYTES);
@@ -585,216 +617,305 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         tma_load_4d(sV + c * (Cfg::BN * 128), &segs.v[seg], &bars.kv_full, c * 64, kv_head, k0, b);
       }
       for (int it = 0; it < total_steps; ++it) {
-        const int st = it % Cfg::QSTAGES;
-        const uint32_t ph = (it / Cfg::QSTAGES) & 1;
         const int head = kv_head * group + it / steps_per_head;
-        const int qb = qb_first + it % steps_per_head;
-        if (!mbar_wait(&bars.q_empty[st], ph ^ 1, abort_flag)) { report_error(status, KID_BWD, 1); break; }
-        mbar_expect_tx(&bars.q_full[st], 2 * Cfg::TILE_BYTES);
-        uint8_t* q_dst = sQ + st * 2 * Cfg::TILE_BYTES;
-        uint8_t* do_dst = q_dst + Cfg::TILE_BYTES;
+        const int q0 = (qb_first + it % steps_per_head) * Cfg::BM;
+        const int qs = it % Cfg::QSTAGES, os = it % Cfg::OSTAGES;
+        if (!mbar_wait(&bars.q_empty[qs], ((it / Cfg::QSTAGES) & 1) ^ 1, abort_flag)) { report_error(status, KID_BWD, 1); break; }
+        mbar_expect_tx(&bars.q_full[qs], Cfg::TILE_BYTES);
 #pragma unroll
-        for (int c = 0; c < Cfg::DCH; ++c) {
-          tma_load_4d(q_dst + c * (Cfg::BM * 128), &tm_q, &bars.q_full[st], c * 64, head, qb * Cfg::BM, b);
-          tma_load_4d(do_dst + c * (Cfg::BM * 128), &tm_do, &bars.q_full[st], c * 64, head, qb * Cfg::BM, b);
-        }
+        for (int c = 0; c < Cfg::DCH; ++c)
+          tma_load_4d(sQ + qs * Cfg::TILE_BYTES + c * (Cfg::BM * 128), &tm_q, &bars.q_full[qs], c * 64, head, q0, b);
+        if (!mbar_wait(&bars.do_empty[os], ((it / Cfg::OSTAGES) & 1) ^ 1, abort_flag)) { report_error(status, KID_BWD, 11); break; }
+        mbar_expect_tx(&bars.do_full[os], Cfg::TILE_BYTES);
+#pragma unroll
+        for (int c = 0; c < Cfg::DCH; ++c)
+          tma_load_4d(sdO + os * Cfg::TILE_BYTES + c * (Cfg::BM * 128), &tm_do, &bars.do_full[os], c * 64, head, q0, b);
       }
     }
-  } else if (warp == 9) {
+  } else if (warp == 13) {
     // ------------------------------------------------------------------------------ MMA issuer
     if (lane == 0 && total_steps > 0) {
-      constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, false, false);   // S, dP: [q, kv], K-major operands
-      constexpr uint32_t idesc_kv = make_idesc_bf16(128, D, true, true);      // dV, dK: A = P^T/dS^T, B = dO/Q (both MN-major)
-      constexpr uint32_t idesc_dq = make_idesc_bf16(128, D, false, true);     // dQ: A = dS (K-major), B = K (MN-major)
+      constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, false, false);   // S^T, dP^T: [key, query], K-major operands
+      constexpr uint32_t idesc_kv = make_idesc_bf16(128, D, false, true);     // dV, dK: A = P^T (TMEM) / dS^T (K-major), B = dO / Q (MN-major)
+      constexpr uint32_t idesc_dq = make_idesc_bf16(128, D, true, true);      // dQ: A = dS^T seen as dS (MN-major), B = K (MN-major)
       bool ok = mbar_wait(&bars.kv_full, 0, abort_flag);
       if (!ok) report_error(status, KID_BWD, 2);
-      const uint32_t k_addr = smem_u32(sK), v_addr = smem_u32(sV), p_addr = smem_u32(sP), ds_addr = smem_u32(sdS);
-      // Base descriptors, built once: one thread issues ~40 MMAs per step and is on the critical path of every hand-off,
-      // so the per-MMA work is kept to two integer adds. "km" = K-major view (LBO 16), "mn" = MN-major view (LBO = tile).
+      // Base descriptors, built once: "km" = K-major view (LBO 16), "mn" = MN-major view (LBO = 64-column chunk).
+      const uint32_t k_addr = smem_u32(sK), ds_addr = smem_u32(sdS);
       const uint64_t k_km = make_smem_desc_sw128(k_addr, 16, 1024), k_mn = make_smem_desc_sw128(k_addr, 128 * 128, 1024);
-      const uint64_t v_km = make_smem_desc_sw128(v_addr, 16, 1024);
-      const uint64_t p_mn = make_smem_desc_sw128(p_addr, 128 * 128, 1024);
+      const uint64_t v_km = make_smem_desc_sw128(smem_u32(sV), 16, 1024);
       const uint64_t ds_mn = make_smem_desc_sw128(ds_addr, 128 * 128, 1024), ds_km = make_smem_desc_sw128(ds_addr, 16, 1024);
-      // S = Q K^T and dP = dO V^T of step `it`
-      auto issue_s_dp = [&](int it) -> bool {
-        const int st = it % Cfg::QSTAGES;
-        const uint32_t q_addr = smem_u32(sQ + st * 2 * Cfg::TILE_BYTES);
-        const uint64_t q_km = make_smem_desc_sw128(q_addr, 16, 1024);
-        const uint64_t do_km = smem_desc_advance(q_km, Cfg::TILE_BYTES);
-        if (!mbar_wait(&bars.q_full[st], (it / Cfg::QSTAGES) & 1, abort_flag)) { report_error(status, KID_BWD, 3); return false; }
-        if (Cfg::SHARE_S_DQ && it > 0) {   // S overwrites the columns dQ of the previous step was read from
-          if (!mbar_wait(&bars.dq_read, (it - 1) & 1, abort_flag)) { report_error(status, KID_BWD, 4); return false; }
-        }
+      const uint64_t q_km0 = make_smem_desc_sw128(smem_u32(sQ), 16, 1024), q_mn0 = make_smem_desc_sw128(smem_u32(sQ), 128 * 128, 1024);
+      const uint64_t do_km0 = make_smem_desc_sw128(smem_u32(sdO), 16, 1024), do_mn0 = make_smem_desc_sw128(smem_u32(sdO), 128 * 128, 1024);
+      // S^T = K Q^T of step `it`
+      auto issue_s = [&](int it) -> bool {
+        const int qs = it % Cfg::QSTAGES;
+        if (!mbar_wait(&bars.q_full[qs], (it / Cfg::QSTAGES) & 1, abort_flag)) { report_error(status, KID_BWD, 3); return false; }
         tcgen05_fence_after();
+        const uint64_t q_km = smem_desc_advance(q_km0, qs * Cfg::TILE_BYTES);
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
           const uint32_t off = (kk >> 2) * (128 * 128) + (kk & 3) * 32;
-          umma_bf16(tmem_base + Cfg::S_COL, smem_desc_advance(q_km, off), smem_desc_advance(k_km, off), idesc_s, kk > 0 ? 1u : 0u);
+          umma_bf16(tmem_base + Cfg::S_COL, smem_desc_advance(k_km, off), smem_desc_advance(q_km, off), idesc_s, kk > 0 ? 1u : 0u);
         }
         umma_commit(&bars.s_full);
+        return true;
+      };
+      // dP^T = V dO^T of step `it`
+      auto issue_dp = [&](int it) -> bool {
+        const int os = it % Cfg::OSTAGES;
+        if (!mbar_wait(&bars.do_full[os], (it / Cfg::OSTAGES) & 1, abort_flag)) { report_error(status, KID_BWD, 12); return false; }
+        tcgen05_fence_after();
+        const uint64_t do_km = smem_desc_advance(do_km0, os * Cfg::TILE_BYTES);
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
           const uint32_t off = (kk >> 2) * (128 * 128) + (kk & 3) * 32;
-          umma_bf16(tmem_base + Cfg::DP_COL, smem_desc_advance(do_km, off), smem_desc_advance(v_km, off), idesc_s, kk > 0 ? 1u : 0u);
+          umma_bf16(tmem_base + Cfg::DP_COL, smem_desc_advance(v_km, off), smem_desc_advance(do_km, off), idesc_s, kk > 0 ? 1u : 0u);
         }
         umma_commit(&bars.dp_full);
         return true;
       };
+      ok = ok && issue_s(0);
+      if (!Cfg::SHARE) ok = ok && issue_dp(0);
       for (int it = 0; it < total_steps && ok; ++it) {
-        const int st = it % Cfg::QSTAGES;
-        const uint64_t q_mn = make_smem_desc_sw128(smem_u32(sQ + st * 2 * Cfg::TILE_BYTES), 128 * 128, 1024);
-        const uint64_t do_mn = smem_desc_advance(q_mn, Cfg::TILE_BYTES);
-        if (!issue_s_dp(it)) break;
-        if (!mbar_wait(&bars.pds_ready, it & 1, abort_flag)) { report_error(status, KID_BWD, 5); break; }
-        if (!Cfg::SHARE_S_DQ && it > 0) {  // separate dQ columns: only the previous dQ must have been read
-          if (!mbar_wait(&bars.dq_read, (it - 1) & 1, abort_flag)) { report_error(status, KID_BWD, 6); break; }
+        const uint32_t par = it & 1;
+        const bool next = it + 1 < total_steps;
+        if (!Cfg::SHARE && next) {        // the compute warps hold S of this step in registers: the next one may overwrite it
+          if (!mbar_wait(&bars.s_read, par, abort_flag)) { report_error(status, KID_BWD, 4); break; }
+          if (!issue_s(it + 1)) break;
         }
+        if (Cfg::SHARE) {                 // dP shares its columns with dQ of the previous step
+          if (it > 0 && !mbar_wait(&bars.dq_read, par ^ 1, abort_flag)) { report_error(status, KID_BWD, 6); break; }
+          if (!issue_dp(it)) break;
+        }
+        // dV += P^T dO : M = 128 keys, N = D, reduction over the 128 query rows
+        if (!mbar_wait(&bars.p_ready, par, abort_flag)) { report_error(status, KID_BWD, 5); break; }
         tcgen05_fence_after();
-        // dQ = dS K : M = 128 query rows, N = D, reduction over the 128 keys. Issued first: the compute threads drain
-        // dQ while the (three times longer) dV/dK MMAs below still run.
+        const uint64_t do_mn = smem_desc_advance(do_mn0, (it % Cfg::OSTAGES) * Cfg::TILE_BYTES);
 #pragma unroll
         for (int kk = 0; kk < 128 / 16; ++kk)
-          umma_bf16(tmem_base + Cfg::DQ_COL, smem_desc_advance(ds_km, (kk >> 2) * (128 * 128) + (kk & 3) * 32),
-                    smem_desc_advance(k_mn, kk * 2048), idesc_dq, kk > 0 ? 1u : 0u);
-        umma_commit(&bars.dq_full);
-        // dV += P^T dO, dK += dS^T Q : M = 128 keys, N = D, reduction over the 128 query rows. The next step's P / dS
-        // are only written after s_full of that step, whose commit also covers these MMAs.
-#pragma unroll
-        for (int kk = 0; kk < 128 / 16; ++kk) {
-          // A: P / dS stored [q rows][kv], kv contiguous -> MN-major with M = kv: two 64-key chunks (LBO), 8-row groups (SBO)
-          // B: dO / Q stored [q rows][d], d contiguous -> MN-major with N = d
-          umma_bf16(tmem_base + Cfg::DV_COL, smem_desc_advance(p_mn, kk * 2048), smem_desc_advance(do_mn, kk * 2048), idesc_kv,
-                    (it > 0 || kk > 0) ? 1u : 0u);
-          umma_bf16(tmem_base + Cfg::DK_COL, smem_desc_advance(ds_mn, kk * 2048), smem_desc_advance(q_mn, kk * 2048), idesc_kv,
-                    (it > 0 || kk > 0) ? 1u : 0u);
+          umma_bf16_ts(tmem_base + Cfg::DV_COL, tmem_base + Cfg::P_COL + (kk >> 2) * Cfg::P_HALF + (kk & 3) * 8,
+                       smem_desc_advance(do_mn, kk * 2048), idesc_kv, (it > 0 || kk > 0) ? 1u : 0u);
+        umma_commit(&bars.p_free);
+        umma_commit(&bars.do_empty[it % Cfg::OSTAGES]);
+        if (next) {
+          if (Cfg::SHARE) {               // S overwrites P: dV must have read it
+            if (!mbar_wait(&bars.p_free, par, abort_flag)) { report_error(status, KID_BWD, 13); break; }
+            if (!issue_s(it + 1)) break;
+          } else {
+            if (!mbar_wait(&bars.dp_read, par, abort_flag)) { report_error(status, KID_BWD, 14); break; }
+            if (!issue_dp(it + 1)) break;
+          }
         }
-        umma_commit(&bars.q_empty[st]);
+        if (!mbar_wait(&bars.ds_ready, par, abort_flag)) { report_error(status, KID_BWD, 15); break; }
+        if (!Cfg::SHARE && it > 0 && !mbar_wait(&bars.dq_read, par ^ 1, abort_flag)) { report_error(status, KID_BWD, 16); break; }
+        tcgen05_fence_after();
+        // dQ = dS K : M = 128 query rows, N = D, reduction over the 128 keys (first: its drain is the longer way)
+#pragma unroll
+        for (int kk = 0; kk < 128 / 16; ++kk)
+          umma_bf16(tmem_base + Cfg::DQ_COL, smem_desc_advance(ds_mn, kk * 2048), smem_desc_advance(k_mn, kk * 2048), idesc_dq,
+                    kk > 0 ? 1u : 0u);
+        umma_commit(&bars.dq_full);
+        // dK += dS^T Q : M = 128 keys, N = D, reduction over the 128 query rows
+        const uint64_t q_mn = smem_desc_advance(q_mn0, (it % Cfg::QSTAGES) * Cfg::TILE_BYTES);
+#pragma unroll
+        for (int kk = 0; kk < 128 / 16; ++kk)
+          umma_bf16(tmem_base + Cfg::DK_COL, smem_desc_advance(ds_km, (kk >> 2) * (128 * 128) + (kk & 3) * 32),
+                    smem_desc_advance(q_mn, kk * 2048), idesc_kv, (it > 0 || kk > 0) ? 1u : 0u);
+        umma_commit(&bars.ds_free);
+        umma_commit(&bars.q_empty[it % Cfg::QSTAGES]);
       }
       if (ok) umma_commit(&bars.acc_full);
     }
-  } else {
-    // ------------------------------------------------------------------------------ compute threads (warps 0..7)
-    // Thread pair (t, t + 128) shares query row t (TMEM lane t): `half` 0 owns score columns 0..63, dQ columns
-    // 0..D/2-1 and the dV output, `half` 1 the rest and dK. Nothing has to be exchanged between the two.
-    const int t = threadIdx.x & 127;
-    const int half = threadIdx.x >> 7;
-    const uint32_t t_lane = tmem_base + (uint32_t((warp & 3) * 32) << 16);
-    const float sl2 = p.scale * LOG2E;
-    bool ok = total_steps > 0;
-    const bool prof_on = PROF && p.prof != nullptr && threadIdx.x == 0;
-    long long pacc[4] = {0, 0, 0, 0};
-    const long long pstart = prof_clock(prof_on);
+  } else if (warp == 14) {
+    // ------------------------------------------------------------------------------ row statistics (lse, delta) of a step's queries
     for (int it = 0; it < total_steps; ++it) {
-      const long long pt0 = prof_clock(prof_on);
+      const int st = it & 1;
       const int head = kv_head * group + it / steps_per_head;
-      const int qb = qb_first + it % steps_per_head;
-      const int row = qb * Cfg::BM + t;
-      const bool row_ok = row < p.Sq;
-      const long long stat_idx = ((long long)b * p.hq + head) * p.Sq + (row_ok ? row : 0);
-      const float lse2 = row_ok ? LSE[stat_idx] * LOG2E : 0.f;
-      const float dlt = row_ok ? DELTA[stat_idx] : 0.f;
-      const bool need_mask = (diag && k0 + Cfg::BN - 1 > qb * Cfg::BM) || (k0 + Cfg::BN > p.Sk) || !row_ok;
-      if (!mbar_wait(&bars.s_full, it & 1, abort_flag)) { if (lane == 0) report_error(status, KID_BWD, 7); ok = false; break; }
-      if (!mbar_wait(&bars.dp_full, it & 1, abort_flag)) { if (lane == 0) report_error(status, KID_BWD, 8); ok = false; break; }
+      const int q0 = (qb_first + it % steps_per_head) * Cfg::BM;
+      const long long base = ((long long)b * p.hq + head) * p.Sq;
+      float l[4], dl[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int row = q0 + lane + 32 * i;
+        // rows beyond Sq: exp2(0 - inf) = 0
+        l[i] = row < p.Sq ? LSE[base + row] * LOG2E : INFINITY;
+        dl[i] = row < p.Sq ? DELTA[base + row] * p.scale : 0.f;
+      }
+      if (!mbar_wait(&bars.st_empty[st], ((it >> 1) & 1) ^ 1, abort_flag)) { if (lane == 0) report_error(status, KID_BWD, 17); break; }
+      float* dst = sStat + st * 2 * Cfg::BM;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        dst[lane + 32 * i] = l[i];
+        dst[Cfg::BM + lane + 32 * i] = dl[i];
+      }
+      mbar_arrive(&bars.st_full[st]);
+    }
+  } else if (warp >= 8 && warp < 12) {
+    // ------------------------------------------------------------------------------ dQ of every step -> fp32 workspace
+    // Warp w owns 32 query rows: it stages 32 columns at a time in one of its two buffers and hands them to TMA reduce-adds.
+    regs_dec<BWD_REGS_DRAIN>();
+    const int quarter = warp & 3;
+    const uint32_t t_lane = tmem_base + (uint32_t(quarter * 32) << 16) + Cfg::DQ_COL;
+    uint8_t* stg = sDQ + quarter * 8192;
+    const bool prof_on = PROF && p.prof != nullptr && threadIdx.x == 256;
+    long long pacc[2] = {0, 0};
+    for (int it = 0; it < total_steps; ++it) {
+      const int head = kv_head * group + it / steps_per_head;
+      const int row0 = (qb_first + it % steps_per_head) * Cfg::BM + quarter * 32;
+      const long long pt0 = prof_clock(prof_on);
+      if (!mbar_wait(&bars.dq_full, it & 1, abort_flag)) { if (lane == 0) report_error(status, KID_BWD, 9); break; }
       tcgen05_fence_after();
       const long long pt1 = prof_clock(prof_on);
-      uint32_t rs[64], rd[64];                       // this thread's 64 score / dP columns, one batched TMEM read
 #pragma unroll
-      for (int cc = 0; cc < 2; ++cc) {
-        tmem_ld_32x32b_x32_at(t_lane + Cfg::S_COL + (half * 2 + cc) * 32, rs, cc * 32);
-        tmem_ld_32x32b_x32_at(t_lane + Cfg::DP_COL + (half * 2 + cc) * 32, rd, cc * 32);
-      }
-      tmem_ld_wait();
-      const float dlt_s = dlt * p.scale;
-#pragma unroll
-      for (int cc = 0; cc < 2; ++cc) {
-        const int c = half * 2 + cc;
-        uint32_t pp[16], dd[16];
-#pragma unroll
-        for (int e = 0; e < 32; e += 2) {
-          float p0 = fast_exp2(__uint_as_float(rs[cc * 32 + e]) * sl2 - lse2);
-          float p1 = fast_exp2(__uint_as_float(rs[cc * 32 + e + 1]) * sl2 - lse2);
-          if (need_mask) {
-            const int col = k0 + c * 32 + e;
-            if (!row_ok || (diag && col > row) || col >= p.Sk) p0 = 0.f;
-            if (!row_ok || (diag && col + 1 > row) || col + 1 >= p.Sk) p1 = 0.f;
-          }
-          const float d0 = p0 * (__uint_as_float(rd[cc * 32 + e]) * p.scale - dlt_s);
-          const float d1 = p1 * (__uint_as_float(rd[cc * 32 + e + 1]) * p.scale - dlt_s);
-          pp[e >> 1] = pack_bf16(p0, p1);
-          dd[e >> 1] = pack_bf16(d0, d1);
+      for (int r_ = 0; r_ < D / 64; ++r_) {
+        uint32_t r[64];
+        tmem_ld_32x32b_x32_at(t_lane + r_ * 64, r, 0);
+        tmem_ld_32x32b_x32_at(t_lane + r_ * 64 + 32, r, 32);
+        tmem_ld_wait();
+        if (r_ == D / 64 - 1) {
+          tcgen05_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars.dq_read);
         }
-        const uint32_t chunk_off = ((c * 32) >> 6) * (128 * 128);
-        const int u0 = ((c * 32) & 63) >> 3;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const uint32_t off = chunk_off + sw128_offset(t, u0 + u);
-          *reinterpret_cast<uint4*>(sP + off) = make_uint4(pp[4 * u], pp[4 * u + 1], pp[4 * u + 2], pp[4 * u + 3]);
-          *reinterpret_cast<uint4*>(sdS + off) = make_uint4(dd[4 * u], dd[4 * u + 1], dd[4 * u + 2], dd[4 * u + 3]);
-        }
-      }
-      tcgen05_fence_before();
-      fence_proxy_async_smem();
-      mbar_arrive(&bars.pds_ready);
-      const long long pt2 = prof_clock(prof_on);
-      // dQ tile of this step -> fp32 workspace
-      if (!mbar_wait(&bars.dq_full, it & 1, abort_flag)) { if (lane == 0) report_error(status, KID_BWD, 9); ok = false; break; }
-      tcgen05_fence_after();
-      const long long pt3 = prof_clock(prof_on);
-      if (Cfg::DQ_TMA) {
-        // round r: `half` h stages dQ columns [32 (h R + r), +32) of its row (R = D / 64 rounds); thread 0 hands both
-        // 128 x 32 buffers to TMA
-#pragma unroll 1
-        for (int r_ = 0; r_ < D / 64; ++r_) {
-          uint32_t r[32];
-          tmem_ld_32x32b_x32(t_lane + Cfg::DQ_COL + (half * (D / 64) + r_) * 32, r);
-          tmem_ld_wait();
-          if (threadIdx.x == 0) tma_store_wait_read<0>();   // the previous reduce has finished reading the staging buffers
-          asm volatile("bar.sync 1, 256;" ::: "memory");
+        for (int h = 0; h < 2; ++h) {
+          if (lane == 0) tma_store_wait_read<1>();          // the reduce before the last has finished reading this buffer
+          __syncwarp();
 #pragma unroll
           for (int u = 0; u < 8; ++u)
-            *reinterpret_cast<uint4*>(sDQ + half * (128 * 128) + sw128_offset(t, u)) =
-                make_uint4(r[4 * u], r[4 * u + 1], r[4 * u + 2], r[4 * u + 3]);
+            *reinterpret_cast<uint4*>(stg + h * 4096 + sw128_offset(lane, u)) =
+                make_uint4(r[h * 32 + 4 * u], r[h * 32 + 4 * u + 1], r[h * 32 + 4 * u + 2], r[h * 32 + 4 * u + 3]);
           fence_proxy_async_smem();
-          asm volatile("bar.sync 1, 256;" ::: "memory");
-          if (threadIdx.x == 0) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-              tma_reduce_add_4d(&tm_dq, sDQ + h * (128 * 128), (h * (D / 64) + r_) * 32, head, qb * Cfg::BM, b);
+          __syncwarp();
+          if (lane == 0) {
+            if (row0 < p.Sq) tma_reduce_add_4d(&tm_dq, stg + h * 4096, r_ * 64 + h * 32, head, row0, b);
             tma_store_commit();
           }
         }
-      } else {
-        float* dq_row = dq_ws + (((long long)b * p.Sq + (row_ok ? row : 0)) * p.hq + head) * D + half * (D / 2);
-#pragma unroll 1
-        for (int c = 0; c < D / 64; ++c) {
-          uint32_t r[32];
-          tmem_ld_32x32b_x32(t_lane + Cfg::DQ_COL + half * (D / 2) + c * 32, r);
-          tmem_ld_wait();
-          if (row_ok) {
-#pragma unroll
-            for (int e = 0; e < 32; e += 4)
-              red_add_v4(dq_row + c * 32 + e, __uint_as_float(r[e]), __uint_as_float(r[e + 1]), __uint_as_float(r[e + 2]),
-                         __uint_as_float(r[e + 3]));
-          }
-        }
       }
+      if (prof_on) { const long long pt2 = clock64(); pacc[0] += pt1 - pt0; pacc[1] += pt2 - pt1; }
+    }
+    if (lane == 0) tma_store_wait<0>();
+    if (prof_on) {
+      atomicAdd(&p.prof[2], (unsigned long long)pacc[0]);
+      atomicAdd(&p.prof[3], (unsigned long long)pacc[1]);
+    }
+  } else if (warp < 8) {
+    // ------------------------------------------------------------------------------ compute threads (warps 0..7)
+    regs_inc<BWD_REGS_COMPUTE>();
+    // Thread pair (t, t + 128) shares key k0 + t (TMEM lane t): `half` 0 owns query columns 0..63 of a step and
+    // the dV output, `half` 1 the rest and dK. Nothing has to be exchanged between the two.
+    const int t = threadIdx.x & 127;
+    const int half = threadIdx.x >> 7;
+    const int quarter = warp & 3;
+    const uint32_t t_lane = tmem_base + (uint32_t(quarter * 32) << 16);
+    const float sl2 = p.scale * LOG2E;
+    const int key = k0 + t;
+    bool ok = total_steps > 0;
+    const bool prof_on = PROF && p.prof != nullptr && threadIdx.x == 0;
+    long long pacc[2] = {0, 0};
+    const long long pstart = prof_clock(prof_on);
+    for (int it = 0; it < total_steps; ++it) {
+      const long long pt0 = prof_clock(prof_on);
+      const uint32_t par = it & 1;
+      const int qcol0 = (qb_first + it % steps_per_head) * Cfg::BM + half * 64;     // first query of this thread's columns
+      const bool need_mask = (diag && k0 + Cfg::BN - 1 > qcol0) || (k0 + Cfg::BN > p.Sk);
+      const int hidden = key >= p.Sk ? 64 : (diag ? key - qcol0 : 0);              // columns [0, hidden) do not see this key
+      const float* st_l = sStat + par * 2 * Cfg::BM + half * 64;
+      const float* st_d = st_l + Cfg::BM;
+      if (!mbar_wait(&bars.st_full[par], (it >> 1) & 1, abort_flag)) { if (lane == 0) report_error(status, KID_BWD, 18); ok = false; break; }
+      if (!mbar_wait(&bars.s_full, par, abort_flag)) { if (lane == 0) report_error(status, KID_BWD, 7); ok = false; break; }
+      tcgen05_fence_after();
+      const long long pt1 = prof_clock(prof_on);
+      uint32_t s[64];
+      tmem_ld_32x32b_x32_at(t_lane + Cfg::S_COL + half * 64, s, 0);
+      tmem_ld_32x32b_x32_at(t_lane + Cfg::S_COL + half * 64 + 32, s, 32);
+      tmem_ld_wait();
+      if (!Cfg::SHARE) {
+        tcgen05_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars.s_read);
+      }
+      uint32_t pk[32];                        // P^T of this thread's 64 queries, bf16 pairs
+      // The masked and the plain form are separate code: a test of need_mask inside the loop costs a branch per element group,
+      // which took the scheduler's freedom away (d = 64, 32768 keys: 26.7 ms with it, 17.2 without).
+      auto exponentials = [&](auto masked) {
+#pragma unroll
+        for (int e = 0; e < 64; e += 4) {
+          const float4 lv = *reinterpret_cast<const float4*>(st_l + e);
+          float pv[4] = {fast_exp2(__uint_as_float(s[e]) * sl2 - lv.x), fast_exp2(__uint_as_float(s[e + 1]) * sl2 - lv.y),
+                         fast_exp2(__uint_as_float(s[e + 2]) * sl2 - lv.z), fast_exp2(__uint_as_float(s[e + 3]) * sl2 - lv.w)};
+          if constexpr (decltype(masked)::value) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) pv[i] = e + i < hidden ? 0.f : pv[i];
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) s[e + i] = __float_as_uint(pv[i]);
+          pk[e >> 1] = pack_bf16(pv[0], pv[1]);
+          pk[(e >> 1) + 1] = pack_bf16(pv[2], pv[3]);
+        }
+      };
+      if (need_mask) exponentials(std::true_type{});
+      else exponentials(std::false_type{});
+      if (!Cfg::SHARE && it > 0) {                                  // the dV MMA of the previous step has read its P
+        if (!mbar_wait(&bars.p_free, par ^ 1, abort_flag)) { if (lane == 0) report_error(status, KID_BWD, 19); ok = false; break; }
+        tcgen05_fence_after();
+      }
+      tmem_st_32x32b_x32(t_lane + Cfg::P_COL + half * Cfg::P_HALF, pk);
+      tmem_st_wait();
       tcgen05_fence_before();
-      mbar_arrive(&bars.dq_read);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars.p_ready);
+      const long long pt4 = prof_clock(prof_on);
+      if (!mbar_wait(&bars.dp_full, par, abort_flag)) { if (lane == 0) report_error(status, KID_BWD, 8); ok = false; break; }
+      tcgen05_fence_after();
+      const long long pt5 = prof_clock(prof_on);
+      uint32_t dp[64];
+      tmem_ld_32x32b_x32_at(t_lane + Cfg::DP_COL + half * 64, dp, 0);
+      tmem_ld_32x32b_x32_at(t_lane + Cfg::DP_COL + half * 64 + 32, dp, 32);
+      tmem_ld_wait();
+      if (!Cfg::SHARE) {
+        tcgen05_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars.dp_read);
+      }
+#pragma unroll
+      for (int e = 0; e < 64; e += 4) {
+        const float4 dv = *reinterpret_cast<const float4*>(st_d + e);
+        const float d0 = __uint_as_float(s[e]) * (__uint_as_float(dp[e]) * p.scale - dv.x);
+        const float d1 = __uint_as_float(s[e + 1]) * (__uint_as_float(dp[e + 1]) * p.scale - dv.y);
+        const float d2 = __uint_as_float(s[e + 2]) * (__uint_as_float(dp[e + 2]) * p.scale - dv.z);
+        const float d3 = __uint_as_float(s[e + 3]) * (__uint_as_float(dp[e + 3]) * p.scale - dv.w);
+        pk[e >> 1] = pack_bf16(d0, d1);
+        pk[(e >> 1) + 1] = pack_bf16(d2, d3);
+      }
+      // the dQ and dK MMAs of the previous step have read its dS
+      if (it > 0 && !mbar_wait(&bars.ds_free, par ^ 1, abort_flag)) { if (lane == 0) report_error(status, KID_BWD, 20); ok = false; break; }
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        *reinterpret_cast<uint4*>(sdS + half * (128 * 128) + sw128_offset(t, u)) =
+            make_uint4(pk[4 * u], pk[4 * u + 1], pk[4 * u + 2], pk[4 * u + 3]);
+      tcgen05_fence_before();                 // (also orders the reads of dP before the dQ MMA that may reuse its columns)
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(&bars.ds_ready);
+        mbar_arrive(&bars.st_empty[par]);
+      }
       if (prof_on) {
-        const long long pt4 = clock64();
-        pacc[0] += pt1 - pt0; pacc[1] += pt2 - pt1; pacc[2] += pt3 - pt2; pacc[3] += pt4 - pt3;
+        const long long pt6 = clock64();
+        pacc[0] += (pt1 - pt0) + (pt5 - pt4);
+        pacc[1] += (pt4 - pt1) + (pt6 - pt5);
       }
     }
     if (prof_on) {
-      for (int i = 0; i < 4; ++i) atomicAdd(&p.prof[i], (unsigned long long)pacc[i]);
+      for (int i = 0; i < 2; ++i) atomicAdd(&p.prof[i], (unsigned long long)pacc[i]);
       atomicAdd(&p.prof[4], (unsigned long long)total_steps);
       atomicAdd(&p.prof[5], (unsigned long long)(clock64() - pstart));
       atomicAdd(&p.prof[6], 1ull);
     }
-    if (Cfg::DQ_TMA && threadIdx.x == 0) tma_store_wait<0>();
     // dK, dV of this key block (thread t <-> key k0 + t); fp32 when they are partials of a multi-rank reduction
-    const int key = k0 + t;
     const long long seg_off = (long long)seg * p.seg_stride;
     if (total_steps == 0) {
       if (key < p.Sk) {
@@ -886,7 +1007,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     for (int i = 0; i < 2000; ++i) __nanosleep(1000);
     __syncthreads();
   }
-  if (warp == 9) {
+  if (warp == 13) {
     tcgen05_fence_after();
     tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
   }
@@ -924,20 +1045,22 @@ static int launch_fwd(const CUtensorMap& mq, const KVSegs& segs, void* o, float*
 
 template <int D, bool OUT_F32, bool PROF = false>
 static int launch_bwd(const CUtensorMap& mq, const KVSegs& segs, const CUtensorMap& mdo, const CUtensorMap& mdq, const float* lse,
-                      const float* delta, float* dq_ws, void* dk, void* dv, const BwdParams& p, KernelStatus* st,
-                      cudaStream_t stream) {
+                      const float* delta, void* dk, void* dv, const BwdParams& p, KernelStatus* st, cudaStream_t stream) {
   if (!PROF && p.prof != nullptr)
-    return launch_bwd<D, OUT_F32, true>(mq, segs, mdo, mdq, lse, delta, dq_ws, dk, dv, p, st, stream);
+    return launch_bwd<D, OUT_F32, true>(mq, segs, mdo, mdq, lse, delta, dk, dv, p, st, stream);
   auto kern = attn_bwd_kernel<D, OUT_F32, PROF>;
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdCfg<D>::SMEM) != cudaSuccess) return -3;
     cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    // the warpgroups share out BWD_REGS registers per thread; with fewer at launch setmaxnreg.inc would wait forever
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess || fa.numRegs != BWD_REGS) return -6;
     configured = true;
   }
   const int num_kb = ((p.Sk + 127) / 128) * p.n_segs;
   const long long grid = (long long)num_kb * p.hkv * p.B;
-  launch_pdl(kern, dim3((unsigned)grid), dim3(BWD_THREADS), BwdCfg<D>::SMEM, stream, mq, segs, mdo, mdq, lse, delta, dq_ws, dk, dv, p, st);
+  launch_pdl(kern, dim3((unsigned)grid), dim3(BWD_THREADS), BwdCfg<D>::SMEM, stream, mq, segs, mdo, mdq, lse, delta, dk, dv, p, st);
   pt_count_launches(1);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
@@ -1008,10 +1131,10 @@ static int attention_bwd_impl(const void* dout, const void* q, const void* const
   if ((rc = make_attn_map(&mq, q, B, Sq, hq, d, q_row, 128))) return rc;
   if ((rc = make_attn_map(&mdo, dout, B, Sq, hq, d, (long long)hq * d, 128))) return rc;
   {
-    // fp32 dQ workspace [B, Sq, hq, d]: 32-column x 128-row boxes for the TMA reduce-add (used by the d = 64 kernel)
+    // fp32 dQ workspace [B, Sq, hq, d]: 32-column x 32-row boxes for the TMA reduce-adds
     uint64_t dims[4] = {(uint64_t)d, (uint64_t)hq, (uint64_t)Sq, (uint64_t)B};
     uint64_t strides[3] = {(uint64_t)d, (uint64_t)hq * d, (uint64_t)hq * d * (uint64_t)Sq};
-    uint32_t box[4] = {32, 1, 128, 1};
+    uint32_t box[4] = {32, 1, 32, 1};
     if ((rc = make_f32_map(&mdq, dq_ws, 4, dims, strides, box))) return rc;
   }
   for (int i = 0; i < n_segs; ++i) {
@@ -1024,10 +1147,10 @@ static int attention_bwd_impl(const void* dout, const void* q, const void* const
     return -12;
   BwdParams p{B, Sq, Sk, hq, hkv, causal, scale, dk_row, dv_row, n_segs, seg_stride, cosT, sinT, rope_seq, g_attn_prof};
   KernelStatus* sw = status_word_attn();
-  if (d == 64) rc = out_f32 ? launch_bwd<64, true>(mq, segs, mdo, mdq, lse, delta, dq_ws, dk, dv, p, sw, st)
-                            : launch_bwd<64, false>(mq, segs, mdo, mdq, lse, delta, dq_ws, dk, dv, p, sw, st);
-  else rc = out_f32 ? launch_bwd<128, true>(mq, segs, mdo, mdq, lse, delta, dq_ws, dk, dv, p, sw, st)
-                    : launch_bwd<128, false>(mq, segs, mdo, mdq, lse, delta, dq_ws, dk, dv, p, sw, st);
+  if (d == 64) rc = out_f32 ? launch_bwd<64, true>(mq, segs, mdo, mdq, lse, delta, dk, dv, p, sw, st)
+                            : launch_bwd<64, false>(mq, segs, mdo, mdq, lse, delta, dk, dv, p, sw, st);
+  else rc = out_f32 ? launch_bwd<128, true>(mq, segs, mdo, mdq, lse, delta, dk, dv, p, sw, st)
+                    : launch_bwd<128, false>(mq, segs, mdo, mdq, lse, delta, dk, dv, p, sw, st);
   if (rc) return rc;
   if (dq != nullptr) {
     const long long n = (long long)B * Sq * hq * d;

@@ -62,6 +62,26 @@ def test_attention_backward(C, B, Sq, Sk, hq, hkv, d, causal):
         torch.testing.assert_close(got.float(), want, rtol=5e-2, atol=5e-2)
 
 
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("Sq,Sk,group,causal", [(1, 1, 1, True), (127, 127, 3, True), (129, 129, 1, True), (385, 385, 4, True),
+                                                (640, 640, 2, True), (128, 300, 1, True), (65, 257, 3, False), (513, 64, 2, False)])
+def test_attention_backward_at_tile_and_ring_edges(C, Sq, Sk, group, causal, d):
+    """One step, a step more or less than the operand rings hold, ragged last blocks on either side, keys no query sees."""
+    q, k, v = rnd(2, Sq, 2 * group, d, seed=1), rnd(2, Sk, 2, d, seed=2), rnd(2, Sk, 2, d, seed=3)
+    do = rnd(2, Sq, 2 * group, d, seed=4)
+    scale = 1.0 / math.sqrt(d)
+    o_ref, lse_ref = ref.attention_fwd(q, k, v, causal, scale)
+    want = ref.attention_bwd(do, q, k, v, o_ref, lse_ref, causal, scale)
+    got = C.attention_bwd(do, q, k, v, o_ref, lse_ref, causal, scale)
+    torch.cuda.synchronize()
+    assert C.kernel_status() == 0
+    # P and dS are rounded to bf16 (2^-9) before the second matrix products: the error of a sum of such terms stays below
+    # 2^-9 of the root of its sum of squares, with a factor of four for the cancellation in dS
+    for name, g, w in zip(("dq", "dk", "dv"), got, want):
+        err = float((g.float() - w).norm())
+        assert err <= 1e-2 * float(w.norm()) + 2e-3 * w.numel() ** 0.5, f"{name}: {err} of {float(w.norm())}"
+
+
 @pytest.mark.parametrize("B,S,hq,hkv,d", [(2, 256, 4, 2, 64), (1, 300, 4, 4, 64), (2, 256, 2, 1, 128), (3, 128, 2, 2, 64)])
 def test_attention_backward_with_inverse_rope_on_dq_dk(C, B, S, hq, hkv, d):
     """dq / dk un-rotated inside the backward (dq in the fp32->bf16 conversion, dk in the epilogue) vs the RoPE kernel."""
