@@ -300,6 +300,21 @@ __device__ __forceinline__ void tmem_ld_32x32b_x32_at(uint32_t taddr, uint32_t (
       : "r"(taddr)
       : "memory");
 }
+// r[off .. off+32) of a larger register array -> 32 lanes x 32 columns
+template <int N>
+__device__ __forceinline__ void tmem_st_32x32b_x32_at(uint32_t taddr, const uint32_t (&r)[N], int off) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
+      "r"(r[off + 0]), "r"(r[off + 1]), "r"(r[off + 2]), "r"(r[off + 3]), "r"(r[off + 4]), "r"(r[off + 5]), "r"(r[off + 6]),
+      "r"(r[off + 7]), "r"(r[off + 8]), "r"(r[off + 9]), "r"(r[off + 10]), "r"(r[off + 11]), "r"(r[off + 12]),
+      "r"(r[off + 13]), "r"(r[off + 14]), "r"(r[off + 15]), "r"(r[off + 16]), "r"(r[off + 17]), "r"(r[off + 18]),
+      "r"(r[off + 19]), "r"(r[off + 20]), "r"(r[off + 21]), "r"(r[off + 22]), "r"(r[off + 23]), "r"(r[off + 24]),
+      "r"(r[off + 25]), "r"(r[off + 26]), "r"(r[off + 27]), "r"(r[off + 28]), "r"(r[off + 29]), "r"(r[off + 30]),
+      "r"(r[off + 31])
+      : "memory");
+}
 __device__ __forceinline__ void tmem_st_32x32b_x16(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
