@@ -50,6 +50,7 @@ int pt_ce_grad(void* logits, const long long* targets, const float* lse, long lo
                long long vocab_start, cudaStream_t st);
 int pt_accumulate(float* acc, const void* g, long long n, int g_is_f32, cudaStream_t st);
 int pt_add(const void* a, const void* b, void* out, long long n, cudaStream_t st);
+int pt_scale(float* x, const float* coef, long long n, cudaStream_t st);
 int pt_adamw_multi(void** params, const float** grads, float** ms, float** vs, float** masters,
                    const long long* numels, int count, int param_is_bf16, int step, float lr, float beta1, float beta2,
                    float eps, float wd, cudaStream_t st);
@@ -421,6 +422,14 @@ void adamw_multi_(std::vector<Tensor> params, std::vector<Tensor> grads, std::ve
                 "adamw: parameters must be bf16 or fp32");
 }
 
+void scale_(Tensor& x, const Tensor& coef) {
+  PT_CHECK_F32(x); PT_CHECK_F32(coef);
+  TORCH_CHECK(x.is_contiguous() && coef.numel() == 1 && coef.device() == x.device(),
+              "scale_: a contiguous tensor and one coefficient on its device");
+  c10::cuda::CUDAGuard guard(x.device());
+  PT_CHECK_RC(pt_scale(x.data_ptr<float>(), coef.data_ptr<float>(), x.numel(), stream()), "scale_");
+}
+
 void merge_attention_(Tensor& out, Tensor& lse, const Tensor& bo, const Tensor& bl) {
   PT_CHECK_F32(out); PT_CHECK_F32(lse); PT_CHECK_BF16(bo); PT_CHECK_F32(bl);
   TORCH_CHECK(out.dim() == 4 && out.is_contiguous() && bo.is_contiguous() && bo.sizes() == out.sizes() &&
@@ -670,6 +679,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("accumulate_", &accumulate_);
   m.def("add", &add);
   m.def("adamw_multi_", &adamw_multi_);
+  m.def("scale_", &scale_);
   m.def("merge_attention_", &merge_attention_);
   m.def("attention_fwd", &attention_fwd);
   m.def("attention_bwd", &attention_bwd, py::arg("dout"), py::arg("q"), py::arg("k"), py::arg("v"), py::arg("o"),

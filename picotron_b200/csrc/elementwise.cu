@@ -387,47 +387,123 @@ __global__ void add_kernel(const bf16* __restrict__ a, const bf16* __restrict__ 
 // ---------------------------------------------------------------------------------------------
 // multi-tensor AdamW (decoupled weight decay), fp32 gradients, fp32 or bf16 moments, optional fp32 master
 // ---------------------------------------------------------------------------------------------
-constexpr int ADAM_MAX_TENSORS = 24;
-constexpr int ADAM_MAX_BLOCKS = 320;
-constexpr int ADAM_CHUNK = 65536;
+// Bound by memory: 30 bytes per parameter (gradient, moments and master in; moments, master and bf16 weight out). One launch
+// takes up to 256 tensors (their table travels as a kernel parameter), one block one chunk of 4096 elements of one tensor,
+// found by bisection of the chunk prefix sums, so that the grid fills the chip whatever the tensors' sizes; 16-byte accesses
+// where every pointer of the tensor allows them. Clipping + AdamW of 667M parameters (two layers of the 7B shape with its
+// embedding and head): 6.64 -> 3.67 ms, 96 % of the copy rate (before: launches of at most 320 blocks, 4-byte accesses, and a
+// library multiply at 3.1 TB/s for the clipping).
+constexpr int ADAM_MAX_TENSORS = 256;
+constexpr int ADAM_THREADS = 256;
+constexpr int ADAM_CHUNK = 4096;
 
-struct AdamArgs {
-  void* param[ADAM_MAX_TENSORS];
-  const float* grad[ADAM_MAX_TENSORS];
-  float* m[ADAM_MAX_TENSORS];
-  float* v[ADAM_MAX_TENSORS];
-  float* master[ADAM_MAX_TENSORS];
-  long long numel[ADAM_MAX_TENSORS];
-  unsigned char block_tensor[ADAM_MAX_BLOCKS];
-  int block_chunk[ADAM_MAX_BLOCKS];
+struct AdamTensor {
+  void* param;
+  const float* grad;
+  float* m;
+  float* v;
+  float* master;
+  long long numel;
 };
+struct AdamArgs {
+  AdamTensor t[ADAM_MAX_TENSORS];
+  unsigned first_block[ADAM_MAX_TENSORS + 1];      // first block of each tensor; [count] = grid size
+  unsigned char vec[ADAM_MAX_TENSORS];             // 1: every pointer is aligned for 4-element accesses
+  int count;
+};
+static_assert(sizeof(AdamArgs) <= 32000, "kernel parameter limit");
+
+__device__ __forceinline__ void adam_update(float& w, float& m, float& v, float g, float lr, float beta1, float beta2, float eps,
+                                            float wd, float bc1, float bc2_sqrt) {
+  m = m * beta1 + g * (1.f - beta1);
+  v = v * beta2 + g * g * (1.f - beta2);
+  w = w * (1.f - lr * wd);
+  w -= (lr / bc1) * (m / (sqrtf(v) / bc2_sqrt + eps));
+}
 
 template <bool PARAM_BF16>
-__global__ void __launch_bounds__(512)
+__global__ void __launch_bounds__(ADAM_THREADS)
 adamw_kernel(const __grid_constant__ AdamArgs args, float lr, float beta1, float beta2, float eps, float wd,
              float bc1, float bc2_sqrt) {
-  const int ti = args.block_tensor[blockIdx.x];
-  const long long base = (long long)args.block_chunk[blockIdx.x] * ADAM_CHUNK;
-  const long long n = args.numel[ti];
-  const float* g = args.grad[ti];
-  float* m = args.m[ti];
-  float* v = args.v[ti];
-  float* mw = args.master[ti];
-  for (long long i = base + threadIdx.x; i < base + ADAM_CHUNK && i < n; i += blockDim.x) {
+  int lo = 0, hi = args.count;                     // the tensor of this block: first_block[lo] <= blockIdx.x < first_block[lo + 1]
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (args.first_block[mid] <= blockIdx.x) lo = mid;
+    else hi = mid;
+  }
+  const AdamTensor& t = args.t[lo];
+  const long long base = (long long)(blockIdx.x - args.first_block[lo]) * ADAM_CHUNK;
+  const long long end = min(base + ADAM_CHUNK, t.numel);
+  if (args.vec[lo] && end - base == ADAM_CHUNK) {
+    constexpr int ITERS = ADAM_CHUNK / (4 * ADAM_THREADS);
+#pragma unroll 2
+    for (int k = 0; k < ITERS; ++k) {
+      const long long i = base + (long long)(k * ADAM_THREADS + threadIdx.x) * 4;
+      const float4 g = __ldcs(reinterpret_cast<const float4*>(t.grad + i));
+      float4 m = __ldcs(reinterpret_cast<const float4*>(t.m + i));
+      float4 v = __ldcs(reinterpret_cast<const float4*>(t.v + i));
+      float4 w;
+      if (t.master != nullptr) {
+        w = __ldcs(reinterpret_cast<const float4*>(t.master + i));
+      } else if (PARAM_BF16) {
+        const uint2 q = *reinterpret_cast<const uint2*>(reinterpret_cast<const bf16*>(t.param) + i);
+        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&q.x));
+        const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&q.y));
+        w = make_float4(a.x, a.y, b.x, b.y);
+      } else {
+        w = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(t.param) + i);
+      }
+      adam_update(w.x, m.x, v.x, g.x, lr, beta1, beta2, eps, wd, bc1, bc2_sqrt);
+      adam_update(w.y, m.y, v.y, g.y, lr, beta1, beta2, eps, wd, bc1, bc2_sqrt);
+      adam_update(w.z, m.z, v.z, g.z, lr, beta1, beta2, eps, wd, bc1, bc2_sqrt);
+      adam_update(w.w, m.w, v.w, g.w, lr, beta1, beta2, eps, wd, bc1, bc2_sqrt);
+      __stcs(reinterpret_cast<float4*>(t.m + i), m);
+      __stcs(reinterpret_cast<float4*>(t.v + i), v);
+      if (t.master != nullptr) __stcs(reinterpret_cast<float4*>(t.master + i), w);
+      if (PARAM_BF16) {
+        uint2 q;
+        q.x = pack_bf16(w.x, w.y);
+        q.y = pack_bf16(w.z, w.w);
+        *reinterpret_cast<uint2*>(reinterpret_cast<bf16*>(t.param) + i) = q;
+      } else {
+        *reinterpret_cast<float4*>(reinterpret_cast<float*>(t.param) + i) = w;
+      }
+    }
+    return;
+  }
+  for (long long i = base + threadIdx.x; i < end; i += ADAM_THREADS) {
     float w;
-    if (mw != nullptr) w = mw[i];
-    else if (PARAM_BF16) w = __bfloat162float(reinterpret_cast<bf16*>(args.param[ti])[i]);
-    else w = reinterpret_cast<float*>(args.param[ti])[i];
-    const float gi = g[i];
-    const float mi = m[i] * beta1 + gi * (1.f - beta1);
-    const float vi = v[i] * beta2 + gi * gi * (1.f - beta2);
-    w = w * (1.f - lr * wd);
-    w -= (lr / bc1) * (mi / (sqrtf(vi) / bc2_sqrt + eps));
-    m[i] = mi;
-    v[i] = vi;
-    if (mw != nullptr) mw[i] = w;
-    if (PARAM_BF16) reinterpret_cast<bf16*>(args.param[ti])[i] = __float2bfloat16(w);
-    else reinterpret_cast<float*>(args.param[ti])[i] = w;
+    if (t.master != nullptr) w = t.master[i];
+    else if (PARAM_BF16) w = __bfloat162float(reinterpret_cast<bf16*>(t.param)[i]);
+    else w = reinterpret_cast<float*>(t.param)[i];
+    float m = t.m[i], v = t.v[i];
+    adam_update(w, m, v, t.grad[i], lr, beta1, beta2, eps, wd, bc1, bc2_sqrt);
+    t.m[i] = m;
+    t.v[i] = v;
+    if (t.master != nullptr) t.master[i] = w;
+    if (PARAM_BF16) reinterpret_cast<bf16*>(t.param)[i] = __float2bfloat16(w);
+    else reinterpret_cast<float*>(t.param)[i] = w;
+  }
+}
+
+// x *= *coef over a contiguous fp32 buffer (gradient clipping). Bound by memory: 8 bytes per element; a coefficient of exactly
+// 1 (nothing to clip) leaves the buffer untouched without reading it.
+constexpr int SCALE_CHUNK = 8192;
+__global__ void __launch_bounds__(256) scale_kernel(float* __restrict__ x, const float* __restrict__ coef, long long n) {
+  const float c = *coef;
+  if (c == 1.f) return;
+  const long long base = (long long)blockIdx.x * SCALE_CHUNK;
+  const bool aligned = (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+  if (aligned && base + SCALE_CHUNK <= n) {
+#pragma unroll
+    for (int k = 0; k < SCALE_CHUNK / 1024; ++k) {
+      float4* q = reinterpret_cast<float4*>(x + base) + k * 256 + threadIdx.x;
+      float4 v = __ldcs(q);
+      v.x *= c; v.y *= c; v.z *= c; v.w *= c;
+      __stcs(q, v);
+    }
+  } else {
+    for (long long i = base + threadIdx.x; i < n && i < base + SCALE_CHUNK; i += 256) x[i] *= c;
   }
 }
 
@@ -897,41 +973,39 @@ extern "C" int pt_adamw_multi(void** params, const float** grads, float** ms, fl
   const float bc1 = 1.f - powf(beta1, (float)step);
   const float bc2_sqrt = sqrtf(1.f - powf(beta2, (float)step));
   AdamArgs args;
-  int nt = 0, nb = 0;
+  args.count = 0;
+  long long blocks = 0;
   auto flush = [&]() -> int {
-    if (nb == 0) return 0;
+    if (args.count == 0) return 0;
+    args.first_block[args.count] = (unsigned)blocks;
     if (param_is_bf16)
-      adamw_kernel<true><<<nb, 512, 0, st>>>(args, lr, beta1, beta2, eps, wd, bc1, bc2_sqrt);
+      adamw_kernel<true><<<(unsigned)blocks, ADAM_THREADS, 0, st>>>(args, lr, beta1, beta2, eps, wd, bc1, bc2_sqrt);
     else
-      adamw_kernel<false><<<nb, 512, 0, st>>>(args, lr, beta1, beta2, eps, wd, bc1, bc2_sqrt);
-    nt = nb = 0;
+      adamw_kernel<false><<<(unsigned)blocks, ADAM_THREADS, 0, st>>>(args, lr, beta1, beta2, eps, wd, bc1, bc2_sqrt);
+    args.count = 0;
+    blocks = 0;
     return check_launch();
   };
   for (int i = 0; i < count; ++i) {
     const long long n = numels[i];
     if (n == 0) continue;
-    long long chunks = (n + ADAM_CHUNK - 1) / ADAM_CHUNK;
-    long long c0 = 0;
-    while (c0 < chunks) {
-      if (nt == ADAM_MAX_TENSORS || nb == ADAM_MAX_BLOCKS) {
-        if (int rc = flush()) return rc;
-      }
-      args.param[nt] = params[i];
-      args.grad[nt] = grads[i];
-      args.m[nt] = ms[i];
-      args.v[nt] = vs[i];
-      args.master[nt] = masters[i];
-      args.numel[nt] = n;
-      while (c0 < chunks && nb < ADAM_MAX_BLOCKS) {
-        args.block_tensor[nb] = (unsigned char)nt;
-        args.block_chunk[nb] = (int)c0;
-        ++nb;
-        ++c0;
-      }
-      ++nt;
-    }
+    const long long chunks = (n + ADAM_CHUNK - 1) / ADAM_CHUNK;
+    if (args.count == ADAM_MAX_TENSORS || (args.count > 0 && blocks + chunks > 0x7fffffffLL))
+      if (int rc = flush()) return rc;
+    const uintptr_t f32s = (uintptr_t)grads[i] | (uintptr_t)ms[i] | (uintptr_t)vs[i] | (uintptr_t)masters[i];
+    const int k = args.count++;
+    args.t[k] = AdamTensor{params[i], grads[i], ms[i], vs[i], masters[i], n};
+    args.vec[k] = (f32s & 15) == 0 && ((uintptr_t)params[i] & (param_is_bf16 ? 7 : 15)) == 0;
+    args.first_block[k] = (unsigned)blocks;
+    blocks += chunks;
   }
   return flush();
+}
+
+extern "C" int pt_scale(float* x, const float* coef, long long n, cudaStream_t st) {
+  if (n == 0) return 0;
+  scale_kernel<<<(unsigned)((n + SCALE_CHUNK - 1) / SCALE_CHUNK), 256, 0, st>>>(x, coef, n);
+  return check_launch();
 }
 
 extern "C" int pt_merge_attention(float* out, float* lse, const void* bo, const float* bl, int B, int S, int h, int d,

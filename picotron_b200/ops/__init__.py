@@ -240,6 +240,14 @@ def accumulate_(main_grad, grad):
     ref.accumulate_(main_grad, grad)
 
 
+def scale_(x, coef):
+    """``x *= coef`` in place; ``coef`` is a one-element tensor on the device of ``x`` (no host synchronisation)."""
+    if x.is_cuda and x.dtype == torch.float32 and x.is_contiguous() and coef.device == x.device:
+        _c().scale_(x, coef.to(x.dtype))
+        return x
+    return x.mul_(coef.to(x.dtype))
+
+
 def merge_attention_(out, lse, block_out, block_lse):
     if out.is_cuda:
         _c().merge_attention_(out, lse, block_out, block_lse)
@@ -250,7 +258,7 @@ def merge_attention_(out, lse, block_out, block_lse):
 # ------------------------------------------------------------------ checked mode
 _CHECKED_OPS = ("rmsnorm_fwd", "add_rmsnorm_fwd", "rmsnorm_bwd", "rope_", "swiglu_fwd", "swiglu_bwd", "linear_swiglu_fwd",
                 "linear_rope_fwd", "linear_add_fwd", "linear_dgrad_swiglu_bwd", "linear_fwd", "linear_dgrad", "linear_wgrad", "attention_fwd", "attention_bwd",
-                "embedding_fwd", "embedding_bwd", "ce_stats", "linear_ce_stats", "ce_grad_", "add", "accumulate_", "merge_attention_")
+                "embedding_fwd", "embedding_bwd", "ce_stats", "linear_ce_stats", "ce_grad_", "add", "accumulate_", "scale_", "merge_attention_")
 _UNCHECKED = {}
 
 

@@ -23,6 +23,7 @@ from typing import Iterable
 import torch
 import torch.distributed as dist
 
+from . import ops
 from .ops import reference as ref
 from .ops import _ext
 
@@ -251,7 +252,7 @@ def clip_grad_norm_(model, max_norm: float) -> torch.Tensor:
     norm = sq.clamp_min(0).sqrt()
     coef = torch.clamp(max_norm / (norm + 1e-6), max=1.0).float()
     if manager is not None:
-        manager.flat.mul_(coef.to(manager.flat.dtype))
+        ops.scale_(manager.flat, coef)
     else:
         for x in grads.values():
             if x is not None:

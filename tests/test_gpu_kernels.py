@@ -359,3 +359,35 @@ def test_adamw_multi_tensor(C, master):
     if master:
         for a, b in zip(masters, rmw):
             torch.testing.assert_close(a, b, rtol=1e-4, atol=1e-5)
+
+
+@pytest.mark.parametrize("dtype,offset,count", [(torch.bfloat16, 0, 3), (torch.bfloat16, 1, 3), (torch.float32, 0, 3),
+                                                (torch.float32, 1, 3), (torch.bfloat16, 0, 300)])
+def test_adamw_chunk_edges_alignment_and_table_size(C, dtype, offset, count):
+    """Sizes around a block's 4096 elements, slices that start off a 16-byte boundary, more tensors than one launch takes."""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    sizes = [(1, 4095, 4096, 4097, 12289, 5)[i % 6] for i in range(2 * count)]
+    new = lambda n, dt: torch.randn(n + offset, device="cuda", generator=g).to(dt)[offset:]
+    params, grads = [new(n, dtype) for n in sizes], [new(n, torch.float32) for n in sizes]
+    ms, vs = [new(n, torch.float32) for n in sizes], [new(n, torch.float32).abs() for n in sizes]
+    masters = [None] * len(sizes)
+    want = [x.clone() for x in params], [x.clone() for x in ms], [x.clone() for x in vs]
+    C.adamw_multi_(params, grads, ms, vs, masters, 3, 1e-2, 0.9, 0.999, 1e-8, 0.01)
+    ref.adamw_step_(want[0], grads, want[1], want[2], masters, 3, 1e-2, 0.9, 0.999, 1e-8, 0.01)
+    # fp32 arithmetic in another order: a few ulps; a bf16 weight may round to its other neighbour, and
+    # neighbours (8 significant bits) are between 2^-8 and 2^-7 of their value apart
+    tol = dict(rtol=2 ** -7, atol=1e-6) if dtype == torch.bfloat16 else dict(rtol=1e-5, atol=1e-5)
+    for got, exp, t in ((params, want[0], tol), (ms, want[1], dict(rtol=1e-5, atol=1e-6)), (vs, want[2], dict(rtol=1e-5, atol=1e-6))):
+        for a, b in zip(got, exp):
+            torch.testing.assert_close(a, b, **t)
+
+
+@pytest.mark.parametrize("n", [1, 8191, 8192, 8193, 40000])
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("c", [0.37, 1.0])
+def test_scale_by_a_device_coefficient(C, n, offset, c):
+    x = torch.randn(n + offset + 3, device="cuda")
+    want = x.clone()
+    want[offset:offset + n] *= c
+    C.scale_(x[offset:offset + n], torch.tensor(c, device="cuda"))
+    assert torch.equal(x, want)
