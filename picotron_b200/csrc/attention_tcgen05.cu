@@ -377,10 +377,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 // ---------------------------------------------------------------------------------------------------------
 // backward helpers: delta = rowsum(dO * O) and fp32 -> bf16 conversion of dQ
 // ---------------------------------------------------------------------------------------------------------
-// D / 8 threads per (b, s, head) row, 16 bytes of dO and of O per thread, reduced with shuffles inside the group.
+// D / 8 threads per (b, s, head) row, 16 bytes of dO and of O per thread, reduced with shuffles inside the group. The fp32
+// workspace that dQ is accumulated in is cleared on the way (a fill of its own was one more launch and as many bytes).
 template <int D>
 __global__ void __launch_bounds__(256)
-delta_kernel(const bf16* __restrict__ dO, const bf16* __restrict__ O, float* __restrict__ delta, int B, int S, int h) {
+delta_kernel(const bf16* __restrict__ dO, const bf16* __restrict__ O, float* __restrict__ delta, float* __restrict__ dq_ws, int B,
+             int S, int h) {
   constexpr int TPR = D / 8;
   pdl_enter();
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -391,6 +393,10 @@ delta_kernel(const bf16* __restrict__ dO, const bf16* __restrict__ O, float* __r
   const uint4 a = *reinterpret_cast<const uint4*>(dO + r * D + part * 8);
   const uint4 o = *reinterpret_cast<const uint4*>(O + r * D + part * 8);
   const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, ow[4] = {o.x, o.y, o.z, o.w};
+  if (rid < total) {
+    float4* z = reinterpret_cast<float4*>(dq_ws + r * D + part * 8);
+    z[0] = z[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
   float acc = 0.f;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -1096,7 +1102,8 @@ extern "C" int pt_attention_fwd(const void* q, const void* k, const void* v, voi
 }
 
 // Backward over `n_segs` K/V segments (see pt_attention_fwd_segs). dout, o [B,Sq,hq,d] bf16 contiguous; lse [B,hq,Sq];
-// delta_in optional (else computed into delta_ws [B,hq,Sq]); dq_ws fp32 [B,Sq,hq,d] zero-initialised scratch; dq bf16 with
+// delta_in optional (else computed into delta_ws [B,hq,Sq]); dq_ws fp32 [B,Sq,hq,d] scratch, cleared together with the computation of
+// delta and therefore to be handed in zeroed where delta_in is given; dq bf16 with
 // token stride dq_row. dk/dv: outputs of segment i start i*seg_stride elements after dk/dv, token strides dk_row/dv_row,
 // bf16 or (out_f32) fp32 -- fp32 is used when they are partial sums that another rank reduces.
 static int attention_bwd_impl(const void* dout, const void* q, const void* const* k_ptrs, const void* const* v_ptrs,
@@ -1115,8 +1122,8 @@ static int attention_bwd_impl(const void* dout, const void* q, const void* const
   if (delta == nullptr) {
     const long long threads = (long long)B * Sq * hq * (d / 8);
     const unsigned blocks = (unsigned)((threads + 255) / 256);
-    if (d == 64) launch_pdl(delta_kernel<64>, dim3(blocks), dim3(256), 0, st, (const bf16*)dout, (const bf16*)o, delta_ws, B, Sq, hq);
-    else launch_pdl(delta_kernel<128>, dim3(blocks), dim3(256), 0, st, (const bf16*)dout, (const bf16*)o, delta_ws, B, Sq, hq);
+    if (d == 64) launch_pdl(delta_kernel<64>, dim3(blocks), dim3(256), 0, st, (const bf16*)dout, (const bf16*)o, delta_ws, dq_ws, B, Sq, hq);
+    else launch_pdl(delta_kernel<128>, dim3(blocks), dim3(256), 0, st, (const bf16*)dout, (const bf16*)o, delta_ws, dq_ws, B, Sq, hq);
     pt_count_launches(1);
     delta = delta_ws;
   }

@@ -485,7 +485,7 @@ std::vector<Tensor> attention_bwd(const Tensor& dout, const Tensor& q, const Ten
   }
   auto f = q.options().dtype(at::kFloat);
   Tensor delta_ws = torch::empty({B, hq, Sq}, f);
-  Tensor dq_ws = torch::zeros({B, Sq, hq, d}, f);
+  Tensor dq_ws = delta.has_value() ? torch::zeros({B, Sq, hq, d}, f) : torch::empty({B, Sq, hq, d}, f);
   if (delta.has_value()) { PT_CHECK_F32(*delta); TORCH_CHECK(delta->is_contiguous() && delta->numel() == delta_ws.numel()); }
   const float* cosp = nullptr;
   const float* sinp = nullptr;
@@ -509,6 +509,101 @@ std::vector<Tensor> attention_bwd(const Tensor& dout, const Tensor& q, const Ten
                                     token_stride(dv, "dv"), causal ? 1 : 0, (float)scale, cosp, sinp, rope_seq, stream()),
               "attention_bwd");
   return {dq, dk, dv};
+}
+
+// ---------------------------------------------------------------------------------------------
+// A decoder layer's launches in one call (one GPU per layer: no tensor, sequence or context parallelism). Small models and
+// short sequences are bound by the host: from Python every launch costs 12 to 20 us, more than most of their kernels take.
+// The kernels, their order and the fallbacks are those of the layer node's Python path.
+// ---------------------------------------------------------------------------------------------
+struct LayerDims {
+  int64_t B, S, hq, hkv, d;
+};
+
+std::vector<Tensor> split_qkv(const Tensor& qkv, const LayerDims& n) {
+  return {qkv.narrow(1, 0, n.hq * n.d).view({n.B, n.S, n.hq, n.d}),
+          qkv.narrow(1, n.hq * n.d, n.hkv * n.d).view({n.B, n.S, n.hkv, n.d}),
+          qkv.narrow(1, (n.hq + n.hkv) * n.d, n.hkv * n.d).view({n.B, n.S, n.hkv, n.d})};
+}
+
+bool all_bf16_cuda(std::initializer_list<const Tensor*> ts) {
+  for (const Tensor* t : ts)
+    if (!t->is_cuda() || t->scalar_type() != at::kBFloat16) return false;
+  return true;
+}
+
+// Returns {x_out, h1, rstd1, qkv, o, lse, x_mid, rstd2, h2, gu, a}, or {} (nothing launched) for operands that are not bf16.
+std::vector<Tensor> decoder_layer_fwd(const Tensor& x, const Tensor& ln1, const Tensor& w_qkv, const Tensor& cosT, const Tensor& sinT,
+                                      const Tensor& wo, const Tensor& ln2, const Tensor& w_gu, const Tensor& wd, double eps, int64_t B,
+                                      int64_t S, int64_t hq, int64_t hkv, int64_t d, double scale) {
+  if (!all_bf16_cuda({&x, &ln1, &w_qkv, &wo, &ln2, &w_gu, &wd})) return {};
+  const LayerDims n{B, S, hq, hkv, d};
+  auto n1 = rmsnorm_fwd(x, ln1, eps);
+  Tensor qkv = gemm_rope(n1[0], w_qkv, cosT, sinT, hq + hkv, d, S);
+  if (!qkv.defined()) {
+    qkv = gemm(n1[0], w_qkv, false, false, c10::nullopt, false);
+    rope_(qkv, cosT, sinT, hq + hkv, d, S, false);
+  }
+  auto parts = split_qkv(qkv, n);
+  auto att = attention_fwd(parts[0], parts[1], parts[2], true, scale);
+  const Tensor o2 = att[0].view({B * S, hq * d});
+  auto n2 = add_rmsnorm_fwd(x, gemm(o2, wo, false, false, c10::nullopt, false), ln2, eps);      // {x_mid, h2, rstd2}
+  auto mlp = gemm_swiglu(n2[1], w_gu);
+  if (mlp.empty()) {
+    Tensor gu = gemm(n2[1], w_gu, false, false, c10::nullopt, false);
+    mlp = {gu, swiglu_fwd(gu)};
+  }
+  Tensor out = gemm_add(mlp[1], wd, n2[0]);
+  if (!out.defined()) out = ::add(n2[0], gemm(mlp[1], wd, false, false, c10::nullopt, false));
+  return {out, n1[0], n1[1], qkv, o2, att[1], n2[0], n2[2], n2[1], mlp[0], mlp[1]};
+}
+
+// The fp32 regions of parameters that one GEMM accumulates into together, as one [rows, cols] tensor; undefined unless they
+// are adjacent in one storage.
+Tensor packed_region(const std::vector<Tensor>& parts) {
+  const Tensor& f = parts[0];
+  int64_t rows = 0;
+  for (const Tensor& t : parts) {
+    if (t.dim() != 2 || !t.is_contiguous() || t.size(1) != f.size(1) || t.scalar_type() != at::kFloat || !t.is_cuda() ||
+        t.storage().data() != f.storage().data() || t.storage_offset() != f.storage_offset() + rows * f.size(1))
+      return Tensor();
+    rows += t.size(0);
+  }
+  return parts.size() == 1 ? f : f.as_strided({rows, f.size(1)}, {f.size(1), 1}, f.storage_offset());
+}
+
+// Backward of decoder_layer_fwd; the weight gradients are added to the fp32 regions `mg` (q, k, v, out, gate, up, down, norm 1,
+// norm 2). `saved` = {x, rstd1, h1, qkv, o, lse, x_mid, rstd2, h2, gu, a}. Returns dx, or an undefined tensor (nothing launched).
+Tensor decoder_layer_bwd(const Tensor& dout, const std::vector<Tensor>& saved, const Tensor& ln1, const Tensor& w_qkv,
+                         const Tensor& cosT, const Tensor& sinT, const Tensor& wo, const Tensor& ln2, const Tensor& w_gu,
+                         const Tensor& wd, const std::vector<Tensor>& mg, int64_t B, int64_t S, int64_t hq, int64_t hkv, int64_t d,
+                         double scale) {
+  TORCH_CHECK(saved.size() == 11 && mg.size() == 9);
+  if (!all_bf16_cuda({&dout, &ln1, &w_qkv, &wo, &ln2, &w_gu, &wd})) return Tensor();
+  const Tensor mg_qkv = packed_region({mg[0], mg[1], mg[2]}), mg_o = packed_region({mg[3]}), mg_gu = packed_region({mg[4], mg[5]}),
+               mg_d = packed_region({mg[6]});
+  if (!mg_qkv.defined() || !mg_o.defined() || !mg_gu.defined() || !mg_d.defined()) return Tensor();
+  for (int i = 7; i < 9; ++i)
+    if (!mg[i].is_cuda() || mg[i].scalar_type() != at::kFloat || !mg[i].is_contiguous()) return Tensor();
+  const Tensor &x = saved[0], &rstd1 = saved[1], &h1 = saved[2], &qkv = saved[3], &o2 = saved[4], &lse = saved[5], &x_mid = saved[6],
+               &rstd2 = saved[7], &h2 = saved[8], &gu = saved[9], &a = saved[10];
+  const LayerDims n{B, S, hq, hkv, d};
+  Tensor dgu = gemm_dgrad_swiglu_bwd(dout, wd, gu);
+  if (!dgu.defined()) dgu = swiglu_bwd(gu, gemm(dout, wd, false, true, c10::nullopt, false));
+  gemm(dout, a, true, true, mg_d, true);
+  Tensor dh = gemm(dgu, w_gu, false, true, c10::nullopt, false);
+  gemm(dgu, h2, true, true, mg_gu, true);
+  dgu = Tensor();
+  const Tensor dx_mid = rmsnorm_bwd(dh, x_mid, ln2, rstd2, dout, mg[8])[0];
+  dh = gemm(dx_mid, wo, false, true, c10::nullopt, false);                     // dL/d(attention output)
+  gemm(dx_mid, o2, true, true, mg_o, true);
+  auto parts = split_qkv(qkv, n);
+  Tensor dqkv = torch::empty_like(qkv);
+  attention_bwd(dh.view({B, S, hq, d}), parts[0], parts[1], parts[2], o2.view({B, S, hq, d}), lse, true, scale, c10::nullopt,
+                split_qkv(dqkv, n), cosT, sinT);
+  dh = gemm(dqkv, w_qkv, false, true, c10::nullopt, false);
+  gemm(dqkv, h1, true, true, mg_qkv, true);
+  return rmsnorm_bwd(dh, x, ln1, rstd1, dx_mid, mg[7])[0];
 }
 
 void allreduce_symm(std::vector<int64_t> buf_ptrs, std::vector<int64_t> flag_ptrs, int64_t mc_ptr, int64_t offset_elems,
@@ -555,7 +650,8 @@ Tensor attention_bwd_segs(const Tensor& dout, const Tensor& q, std::vector<int64
   const void* kp[8]; const void* vp[8];
   for (int i = 0; i < n; ++i) { kp[i] = reinterpret_cast<const void*>(k_ptrs[i]); vp[i] = reinterpret_cast<const void*>(v_ptrs[i]); }
   auto dq = torch::empty({B, Sq, hq, d}, q.options());
-  auto dq_ws = torch::zeros({B, Sq, hq, d}, q.options().dtype(at::kFloat));
+  const auto f32 = q.options().dtype(at::kFloat);
+  auto dq_ws = delta.has_value() ? torch::zeros({B, Sq, hq, d}, f32) : torch::empty({B, Sq, hq, d}, f32);
   auto delta_ws = torch::empty({B, hq, Sq}, q.options().dtype(at::kFloat));
   float* part = reinterpret_cast<float*>(partial_ptr);
   const long long per = (long long)B * Sk * hkv * d;
@@ -679,6 +775,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("accumulate_", &accumulate_);
   m.def("add", &add);
   m.def("adamw_multi_", &adamw_multi_);
+  m.def("decoder_layer_fwd", &decoder_layer_fwd);
+  m.def("decoder_layer_bwd", &decoder_layer_bwd);
   m.def("scale_", &scale_);
   m.def("merge_attention_", &merge_attention_);
   m.def("attention_fwd", &attention_fwd);

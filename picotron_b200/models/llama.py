@@ -362,6 +362,17 @@ class DecoderLayerFn(torch.autograd.Function):
         w_qkv = layer.packed_qkv()
         w_gu = layer.packed_gu()
 
+        if tp_group is None and not att.cp_enabled and ops.runs_layer_natively(x2):
+            cos, sin = layer.rope(x.device)
+            r = ops.decoder_layer_fwd(x2, ln1_w, w_qkv, cos, sin, wo, ln2_w, w_gu, wd, layer.eps, B, S, hq, hkv, d, layer.sm_scale)
+            if r:
+                out, h1, rstd1, qkv, o2, lse, x_mid, rstd2, h2, gu, a = r
+                ctx.save_for_backward(x2, rstd1, h1, qkv, o2, lse, x_mid, rstd2, h2, gu, a)
+                ctx.layer = layer
+                ctx.dims = (B, S, H, S_in)
+                ctx.sp_group = None
+                return out.view(B, S_in, H)
+
         h1, rstd1 = ops.rmsnorm_fwd(x2, ln1_w, layer.eps)
         h1_all = tpc.gather_tokens(h1, sp_group) if sp_group is not None else h1
         cos, sin = layer.rope(x.device)
@@ -417,6 +428,19 @@ class DecoderLayerFn(torch.autograd.Function):
         if not dout2.is_contiguous():
             dout2 = dout2.contiguous()
         sp = sp_group is not None
+        if not sp and tp_group is None and not att.cp_enabled and pgm.get().cp_dp_world_size == 1 and ops.runs_layer_natively(dout2):
+            # (with several data-parallel replicas a bucket's all-reduce starts as soon as its last gradient is there)
+            params = (att.q_proj.weight, att.k_proj.weight, att.v_proj.weight, wo, mlp.gate_proj.weight, mlp.up_proj.weight, wd,
+                      ln1.weight, ln2.weight)
+            grads = [getattr(p, "main_grad", None) for p in params]
+            if all(g is not None for g in grads):
+                cos, sin = layer.rope(dout.device)
+                dx = ops.decoder_layer_bwd(dout2, [x2, rstd1, h1, qkv, o2, lse, x_mid, rstd2, h2, gu, a], ln1.weight, w_qkv, cos, sin,
+                                           wo, ln2.weight, w_gu, wd, grads, B, S, hq, hkv, d, layer.sm_scale)
+                if dx is not None:
+                    for p in params:
+                        notify_grad_ready(p)
+                    return dx.view(B, S_in, H), None, None, None, None, None, None, None, None, None, None
         dout_all = tpc.gather_tokens(dout2, sp_group) if sp else dout2      # backward of the forward's reduce-scatter
 
         # ---- MLP

@@ -184,6 +184,23 @@ def attention_bwd(do, q, k, v, o, lse, causal: bool, scale: Optional[float] = No
     return res
 
 
+# ------------------------------------------------------------------ a decoder layer's launches in one native call
+def runs_layer_natively(x) -> bool:
+    """Whether :func:`decoder_layer_fwd` / :func:`decoder_layer_bwd` may be used for ``x``: bf16 on the GPU, with the fused
+    epilogues on. Checked mode looks at every single op and keeps the separate calls."""
+    return x.is_cuda and x.dtype == torch.bfloat16 and FUSE_GEMM_EPILOGUES and not _UNCHECKED
+
+
+def decoder_layer_fwd(*args):
+    """``(x_out, h1, rstd1, qkv, o, lse, x_mid, rstd2, h2, gu, a)`` of a layer on one GPU, or ``[]`` if it is not covered."""
+    return _c().decoder_layer_fwd(*args)
+
+
+def decoder_layer_bwd(*args):
+    """``dx`` of a layer whose weight gradients go into fp32 regions, or None (and nothing launched) if it is not covered."""
+    return _c().decoder_layer_bwd(*args)
+
+
 # ------------------------------------------------------------------ embedding
 def embedding_fwd(ids, w, vocab_start: int = 0):
     if w.is_cuda:
