@@ -6,6 +6,8 @@
 // accumulation; train.py:209,235 AdamW; context_parallel.py:157-187 LSE merge).
 // All of them are bandwidth-bound: 16-byte vector accesses, fp32 math, one pass over HBM per tensor.
 #include "common.cuh"
+
+#include <type_traits>
 #include "noalloc.h"
 
 namespace pt {
@@ -550,228 +552,231 @@ static inline int check_launch(int n = 1) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// Row-block RMSNorm kernels (the ones the training step runs). A CTA of 256 threads owns fixed columns -- thread t
-// holds the 16-byte chunks t, t + 256, ... of a row -- and walks the rows R at a time: all loads of the R rows are
-// issued before the first reduction, the R row sums are reduced together (one CTA barrier per R rows, double-buffered
-// scratch), and because the columns of a thread never change, the weight and the weight-gradient accumulators live
-// in registers for the whole kernel. (One CTA per row forward and one warp per row backward, which these replace, reached
-// 0.3-0.4 of the copy bandwidth: every row was a load -> reduce -> store chain with nothing else in flight in that warp.)
+// RMSNorm kernels of the training step. Bound by memory: 4 (forward), 8 (with the residual add) and 8 (backward) bytes per
+// element. A TEAM of 32, 64, 128 or 256 threads holds one row, at most 4 16-byte chunks per thread, so that a row is one batch
+// of loads, one reduction among the team's own warps and one batch of stores, and a CTA of 256 threads works on 256 / TEAM
+// independent rows. Forward: one row per team and a CTA for every 256 / TEAM rows. Backward: two CTAs per SM walk the rows; a
+// thread's columns never change, so the weight gradient is summed in registers, then over the CTA's teams in shared memory, and
+// added to the destination once per CTA.
 //   forward :  x_new = x (+ delta); rstd = rsqrt(mean(x_new^2) + eps); y = x_new * rstd * w
 //   backward:  dx = rstd * (w*dy - xhat * mean(xhat*w*dy)) (+ dres);  dw_acc += sum_rows dy * xhat   (fp32 reductions)
-// H % 8 == 0, H <= 8 * 256 * NC.
+// H % 8 == 0, H <= 8 * 4 * TEAM. (Before, the whole CTA held four rows at a time: at H = 576 two thirds of its threads had no
+// column, and every four rows waited for one CTA barrier. Measured then
+// and now, us, launch included: forward / with add / backward of 8192 x 576: 14.3 -> 12.3 / 17.1 -> 14.3 / 26.6 -> 16.4;
+// 4096 x 960: 12.3 -> 10.2 / 14.3 -> 13.2 / 20.5 -> 16.4; 4096 x 2048: 14.3 / 20.5 -> 18.4 / 24.6 -> 22.6.)
 // ---------------------------------------------------------------------------------------------
 constexpr int ROWS_THREADS = 256;
 
-// sums[r] over the CTA for r < R; `red` is [2][R][8] floats, `it` alternates the half that is written
-template <int R>
-__device__ __forceinline__ void block_sum_rows(float (&v)[R], float* red, int it) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float* buf = red + (it & 1) * R * 8;
+// sum of v over the team; `red` has 8 floats per parity of `it`
+template <int TEAM>
+__device__ __forceinline__ float team_sum(float v, float* red, int it) {
+  v = warp_sum(v);
+  if constexpr (TEAM > 32) {
+    constexpr int WARPS = TEAM / 32;
+    const int warp = threadIdx.x >> 5, team = threadIdx.x / TEAM;
+    float* buf = red + (it & 1) * 8;
+    if ((threadIdx.x & 31) == 0) buf[warp] = v;
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "n"(TEAM) : "memory");
+    v = 0.f;
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    v[r] = warp_sum(v[r]);
-    if (lane == 0) buf[r * 8 + warp] = v[r];
+    for (int i = 0; i < WARPS; ++i) v += buf[team * WARPS + i];
   }
-  __syncthreads();
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const float4 a = *reinterpret_cast<const float4*>(buf + r * 8), b = *reinterpret_cast<const float4*>(buf + r * 8 + 4);
-    v[r] = (a.x + a.y) + (a.z + a.w) + (b.x + b.y) + (b.z + b.w);
-  }
+  return v;
 }
 
-template <bool ADD, int NC, int R>
+template <bool ADD, int TEAM, int NC>
 __global__ void __launch_bounds__(ROWS_THREADS)
 rmsnorm_fwd_rows_kernel(const bf16* __restrict__ x, const bf16* __restrict__ delta, const bf16* __restrict__ w,
                         bf16* __restrict__ x_new, bf16* __restrict__ y, float* __restrict__ rstd_out, int T, int H, float eps) {
-  __shared__ __align__(16) float red[2 * R * 8];
+  __shared__ float red[2 * 8];
   pdl_enter();
-  const int nchunk = H / 8;
-  bf16x8 wv[NC];
+  const int nchunk = H / 8, tid = threadIdx.x % TEAM;
+  const long long row = (long long)blockIdx.x * (ROWS_THREADS / TEAM) + threadIdx.x / TEAM;
+  if (row >= T) return;                              // (a whole team: its barrier is its own)
+  bf16x8 px[NC], pd[NC], wv[NC];
 #pragma unroll
   for (int i = 0; i < NC; ++i) {
-    const int c = threadIdx.x + i * ROWS_THREADS;
-    if (c < nchunk) wv[i] = *reinterpret_cast<const bf16x8*>(w + c * 8);
-  }
-  int it = 0;
-  for (long long row0 = (long long)blockIdx.x * R; row0 < T; row0 += (long long)gridDim.x * R, ++it) {
-    bf16x8 px[R][NC], pd[R][NC];
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-#pragma unroll
-      for (int i = 0; i < NC; ++i) {
-        const int c = threadIdx.x + i * ROWS_THREADS;
-        if (row0 + r < T && c < nchunk) {
-          px[r][i] = *reinterpret_cast<const bf16x8*>(x + (row0 + r) * H + c * 8);
-          if (ADD) pd[r][i] = *reinterpret_cast<const bf16x8*>(delta + (row0 + r) * H + c * 8);
-        }
-      }
-    float ss[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      ss[r] = 0.f;
-#pragma unroll
-      for (int i = 0; i < NC; ++i) {
-        const int c = threadIdx.x + i * ROWS_THREADS;
-        if (row0 + r < T && c < nchunk) {
-          float v[8];
-          unpack8(px[r][i], v);
-          if (ADD) {
-            float d[8];
-            unpack8(pd[r][i], d);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] += d[j];
-            px[r][i] = pack8(v);                       // the rounded residual stream is what the backward sees
-            *reinterpret_cast<bf16x8*>(x_new + (row0 + r) * H + c * 8) = px[r][i];
-            unpack8(px[r][i], v);
-          }
-#pragma unroll
-          for (int j = 0; j < 8; ++j) ss[r] += v[j] * v[j];
-        }
-      }
+    const int c = tid + i * TEAM;
+    if (c < nchunk) {
+      px[i] = *reinterpret_cast<const bf16x8*>(x + row * H + c * 8);
+      if (ADD) pd[i] = *reinterpret_cast<const bf16x8*>(delta + row * H + c * 8);
+      wv[i] = *reinterpret_cast<const bf16x8*>(w + c * 8);
     }
-    block_sum_rows<R>(ss, red, it);
+  }
+  float ss = 0.f;
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      if (row0 + r >= T) continue;
-      const float rstd = rsqrtf(ss[r] / (float)H + eps);
-      if (threadIdx.x == 0) rstd_out[row0 + r] = rstd;
+  for (int i = 0; i < NC; ++i) {
+    const int c = tid + i * TEAM;
+    if (c < nchunk) {
+      float v[8];
+      unpack8(px[i], v);
+      if (ADD) {
+        float d[8];
+        unpack8(pd[i], d);
 #pragma unroll
-      for (int i = 0; i < NC; ++i) {
-        const int c = threadIdx.x + i * ROWS_THREADS;
-        if (c < nchunk) {
-          float v[8], ww[8], o[8];
-          unpack8(px[r][i], v);
-          unpack8(wv[i], ww);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] = v[j] * rstd * ww[j];
-          *reinterpret_cast<bf16x8*>(y + (row0 + r) * H + c * 8) = pack8(o);
-        }
+        for (int j = 0; j < 8; ++j) v[j] += d[j];
+        px[i] = pack8(v);                              // the rounded residual stream is what the backward sees
+        *reinterpret_cast<bf16x8*>(x_new + row * H + c * 8) = px[i];
+        unpack8(px[i], v);
       }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) ss += v[j] * v[j];
+    }
+  }
+  const float rstd = rsqrtf(team_sum<TEAM>(ss, red, 0) / (float)H + eps);
+  if (tid == 0) rstd_out[row] = rstd;
+#pragma unroll
+  for (int i = 0; i < NC; ++i) {
+    const int c = tid + i * TEAM;
+    if (c < nchunk) {
+      float v[8], ww[8], o[8];
+      unpack8(px[i], v);
+      unpack8(wv[i], ww);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[j] = v[j] * rstd * ww[j];
+      *reinterpret_cast<bf16x8*>(y + row * H + c * 8) = pack8(o);
     }
   }
 }
 
-template <int NC, int R>
-__global__ void __launch_bounds__(ROWS_THREADS)
+template <int TEAM, int NC>
+__global__ void __launch_bounds__(ROWS_THREADS, NC <= 2 ? 3 : 2)
 rmsnorm_bwd_rows_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, const bf16* __restrict__ w,
                         const float* __restrict__ rstd_in, const bf16* __restrict__ dres, bf16* __restrict__ dx,
                         float* __restrict__ dw_acc, int T, int H) {
-  __shared__ __align__(16) float red[2 * R * 8];
+  constexpr int TEAMS = ROWS_THREADS / TEAM;
+  __shared__ float red[2 * 8];
+  __shared__ __align__(16) float comb[TEAMS > 1 ? TEAMS * TEAM * NC * 8 : 4];
   pdl_enter();
-  const int nchunk = H / 8;
+  const int nchunk = H / 8, tid = threadIdx.x % TEAM, team = threadIdx.x / TEAM;
   bf16x8 wv[NC];
   float dwacc[NC][8];
 #pragma unroll
   for (int i = 0; i < NC; ++i) {
-    const int c = threadIdx.x + i * ROWS_THREADS;
+    const int c = tid + i * TEAM;
     if (c < nchunk) wv[i] = *reinterpret_cast<const bf16x8*>(w + c * 8);
 #pragma unroll
     for (int j = 0; j < 8; ++j) dwacc[i][j] = 0.f;
   }
   int it = 0;
-  for (long long row0 = (long long)blockIdx.x * R; row0 < T; row0 += (long long)gridDim.x * R, ++it) {
-    bf16x8 px[R][NC], pdy[R][NC], pr[R][NC];
-    float rstd[R];
+  for (long long row = (long long)blockIdx.x * TEAMS + team; row < T; row += (long long)gridDim.x * TEAMS, ++it) {
+    bf16x8 px[NC], pdy[NC], pr[NC];
+    const float rstd = rstd_in[row];
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      rstd[r] = row0 + r < T ? rstd_in[row0 + r] : 0.f;
+    for (int i = 0; i < NC; ++i) {
+      const int c = tid + i * TEAM;
+      if (c < nchunk) {
+        px[i] = *reinterpret_cast<const bf16x8*>(x + row * H + c * 8);
+        pdy[i] = *reinterpret_cast<const bf16x8*>(dy + row * H + c * 8);
+        if (dres != nullptr) pr[i] = *reinterpret_cast<const bf16x8*>(dres + row * H + c * 8);
+      }
+    }
+    float dot = 0.f;
 #pragma unroll
-      for (int i = 0; i < NC; ++i) {
-        const int c = threadIdx.x + i * ROWS_THREADS;
-        if (row0 + r < T && c < nchunk) {
-          px[r][i] = *reinterpret_cast<const bf16x8*>(x + (row0 + r) * H + c * 8);
-          pdy[r][i] = *reinterpret_cast<const bf16x8*>(dy + (row0 + r) * H + c * 8);
-          if (dres != nullptr) pr[r][i] = *reinterpret_cast<const bf16x8*>(dres + (row0 + r) * H + c * 8);
+    for (int i = 0; i < NC; ++i) {
+      const int c = tid + i * TEAM;
+      if (c < nchunk) {
+        float xv[8], dv[8], ww[8];
+        unpack8(px[i], xv);
+        unpack8(pdy[i], dv);
+        unpack8(wv[i], ww);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float xh = xv[j] * rstd;
+          dot += xh * dv[j] * ww[j];
+          dwacc[i][j] += dv[j] * xh;
         }
       }
     }
-    float dot[R];
+    const float cmean = team_sum<TEAM>(dot, red, it) / (float)H;
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      dot[r] = 0.f;
+    for (int i = 0; i < NC; ++i) {
+      const int c = tid + i * TEAM;
+      if (c < nchunk) {
+        float xv[8], dv[8], ww[8], o[8];
+        unpack8(px[i], xv);
+        unpack8(pdy[i], dv);
+        unpack8(wv[i], ww);
 #pragma unroll
-      for (int i = 0; i < NC; ++i) {
-        const int c = threadIdx.x + i * ROWS_THREADS;
-        if (row0 + r < T && c < nchunk) {
-          float xv[8], dv[8], ww[8];
-          unpack8(px[r][i], xv);
-          unpack8(pdy[r][i], dv);
-          unpack8(wv[i], ww);
+        for (int j = 0; j < 8; ++j) o[j] = (dv[j] * ww[j] - xv[j] * rstd * cmean) * rstd;
+        if (dres != nullptr) {
+          float rr[8];
+          unpack8(pr[i], rr);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float xh = xv[j] * rstd[r];
-            dot[r] += xh * dv[j] * ww[j];
-            dwacc[i][j] += dv[j] * xh;
-          }
+          for (int j = 0; j < 8; ++j) o[j] += rr[j];
         }
-      }
-    }
-    block_sum_rows<R>(dot, red, it);
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      if (row0 + r >= T) continue;
-      const float cmean = dot[r] / (float)H;
-#pragma unroll
-      for (int i = 0; i < NC; ++i) {
-        const int c = threadIdx.x + i * ROWS_THREADS;
-        if (c < nchunk) {
-          float xv[8], dv[8], ww[8], o[8];
-          unpack8(px[r][i], xv);
-          unpack8(pdy[r][i], dv);
-          unpack8(wv[i], ww);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] = (dv[j] * ww[j] - xv[j] * rstd[r] * cmean) * rstd[r];
-          if (dres != nullptr) {
-            float rr[8];
-            unpack8(pr[r][i], rr);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) o[j] += rr[j];
-          }
-          *reinterpret_cast<bf16x8*>(dx + (row0 + r) * H + c * 8) = pack8(o);
-        }
+        *reinterpret_cast<bf16x8*>(dx + row * H + c * 8) = pack8(o);
       }
     }
   }
+  auto red_add = [&](float* dst, float4 v) {
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+  };
+  if constexpr (TEAMS == 1) {
 #pragma unroll
-  for (int i = 0; i < NC; ++i) {
-    const int c = threadIdx.x + i * ROWS_THREADS;
-    if (c < nchunk) {
-      float* dst = dw_acc + c * 8;
-      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(dwacc[i][0]), "f"(dwacc[i][1]),
-                   "f"(dwacc[i][2]), "f"(dwacc[i][3]) : "memory");
-      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + 4), "f"(dwacc[i][4]), "f"(dwacc[i][5]),
-                   "f"(dwacc[i][6]), "f"(dwacc[i][7]) : "memory");
+    for (int i = 0; i < NC; ++i) {
+      const int c = tid + i * TEAM;
+      if (c < nchunk) {
+        red_add(dw_acc + c * 8, make_float4(dwacc[i][0], dwacc[i][1], dwacc[i][2], dwacc[i][3]));
+        red_add(dw_acc + c * 8 + 4, make_float4(dwacc[i][4], dwacc[i][5], dwacc[i][6], dwacc[i][7]));
+      }
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < NC; ++i) {
+      float4* q = reinterpret_cast<float4*>(comb + (team * TEAM * NC + tid + i * TEAM) * 8);
+      q[0] = make_float4(dwacc[i][0], dwacc[i][1], dwacc[i][2], dwacc[i][3]);
+      q[1] = make_float4(dwacc[i][4], dwacc[i][5], dwacc[i][6], dwacc[i][7]);
+    }
+    __syncthreads();
+    for (int c4 = threadIdx.x; c4 < H / 4; c4 += ROWS_THREADS) {
+      float4 v = *reinterpret_cast<const float4*>(comb + c4 * 4);
+#pragma unroll
+      for (int t = 1; t < TEAMS; ++t) {
+        const float4 u = *reinterpret_cast<const float4*>(comb + t * TEAM * NC * 8 + c4 * 4);
+        v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+      }
+      red_add(dw_acc + c4 * 4, v);
     }
   }
 }
 
-// grid of a row-block kernel: every CTA gets work, at most `per_sm` CTAs per SM
-static inline int rows_grid(int T, int R, int num_sms, int per_sm) {
-  const int want = (T + R - 1) / R, cap = num_sms * per_sm;
-  return want < cap ? want : cap;
+// The smallest team whose threads hold a row with at most four chunks each: calls f(team, chunks per thread) as constants.
+// The backward of a wide row takes two chunks per thread: half the registers make room for a third CTA per SM (4096 x 2048:
+// 26.6 us with four chunks, 22.6 with two; 32768 x 2048: 119 and 104), while narrow rows are better off without barriers
+// (8192 x 576: 16.4 us with 32 threads per row, 18.5 with 64).
+template <typename F>
+static void with_team(int H, bool backward, F f) {
+  const int nchunk = H / 8;
+#define PT_TEAM(TEAM, NC) f(std::integral_constant<int, TEAM>{}, std::integral_constant<int, NC>{})
+  if (nchunk <= 32) PT_TEAM(32, 1);
+  else if (nchunk <= 64) PT_TEAM(32, 2);
+  else if (nchunk <= 96) PT_TEAM(32, 3);
+  else if (nchunk <= 128) PT_TEAM(32, 4);
+  else if (backward && nchunk <= 256) PT_TEAM(128, 2);
+  else if (backward && nchunk <= 512) PT_TEAM(256, 2);
+  else if (nchunk <= 192) PT_TEAM(64, 3);
+  else if (nchunk <= 256) PT_TEAM(64, 4);
+  else if (nchunk <= 384) PT_TEAM(128, 3);
+  else if (nchunk <= 512) PT_TEAM(128, 4);
+  else PT_TEAM(256, 4);
+#undef PT_TEAM
 }
 
 extern "C" int pt_rmsnorm_fwd(const void* x, const void* delta, const void* w, void* x_new, void* y, float* rstd,
                               int T, int H, float eps, cudaStream_t st) {
   if (H % 8 || H > 8 * ROWS_THREADS * 4) return -10;
   if (T == 0) return 0;
-  static int num_sms = 0;
-  if (num_sms == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
-  }
-  const int nc = (H / 8 + ROWS_THREADS - 1) / ROWS_THREADS;
-#define PT_NORM_FWD(ADD, NC, R)                                                                                      \
-  launch_pdl(rmsnorm_fwd_rows_kernel<ADD, NC, R>, dim3(rows_grid(T, R, num_sms, 4)), dim3(ROWS_THREADS), 0, st,      \
-             (const bf16*)x, (const bf16*)delta, (const bf16*)w, (bf16*)x_new, (bf16*)y, rstd, T, H, eps)
-  if (delta != nullptr) {
-    if (nc <= 1) PT_NORM_FWD(true, 1, 4); else if (nc <= 2) PT_NORM_FWD(true, 2, 2); else PT_NORM_FWD(true, 4, 1);
-  } else {
-    if (nc <= 1) PT_NORM_FWD(false, 1, 4); else if (nc <= 2) PT_NORM_FWD(false, 2, 2); else PT_NORM_FWD(false, 4, 1);
-  }
-#undef PT_NORM_FWD
+  with_team(H, false, [&](auto team, auto nc) {
+    constexpr int TEAM = decltype(team)::value, NC = decltype(nc)::value, ROWS = ROWS_THREADS / TEAM;
+    const dim3 grid((unsigned)((T + ROWS - 1) / ROWS));
+    if (delta != nullptr)
+      launch_pdl(rmsnorm_fwd_rows_kernel<true, TEAM, NC>, grid, dim3(ROWS_THREADS), 0, st, (const bf16*)x, (const bf16*)delta,
+                 (const bf16*)w, (bf16*)x_new, (bf16*)y, rstd, T, H, eps);
+    else
+      launch_pdl(rmsnorm_fwd_rows_kernel<false, TEAM, NC>, grid, dim3(ROWS_THREADS), 0, st, (const bf16*)x, (const bf16*)delta,
+                 (const bf16*)w, (bf16*)x_new, (bf16*)y, rstd, T, H, eps);
+  });
   return check_launch();
 }
 
@@ -809,12 +814,12 @@ extern "C" int pt_rmsnorm_bwd_acc(const void* dy, const void* x, const void* w, 
                                   void* dx, float* dw_acc, int T, int H, int num_sms, cudaStream_t st) {
   if (H % 8 || H > 8 * ROWS_THREADS * 4 || (reinterpret_cast<uintptr_t>(dw_acc) & 15)) return 1;
   if (T == 0) return 0;
-  const int nc = (H / 8 + ROWS_THREADS - 1) / ROWS_THREADS;
-#define PT_NORM_BWD_ROWS(NC, R)                                                                                      \
-  launch_pdl(rmsnorm_bwd_rows_kernel<NC, R>, dim3(rows_grid(T, R, num_sms, 2)), dim3(ROWS_THREADS), 0, st,           \
-             (const bf16*)dy, (const bf16*)x, (const bf16*)w, rstd, (const bf16*)dres, (bf16*)dx, dw_acc, T, H)
-  if (nc <= 1) PT_NORM_BWD_ROWS(1, 4); else if (nc <= 2) PT_NORM_BWD_ROWS(2, 2); else PT_NORM_BWD_ROWS(4, 1);
-#undef PT_NORM_BWD_ROWS
+  with_team(H, true, [&](auto team, auto nc) {
+    constexpr int TEAM = decltype(team)::value, NC = decltype(nc)::value, ROWS = ROWS_THREADS / TEAM;
+    const int want = (T + ROWS - 1) / ROWS, cap = (NC <= 2 ? 3 : 2) * num_sms;
+    launch_pdl(rmsnorm_bwd_rows_kernel<TEAM, NC>, dim3((unsigned)(want < cap ? want : cap)), dim3(ROWS_THREADS), 0, st,
+               (const bf16*)dy, (const bf16*)x, (const bf16*)w, rstd, (const bf16*)dres, (bf16*)dx, dw_acc, T, H);
+  });
   return check_launch();
 }
 

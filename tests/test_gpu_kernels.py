@@ -251,6 +251,26 @@ def test_rmsnorm_fwd_bwd(C, T, H):
     torch.testing.assert_close(dx0.float(), ref.rmsnorm_bwd(dy, x, w, rstd_ref)[0].float(), rtol=2e-2, atol=3e-2)
 
 
+@pytest.mark.parametrize("T", [1, 9, 2500])
+@pytest.mark.parametrize("H", [8, 256, 264, 576, 960, 1024, 1032, 1544, 2056, 3080, 4104, 8192])
+def test_rmsnorm_at_the_edges_of_its_team_sizes(C, T, H):
+    """Row widths on both sides of every change of threads per row and chunks per thread, with more rows than one pass covers."""
+    x, d, dy = bf(T, H, seed=1), bf(T, H, seed=2), bf(T, H, seed=3)
+    w = (1 + 0.1 * bf(H, seed=4).float()).to(torch.bfloat16)
+    xn, y, rstd = C.add_rmsnorm_fwd(x, d, w, 1e-5)
+    xn_ref, y_ref, rstd_ref = ref.add_rmsnorm_fwd(x, d, w, 1e-5)
+    assert torch.equal(xn, xn_ref)
+    torch.testing.assert_close(rstd, rstd_ref, rtol=1e-5, atol=0)           # fp32 sums of at most 8192 squares in another order
+    torch.testing.assert_close(y, y_ref, rtol=2 ** -7, atol=0)              # bf16 neighbours
+    torch.testing.assert_close(C.rmsnorm_fwd(xn, w, 1e-5)[0], y, rtol=2 ** -7, atol=0)
+    acc = torch.full((H,), 0.5, device="cuda")
+    dx, _ = C.rmsnorm_bwd(dy, xn, w, rstd, d, acc)
+    dx_ref, dw_ref = ref.rmsnorm_bwd(dy, xn, w, rstd, d)
+    # fp32 terms of size up to |dy| + |dres|, rounded once to bf16
+    torch.testing.assert_close(dx.float(), dx_ref.float(), rtol=2 ** -7, atol=2e-3)
+    torch.testing.assert_close(acc - 0.5, dw_ref, rtol=1e-4, atol=1e-5 * T ** 0.5 * 16)
+
+
 @pytest.mark.parametrize("T,H", [(513, 2048), (64, 768), (33, 256), (40, 4096), (9, 320)])
 def test_rmsnorm_bwd_accumulates_into_fp32_destination(C, T, H):
     """dw added in place to an fp32 vector (a gradient-bucket slice), also when that slice is not 16-byte aligned."""
