@@ -207,6 +207,9 @@ class _SingleProcessGrid:
         return "TP(1)-CP(1)-PP(1)-DP(1)-Rank(0)"
 
 
+_SINGLE_PROCESS = _SingleProcessGrid()      # (the layers ask for the grid several times per pass)
+
+
 class LayoutGrid(_SingleProcessGrid):
     """Coordinates of ONE rank of a tp x pp grid without any communicator: enough to construct that rank's modules on
     the meta device and read off its parameter names and shard shapes (offline tools such as checkpoint resharding)."""
@@ -235,10 +238,7 @@ def layout_grid(tp_rank: int, tp_size: int, pp_rank: int, pp_size: int):
 
 def get() -> "ProcessGroupManager":
     """The active grid; a size-1 stand-in when ``setup_process_group_manager`` was never called."""
-    global process_group_manager
-    if process_group_manager is None:
-        return _SingleProcessGrid()  # type: ignore[return-value]
-    return process_group_manager
+    return process_group_manager if process_group_manager is not None else _SINGLE_PROCESS  # type: ignore[return-value]
 
 
 def reset() -> None:
