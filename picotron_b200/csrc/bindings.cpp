@@ -23,6 +23,7 @@ int pt_ce_combine(const void* part, float* rowmax, float* sumexp, long long T, i
 void* pt_status_word();
 void pt_attention_set_profile(unsigned long long* counters);
 void pt_gemm_set_group_m(int g);
+void pt_gemm_set_tile_n(int n);
 int pt_gemm_get_group_m();
 void pt_gemm_set_tma_epilogue(int on);
 int pt_gemm_get_tma_epilogue();
@@ -791,6 +792,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("get_gemm_tma_epilogue", []() { return pt_gemm_get_tma_epilogue() != 0; });
   m.def("set_gemm_group_m", [](int64_t g) { pt_gemm_set_group_m((int)g); },
         "CTA-pair GEMM tile numbering: rows of 256-row tiles per group (L2 locality of concurrently running tiles; default 8).");
+  m.def("set_gemm_tile_n", [](int64_t n) { pt_gemm_set_tile_n((int)n); },
+        "columns of the GEMM output tiles: 128, 256, or 0 for the choice by shape (bf16 outputs)");
   m.def("get_gemm_group_m", []() { return (int64_t)pt_gemm_get_group_m(); });
   m.def("attention_set_profile", [](const c10::optional<Tensor>& counters) {
           if (!counters.has_value()) { pt_attention_set_profile(nullptr); return; }

@@ -1,7 +1,7 @@
 // bf16 GEMM for sm_100a on CTA pairs (tcgen05 cta_group::2): D[M,N] = op(A) * op(B), fp32 accumulate in TMEM.
 //
 // Same contract and operand layouts as gemm_tcgen05.cu, but two CTAs (a cluster of 2 on neighbouring SMs)
-// cooperate on one 256x256 output tile: each CTA loads its own 128 rows of A and its own 128 columns of
+// cooperate on one 256x256 (or, where that gives one wave at most, 256x128) output tile: each CTA loads its own 128 rows of A and its own 128 columns of
 // B -- with plain, non-multicast TMA loads -- and one thread of the leader CTA issues a 256-row MMA that
 // reads both CTAs' shared memory and writes both CTAs' tensor memory. Per output element this moves a
 // third less operand data from L2 into shared memory than the single-CTA 128x256 tile (each B half is
@@ -24,7 +24,7 @@
 // 16-byte stores, read-modify-write for the accumulate mode) is kept as a template variant.
 //
 // Fused epilogues (forward GEMMs X W^T with bf16 output only):
-//   SwiGLU  W is the packed [gate; up] weight [2I, K]. The leader CTA loads 128 gate rows, its partner the 128 up rows of
+//   SwiGLU  W is the packed [gate; up] weight [2I, K]. The leader CTA loads 128 (64) gate rows, its partner the up rows of
 //           the same indices, so accumulator columns 0..127 / 128..255 of a tile are gate / up pre-activations of the
 //           same 128 hidden units. The epilogue stores both (the backward needs them) and silu(gate) * up to a second
 //           output, which replaces the separate activation kernel and its pass over the [T, 2I] tensor.
@@ -43,22 +43,18 @@
 #include "common.cuh"
 #include "tensormap.cuh"
 
+#include <type_traits>
+
 extern "C" void pt_count_launches(int n);
 
 namespace pt {
 namespace gemm_pair {
 
 constexpr int BM = 128;        // rows of A per CTA (256 per pair)
-constexpr int BN_HALF = 128;   // columns of B per CTA (256 per pair)
-constexpr int BN = 256;
 constexpr int BK = 64;
 constexpr int UMMA_K = 16;
 constexpr int STAGES = 6;
 constexpr int A_BYTES = BM * BK * 2;        // 16 KiB
-constexpr int B_BYTES = BN_HALF * BK * 2;   // 16 KiB
-constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-constexpr int STAGING_BYTES = 4 * 2 * 4096;   // 4 epilogue warps x 2 buffers of [32 rows][128 B]
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + STAGING_BYTES + 1024;
 constexpr int NUM_THREADS = 192;
 constexpr int TMEM_COLS = 512;
 constexpr unsigned KERNEL_ID = 2;
@@ -68,8 +64,9 @@ enum Epilogue { EPI_NONE = 0, EPI_SWIGLU = 1, EPI_ROPE64 = 2, EPI_ROPE128 = 3, E
 // operand stages and staging buffers per epilogue warp of each variant (see the smem budget in launch())
 __host__ __device__ constexpr int stages_of(int epi) { return epi == EPI_SWIGLU_BWD ? 5 : 6; }
 __host__ __device__ constexpr int staging_bufs_of(int epi) { return epi == EPI_SWIGLU_BWD ? 4 : 2; }
-__host__ __device__ constexpr int smem_bytes_of(int epi) {
-  return stages_of(epi) * STAGE_BYTES + 4 * staging_bufs_of(epi) * 4096 + 1024;
+// a stage holds BM x BK of A and bn / 2 x BK of B; four epilogue warps stage [32 rows][128 B] per buffer
+__host__ __device__ constexpr int smem_bytes_of(int epi, int bn) {
+  return stages_of(epi) * (A_BYTES + bn / 2 * BK * 2) + 4 * staging_bufs_of(epi) * 4096 + 1024;
 }
 
 struct EpiArgs {
@@ -126,14 +123,17 @@ __device__ __forceinline__ float ex2_approx(float x) {
   return y;
 }
 
-// N is the number of output columns, except for EPI_SWIGLU where it is I (tiles pair 128 gate with 128 up columns).
-template <bool A_MN, bool B_MN, int OUT_MODE, bool EPI_TMA, int EPI>
+// N is the number of output columns, except for EPI_SWIGLU where it is I (tiles pair BN / 2 gate with BN / 2 up columns).
+template <bool A_MN, bool B_MN, int OUT_MODE, bool EPI_TMA, int EPI, int BN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                  const __grid_constant__ CUtensorMap tma_d, const __grid_constant__ CUtensorMap tma_h,
                  void* __restrict__ Dptr, int M, int N, int K, long long ldd, KernelStatus* status, EpiArgs ea) {
   static_assert(EPI == EPI_NONE || (EPI_TMA && !A_MN && OUT_MODE == OUT_BF16 && B_MN == (EPI == EPI_SWIGLU_BWD)),
                 "fused epilogues: bf16 output; forward layout, except the SwiGLU backward which rides on the dgrad layout");
+  static_assert(BN == 256 || (BN == 128 && EPI_TMA && OUT_MODE == OUT_BF16 && EPI != EPI_CE), "narrow tiles: bf16 outputs");
+  constexpr int BN_HALF = BN / 2;                 // columns of B per CTA
+  constexpr int B_BYTES = BN_HALF * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
   constexpr int STAGES = stages_of(EPI);          // shadows the namespace constant: the variants differ in their smem split
   pdl_launch_dependents();
   extern __shared__ uint8_t smem_raw[];
@@ -425,7 +425,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         };
         if constexpr (EPI == EPI_SWIGLU) {
 #pragma unroll 1
-          for (int c = 0; c < 2; ++c) {
+          for (int c = 0; c < BN_HALF / 64; ++c) {
             uint32_t g[64], u[64];
             tmem_ld_32x32b_x32_at(t_row + c * 64, g, 0);
             tmem_ld_32x32b_x32_at(t_row + c * 64 + 32, g, 32);
@@ -712,18 +712,39 @@ static int split_k_blocks(int tiles, int num_kb, int clusters) {
   return best;
 }
 
-template <bool A_MN, bool B_MN, int OUT_MODE, bool EPI_TMA, int EPI = EPI_NONE>
+static int g_tile_n = 0;    // 0: by the rule below, 128 / 256: as given (tests, measurements)
+
+// Columns of an output tile (bf16 outputs). A 256 x 256 tile moves the fewest operand bytes per product, but a few hundred
+// tokens or a few hundred columns give only a handful of them for 74 CTA pairs, and then their epilogue, 256 columns one after
+// the other, is a good part of the time. Tiles of 128 columns halve it, at the same time per k-block, wherever they still fit
+// in one wave. Measured with 256 / 128 columns (us): RoPE 256 x 960 x 576: 14.8 / 11.2, SwiGLU 256 x 3072 x 576: 11.2 / 9.7,
+// SwiGLU backward 256 x 3072 x 576: 15.9 / 12.3, residual add 256 x 576 x 1536: 15.6 / 13.8; beyond one wave they lose (RoPE
+// 512 x 6144 x 2048: 24.1 / 27.9, SwiGLU 1024 x 3072 x 576: 11.8 / 13.3), and beyond K = 8192 the epilogue no longer shows.
+static int tile_columns(int M, int n_cols, int K) {
+  if (g_tile_n) return g_tile_n;
+  static int pairs = 0;
+  if (pairs == 0) {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    pairs = sms / 2 > 0 ? sms / 2 : 1;
+  }
+  const long long rows = (M + 2 * BM - 1) / (2 * BM);
+  return rows * ((n_cols + 127) / 128) <= pairs && K <= 8192 ? 128 : 256;
+}
+
+template <bool A_MN, bool B_MN, int OUT_MODE, bool EPI_TMA, int EPI = EPI_NONE, int BN = 256>
 static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& md, void* D, int M, int N, int K,
                   long long ldd, KernelStatus* status, cudaStream_t stream, const CUtensorMap* mh = nullptr,
                   EpiArgs ea = EpiArgs{}) {
-  auto kern = gemm_pair_kernel<A_MN, B_MN, OUT_MODE, EPI_TMA, EPI>;
+  auto kern = gemm_pair_kernel<A_MN, B_MN, OUT_MODE, EPI_TMA, EPI, BN>;
   static int max_clusters = 0;
   if (max_clusters == 0) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes_of(EPI)) != cudaSuccess) return -3;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes_of(EPI, BN)) != cudaSuccess) return -3;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2, 1, 1);
     cfg.blockDim = dim3(NUM_THREADS, 1, 1);
-    cfg.dynamicSmemBytes = smem_bytes_of(EPI);
+    cfg.dynamicSmemBytes = smem_bytes_of(EPI, BN);
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
     attr.val.clusterDim.x = 2;
@@ -738,14 +759,14 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMa
     }
     max_clusters = n;
   }
-  const int n_tiles = (EPI == EPI_SWIGLU) ? (N + BN_HALF - 1) / BN_HALF : (N + BN - 1) / BN;
+  const int n_tiles = (EPI == EPI_SWIGLU) ? (N + BN / 2 - 1) / (BN / 2) : (N + BN - 1) / BN;
   const int tiles = ((M + 2 * BM - 1) / (2 * BM)) * n_tiles;
   const int num_kb = (K + BK - 1) / BK;
   ea.group_m = g_group_m;
   ea.kb_per_split = (OUT_MODE == OUT_F32_ACC && EPI_TMA) ? split_k_blocks(tiles, num_kb, max_clusters) : num_kb;
   const int units = tiles * ((num_kb + ea.kb_per_split - 1) / ea.kb_per_split);
   const int clusters = units < max_clusters ? units : max_clusters;
-  const cudaError_t err = launch_pdl(kern, dim3(2 * clusters), dim3(NUM_THREADS), smem_bytes_of(EPI), stream, ma, mb, md,
+  const cudaError_t err = launch_pdl(kern, dim3(2 * clusters), dim3(NUM_THREADS), smem_bytes_of(EPI, BN), stream, ma, mb, md,
                                      mh ? *mh : md, D, M, N, K, ldd, status, ea);
   pt_count_launches(1);
   return (err == cudaSuccess && cudaGetLastError() == cudaSuccess) ? 0 : -4;
@@ -756,6 +777,7 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMa
 
 extern "C" void pt_gemm_set_group_m(int g) { pt::gemm_pair::g_group_m = g < 1 ? 1 : g; }
 extern "C" int pt_gemm_get_group_m() { return pt::gemm_pair::g_group_m; }
+extern "C" void pt_gemm_set_tile_n(int n) { pt::gemm_pair::g_tile_n = n == 128 || n == 256 ? n : 0; }
 
 // 1 (default): epilogue through shared memory and TMA store / reduce-add; 0: per-thread 16-byte stores.
 static int g_tma_epilogue = 1;
@@ -768,13 +790,14 @@ extern "C" int pt_gemm_bf16_pair(const void* A, const void* B, void* D, int M, i
                                  cudaStream_t stream) {
   using namespace pt;
   using namespace pt::gemm_pair;
+  const int bn = (out_mode == OUT_BF16 && g_tma_epilogue && !a_mn) ? tile_columns(M, N, K) : 256;
   CUtensorMap ma, mb;
   int rc;
   rc = a_mn ? make_bf16_map_2d(&ma, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, 64, BK)
             : make_bf16_map_2d(&ma, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda, BK, BM);
   if (rc) return rc * 10 - 1;    // -21: tensor map of A could not be encoded
   rc = b_mn ? make_bf16_map_2d(&mb, B, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, 64, BK)
-            : make_bf16_map_2d(&mb, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, BK, BN_HALF);
+            : make_bf16_map_2d(&mb, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, BK, bn / 2);
   if (rc) return rc * 10 - 2;    // -22: tensor map of B could not be encoded
   CUtensorMap md = ma;           // unused by the per-thread epilogue
   const bool epi_tma = g_tma_epilogue != 0;
@@ -786,6 +809,9 @@ extern "C" int pt_gemm_bf16_pair(const void* A, const void* B, void* D, int M, i
     if (rc) return rc * 10 - 3;  // -23: tensor map of D could not be encoded
   }
   KernelStatus* st = reinterpret_cast<KernelStatus*>(status);
+  if (bn == 128)
+    return b_mn ? launch<false, true, OUT_BF16, true, EPI_NONE, 128>(ma, mb, md, D, M, N, K, ldd, st, stream)
+                : launch<false, false, OUT_BF16, true, EPI_NONE, 128>(ma, mb, md, D, M, N, K, ldd, st, stream);
 #define PT_GEMM_CASE(AM, BMN, OM)                                                                             \
   if (a_mn == AM && b_mn == BMN && out_mode == OM)                                                            \
     return epi_tma ? launch<AM, BMN, OM, true>(ma, mb, md, D, M, N, K, ldd, st, stream)                       \
@@ -821,7 +847,7 @@ extern "C" int pt_gemm_bf16_fused(const void* A, const void* B, void* D, int M, 
   EpiArgs ea{};
   int n_out = N;
   if (epi == EPI_SWIGLU) {
-    if (inter <= 0 || inter % BN_HALF || H == nullptr || (ldh % 8) || (reinterpret_cast<uintptr_t>(H) & 15)) return 1;
+    if (inter <= 0 || inter % 128 || H == nullptr || (ldh % 8) || (reinterpret_cast<uintptr_t>(H) & 15)) return 1;
     ea.inter = inter;
     n_out = 2 * inter;
   } else if (epi == EPI_ADD) {
@@ -843,6 +869,7 @@ extern "C" int pt_gemm_bf16_fused(const void* A, const void* B, void* D, int M, 
     return -11;
   }
   if (M <= 0 || n_out <= 0 || K <= 0) return 0;
+  const int bn = tile_columns(M, epi == EPI_SWIGLU_BWD ? inter : n_out, K);
   CUtensorMap ma, mb, md, mh;
   int rc;
   if ((rc = make_bf16_map_2d(&ma, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda, BK, BM))) return rc * 10 - 1;
@@ -850,7 +877,7 @@ extern "C" int pt_gemm_bf16_fused(const void* A, const void* B, void* D, int M, 
     // B is stored [K, I] (MN-major operand): 64-column x BK-row boxes, as in the plain dgrad GEMM
     if ((rc = make_bf16_map_2d(&mb, B, (uint64_t)inter, (uint64_t)K, (uint64_t)ldb, 64, BK))) return rc * 10 - 2;
   } else {
-    if ((rc = make_bf16_map_2d(&mb, B, (uint64_t)K, (uint64_t)n_out, (uint64_t)ldb, BK, BN_HALF))) return rc * 10 - 2;
+    if ((rc = make_bf16_map_2d(&mb, B, (uint64_t)K, (uint64_t)n_out, (uint64_t)ldb, BK, bn / 2))) return rc * 10 - 2;
   }
   if ((rc = make_bf16_map_2d(&md, D, (uint64_t)n_out, (uint64_t)M, (uint64_t)ldd, 64, 32))) return rc * 10 - 3;
   mh = md;
@@ -859,11 +886,15 @@ extern "C" int pt_gemm_bf16_fused(const void* A, const void* B, void* D, int M, 
     return rc * 10 - 4;
   if (epi == EPI_SWIGLU && (rc = make_bf16_map_2d(&mh, H, (uint64_t)inter, (uint64_t)M, (uint64_t)ldh, 64, 32))) return rc * 10 - 4;
   KernelStatus* st = reinterpret_cast<KernelStatus*>(status);
-  if (epi == EPI_SWIGLU) return launch<false, false, OUT_BF16, true, EPI_SWIGLU>(ma, mb, md, D, M, inter, K, ldd, st, stream, &mh, ea);
-  if (epi == EPI_ADD) return launch<false, false, OUT_BF16, true, EPI_ADD>(ma, mb, md, D, M, N, K, ldd, st, stream, &mh, ea);
-  if (epi == EPI_SWIGLU_BWD) return launch<false, true, OUT_BF16, true, EPI_SWIGLU_BWD>(ma, mb, md, D, M, inter, K, ldd, st, stream, &mh, ea);
-  if (head_dim == 64) return launch<false, false, OUT_BF16, true, EPI_ROPE64>(ma, mb, md, D, M, N, K, ldd, st, stream, &mh, ea);
-  return launch<false, false, OUT_BF16, true, EPI_ROPE128>(ma, mb, md, D, M, N, K, ldd, st, stream, &mh, ea);
+  auto run = [&](auto width) -> int {
+    constexpr int W = decltype(width)::value;
+    if (epi == EPI_SWIGLU) return launch<false, false, OUT_BF16, true, EPI_SWIGLU, W>(ma, mb, md, D, M, inter, K, ldd, st, stream, &mh, ea);
+    if (epi == EPI_ADD) return launch<false, false, OUT_BF16, true, EPI_ADD, W>(ma, mb, md, D, M, N, K, ldd, st, stream, &mh, ea);
+    if (epi == EPI_SWIGLU_BWD) return launch<false, true, OUT_BF16, true, EPI_SWIGLU_BWD, W>(ma, mb, md, D, M, inter, K, ldd, st, stream, &mh, ea);
+    if (head_dim == 64) return launch<false, false, OUT_BF16, true, EPI_ROPE64, W>(ma, mb, md, D, M, N, K, ldd, st, stream, &mh, ea);
+    return launch<false, false, OUT_BF16, true, EPI_ROPE128, W>(ma, mb, md, D, M, N, K, ldd, st, stream, &mh, ea);
+  };
+  return bn == 128 ? run(std::integral_constant<int, 128>{}) : run(std::integral_constant<int, 256>{});
 }
 
 // LM-head GEMM with the cross-entropy row statistics in its epilogue: D[M, N] = A[M, K] B[N, K]^T (bf16, stored because the
@@ -886,11 +917,11 @@ extern "C" int pt_gemm_bf16_ce(const void* A, const void* B, void* D, int M, int
   ea.ce_tgt = tgt;
   ea.ce_targets = targets;
   ea.ce_vocab_start = vocab_start;
-  ea.ce_tiles = (N + BN - 1) / BN;
+  ea.ce_tiles = (N + 255) / 256;
   CUtensorMap ma, mb, md;
   int rc;
   if ((rc = make_bf16_map_2d(&ma, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda, BK, BM))) return rc * 10 - 1;
-  if ((rc = make_bf16_map_2d(&mb, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, BK, BN_HALF))) return rc * 10 - 2;
+  if ((rc = make_bf16_map_2d(&mb, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, BK, 128))) return rc * 10 - 2;
   if ((rc = make_bf16_map_2d(&md, D, (uint64_t)N, (uint64_t)M, (uint64_t)ldd, 64, 32))) return rc * 10 - 3;
   return launch<false, false, OUT_BF16, true, EPI_CE>(ma, mb, md, D, M, N, K, ldd, reinterpret_cast<KernelStatus*>(status), stream,
                                                       &md, ea);

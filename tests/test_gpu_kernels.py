@@ -411,3 +411,30 @@ def test_scale_by_a_device_coefficient(C, n, offset, c):
     want[offset:offset + n] *= c
     C.scale_(x[offset:offset + n], torch.tensor(c, device="cuda"))
     assert torch.equal(x, want)
+
+
+@pytest.mark.parametrize("T", [1, 128, 255, 257, 600])
+@pytest.mark.parametrize("H,I,hq,hkv,d", [(64, 128, 1, 1, 64), (192, 384, 3, 1, 64), (520, 640, 4, 2, 64), (256, 128, 2, 1, 128)])
+def test_gemm_narrow_tiles_equal_wide_tiles(T, H, I, hq, hkv, d):
+    """128-column against 256-column output tiles: the same products summed in the same order, whatever the tile and epilogue."""
+    from picotron_b200.ops import _ext
+    C = _ext.load()
+    C.set_gemm_pair(True)
+    C.set_gemm_tma_epilogue(True)
+    x, a, gu = bf(T, H, seed=1), bf(T, I, seed=2), bf(T, 2 * I, seed=3)
+    wq, wgu, wd = bf((hq + 2 * hkv) * d, H, seed=4), bf(2 * I, H, seed=5), bf(H, I, seed=6)
+    cos, sin = ref.rope_tables(max(T, 8), d, 10000.0, device="cuda")
+    results = []
+    try:
+        for n in (128, 256, 0):
+            C.set_gemm_tile_n(n)
+            results.append([C.gemm(x, wq, False, False), C.gemm(gu, wgu, False, True), C.gemm(a, wd, False, False),
+                            C.gemm_rope(x, wq, cos, sin, hq + hkv, d, T), *C.gemm_swiglu(x, wgu), C.gemm_add(a, wd, x),
+                            C.gemm_dgrad_swiglu_bwd(x, wd, gu)])
+    finally:
+        C.set_gemm_tile_n(0)
+    _status_ok(C)
+    torch.testing.assert_close(results[0][0].float(), x.float() @ wq.float().t(), rtol=2e-2, atol=2e-2 * math.sqrt(H))
+    for other in results[1:]:
+        for got, want in zip(results[0], other):
+            assert torch.equal(got, want)
