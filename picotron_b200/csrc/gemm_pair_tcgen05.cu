@@ -712,6 +712,34 @@ static int split_k_blocks(int tiles, int num_kb, int clusters) {
   return best;
 }
 
+// fp32 workspace of a split bf16 GEMM: cleared before, rounded into the output after
+__global__ void __launch_bounds__(256) clear_f32_kernel(float4* __restrict__ x, long long n4) {
+  pdl_enter();
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (i < n4) x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+__global__ void __launch_bounds__(256) round_f32_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ out, long long rows,
+                                                        int cols, long long ldd) {
+  pdl_enter();
+  const long long i = ((long long)blockIdx.x * 256 + threadIdx.x) * 8;
+  if (i >= rows * cols) return;                          // cols % 8 == 0: a thread's eight elements lie in one row
+  const float4 a = *reinterpret_cast<const float4*>(x + i), b = *reinterpret_cast<const float4*>(x + i + 4);
+  *reinterpret_cast<uint4*>(out + i / cols * ldd + i % cols) =
+      make_uint4(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w), pack_bf16(b.x, b.y), pack_bf16(b.z, b.w));
+}
+
+static int num_pairs() {
+  static int pairs = 0;
+  if (pairs == 0) {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    pairs = sms / 2 > 0 ? sms / 2 : 1;
+  }
+  return pairs;
+}
+
+static int g_split_dgrad = 1;
 static int g_tile_n = 0;    // 0: by the rule below, 128 / 256: as given (tests, measurements)
 
 // Columns of an output tile (bf16 outputs). A 256 x 256 tile moves the fewest operand bytes per product, but a few hundred
@@ -722,13 +750,7 @@ static int g_tile_n = 0;    // 0: by the rule below, 128 / 256: as given (tests,
 // 512 x 6144 x 2048: 24.1 / 27.9, SwiGLU 1024 x 3072 x 576: 11.8 / 13.3), and beyond K = 8192 the epilogue no longer shows.
 static int tile_columns(int M, int n_cols, int K) {
   if (g_tile_n) return g_tile_n;
-  static int pairs = 0;
-  if (pairs == 0) {
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    pairs = sms / 2 > 0 ? sms / 2 : 1;
-  }
+  const int pairs = num_pairs();
   const long long rows = (M + 2 * BM - 1) / (2 * BM);
   return rows * ((n_cols + 127) / 128) <= pairs && K <= 8192 ? 128 : 256;
 }
@@ -783,6 +805,47 @@ extern "C" void pt_gemm_set_tile_n(int n) { pt::gemm_pair::g_tile_n = n == 128 |
 static int g_tma_epilogue = 1;
 extern "C" void pt_gemm_set_tma_epilogue(int on) { g_tma_epilogue = on; }
 extern "C" int pt_gemm_get_tma_epilogue() { return g_tma_epilogue; }
+
+// Input-gradient GEMMs (bf16 output, long K) with few output tiles: K split over the idle CTA pairs, which add to an fp32
+// workspace that is rounded to bf16 once. pt_gemm_split_elems gives the workspace's size in floats, 0 where splitting does not
+// pay: the time in k-blocks (about 0.33 us each) of split_k_blocks' model with and without a split, plus 24 k-blocks for the two
+// small kernels around it and the workspace's 16 bytes per element and split at 5 TB/s. Measured without / with it (us):
+// 2048 x 576 x 49152 (LM head of the 135M shape): 246 / 105; 512 x 2048 x 16384: 90 / 42; 1024 x 2048 x 128256: 627 / 372;
+// 256 x 4096 x 4096: 34 / 28; and with no gain left at 2048 x 2048 x 128256: 745 / 749.
+// (The sums of a split tile come in any order, as those of dQ and of the weight gradients do; the forward GEMMs are not split.)
+extern "C" long long pt_gemm_split_elems(int M, int N, int K) {
+  using namespace pt::gemm_pair;
+  if (M <= 0 || N % 8 || K <= 0 || !g_split_dgrad) return 0;
+  const int pairs = num_pairs(), kb = (K + BK - 1) / BK;
+  const int tiles = ((M + 2 * BM - 1) / (2 * BM)) * ((N + 255) / 256);
+  if (tiles >= pairs) return 0;
+  const int kbs = split_k_blocks(tiles, kb, pairs);
+  const long long S = (kb + kbs - 1) / kbs;
+  if (S <= 1) return 0;
+  const long long waves = (tiles * S + pairs - 1) / pairs;
+  const long long cost = waves * (kbs + 12) + 24 + (long long)((double)M * N * 4 * (2 + S) / 5e6 / 0.33);
+  return cost + cost / 8 < kb + 12 ? (long long)M * N : 0;
+}
+
+extern "C" void pt_gemm_set_split_dgrad(int on) { pt::gemm_pair::g_split_dgrad = on; }
+
+extern "C" int pt_gemm_bf16_pair(const void* A, const void* B, void* D, int M, int N, int K, long long lda, long long ldb,
+                                 long long ldd, int a_mn, int b_mn, int out_mode, void* status, cudaStream_t stream);
+
+// D[M, N] = A[M, K] B[K, N] (bf16) through the fp32 workspace ws (M * N floats, 16-byte aligned); ldd % 8 == 0, D 16-byte aligned.
+extern "C" int pt_gemm_bf16_split(const void* A, const void* B, void* D, float* ws, int M, int N, int K, long long lda, long long ldb,
+                                  long long ldd, void* status, cudaStream_t stream) {
+  using namespace pt;
+  using namespace pt::gemm_pair;
+  const long long n = (long long)M * N;
+  launch_pdl(clear_f32_kernel, dim3((unsigned)((n / 4 + 255) / 256)), dim3(256), 0, stream, reinterpret_cast<float4*>(ws), n / 4);
+  const int rc = pt_gemm_bf16_pair(A, B, ws, M, N, K, lda, ldb, N, 0, 1, OUT_F32_ACC, status, stream);
+  if (rc) return rc;
+  launch_pdl(round_f32_kernel, dim3((unsigned)((n / 8 + 255) / 256)), dim3(256), 0, stream, (const float*)ws, (__nv_bfloat16*)D,
+             (long long)M, N, ldd);
+  pt_count_launches(2);
+  return cudaGetLastError() == cudaSuccess ? 0 : -4;
+}
 
 // Same contract as pt_gemm_bf16 (gemm_tcgen05.cu). Returns -5 when CTA pairs cannot be scheduled.
 extern "C" int pt_gemm_bf16_pair(const void* A, const void* B, void* D, int M, int N, int K, long long lda,

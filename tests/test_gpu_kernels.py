@@ -438,3 +438,31 @@ def test_gemm_narrow_tiles_equal_wide_tiles(T, H, I, hq, hkv, d):
     for other in results[1:]:
         for got, want in zip(results[0], other):
             assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("T,N,K", [(64, 576, 49152), (2048, 576, 49160), (500, 520, 16392), (512, 2048, 16384), (1, 8, 8200)])
+@pytest.mark.parametrize("into", [False, True])
+def test_gemm_input_gradient_with_k_split(C, T, N, K, into):
+    """Few output tiles behind a long K: parts of K are summed in an fp32 workspace and rounded once; also into rows of a wider
+    output, whose other columns stay as they were."""
+    from picotron_b200.ops import _ext
+    C = _ext.load()
+    C.set_gemm_pair(True)
+    C.set_gemm_tma_epilogue(True)
+    dy, w = bf(T, K, seed=1, scale=0.1), bf(K, N, seed=2, scale=0.1)
+    big = torch.full((T, N + 16), 3.0, device="cuda", dtype=torch.bfloat16)
+    out = big[:, 8:8 + N] if into else None
+    n0 = C.launch_count()
+    y = C.gemm(dy, w, False, True, out, False)
+    assert C.launch_count() - n0 == 3, "this shape should be split"
+    _status_ok(C)
+    want = dy.double() @ w.double()
+    # fp32 sums in another order (2^-24 sqrt(K) of sums of size sqrt(K)), then one rounding to bf16 (2^-9)
+    assert _rel(y, want) < 2.5e-3
+    if into:
+        assert torch.equal(big[:, :8], torch.full_like(big[:, :8], 3.0)) and torch.equal(big[:, 8 + N:], torch.full_like(big[:, :8], 3.0))
+    C.set_gemm_split_dgrad(False)
+    try:
+        assert _rel(C.gemm(dy, w, False, True), want) > 0.9 * _rel(y, want)       # no further off than the unsplit kernel
+    finally:
+        C.set_gemm_split_dgrad(True)
