@@ -262,8 +262,8 @@ def bench_attention_phases():
             C.attention_set_profile(None)
         c = [float(x) for x in counters.tolist()]
         print(f"B={B} S={S} hq={hq} hkv={hkv} d={d}")
-        print(f"  fwd: wait S {c[14] / c[11]:6.0f} | read S + row max {c[8] / c[11]:6.0f} | wait O / rescale {c[9] / c[11]:6.0f} | "
-              f"exp + store P {c[10] / c[11]:6.0f} | blocks per CTA {c[11] / c[13]:5.1f} | loop lifetime {c[12] / c[13]:9.0f}")
+        print(f"  fwd: wait S {c[14] / c[11]:6.0f} | read S + row max {c[8] / c[11]:6.0f} | wait O, rescale, store P {c[9] / c[11]:6.0f} | "
+              f"exponentials {c[10] / c[11]:6.0f} | blocks per CTA {c[11] / c[13]:5.1f} | loop lifetime {c[12] / c[13]:9.0f}")
         print(f"  bwd: wait S, dP {c[0] / c[4]:6.0f} | read + exp + store P, dS {c[1] / c[4]:6.0f} | wait dQ {c[2] / c[4]:6.0f} | "
               f"drain dQ {c[3] / c[4]:6.0f} | steps per CTA {c[4] / c[6]:5.1f} | loop lifetime {c[5] / c[6]:9.0f}")
     print("kernel status:", C.kernel_status())

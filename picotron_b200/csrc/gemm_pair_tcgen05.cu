@@ -1,7 +1,8 @@
 // bf16 GEMM for sm_100a on CTA pairs (tcgen05 cta_group::2): D[M,N] = op(A) * op(B), fp32 accumulate in TMEM.
 //
 // Same contract and operand layouts as gemm_tcgen05.cu, but two CTAs (a cluster of 2 on neighbouring SMs)
-// cooperate on one 256x256 (or, where that gives one wave at most, 256x128) output tile: each CTA loads its own 128 rows of A and its own 128 columns of
+// cooperate on one 256x256 output tile (256x128 where such tiles still give one wave): each CTA loads its own 128 rows of A
+// and its own half of the columns of
 // B -- with plain, non-multicast TMA loads -- and one thread of the leader CTA issues a 256-row MMA that
 // reads both CTAs' shared memory and writes both CTAs' tensor memory. Per output element this moves a
 // third less operand data from L2 into shared memory than the single-CTA 128x256 tile (each B half is
