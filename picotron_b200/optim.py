@@ -3,7 +3,7 @@
 The reference asks ``torch.optim.AdamW`` for ``fused=True`` but never gets it
 (``train.py:203-209``: a ``torch.device`` is compared with the string ``'cuda'``), so its optimizer step
 is the multi-kernel ``foreach`` path on bf16 parameters and bf16 moments. This optimizer performs the
-whole step for all parameters in one kernel launch: it reads the fp32 ``param.main_grad`` (falling back to
+whole step in one kernel launch per 256 parameters: it reads the fp32 ``param.main_grad`` (falling back to
 ``param.grad``), keeps fp32 moments and -- optionally -- an fp32 master copy of each parameter, and
 writes the rounded bf16 parameter back. Update rule and defaults are those of ``torch.optim.AdamW``
 (betas 0.9/0.999, eps 1e-8, decoupled weight decay 0.01).
