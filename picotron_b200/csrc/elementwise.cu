@@ -567,28 +567,61 @@ static inline int check_launch(int n = 1) {
 // ---------------------------------------------------------------------------------------------
 constexpr int ROWS_THREADS = 256;
 
-// sum of v over the team; `red` has 8 floats per parity of `it`
-template <int TEAM>
-__device__ __forceinline__ float team_sum(float v, float* red, int it) {
-  v = warp_sum(v);
-  if constexpr (TEAM > 32) {
-    constexpr int WARPS = TEAM / 32;
-    const int warp = threadIdx.x >> 5, team = threadIdx.x / TEAM;
-    float* buf = red + (it & 1) * 8;
-    if ((threadIdx.x & 31) == 0) buf[warp] = v;
-    asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "n"(TEAM) : "memory");
-    v = 0.f;
+// Sum over a row. Its order is the same for every team size: the 16-byte chunks c, c + 256, ... go to one running sum, 32
+// neighbouring running sums are added by a warp (butterfly), and the eight warp sums so obtained as
+// (((0 + 1) + (2 + 3)) + (4 + 5)) + (6 + 7). So a thread of a small team keeps a running sum per chunk (`acc_of`), each reduced by
+// itself: results do not depend on how a row is dealt to threads. `red` has 8 floats per team and parity of `it`.
+template <int TEAM> __host__ __device__ constexpr int acc_of(int i) { return i % (ROWS_THREADS / TEAM); }
+template <int TEAM, int NC> __host__ __device__ constexpr int accs() { return NC < ROWS_THREADS / TEAM ? NC : ROWS_THREADS / TEAM; }
+
+// Warp sums of four values at once, each as warp_sum gives it: the first two steps of the butterflies share their shuffles,
+// because a lane needs to go on with only one of the values. Value a ends up in the lanes [8 a, 8 a + 8).
+__device__ __forceinline__ float warp_sums4(float v0, float v1, float v2, float v3) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const bool b16 = threadIdx.x & 16, b8 = threadIdx.x & 8;
+  const float k0 = (b16 ? v2 : v0) + __shfl_xor_sync(FULL, b16 ? v0 : v2, 16);
+  const float k1 = (b16 ? v3 : v1) + __shfl_xor_sync(FULL, b16 ? v1 : v3, 16);
+  float k = (b8 ? k1 : k0) + __shfl_xor_sync(FULL, b8 ? k0 : k1, 8);
 #pragma unroll
-    for (int i = 0; i < WARPS; ++i) v += buf[team * WARPS + i];
+  for (int o = 4; o > 0; o >>= 1) k += __shfl_xor_sync(FULL, k, o);
+  return k;
+}
+
+template <int TEAM, int NA>
+__device__ __forceinline__ float row_sum(float (&v)[NA], float* red, int it) {
+  constexpr int WARPS = TEAM / 32;
+  float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  float k = 0.f;
+  if constexpr (NA > 2) {
+    k = warp_sums4(v[0], v[1], v[2], NA > 3 ? v[NA - 1] : 0.f);
+  } else {
+#pragma unroll
+    for (int a = 0; a < NA; ++a) v[a] = warp_sum(v[a]);
   }
-  return v;
+  if constexpr (WARPS == 1) {
+#pragma unroll
+    for (int a = 0; a < NA; ++a) s[a] = NA > 2 ? __shfl_sync(0xffffffffu, k, a * 8) : v[a];
+  } else {
+    const int warp = (threadIdx.x % TEAM) >> 5, team = threadIdx.x / TEAM, lane = threadIdx.x & 31;
+    float* buf = red + ((it & 1) * (ROWS_THREADS / TEAM) + team) * 8;
+    if constexpr (NA > 2) {
+      if (lane % 8 == 0 && lane / 8 < NA) buf[lane / 8 * WARPS + warp] = k;
+    } else if (lane == 0) {
+#pragma unroll
+      for (int a = 0; a < NA; ++a) buf[a * WARPS + warp] = v[a];
+    }
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "n"(TEAM) : "memory");
+#pragma unroll
+    for (int i = 0; i < NA * WARPS; ++i) s[i] = buf[i];
+  }
+  return (((s[0] + s[1]) + (s[2] + s[3])) + (s[4] + s[5])) + (s[6] + s[7]);
 }
 
 template <bool ADD, int TEAM, int NC>
 __global__ void __launch_bounds__(ROWS_THREADS)
 rmsnorm_fwd_rows_kernel(const bf16* __restrict__ x, const bf16* __restrict__ delta, const bf16* __restrict__ w,
                         bf16* __restrict__ x_new, bf16* __restrict__ y, float* __restrict__ rstd_out, int T, int H, float eps) {
-  __shared__ float red[2 * 8];
+  __shared__ __align__(16) float red[ROWS_THREADS / TEAM * 8];
   pdl_enter();
   const int nchunk = H / 8, tid = threadIdx.x % TEAM;
   const long long row = (long long)blockIdx.x * (ROWS_THREADS / TEAM) + threadIdx.x / TEAM;
@@ -603,7 +636,7 @@ rmsnorm_fwd_rows_kernel(const bf16* __restrict__ x, const bf16* __restrict__ del
       wv[i] = *reinterpret_cast<const bf16x8*>(w + c * 8);
     }
   }
-  float ss = 0.f;
+  float ss[accs<TEAM, NC>()] = {};
 #pragma unroll
   for (int i = 0; i < NC; ++i) {
     const int c = tid + i * TEAM;
@@ -620,10 +653,10 @@ rmsnorm_fwd_rows_kernel(const bf16* __restrict__ x, const bf16* __restrict__ del
         unpack8(px[i], v);
       }
 #pragma unroll
-      for (int j = 0; j < 8; ++j) ss += v[j] * v[j];
+      for (int j = 0; j < 8; ++j) ss[acc_of<TEAM>(i)] += v[j] * v[j];
     }
   }
-  const float rstd = rsqrtf(team_sum<TEAM>(ss, red, 0) / (float)H + eps);
+  const float rstd = rsqrtf(row_sum<TEAM>(ss, red, 0) / (float)H + eps);
   if (tid == 0) rstd_out[row] = rstd;
 #pragma unroll
   for (int i = 0; i < NC; ++i) {
@@ -645,7 +678,7 @@ rmsnorm_bwd_rows_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x,
                         const float* __restrict__ rstd_in, const bf16* __restrict__ dres, bf16* __restrict__ dx,
                         float* __restrict__ dw_acc, int T, int H) {
   constexpr int TEAMS = ROWS_THREADS / TEAM;
-  __shared__ float red[2 * 8];
+  __shared__ __align__(16) float red[2 * TEAMS * 8];
   __shared__ __align__(16) float comb[TEAMS > 1 ? TEAMS * TEAM * NC * 8 : 4];
   pdl_enter();
   const int nchunk = H / 8, tid = threadIdx.x % TEAM, team = threadIdx.x / TEAM;
@@ -671,7 +704,7 @@ rmsnorm_bwd_rows_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x,
         if (dres != nullptr) pr[i] = *reinterpret_cast<const bf16x8*>(dres + row * H + c * 8);
       }
     }
-    float dot = 0.f;
+    float dot[accs<TEAM, NC>()] = {};
 #pragma unroll
     for (int i = 0; i < NC; ++i) {
       const int c = tid + i * TEAM;
@@ -683,12 +716,12 @@ rmsnorm_bwd_rows_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x,
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const float xh = xv[j] * rstd;
-          dot += xh * dv[j] * ww[j];
+          dot[acc_of<TEAM>(i)] += xh * dv[j] * ww[j];
           dwacc[i][j] += dv[j] * xh;
         }
       }
     }
-    const float cmean = team_sum<TEAM>(dot, red, it) / (float)H;
+    const float cmean = row_sum<TEAM>(dot, red, it) / (float)H;
 #pragma unroll
     for (int i = 0; i < NC; ++i) {
       const int c = tid + i * TEAM;

@@ -271,6 +271,57 @@ def test_rmsnorm_at_the_edges_of_its_team_sizes(C, T, H):
     torch.testing.assert_close(acc - 0.5, dw_ref, rtol=1e-4, atol=1e-5 * T ** 0.5 * 16)
 
 
+def _row_sum_in_kernel_order(terms):
+    """Sum over the last dimension of an fp32 CPU tensor in the RMSNorm kernels' order: running sums over the 8-element chunks
+    c, c + 256, ..., a butterfly over 32 neighbouring ones, then the eight warp sums."""
+    T, H = terms.shape
+    groups = (H // 8 + 255) // 256
+    c = torch.zeros(T, groups * 256 * 8)
+    c[:, :H] = terms
+    c = c.view(T, groups, 256, 8)
+    run = torch.zeros(T, 256)
+    for g in range(groups):
+        for j in range(8):
+            run = run + c[:, g, :, j]
+    w, lanes = run.view(T, 8, 32), torch.arange(32)
+    for o in (16, 8, 4, 2, 1):
+        w = w + w[:, :, lanes ^ o]
+    s = w[:, :, 0].unbind(1)
+    return (((s[0] + s[1]) + (s[2] + s[3])) + (s[4] + s[5])) + (s[6] + s[7])
+
+
+@pytest.mark.parametrize("H", [576, 960, 1024, 1544, 2048, 2056, 3080, 4096, 8192])
+def test_rmsnorm_row_sums_do_not_depend_on_the_threads_per_row(C, H):
+    """Rows whose sums lose or keep whole groups of terms depending on the order of the additions."""
+    T = 16
+    # forward: in chunks 0..31 one large square per chunk, behind which every following term of the same running sum vanishes
+    x = torch.full((T, H), 0.95)
+    x[:, :256:8] = 4096.0
+    x = x.to(torch.bfloat16)
+    one = torch.ones(H, device="cuda", dtype=torch.bfloat16)
+    _, rstd = C.rmsnorm_fwd(x.cuda(), one, 1e-5)
+    xn, _, rstd_add = C.add_rmsnorm_fwd(x.cuda(), torch.zeros_like(x).cuda(), one, 1e-5)
+    _status_ok(C)
+    want = (_row_sum_in_kernel_order(x.float() ** 2).double() / H + 1e-5).rsqrt()
+    # approximate division and reciprocal root: 2 ulp of 2^-24 and 2^-22.9 relative, halved and summed; the other orders are off
+    # by up to 1e-6
+    for r in (rstd, rstd_add):
+        torch.testing.assert_close(r.cpu().double(), want, rtol=3e-7, atol=0)
+    assert torch.equal(xn.cpu(), x)
+    # backward: 2^30 and -2^30 in different chunks, ones elsewhere; how many ones survive is a matter of the order
+    gen = torch.Generator().manual_seed(H)
+    dy = torch.ones(T, H)
+    for t in range(T):
+        a, b = torch.randperm(H, generator=gen)[:2].tolist()
+        dy[t, a], dy[t, b] = 2.0 ** 30, -2.0 ** 30
+    # x = w = rstd = 1: dx = dy - sum(dy) / H
+    dx, _ = C.rmsnorm_bwd(dy.to(torch.bfloat16).cuda(), torch.ones(T, H, device="cuda", dtype=torch.bfloat16), one,
+                          torch.ones(T, device="cuda"), None)
+    _status_ok(C)
+    want = dy - (_row_sum_in_kernel_order(dy) / H)[:, None]
+    torch.testing.assert_close(dx.float().cpu(), want, rtol=2 ** -8, atol=2 ** -8)
+
+
 @pytest.mark.parametrize("T,H", [(513, 2048), (64, 768), (33, 256), (40, 4096), (9, 320)])
 def test_rmsnorm_bwd_accumulates_into_fp32_destination(C, T, H):
     """dw added in place to an fp32 vector (a gradient-bucket slice), also when that slice is not 16-byte aligned."""
