@@ -62,6 +62,27 @@ def test_attention_backward(C, B, Sq, Sk, hq, hkv, d, causal):
         torch.testing.assert_close(got.float(), want, rtol=5e-2, atol=5e-2)
 
 
+def test_attention_forward_row_sums_keep_their_order(C):
+    """One probability of 1 and 64 that vanish beside it when they are added one by one: a row's sum is that of its neighbour pairs
+    in four running sums (every fourth pair), so exactly the sixteen of the first running sum get lost."""
+    d, keys = 64, 128
+    q, k = torch.zeros(1, 130, 1, d), torch.zeros(1, keys, 1, d)
+    q[..., 0] = 1.0
+    k[0, :, 0, 0] = torch.where(torch.arange(keys) % 2 == 1, -24.125, -300.0)
+    k[0, 0, 0, 0] = 0.0
+    q, k = q.to(torch.bfloat16).cuda(), k.to(torch.bfloat16).cuda()
+    _, lse = C.attention_fwd(q, k, torch.randn_like(k), False, math.log(2.0))
+    torch.cuda.synchronize()
+    assert C.kernel_status() == 0
+    p = torch.exp2(k[0, :, 0, 0].float().cpu())
+    pairs, run = p[0::2] + p[1::2], torch.zeros(4)
+    for i in range(0, keys // 2, 4):
+        run = run + pairs[i:i + 4]
+    want = torch.log(((run[0] + run[1]) + (run[2] + run[3])).double())
+    # the logarithm's error is at most 2^-21.4 = 3.6e-7 there; a sum that keeps the sixteen is off by 16 * 2^-24.125 = 8.7e-7
+    torch.testing.assert_close(lse.double().cpu(), want.expand(lse.shape), rtol=0, atol=4e-7)
+
+
 @pytest.mark.parametrize("d", [64, 128])
 @pytest.mark.parametrize("Sq,Sk,group,causal", [(1, 1, 1, True), (127, 127, 3, True), (129, 129, 1, True), (385, 385, 4, True),
                                                 (640, 640, 2, True), (128, 300, 1, True), (65, 257, 3, False), (513, 64, 2, False)])
