@@ -24,10 +24,11 @@ void* pt_status_word();
 void pt_attention_set_profile(unsigned long long* counters);
 void pt_gemm_set_group_m(int g);
 void pt_gemm_set_tile_n(int n);
-long long pt_gemm_split_elems(int M, int N, int K);
-void pt_gemm_set_split_dgrad(int on);
+int pt_gemm_split_parts(int M, int N, int K, int out_mode);
+long long pt_gemm_split_elems(int M, int N, int K, int out_mode, int parts);
+void pt_gemm_set_split_k(int on);
 int pt_gemm_bf16_split(const void* A, const void* B, void* D, float* ws, int M, int N, int K, long long lda, long long ldb,
-                       long long ldd, void* status, cudaStream_t stream);
+                       long long ldd, int a_mn, int b_mn, int out_mode, int parts, void* status, cudaStream_t stream);
 int pt_gemm_get_group_m();
 void pt_gemm_set_tma_epilogue(int on);
 int pt_gemm_get_tma_epilogue();
@@ -296,13 +297,15 @@ Tensor gemm(const Tensor& a, const Tensor& b, bool trans_a, bool trans_b, const 
     mode = 0;
   }
   const long long ldd = row_stride_2d(d, "out");
-  if (mode == 0 && !trans_a && trans_b && pt_gemm_get_pair() && pt_gemm_get_tma_epilogue() && lda % 8 == 0 && ldb % 8 == 0 &&
-      ldd % 8 == 0 && (((uintptr_t)a.data_ptr() | (uintptr_t)b.data_ptr() | (uintptr_t)d.data_ptr()) & 15) == 0) {
-    const long long elems = pt_gemm_split_elems((int)M, (int)N, (int)K);
-    if (elems > 0) {
-      auto ws = torch::empty({elems}, a.options().dtype(at::kFloat));
+  // input gradients and weight gradients with few output tiles: K in parts (pt_gemm_split_parts)
+  const bool grad = (mode == 0 && !trans_a && trans_b) || (mode == 1 && trans_a && trans_b);
+  if (grad && pt_gemm_get_pair() && pt_gemm_get_tma_epilogue() && lda % 8 == 0 && ldb % 8 == 0 && ldd % (mode == 0 ? 8 : 4) == 0 &&
+      (((uintptr_t)a.data_ptr() | (uintptr_t)b.data_ptr() | (uintptr_t)d.data_ptr()) & 15) == 0) {
+    const int parts = pt_gemm_split_parts((int)M, (int)N, (int)K, mode);
+    if (parts > 1) {
+      auto ws = torch::empty({pt_gemm_split_elems((int)M, (int)N, (int)K, mode, parts)}, a.options().dtype(at::kFloat));
       const int rc = pt_gemm_bf16_split(a.data_ptr(), b.data_ptr(), d.data_ptr(), ws.data_ptr<float>(), (int)M, (int)N, (int)K, lda,
-                                        ldb, ldd, pt_status_word(), stream());
+                                        ldb, ldd, trans_a ? 1 : 0, trans_b ? 1 : 0, mode, parts, pt_status_word(), stream());
       if (rc != -5) {                                    // (CTA pairs cannot be scheduled: the general path below)
         TORCH_CHECK(rc == 0, "gemm (split) failed with code ", rc);
         return d;
@@ -809,8 +812,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("get_gemm_tma_epilogue", []() { return pt_gemm_get_tma_epilogue() != 0; });
   m.def("set_gemm_group_m", [](int64_t g) { pt_gemm_set_group_m((int)g); },
         "CTA-pair GEMM tile numbering: rows of 256-row tiles per group (L2 locality of concurrently running tiles; default 8).");
-  m.def("set_gemm_split_dgrad", [](bool on) { pt_gemm_set_split_dgrad(on ? 1 : 0); },
-        "input-gradient GEMMs with few output tiles: K split over idle CTA pairs (default on)");
+  m.def("set_gemm_split_dgrad", [](bool on) { pt_gemm_set_split_k(on ? 1 : 0); },
+        "input- and weight-gradient GEMMs with few output tiles: K split over idle CTA pairs (default on)");
   m.def("set_gemm_tile_n", [](int64_t n) { pt_gemm_set_tile_n((int)n); },
         "columns of the GEMM output tiles: 128, 256, or 0 for the choice by shape (bf16 outputs)");
   m.def("get_gemm_group_m", []() { return (int64_t)pt_gemm_get_group_m(); });

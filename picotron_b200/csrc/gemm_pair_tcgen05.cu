@@ -21,8 +21,9 @@
 // (64 bf16 or 32 fp32 columns), writes a chunk into a 128B-swizzled 4 KiB staging buffer of its own (two per
 // warp) and one lane hands it to TMA: a tiled store for bf16 / fp32 outputs, a tiled reduce-add for the
 // "accumulate into an fp32 destination" mode, so the weight-gradient GEMMs never read their destination into
-// the SM and a tile's K can be split over several CTA pairs (split_k_blocks). TMA clips rows and columns beyond M and N. The older epilogue (each thread storing its own row with
-// 16-byte stores, read-modify-write for the accumulate mode) is kept as a template variant.
+// the SM. TMA clips rows and columns beyond M and N. The older epilogue (each thread storing its own row with
+// 16-byte stores, read-modify-write for the accumulate mode) is kept as a template variant. Gradient GEMMs of few tiles split K
+// over several CTA pairs, which write slices of a workspace that a small kernel sums (pt_gemm_bf16_split).
 //
 // Fused epilogues (forward GEMMs X W^T with bf16 output only):
 //   SwiGLU  W is the packed [gate; up] weight [2I, K]. The leader CTA loads 128 (64) gate rows, its partner the up rows of
@@ -77,7 +78,9 @@ struct EpiArgs {
   int seq;                // RoPE: row r is at position r % seq
   int rot_cols;           // RoPE: columns [0, rot_cols) are rotated (rotated heads x d)
   int group_m;            // tile numbering: rows of tiles per group (all epilogues)
-  int kb_per_split;       // k-blocks per work unit; a tile is one unit unless its K is split (OUT_F32_ACC only, split_k_blocks)
+  // K split into parts (fp32 outputs without a fused epilogue, pt_gemm_bf16_split): k-blocks per part, rows between the slices of
+  // the destination, and which slice a part goes to (part >> slice_shift). Unsplit: one part with all k-blocks.
+  int kb_per_part, slice_rows, slice_shift;
   // cross-entropy statistics (EPI_CE): per row and per 256-column tile the maximum and the sum of exp(logit - maximum)
   // of the ROUNDED logits go to ce_part[row * ce_tiles + n_blk]; the logit of the row's target column goes to ce_tgt[row]
   float2* ce_part;
@@ -151,11 +154,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   const int num_m = (M + 2 * BM - 1) / (2 * BM);
   const int num_n = (EPI == EPI_SWIGLU) ? (N + BN_HALF - 1) / BN_HALF : (N + BN - 1) / BN;
   const int num_kb = (K + BK - 1) / BK;
-  // Work units: every output tile, once per K split (outermost, so that concurrently running units share operand panels as
-  // before). Several units of a tile add to the same destination with TMA reduce-adds.
+  // Work units: every output tile, once per part of K (outermost, so that concurrently running units share operand panels as
+  // before).
+  constexpr bool PARTS = OUT_MODE != OUT_BF16 && EPI_TMA;
   const int tiles = num_m * num_n;
-  const int kbs = (OUT_MODE == OUT_F32_ACC) ? ea.kb_per_split : num_kb;
-  const int num_tiles = (OUT_MODE == OUT_F32_ACC) ? tiles * ((num_kb + kbs - 1) / kbs) : tiles;
+  const int kbs = PARTS ? ea.kb_per_part : num_kb;
+  const int num_tiles = PARTS ? tiles * ((num_kb + kbs - 1) / kbs) : tiles;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -196,13 +200,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       bool ok = true;
       for (int t = cluster_id; t < num_tiles && ok; t += num_clusters) {
         int m_blk, n_blk;
-        const int split = (OUT_MODE == OUT_F32_ACC) ? t / tiles : 0;
-        tile_coords(t - split * tiles, num_m, num_n, ea.group_m, m_blk, n_blk);
+        const int part = PARTS ? t / tiles : 0;
+        tile_coords(t - part * tiles, num_m, num_n, ea.group_m, m_blk, n_blk);
         const int row0 = m_blk * 2 * BM + (int)rank * BM;          // this CTA's rows of A
         // this CTA's columns of B (SwiGLU: gate rows for the leader, the up rows of the same units for its partner)
         const int col0 = (EPI == EPI_SWIGLU) ? n_blk * BN_HALF + (int)rank * ea.inter : n_blk * BN + (int)rank * BN_HALF;
-        const int kb_end = min(num_kb, (split + 1) * kbs);
-        for (int kb = split * kbs; kb < kb_end; ++kb) {
+        const int kb_end = min(num_kb, (part + 1) * kbs);
+        for (int kb = part * kbs; kb < kb_end; ++kb) {
           if (!mbar_wait(&bars.empty[stage], phase ^ 1, abort_flag)) {
             report_error(status, KERNEL_ID, 1);
             ok = false;
@@ -251,8 +255,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         }
         tcgen05_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
-        const int split = (OUT_MODE == OUT_F32_ACC) ? t / tiles : 0;
-        const int num_here = min(num_kb - split * kbs, kbs);
+        const int part = PARTS ? t / tiles : 0;
+        const int num_here = min(num_kb - part * kbs, kbs);
         for (int kb = 0; kb < num_here; ++kb) {
           if (!mbar_wait(&bars.full[stage], phase, abort_flag)) {
             report_error(status, KERNEL_ID, 3);
@@ -541,7 +545,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       int buf = 0;
       for (int t = cluster_id; t < num_tiles && ok; t += num_clusters, ++local) {
         int m_blk, n_blk;
-        tile_coords(t % tiles, num_m, num_n, ea.group_m, m_blk, n_blk);
+        const int part = PARTS ? t / tiles : 0;
+        tile_coords(t - part * tiles, num_m, num_n, ea.group_m, m_blk, n_blk);
+        const int slice_row0 = PARTS ? (part >> ea.slice_shift) * ea.slice_rows : 0;
         const int acc = local & 1;
         const uint32_t acc_phase = (local >> 1) & 1;
         if (!mbar_wait(&bars.tmem_full[acc], acc_phase, abort_flag)) {
@@ -584,8 +590,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
           if (lane == 0) {
             const int col0 = n_blk * BN + c * CH_COLS;
             if (row0 < M && col0 < N) {
-              if (OUT_MODE == OUT_F32_ACC) tma_reduce_add_2d(&tma_d, dst, col0, row0);
-              else tma_store_2d(&tma_d, dst, col0, row0);
+              if (OUT_MODE == OUT_F32_ACC) tma_reduce_add_2d(&tma_d, dst, col0, slice_row0 + row0);
+              else tma_store_2d(&tma_d, dst, col0, slice_row0 + row0);
             }
             tma_store_commit();
           }
@@ -691,42 +697,42 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
 
 static int g_group_m = 8;   // rows of 256-row tiles per group; measured on the model's shapes: 8 and 16 beat 4 by ~1 %, 1 is worst
 
-// k-blocks per work unit of a GEMM that accumulates into fp32 (weight gradients: K is the number of tokens). With few output
-// tiles a unit per tile leaves most CTA pairs idle behind a long K loop, so K is split over the idle pairs. A unit costs its
-// k-blocks plus about 12 k-blocks' time for its epilogue and the reduce-add traffic of its tile (fitted to a sweep of 1..16
-// splits over the shapes of 20M to 1.7B models); the S with the least waves * unit time wins, S = 1 whenever the tiles alone
-// fill the pairs. Measured (us per launch): 576x576, 8192 tokens: 45.6 -> 12.4 (S = 8); 3072x576, 1803 tokens: 15.5 -> 11.9
-// (S = 2); 6144x2048, 4096 tokens: 82 with S = 1 (chosen), 89 with S = 2.
-static int split_k_blocks(int tiles, int num_kb, int clusters) {
-  constexpr int EPI_KB = 12, MIN_KB = 4;
-  int best = num_kb;
-  long long best_cost = -1;
-  for (int S = 1; S <= 32 && (S == 1 || num_kb / S >= MIN_KB); ++S) {
-    const int kbs = (num_kb + S - 1) / S;
-    const int units = tiles * ((num_kb + kbs - 1) / kbs);
-    const long long cost = (long long)((units + clusters - 1) / clusters) * (kbs + EPI_KB);
-    if (best_cost < 0 || cost < best_cost) {
-      best = kbs;
-      best_cost = cost;
-    }
-  }
-  return best;
-}
-
-// fp32 workspace of a split bf16 GEMM: cleared before, rounded into the output after
+// K-split GEMMs keep their parts in slices of an fp32 workspace: cleared before where two parts add to a slice, summed after in the
+// order of the slices.
 __global__ void __launch_bounds__(256) clear_f32_kernel(float4* __restrict__ x, long long n4) {
   pdl_enter();
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
   if (i < n4) x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
-__global__ void __launch_bounds__(256) round_f32_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ out, long long rows,
-                                                        int cols, long long ldd) {
+// out[r, c] = sum over the slices (bf16), or out[r, c] += that sum (fp32, one atomic per element as the unsplit epilogue's
+// reduce-add). Bound by the workspace's bytes, which lie in L2; four columns per thread.
+template <bool TO_BF16>
+__global__ void __launch_bounds__(256) sum_slices_kernel(const float* __restrict__ ws, int slices, long long slice_elems, void* __restrict__ out,
+                                                         int rows, int cols, int ws_cols, long long ldd) {
   pdl_enter();
-  const long long i = ((long long)blockIdx.x * 256 + threadIdx.x) * 8;
-  if (i >= rows * cols) return;                          // cols % 8 == 0: a thread's eight elements lie in one row
-  const float4 a = *reinterpret_cast<const float4*>(x + i), b = *reinterpret_cast<const float4*>(x + i + 4);
-  *reinterpret_cast<uint4*>(out + i / cols * ldd + i % cols) =
-      make_uint4(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w), pack_bf16(b.x, b.y), pack_bf16(b.z, b.w));
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  const int quads = ws_cols / 4;
+  const long long r = i / quads;
+  const int c = (int)(i - r * quads) * 4;
+  if (r >= rows) return;
+  const float* src = ws + r * ws_cols + c;
+  float4 v = *reinterpret_cast<const float4*>(src);
+#pragma unroll 4
+  for (int k = 1; k < slices; ++k) {
+    const float4 u = *reinterpret_cast<const float4*>(src + k * slice_elems);
+    v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+  }
+  if (TO_BF16) {
+    *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(out) + r * ldd + c) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+  } else {
+    float* dst = reinterpret_cast<float*>(out) + r * ldd + c;
+    if (c + 4 <= cols) {
+      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+    } else {
+      const float e[4] = {v.x, v.y, v.z, v.w};
+      for (int j = 0; j < 4 && c + j < cols; ++j) atomicAdd(dst + j, e[j]);
+    }
+  }
 }
 
 static int num_pairs() {
@@ -740,7 +746,7 @@ static int num_pairs() {
   return pairs;
 }
 
-static int g_split_dgrad = 1;
+static int g_split_k = 1;
 static int g_tile_n = 0;    // 0: by the rule below, 128 / 256: as given (tests, measurements)
 
 // Columns of an output tile (bf16 outputs). A 256 x 256 tile moves the fewest operand bytes per product, but a few hundred
@@ -786,8 +792,8 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMa
   const int tiles = ((M + 2 * BM - 1) / (2 * BM)) * n_tiles;
   const int num_kb = (K + BK - 1) / BK;
   ea.group_m = g_group_m;
-  ea.kb_per_split = (OUT_MODE == OUT_F32_ACC && EPI_TMA) ? split_k_blocks(tiles, num_kb, max_clusters) : num_kb;
-  const int units = tiles * ((num_kb + ea.kb_per_split - 1) / ea.kb_per_split);
+  if (ea.kb_per_part <= 0) ea.kb_per_part = num_kb;
+  const int units = tiles * ((num_kb + ea.kb_per_part - 1) / ea.kb_per_part);
   const int clusters = units < max_clusters ? units : max_clusters;
   const cudaError_t err = launch_pdl(kern, dim3(2 * clusters), dim3(NUM_THREADS), smem_bytes_of(EPI, BN), stream, ma, mb, md,
                                      mh ? *mh : md, D, M, N, K, ldd, status, ea);
@@ -807,44 +813,98 @@ static int g_tma_epilogue = 1;
 extern "C" void pt_gemm_set_tma_epilogue(int on) { g_tma_epilogue = on; }
 extern "C" int pt_gemm_get_tma_epilogue() { return g_tma_epilogue; }
 
-// Input-gradient GEMMs (bf16 output, long K) with few output tiles: K split over the idle CTA pairs, which add to an fp32
-// workspace that is rounded to bf16 once. pt_gemm_split_elems gives the workspace's size in floats, 0 where splitting does not
-// pay: the time in k-blocks (about 0.33 us each) of split_k_blocks' model with and without a split, plus 24 k-blocks for the two
-// small kernels around it and the workspace's 16 bytes per element and split at 5 TB/s. Measured without / with it (us):
-// 2048 x 576 x 49152 (LM head of the 135M shape): 246 / 105; 512 x 2048 x 16384: 90 / 42; 1024 x 2048 x 128256: 627 / 372;
-// 256 x 4096 x 4096: 34 / 28; and with no gain left at 2048 x 2048 x 128256: 745 / 749.
-// (The sums of a split tile come in any order, as those of dQ and of the weight gradients do; the forward GEMMs are not split.)
-extern "C" long long pt_gemm_split_elems(int M, int N, int K) {
+extern "C" void pt_gemm_set_split_k(int on) { pt::gemm_pair::g_split_k = on; }
+
+namespace pt {
+namespace gemm_pair {
+struct SplitPlan {
+  int parts, kb_per_part, slices, shift, slice_rows, ws_cols;
+};
+// Two parts add to a slice of an input gradient's workspace (a sum of two is the same in either order); the parts of a weight
+// gradient, whose result has to be read and written anyway, each store a slice of their own.
+static SplitPlan split_plan(int M, int N, int K, int out_mode, int parts) {
+  SplitPlan s;
+  const int kb = (K + BK - 1) / BK;
+  s.kb_per_part = (kb + parts - 1) / parts;
+  s.parts = (kb + s.kb_per_part - 1) / s.kb_per_part;
+  s.shift = out_mode == OUT_BF16 ? 1 : 0;
+  s.slices = (s.parts + s.shift) >> s.shift;
+  s.slice_rows = (M + 31) / 32 * 32;        // the epilogue writes 32 rows at a time
+  s.ws_cols = (N + 3) / 4 * 4;
+  return s;
+}
+static int run_pair(const void* A, const void* B, void* D, int M, int N, int K, long long lda, long long ldb, long long ldd, int a_mn,
+                    int b_mn, int out_mode, const SplitPlan* split, void* status, cudaStream_t stream);
+}  // namespace gemm_pair
+}  // namespace pt
+
+// How many parts K is split into when D[M, N] has few tiles behind a long K; 1: not at all. In k-blocks of 0.33 us, a wave of tiles
+// takes its k-blocks plus a constant, and a split adds its further kernels and the workspace's traffic. Measured without / with it (us):
+// weight gradients (out_mode OUT_F32_ACC; K is the number of tokens; constants fitted to a sweep of 1 to 32 parts over the shapes
+// of 20M to 1.7B models and 256 to 32,768 tokens, 3 % off; a split has to give 5 %): 576 x 576, 8192 tokens: 45.7 / 16.2; 3072 x
+// 576, 4096 tokens: 27.3 / 21.2; 512 x 512, 512 tokens: 8.4 / 8.1 (not split); 2048 x 2048, 4096 tokens: 29.4 / 36.4 (not split).
+// Input gradients (OUT_BF16; the constants are on the safe side, so that it is split where it gives about a quarter): 2048 x 576 x
+// 49152 (LM head of the 135M shape): 241 / 103; 512 x 2048 x 16384: 84.7 / 35.4; 256 x 4096 x 4096: 25.0 / 18.7; 512 x 512 x 2048:
+// 13.8 / 11.4 (not split); 2048 x 2048 x 49152: 282 / 300 (not split).
+// (Weight gradients with every part added to the destination by itself needed 3 us less, but their results changed from run to run
+// and were rounded once per part. The forward GEMMs are not split.)
+extern "C" int pt_gemm_split_parts(int M, int N, int K, int out_mode) {
   using namespace pt::gemm_pair;
-  if (M <= 0 || N % 8 || K <= 0 || !g_split_dgrad) return 0;
+  const bool wgrad = out_mode == OUT_F32_ACC;
+  if (M <= 0 || N <= 0 || K <= 0 || !g_split_k || (!wgrad && N % 8)) return 1;
   const int pairs = num_pairs(), kb = (K + BK - 1) / BK;
   const int tiles = ((M + 2 * BM - 1) / (2 * BM)) * ((N + 255) / 256);
-  if (tiles >= pairs) return 0;
-  const int kbs = split_k_blocks(tiles, kb, pairs);
-  const long long S = (kb + kbs - 1) / kbs;
-  if (S <= 1) return 0;
-  const long long waves = (tiles * S + pairs - 1) / pairs;
-  const long long cost = waves * (kbs + 12) + 24 + (long long)((double)M * N * 4 * (2 + S) / 5e6 / 0.33);
-  return cost + cost / 8 < kb + 12 ? (long long)M * N : 0;
+  if (tiles >= pairs) return 1;
+  constexpr int MIN_KB = 4, MAX_PARTS = 32;
+  const double mbytes = (double)M * N * 4e-6;
+  const int wave_kb = wgrad ? 3 : 12, other_kb = wgrad ? 16 : 0;      // other_kb: launches, split or not
+  auto cost = [&](const SplitPlan& p, bool whole) {
+    double c = other_kb + (double)((tiles * p.parts + pairs - 1) / pairs) * (p.kb_per_part + wave_kb);
+    if (whole) c += wgrad ? 2 + 0.27 * mbytes * (2 * p.slices + 2) : 24 + 0.6 * mbytes * (2 + p.parts);
+    return c;
+  };
+  // input gradients: the parts with the shortest waves first, then whether they pay (their traffic is a fraction of the tiles' time)
+  int best = 1;
+  double best_cost = other_kb + kb + wave_kb;
+  for (int parts = 2; parts <= MAX_PARTS && kb / parts >= MIN_KB; ++parts) {
+    const double c = cost(split_plan(M, N, K, out_mode, parts), wgrad);
+    if (c < best_cost) {
+      best = parts;
+      best_cost = c;
+    }
+  }
+  if (best == 1) return 1;
+  const double gain = wgrad ? 0.95 : 1 / 1.125;
+  return cost(split_plan(M, N, K, out_mode, best), true) < gain * (other_kb + kb + wave_kb) ? best : 1;
 }
 
-extern "C" void pt_gemm_set_split_dgrad(int on) { pt::gemm_pair::g_split_dgrad = on; }
+// Floats of workspace for pt_gemm_bf16_split with `parts` parts.
+extern "C" long long pt_gemm_split_elems(int M, int N, int K, int out_mode, int parts) {
+  const pt::gemm_pair::SplitPlan p = pt::gemm_pair::split_plan(M, N, K, out_mode, parts);
+  return (long long)p.slices * p.slice_rows * p.ws_cols;
+}
 
-extern "C" int pt_gemm_bf16_pair(const void* A, const void* B, void* D, int M, int N, int K, long long lda, long long ldb,
-                                 long long ldd, int a_mn, int b_mn, int out_mode, void* status, cudaStream_t stream);
-
-// D[M, N] = A[M, K] B[K, N] (bf16) through the fp32 workspace ws (M * N floats, 16-byte aligned); ldd % 8 == 0, D 16-byte aligned.
+// GEMM with K in `parts` parts, each computed by CTA pairs of its own, through the fp32 workspace ws (pt_gemm_split_elems floats,
+// 16-byte aligned). out_mode OUT_BF16: D = op(A) op(B), rounded once (N % 8 == 0, ldd % 8 == 0); OUT_F32_ACC: D += op(A) op(B) with
+// one addition per element (ldd % 4 == 0). The result does not depend on the order in which the parts finish.
 extern "C" int pt_gemm_bf16_split(const void* A, const void* B, void* D, float* ws, int M, int N, int K, long long lda, long long ldb,
-                                  long long ldd, void* status, cudaStream_t stream) {
+                                  long long ldd, int a_mn, int b_mn, int out_mode, int parts, void* status, cudaStream_t stream) {
   using namespace pt;
   using namespace pt::gemm_pair;
-  const long long n = (long long)M * N;
-  launch_pdl(clear_f32_kernel, dim3((unsigned)((n / 4 + 255) / 256)), dim3(256), 0, stream, reinterpret_cast<float4*>(ws), n / 4);
-  const int rc = pt_gemm_bf16_pair(A, B, ws, M, N, K, lda, ldb, N, 0, 1, OUT_F32_ACC, status, stream);
+  const SplitPlan p = split_plan(M, N, K, out_mode, parts);
+  const long long slice_elems = (long long)p.slice_rows * p.ws_cols, n4 = p.slices * slice_elems / 4;
+  if (p.shift > 0) {
+    launch_pdl(clear_f32_kernel, dim3((unsigned)((n4 + 255) / 256)), dim3(256), 0, stream, reinterpret_cast<float4*>(ws), n4);
+    pt_count_launches(1);
+  }
+  const int rc = run_pair(A, B, ws, M, N, K, lda, ldb, p.ws_cols, a_mn, b_mn, p.shift > 0 ? OUT_F32_ACC : OUT_F32, &p, status, stream);
   if (rc) return rc;
-  launch_pdl(round_f32_kernel, dim3((unsigned)((n / 8 + 255) / 256)), dim3(256), 0, stream, (const float*)ws, (__nv_bfloat16*)D,
-             (long long)M, N, ldd);
-  pt_count_launches(2);
+  const dim3 grid((unsigned)(((long long)M * (p.ws_cols / 4) + 255) / 256));
+  if (out_mode == OUT_BF16)
+    launch_pdl(sum_slices_kernel<true>, grid, dim3(256), 0, stream, (const float*)ws, p.slices, slice_elems, D, M, N, p.ws_cols, ldd);
+  else
+    launch_pdl(sum_slices_kernel<false>, grid, dim3(256), 0, stream, (const float*)ws, p.slices, slice_elems, D, M, N, p.ws_cols, ldd);
+  pt_count_launches(1);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 
@@ -852,6 +912,12 @@ extern "C" int pt_gemm_bf16_split(const void* A, const void* B, void* D, float* 
 extern "C" int pt_gemm_bf16_pair(const void* A, const void* B, void* D, int M, int N, int K, long long lda,
                                  long long ldb, long long ldd, int a_mn, int b_mn, int out_mode, void* status,
                                  cudaStream_t stream) {
+  return pt::gemm_pair::run_pair(A, B, D, M, N, K, lda, ldb, ldd, a_mn, b_mn, out_mode, nullptr, status, stream);
+}
+
+static int pt::gemm_pair::run_pair(const void* A, const void* B, void* D, int M, int N, int K, long long lda, long long ldb,
+                                   long long ldd, int a_mn, int b_mn, int out_mode, const SplitPlan* split, void* status,
+                                   cudaStream_t stream) {
   using namespace pt;
   using namespace pt::gemm_pair;
   const int bn = (out_mode == OUT_BF16 && g_tma_epilogue && !a_mn) ? tile_columns(M, N, K) : 256;
@@ -866,11 +932,17 @@ extern "C" int pt_gemm_bf16_pair(const void* A, const void* B, void* D, int M, i
   CUtensorMap md = ma;           // unused by the per-thread epilogue
   const bool epi_tma = g_tma_epilogue != 0;
   if (epi_tma) {
-    uint64_t dims[2] = {(uint64_t)N, (uint64_t)M};
+    uint64_t dims[2] = {(uint64_t)N, split ? (uint64_t)split->slices * split->slice_rows : (uint64_t)M};
     uint64_t strides[1] = {(uint64_t)ldd};
     uint32_t box_bf16[2] = {64, 32}, box_f32[2] = {32, 32};
     rc = out_mode == OUT_BF16 ? make_bf16_map(&md, D, 2, dims, strides, box_bf16) : make_f32_map(&md, D, 2, dims, strides, box_f32);
     if (rc) return rc * 10 - 3;  // -23: tensor map of D could not be encoded
+  }
+  EpiArgs ea{};
+  if (split) {
+    ea.kb_per_part = split->kb_per_part;
+    ea.slice_rows = split->slice_rows;
+    ea.slice_shift = split->shift;
   }
   KernelStatus* st = reinterpret_cast<KernelStatus*>(status);
   if (bn == 128)
@@ -878,7 +950,7 @@ extern "C" int pt_gemm_bf16_pair(const void* A, const void* B, void* D, int M, i
                 : launch<false, false, OUT_BF16, true, EPI_NONE, 128>(ma, mb, md, D, M, N, K, ldd, st, stream);
 #define PT_GEMM_CASE(AM, BMN, OM)                                                                             \
   if (a_mn == AM && b_mn == BMN && out_mode == OM)                                                            \
-    return epi_tma ? launch<AM, BMN, OM, true>(ma, mb, md, D, M, N, K, ldd, st, stream)                       \
+    return epi_tma ? launch<AM, BMN, OM, true>(ma, mb, md, D, M, N, K, ldd, st, stream, nullptr, ea)          \
                    : launch<AM, BMN, OM, false>(ma, mb, md, D, M, N, K, ldd, st, stream);
   PT_GEMM_CASE(0, 0, 0) PT_GEMM_CASE(0, 0, 1) PT_GEMM_CASE(0, 0, 2)
   PT_GEMM_CASE(0, 1, 0) PT_GEMM_CASE(0, 1, 1) PT_GEMM_CASE(0, 1, 2)

@@ -93,6 +93,46 @@ def test_gemm_fp32_accumulation_with_k_split_over_cta_pairs(M, N, K):
     assert _rel(acc - 0.5, a.double().t() @ b.double()) < 1e-5
 
 
+@pytest.mark.parametrize("M,N,K", [(576, 576, 8192), (573, 569, 4100), (264, 520, 32768), (8, 8, 16384)])
+def test_gemm_weight_gradient_parts_are_repeatable_and_rounded_once(C, M, N, K):
+    """The parts of K add up in a fixed order and reach the destination in one addition, also where rows and columns end within a
+    tile, a quad of columns and a strided destination."""
+    from picotron_b200.ops import _ext
+    C = _ext.load()
+    C.set_gemm_pair(True)
+    C.set_gemm_tma_epilogue(True)
+    wide = lambda n: (n + 7) // 8 * 8
+    a, b = bf(K, wide(M), seed=81)[:, :M], bf(K, wide(N), seed=82)[:, :N]
+    want = a.double().t() @ b.double()
+    base = 2.0 ** 20
+    first = None
+    for _ in range(12):
+        big = torch.full((M, wide(N) + 8), base, device="cuda")
+        n0 = C.launch_count()
+        C.gemm(a, b, True, True, big[:, :N], True)
+        assert C.launch_count() - n0 == 2, "this shape should be split"
+        first = big if first is None else first
+        assert torch.equal(big, first)
+    _status_ok(C)
+    assert bool((big[:, N:] == base).all())
+    # one rounding at 2^20 (half an ulp: 2^-4) of a sum that is itself good to 1e-5 of its size
+    err = float((big[:, :N].double() - base - want).abs().max())
+    assert err <= 2 ** -4 + 1e-5 * float(want.abs().max()), err
+
+
+@pytest.mark.parametrize("T,N,K", [(64, 576, 49152), (500, 520, 16392), (300, 2048, 16384)])
+def test_gemm_input_gradient_parts_are_repeatable(C, T, N, K):
+    from picotron_b200.ops import _ext
+    C = _ext.load()
+    C.set_gemm_pair(True)
+    C.set_gemm_tma_epilogue(True)
+    dy, w = bf(T, K, seed=1, scale=0.1), bf(K, N, seed=2, scale=0.1)
+    first = C.gemm(dy, w, False, True)
+    for _ in range(12):
+        assert torch.equal(C.gemm(dy, w, False, True), first)
+    _status_ok(C)
+
+
 @pytest.mark.parametrize("T,I,K", [(256, 128, 64), (300, 384, 320), (1024, 2048, 512), (4096, 1024, 2048)])
 def test_gemm_with_swiglu_epilogue(T, I, K):
     """gate/up GEMM whose epilogue also writes silu(gate) * up, against the two separate kernels and fp32 math."""
