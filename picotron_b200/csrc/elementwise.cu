@@ -415,12 +415,12 @@ struct AdamArgs {
 };
 static_assert(sizeof(AdamArgs) <= 32000, "kernel parameter limit");
 
+// (Explicit fused operations: left to the compiler, the whole and the partial chunks of a tensor were rounded differently.)
 __device__ __forceinline__ void adam_update(float& w, float& m, float& v, float g, float lr, float beta1, float beta2, float eps,
                                             float wd, float bc1, float bc2_sqrt) {
-  m = m * beta1 + g * (1.f - beta1);
-  v = v * beta2 + g * g * (1.f - beta2);
-  w = w * (1.f - lr * wd);
-  w -= (lr / bc1) * (m / (sqrtf(v) / bc2_sqrt + eps));
+  m = fmaf(g, 1.f - beta1, m * beta1);
+  v = fmaf(g * g, 1.f - beta2, v * beta2);
+  w = fmaf(w, 1.f - lr * wd, -((lr / bc1) * (m / (sqrtf(v) / bc2_sqrt + eps))));
 }
 
 template <bool PARAM_BF16>

@@ -493,6 +493,24 @@ def test_adamw_chunk_edges_alignment_and_table_size(C, dtype, offset, count):
             torch.testing.assert_close(a, b, **t)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("master", [False, True])
+def test_adamw_does_not_depend_on_an_elements_place(C, dtype, master):
+    """The same 2048 elements in a whole chunk (16-byte accesses), in a tensor's last chunk and off the alignment: equal bits."""
+    g = torch.Generator(device="cuda").manual_seed(9)
+    draw = lambda scale: torch.randn(2048, device="cuda", generator=g) * scale
+    p, grad, m, v, w = draw(1.0).to(dtype), draw(1e-3), draw(1e-3), draw(1e-3) ** 2, draw(1.0)
+    place = lambda x, off: torch.cat([x.new_zeros(off), x, x, x])[off:]
+    results = []
+    for off in (0, 1):
+        t = [place(x, off) for x in (p, grad, m, v, w)]
+        C.adamw_multi_([t[0]], [t[1]], [t[2]], [t[3]], [t[4] if master else None], 3, 1e-3, 0.9, 0.999, 1e-8, 0.01)
+        results += [[x[i:i + 2048] for x in t] for i in (0, 2048, 4096)]
+    for r in results[1:]:
+        for a, b in zip(results[0], r):
+            assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("n", [1, 8191, 8192, 8193, 40000])
 @pytest.mark.parametrize("offset", [0, 1])
 @pytest.mark.parametrize("c", [0.37, 1.0])
