@@ -331,8 +331,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       if (j > 0) {
         // P_{j-1} and O (tensor memory) may be touched once the MMA O += P_{j-1} V_{j-1} has completed
         if (!mbar_wait(&bars.o_full, (j - 1) & 1, abort_flag)) { if (lane == 0) report_error(status, KID_FWD, 8); ok = false; break; }
+        tcgen05_fence_after();                                    // (also for the store of P_j below)
         if (__any_sync(0xffffffffu, move)) {
-          tcgen05_fence_after();
 #pragma unroll
           for (int c = 0; c < D / 32; ++c) {
             uint32_t r[32];

@@ -1,0 +1,51 @@
+"""What the memory model asks of the kernels and no run can be relied on to show, read from their sources."""
+import glob
+import os
+import re
+
+import pytest
+
+import picotron_b200
+
+CSRC = os.path.join(os.path.dirname(picotron_b200.__file__), "csrc")
+TOKENS = re.compile(r"[{}]|mbar_wait\(|tcgen05_fence_after\(\)|(?:tmem_(?:ld|st)_32x32b|umma_bf16)\w*\(")
+
+
+def unfenced_accesses(src):
+    """Lines of tensor-memory accesses and MMAs that follow an mbarrier wait without tcgen05.fence::after_thread_sync on every
+    way between the two (a fence in a block that is entered conditionally counts inside that block only)."""
+    src = re.sub(r"//[^\n]*", "", src)
+    depth, waits, fences, found = 0, [], [], []      # waits: depths of those not fenced yet; fences: depths of conditional fences
+    for m in TOKENS.finditer(src):
+        token = m.group(0)
+        if token == "{":
+            depth += 1
+        elif token == "}":
+            depth -= 1
+            fences = [f for f in fences if f <= depth]
+        elif token == "mbar_wait(":
+            statement = src[max(src.rfind(c, 0, m.start()) for c in ";{}"):m.start()]
+            # `if (ok && mbar_wait(..)) {`: what depends on the wait stands in the block that follows
+            waits.append(depth + (1 if "if" in statement and not statement.rstrip().endswith("!") else 0))
+            fences = []
+        elif token.startswith("tcgen05_fence"):
+            waits = [w for w in waits if w < depth]
+            if waits:
+                fences.append(depth)
+        elif waits and not fences:
+            found.append(src.count("\n", 0, m.start()) + 1)
+    return found
+
+
+@pytest.mark.parametrize("path", sorted(glob.glob(os.path.join(CSRC, "*tcgen05.cu"))), ids=os.path.basename)
+def test_tensor_memory_is_fenced_after_every_wait(path):
+    with open(path) as f:
+        assert unfenced_accesses(f.read()) == []
+
+
+def test_the_check_sees_a_missing_and_a_conditional_fence():
+    wait = "if (!mbar_wait(&b, 0, a)) { break; }\n"
+    assert unfenced_accesses(wait + "tcgen05_fence_after();\ntmem_st_32x32b_x32(t, r);") == []
+    assert unfenced_accesses(wait + "tmem_st_32x32b_x32(t, r);") == [2]
+    assert unfenced_accesses(wait + "if (m) { tcgen05_fence_after(); tmem_ld_32x32b_x32(t, r); }\ntmem_st_32x32b_x32(t, r);") == [3]
+    assert unfenced_accesses("if (ok && mbar_wait(&b, 0, a)) {\ntcgen05_fence_after();\ntmem_ld_32x32b_x32(t, r); }") == []
