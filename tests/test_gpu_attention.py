@@ -62,6 +62,36 @@ def test_attention_backward(C, B, Sq, Sk, hq, hkv, d, causal):
         torch.testing.assert_close(got.float(), want, rtol=5e-2, atol=5e-2)
 
 
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("Sq,Sk,causal", [(517, 517, True), (300, 517, False), (129, 640, False)])
+@pytest.mark.parametrize("rows", ["all", "some", "none"])
+def test_attention_forward_moves_its_reference_maximum(C, Sq, Sk, causal, d, rows):
+    """Keys that grow with every 64 (or shrink: no move after the first block), so that a row's maximum jumps by far more than the
+    2^8 beyond which the accumulated output is rescaled: for every row, for one row in five (the others of its warp stay), for none."""
+    hq, hkv = 4, 2
+    grow = 1.0 + 2.0 * (torch.arange(Sk, device="cuda") // 64)
+    if rows == "none":
+        grow = grow.flip(0)
+    q, k, v = rnd(2, Sq, hq, d, seed=1), rnd(2, Sk, hkv, d, seed=2), rnd(2, Sk, hkv, d, seed=3)
+    k = (k.float() * grow[:, None, None]).to(torch.bfloat16)
+    if rows == "some":
+        q = (q.float() * (torch.arange(Sq, device="cuda") % 5 == 0)[:, None, None]).to(torch.bfloat16)
+    scale = 1.0 / math.sqrt(d)
+    s = torch.einsum("bqhd,bkhd->bhqk", q.float(), k.float().repeat_interleave(hq // hkv, 2)) * scale * math.log2(math.e)
+    if causal:
+        s = s.masked_fill(torch.ones(Sq, Sk, device="cuda", dtype=torch.bool).triu(1), -math.inf)
+    blocks = torch.stack([b.amax(-1) for b in s.split(128 if d == 64 else 64, dim=-1)])
+    jumps = ((blocks[1:] > blocks.cummax(0).values[:-1] + 8).sum(0) >= (2 if d == 64 else 3)).float().mean()
+    assert (jumps > 0.25 if rows == "all" else 0.05 < jumps < 0.2 if rows == "some" else jumps == 0), "the inputs miss their purpose"
+    o, lse = C.attention_fwd(q, k, v, causal, scale)
+    torch.cuda.synchronize()
+    assert C.kernel_status() == 0
+    o_ref, lse_ref = ref.attention_fwd(q, k, v, causal, scale)
+    # scores up to a few hundred with fp32 sums (2^-24 of the sum of their terms' sizes); probabilities rounded to bf16 (2^-9)
+    torch.testing.assert_close(lse, lse_ref, rtol=1e-5, atol=1e-3)
+    torch.testing.assert_close(o.float(), o_ref.float(), rtol=2e-2, atol=2e-2)
+
+
 def test_attention_forward_row_sums_keep_their_order(C):
     """One probability of 1 and 64 that vanish beside it when they are added one by one: a row's sum is that of its neighbour pairs
     in four running sums (every fourth pair), so exactly the sixteen of the first running sum get lost."""
