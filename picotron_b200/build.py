@@ -9,6 +9,7 @@ their sources (or ``common.cuh``) are newer. nvcc cross-compiles, so no GPU is n
 from __future__ import annotations
 
 import os
+import re
 import subprocess
 import sys
 import sysconfig
@@ -41,6 +42,27 @@ def _run(cmd, log_name=None):
         raise RuntimeError(f"build step failed: {' '.join(cmd)}\n{res.stdout}\n{res.stderr}")
 
 
+# Kernels whose warpgroups redistribute the registers of the launch (setmaxnreg) depend on an exact count: with fewer, the warps
+# that ask for more would wait forever. Substring of the kernel's name, registers per thread.
+FIXED_REGISTERS = {"attn_bwd_kernel": 128}
+
+
+def check_registers(log: str, fixed=None) -> None:
+    """Raise if ``-Xptxas -v`` reports another register count than a kernel of ``fixed`` depends on."""
+    kernel = None
+    for line in log.splitlines():
+        entry = re.search(r"Compiling entry function '(\S+)'", line)
+        if entry:
+            kernel = entry.group(1)
+        used = re.search(r"Used (\d+) registers", line)
+        if used and kernel:
+            for name, want in (FIXED_REGISTERS if fixed is None else fixed).items():
+                if name in kernel and int(used.group(1)) != want:
+                    raise RuntimeError(f"{kernel} uses {used.group(1)} registers per thread; its warpgroups share out {want} "
+                                       "(setmaxnreg): adapt the split in its source to this compiler")
+            kernel = None
+
+
 def build(verbose: bool = True) -> str:
     import torch
     from torch.utils import cpp_extension as ce
@@ -70,6 +92,7 @@ def build(verbose: bool = True) -> str:
             print(f"[picotron_b200.build] compiling {len(jobs)} file(s) for sm_100a", flush=True)
         with ThreadPoolExecutor(max_workers=min(8, len(jobs))) as ex:
             list(ex.map(lambda j: _run(*j), jobs))
+    check_registers(ptxas_report())
     target = ext_path()
     if jobs or _newer(objs, target):
         libs = []

@@ -1085,7 +1085,8 @@ static int launch_bwd(const CUtensorMap& mq, const KVSegs& segs, const CUtensorM
   if (!configured) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdCfg<D>::SMEM) != cudaSuccess) return -3;
     cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    // the warpgroups share out BWD_REGS registers per thread; with fewer at launch setmaxnreg.inc would wait forever
+    // the warpgroups share out BWD_REGS registers per thread; with fewer at launch setmaxnreg.inc would wait forever (the build
+    // fails for another count, build.py: FIXED_REGISTERS)
     cudaFuncAttributes fa;
     if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess || fa.numRegs != BWD_REGS) return -6;
     configured = true;

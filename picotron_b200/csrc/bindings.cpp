@@ -108,6 +108,14 @@ inline cudaStream_t stream() { return at::cuda::getCurrentCUDAStream().stream();
 inline int num_sms() { return at::cuda::getCurrentDeviceProperties()->multiProcessorCount; }
 
 #define PT_CHECK_RC(rc, what) TORCH_CHECK((rc) == 0, what, " failed with code ", (rc))
+// (-6: the attention backward was compiled with another register count than its warpgroups share out)
+#define PT_CHECK_BWD_RC(rc, what)                                                                                              \
+  do {                                                                                                                         \
+    const int rc_ = (rc);                                                                                                      \
+    TORCH_CHECK(rc_ != -6, what, ": this build of the kernel has another number of registers per thread than its warpgroups "  \
+                "share out; rebuild with python -m picotron_b200.build");                                                      \
+    PT_CHECK_RC(rc_, what);                                                                                                    \
+  } while (0)
 #define PT_CHECK_BF16(t) TORCH_CHECK((t).is_cuda() && (t).scalar_type() == at::kBFloat16, #t " must be a CUDA bf16 tensor")
 #define PT_CHECK_F32(t) TORCH_CHECK((t).is_cuda() && (t).scalar_type() == at::kFloat, #t " must be a CUDA fp32 tensor")
 
@@ -522,7 +530,7 @@ std::vector<Tensor> attention_bwd(const Tensor& dout, const Tensor& q, const Ten
     TORCH_CHECK(Sq == Sk, "attention_bwd: rope fusion needs self-attention (Sq == Sk)");
     rope_seq = Sq;                       // row b*Sq + i of the flattened tokens is at position i
   }
-  PT_CHECK_RC(pt_attention_bwd_rope(dout.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(),
+  PT_CHECK_BWD_RC(pt_attention_bwd_rope(dout.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(),
                                     lse.data_ptr<float>(), delta.has_value() ? delta->data_ptr<float>() : nullptr,
                                     delta_ws.data_ptr<float>(), dq_ws.data_ptr<float>(), dq.data_ptr(), dk.data_ptr(),
                                     dv.data_ptr(), B, Sq, Sk, hq, hkv, d, token_stride(q, "q"), token_stride(k, "k"),
@@ -676,7 +684,7 @@ Tensor attention_bwd_segs(const Tensor& dout, const Tensor& q, std::vector<int64
   auto delta_ws = torch::empty({B, hq, Sq}, q.options().dtype(at::kFloat));
   float* part = reinterpret_cast<float*>(partial_ptr);
   const long long per = (long long)B * Sk * hkv * d;
-  PT_CHECK_RC(pt_attention_bwd_segs(dout.data_ptr(), q.data_ptr(), kp, vp, n, o.data_ptr(), lse.data_ptr<float>(),
+  PT_CHECK_BWD_RC(pt_attention_bwd_segs(dout.data_ptr(), q.data_ptr(), kp, vp, n, o.data_ptr(), lse.data_ptr<float>(),
                                     delta.has_value() ? delta->data_ptr<float>() : nullptr, delta_ws.data_ptr<float>(),
                                     dq_ws.data_ptr<float>(), dq.data_ptr(), part, part + per,
                                     1, seg_stride, B, Sq, (int)Sk, hq, (int)hkv, d, token_stride(q, "q"), kv_row, kv_row,

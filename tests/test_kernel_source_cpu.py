@@ -49,3 +49,18 @@ def test_the_check_sees_a_missing_and_a_conditional_fence():
     assert unfenced_accesses(wait + "tmem_st_32x32b_x32(t, r);") == [2]
     assert unfenced_accesses(wait + "if (m) { tcgen05_fence_after(); tmem_ld_32x32b_x32(t, r); }\ntmem_st_32x32b_x32(t, r);") == [3]
     assert unfenced_accesses("if (ok && mbar_wait(&b, 0, a)) {\ntcgen05_fence_after();\ntmem_ld_32x32b_x32(t, r); }") == []
+
+
+def test_a_build_with_other_register_counts_than_a_kernel_depends_on_fails():
+    from picotron_b200 import build
+    log = ("ptxas info    : Compiling entry function '_ZN2pt4attn15attn_bwd_kernelILi64ELb0ELb0EEEv' for 'sm_100a'\n"
+           "ptxas info    : Function properties for _ZN2pt4attn15attn_bwd_kernelILi64ELb0ELb0EEEv\n"
+           "    0 bytes stack frame, 0 bytes spill stores, 0 bytes spill loads\n"
+           "ptxas info    : Used {} registers, used 1 barriers\n"
+           "ptxas info    : Compiling entry function '_Z10add_kernel' for 'sm_100a'\n"
+           "ptxas info    : Used 32 registers\n")
+    build.check_registers(log.format(128))
+    with pytest.raises(RuntimeError, match="attn_bwd_kernel.*126 registers"):
+        build.check_registers(log.format(126))
+    with open(os.path.join(CSRC, "attention_tcgen05.cu")) as f:
+        assert f"BWD_REGS = {build.FIXED_REGISTERS['attn_bwd_kernel']}," in f.read()
