@@ -774,24 +774,44 @@ rmsnorm_bwd_rows_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x,
   }
 }
 
-// The smallest team whose threads hold a row with at most four chunks each: calls f(team, chunks per thread) as constants.
-// The backward of a wide row takes two chunks per thread: half the registers make room for a third CTA per SM (4096 x 2048:
-// 26.6 us with four chunks, 22.6 with two; 32768 x 2048: 119 and 104), while narrow rows are better off without barriers
-// (8192 x 576: 16.4 us with 32 threads per row, 18.5 with 64).
+// Calls f(team, chunks per thread) as constants for the forward. With many rows the smallest team whose threads hold a row with at
+// most four chunks each; with few rows a larger one, as long as its CTAs are at most four per SM, because then the latency of one
+// row's loads and sums is all there is. Measured forward / with add (us): 1803 x 576: 32 threads 3.9 / 6.1, 64 threads 2.7 / 3.7;
+// 256 x 576: 1.7 / 2.2 and with 256 threads 1.4 / 1.7; 512 x 2048: 64 threads 4.5 / 6.9, 256 threads 2.6 / 3.6; and with many rows
+// 8192 x 576: 32 threads 6.7 / 9.7, 64 threads 7.9 / 10.5.
+template <int TEAM, typename F>
+static void with_chunks(int nchunk, F f) {
+#define PT_TEAM(NC) f(std::integral_constant<int, TEAM>{}, std::integral_constant<int, NC>{})
+  if (nchunk <= TEAM) PT_TEAM(1);
+  else if (nchunk <= 2 * TEAM) PT_TEAM(2);
+  else if (nchunk <= 3 * TEAM) PT_TEAM(3);
+  else PT_TEAM(4);
+#undef PT_TEAM
+}
 template <typename F>
-static void with_team(int H, bool backward, F f) {
+static void with_forward_team(int T, int H, int num_sms, F f) {
+  const int nchunk = H / 8;
+  int team = nchunk <= 128 ? 32 : nchunk <= 256 ? 64 : nchunk <= 512 ? 128 : 256;
+  while (team < 256 && (long long)T * (2 * team) <= 4LL * num_sms * ROWS_THREADS) team *= 2;
+  if (team == 32) with_chunks<32>(nchunk, f);
+  else if (team == 64) with_chunks<64>(nchunk, f);
+  else if (team == 128) with_chunks<128>(nchunk, f);
+  else with_chunks<256>(nchunk, f);
+}
+
+// The same for the backward, whose weight-gradient sums favour few, long-lived CTAs. A wide row takes two chunks per thread: half
+// the registers make room for a third CTA per SM (4096 x 2048: 26.6 us with four chunks, 22.6 with two; 32768 x 2048: 119 and 104),
+// while narrow rows are better off without barriers (8192 x 576: 16.4 us with 32 threads per row, 18.5 with 64).
+template <typename F>
+static void with_backward_team(int H, F f) {
   const int nchunk = H / 8;
 #define PT_TEAM(TEAM, NC) f(std::integral_constant<int, TEAM>{}, std::integral_constant<int, NC>{})
   if (nchunk <= 32) PT_TEAM(32, 1);
   else if (nchunk <= 64) PT_TEAM(32, 2);
   else if (nchunk <= 96) PT_TEAM(32, 3);
   else if (nchunk <= 128) PT_TEAM(32, 4);
-  else if (backward && nchunk <= 256) PT_TEAM(128, 2);
-  else if (backward && nchunk <= 512) PT_TEAM(256, 2);
-  else if (nchunk <= 192) PT_TEAM(64, 3);
-  else if (nchunk <= 256) PT_TEAM(64, 4);
-  else if (nchunk <= 384) PT_TEAM(128, 3);
-  else if (nchunk <= 512) PT_TEAM(128, 4);
+  else if (nchunk <= 256) PT_TEAM(128, 2);
+  else if (nchunk <= 512) PT_TEAM(256, 2);
   else PT_TEAM(256, 4);
 #undef PT_TEAM
 }
@@ -800,7 +820,13 @@ extern "C" int pt_rmsnorm_fwd(const void* x, const void* delta, const void* w, v
                               int T, int H, float eps, cudaStream_t st) {
   if (H % 8 || H > 8 * ROWS_THREADS * 4) return -10;
   if (T == 0) return 0;
-  with_team(H, false, [&](auto team, auto nc) {
+  static int num_sms = 0;
+  if (num_sms == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
+  }
+  with_forward_team(T, H, num_sms, [&](auto team, auto nc) {
     constexpr int TEAM = decltype(team)::value, NC = decltype(nc)::value, ROWS = ROWS_THREADS / TEAM;
     const dim3 grid((unsigned)((T + ROWS - 1) / ROWS));
     if (delta != nullptr)
@@ -847,7 +873,7 @@ extern "C" int pt_rmsnorm_bwd_acc(const void* dy, const void* x, const void* w, 
                                   void* dx, float* dw_acc, int T, int H, int num_sms, cudaStream_t st) {
   if (H % 8 || H > 8 * ROWS_THREADS * 4 || (reinterpret_cast<uintptr_t>(dw_acc) & 15)) return 1;
   if (T == 0) return 0;
-  with_team(H, true, [&](auto team, auto nc) {
+  with_backward_team(H, [&](auto team, auto nc) {
     constexpr int TEAM = decltype(team)::value, NC = decltype(nc)::value, ROWS = ROWS_THREADS / TEAM;
     const int want = (T + ROWS - 1) / ROWS, cap = (NC <= 2 ? 3 : 2) * num_sms;
     launch_pdl(rmsnorm_bwd_rows_kernel<TEAM, NC>, dim3((unsigned)(want < cap ? want : cap)), dim3(ROWS_THREADS), 0, st,

@@ -330,10 +330,10 @@ def _row_sum_in_kernel_order(terms):
     return (((s[0] + s[1]) + (s[2] + s[3])) + (s[4] + s[5])) + (s[6] + s[7])
 
 
+@pytest.mark.parametrize("T", [16, 1000, 2500])
 @pytest.mark.parametrize("H", [576, 960, 1024, 1544, 2048, 2056, 3080, 4096, 8192])
-def test_rmsnorm_row_sums_do_not_depend_on_the_threads_per_row(C, H):
-    """Rows whose sums lose or keep whole groups of terms depending on the order of the additions."""
-    T = 16
+def test_rmsnorm_row_sums_do_not_depend_on_the_threads_per_row(C, H, T):
+    """Rows whose sums lose or keep whole groups of terms depending on the order of the additions; few rows get more threads each."""
     # forward: in chunks 0..31 one large square per chunk, behind which every following term of the same running sum vanishes
     x = torch.full((T, H), 0.95)
     x[:, :256:8] = 4096.0
@@ -342,7 +342,7 @@ def test_rmsnorm_row_sums_do_not_depend_on_the_threads_per_row(C, H):
     _, rstd = C.rmsnorm_fwd(x.cuda(), one, 1e-5)
     xn, _, rstd_add = C.add_rmsnorm_fwd(x.cuda(), torch.zeros_like(x).cuda(), one, 1e-5)
     _status_ok(C)
-    want = (_row_sum_in_kernel_order(x.float() ** 2).double() / H + 1e-5).rsqrt()
+    want = (_row_sum_in_kernel_order(x[:1].float() ** 2).double() / H + 1e-5).rsqrt().expand(T)
     # approximate division and reciprocal root: 2 ulp of 2^-24 and 2^-22.9 relative, halved and summed; the other orders are off
     # by up to 1e-6
     for r in (rstd, rstd_add):
@@ -350,15 +350,16 @@ def test_rmsnorm_row_sums_do_not_depend_on_the_threads_per_row(C, H):
     assert torch.equal(xn.cpu(), x)
     # backward: 2^30 and -2^30 in different chunks, ones elsewhere; how many ones survive is a matter of the order
     gen = torch.Generator().manual_seed(H)
-    dy = torch.ones(T, H)
-    for t in range(T):
+    dy = torch.ones(16, H)
+    for row in dy:
         a, b = torch.randperm(H, generator=gen)[:2].tolist()
-        dy[t, a], dy[t, b] = 2.0 ** 30, -2.0 ** 30
+        row[a], row[b] = 2.0 ** 30, -2.0 ** 30
+    want = (dy - (_row_sum_in_kernel_order(dy) / H)[:, None]).repeat(157, 1)[:T]
+    dy = dy.repeat(157, 1)[:T]
     # x = w = rstd = 1: dx = dy - sum(dy) / H
     dx, _ = C.rmsnorm_bwd(dy.to(torch.bfloat16).cuda(), torch.ones(T, H, device="cuda", dtype=torch.bfloat16), one,
                           torch.ones(T, device="cuda"), None)
     _status_ok(C)
-    want = dy - (_row_sum_in_kernel_order(dy) / H)[:, None]
     torch.testing.assert_close(dx.float().cpu(), want, rtol=2 ** -8, atol=2 ** -8)
 
 
