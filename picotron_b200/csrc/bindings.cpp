@@ -821,9 +821,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("set_gemm_group_m", [](int64_t g) { pt_gemm_set_group_m((int)g); },
         "CTA-pair GEMM tile numbering: rows of 256-row tiles per group (L2 locality of concurrently running tiles; default 8).");
   m.def("set_gemm_split_dgrad", [](bool on) { pt_gemm_set_split_k(on ? 1 : 0); },
-        "input- and weight-gradient GEMMs with few output tiles: K split over idle CTA pairs (default on)");
+        "input- and weight-gradient GEMMs with few output tiles: K split over idle CTA pairs (default on; for the calling thread)");
   m.def("set_gemm_tile_n", [](int64_t n) { pt_gemm_set_tile_n((int)n); },
-        "columns of the GEMM output tiles: 128, 256, or 0 for the choice by shape (bf16 outputs)");
+        "columns of the GEMM output tiles: 128, 256, or 0 for the choice by shape (bf16 outputs; for the calling thread)");
   m.def("get_gemm_group_m", []() { return (int64_t)pt_gemm_get_group_m(); });
   m.def("attention_set_profile", [](const c10::optional<Tensor>& counters) {
           if (!counters.has_value()) { pt_attention_set_profile(nullptr); return; }

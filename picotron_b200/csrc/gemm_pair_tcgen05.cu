@@ -746,8 +746,9 @@ static int num_pairs() {
   return pairs;
 }
 
-static int g_split_k = 1;
-static int g_tile_n = 0;    // 0: by the rule below, 128 / 256: as given (tests, measurements)
+// Switches for tests and measurements, of the calling thread only: other threads' launches keep the rules.
+static thread_local int g_split_k = 1;
+static thread_local int g_tile_n = 0;    // 0: by the rule below, 128 / 256: as given (tests, measurements)
 
 // Columns of an output tile (bf16 outputs). A 256 x 256 tile moves the fewest operand bytes per product, but a few hundred
 // tokens or a few hundred columns give only a handful of them for 74 CTA pairs, and then their epilogue, 256 columns one after

@@ -576,3 +576,35 @@ def test_gemm_input_gradient_with_k_split(C, T, N, K, into):
         assert _rel(C.gemm(dy, w, False, True), want) > 0.9 * _rel(y, want)       # no further off than the unsplit kernel
     finally:
         C.set_gemm_split_dgrad(True)
+
+
+def test_gemm_switches_are_those_of_the_calling_thread(C):
+    """A thread that switches the K split off for itself leaves the launches of the others as they were."""
+    import threading
+    C.set_gemm_pair(True)
+    C.set_gemm_tma_epilogue(True)
+    dy, w = bf(64, 49152, seed=1, scale=0.1), bf(49152, 576, seed=2, scale=0.1)
+
+    def launches():
+        n0 = C.launch_count()
+        C.gemm(dy, w, False, True)
+        return C.launch_count() - n0
+
+    counts = [launches()]
+    switched, looked = threading.Event(), threading.Event()
+
+    def other():
+        C.set_gemm_split_dgrad(False)
+        counts.append(launches())
+        switched.set()
+        looked.wait(60)
+        C.set_gemm_split_dgrad(True)
+
+    t = threading.Thread(target=other)
+    t.start()
+    switched.wait(60)
+    counts.append(launches())
+    looked.set()
+    t.join()
+    _status_ok(C)
+    assert counts[0] == counts[2] > counts[1] == 1
