@@ -555,9 +555,9 @@ static inline int check_launch(int n = 1) {
 // RMSNorm kernels of the training step. Bound by memory: 4 (forward), 8 (with the residual add) and 8 (backward) bytes per
 // element. A TEAM of 32, 64, 128 or 256 threads holds one row, at most 4 16-byte chunks per thread, so that a row is one batch
 // of loads, one reduction among the team's own warps and one batch of stores, and a CTA of 256 threads works on 256 / TEAM
-// independent rows. Forward: one row per team and a CTA for every 256 / TEAM rows. Backward: two CTAs per SM walk the rows; a
-// thread's columns never change, so the weight gradient is summed in registers, then over the CTA's teams in shared memory, and
-// added to the destination once per CTA.
+// independent rows. Forward: one row per team and a CTA for every 256 / TEAM rows. Backward: three CTAs per SM (two where a thread
+// holds more than two chunks) walk the rows; a thread's columns never change, so the weight gradient is summed in registers, then
+// over the CTA's teams in shared memory, and added to the destination once per CTA.
 //   forward :  x_new = x (+ delta); rstd = rsqrt(mean(x_new^2) + eps); y = x_new * rstd * w
 //   backward:  dx = rstd * (w*dy - xhat * mean(xhat*w*dy)) (+ dres);  dw_acc += sum_rows dy * xhat   (fp32 reductions)
 // H % 8 == 0, H <= 8 * 4 * TEAM. (Before, the whole CTA held four rows at a time: at H = 576 two thirds of its threads had no
