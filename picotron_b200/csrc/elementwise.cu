@@ -393,8 +393,9 @@ __global__ void add_kernel(const bf16* __restrict__ a, const bf16* __restrict__ 
 // takes up to 256 tensors (their table travels as a kernel parameter), one block one chunk of 4096 elements of one tensor,
 // found by bisection of the chunk prefix sums, so that the grid fills the chip whatever the tensors' sizes; 16-byte accesses
 // where every pointer of the tensor allows them. Clipping + AdamW of 667M parameters (two layers of the 7B shape with its
-// embedding and head): 6.64 -> 3.67 ms, 96 % of the copy rate (before: launches of at most 320 blocks, 4-byte accesses, and a
-// library multiply at 3.1 TB/s for the clipping).
+// embedding and head): 6.72 -> 4.42 ms when the gradients are scaled (42 bytes per parameter, 0.98 of the copy rate), 6.77 -> 3.69 ms
+// when there is nothing to clip (34 bytes, 0.95). (Before: launches of at most 320 blocks, 4-byte accesses, and a library multiply
+// at 3.1 TB/s for the clipping, also by 1.)
 constexpr int ADAM_MAX_TENSORS = 256;
 constexpr int ADAM_THREADS = 256;
 constexpr int ADAM_CHUNK = 4096;
@@ -562,8 +563,9 @@ static inline int check_launch(int n = 1) {
 //   backward:  dx = rstd * (w*dy - xhat * mean(xhat*w*dy)) (+ dres);  dw_acc += sum_rows dy * xhat   (fp32 reductions)
 // H % 8 == 0, H <= 8 * 4 * TEAM. (Before, the whole CTA held four rows at a time: at H = 576 two thirds of its threads had no
 // column, and every four rows waited for one CTA barrier. Measured then
-// and now, us, launch included: forward / with add / backward of 8192 x 576: 14.3 -> 12.3 / 17.1 -> 14.3 / 26.6 -> 16.4;
-// 4096 x 960: 12.3 -> 10.2 / 14.3 -> 13.2 / 20.5 -> 16.4; 4096 x 2048: 14.3 / 20.5 -> 18.4 / 24.6 -> 22.6.)
+// and now, us, launch included: forward / with add / backward of 8192 x 576: 15.2 -> 11.3 / 17.5 -> 15.0 / 27.6 -> 17.5;
+// 4096 x 960: 12.3 -> 10.2 / 14.4 / 20.6 -> 16.4; 4096 x 2048: 14.3 / 20.5 -> 18.5 / 24.6 -> 22.6; wide rows gain nothing: 4096 x
+// 4096: 20.5 -> 21.4 / 30.7 / 41.9 -> 43.0, 32768 x 2048: 56.3 -> 59.4 / 95.1 -> 94.2 / 110.6 -> 104.4.)
 // ---------------------------------------------------------------------------------------------
 constexpr int ROWS_THREADS = 256;
 
