@@ -140,7 +140,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   uint8_t* sK = sQ + Cfg::Q_BYTES;
   uint8_t* sV = sK + Cfg::STAGES * Cfg::KV_BYTES;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int num_qb = (p.Sq + Cfg::BM - 1) / Cfg::BM;
   // Work order. Causal: the heaviest query blocks of ALL heads first (longest job first), so that the last CTAs to start are
   // the lightest; head by head, the last head's heavy blocks ran alone at the end. Measured forward / backward (us): 8192 x 32
@@ -190,7 +190,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 
   if (warp == 4) {
     // ------------------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(&bars.q_full, Cfg::Q_BYTES);
 #pragma unroll
       for (int c = 0; c < Cfg::DCH; ++c) tma_load_4d(sQ + c * (Cfg::BM * 128), &tm_q, &bars.q_full, c * 64, head, q0, b);
@@ -212,7 +212,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     }
   } else if (warp == 5) {
     // ------------------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_s = make_idesc_bf16(Cfg::BM, BN, false, false);
       constexpr uint32_t idesc_o = make_idesc_bf16(Cfg::BM, D, false, true);
       bool ok = mbar_wait(&bars.q_full, 0, abort_flag);
@@ -575,7 +575,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   uint8_t* sDQ = sdS + Cfg::DS_BYTES;                                 // per drain warp two of [32 rows][32 fp32], 128B swizzle
   float* sStat = reinterpret_cast<float*>(sDQ + Cfg::DQ_BYTES);       // [stage][-lse * log2(e) | -delta * scale][128]
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int bps = (p.Sk + Cfg::BN - 1) / Cfg::BN;         // key blocks per segment
   const int num_kb = bps * p.n_segs;
   // causal: the first (heaviest) key blocks of all heads first, full attention: head by head (see the forward)
@@ -640,7 +640,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   if (warp >= 12) regs_dec<BWD_REGS_REST>();
   if (warp == 12) {
     // ------------------------------------------------------------------------------ TMA producer
-    if (lane == 0 && total_steps > 0) {
+    if (total_steps > 0 && elect_one()) {
       mbar_expect_tx(&bars.kv_full, 2 * Cfg::TILE_BYTES);
 #pragma unroll
       for (int c = 0; c < Cfg::DCH; ++c) {
@@ -665,7 +665,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     }
   } else if (warp == 13) {
     // ------------------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && total_steps > 0) {
+    if (total_steps > 0 && elect_one()) {
       constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, false, false);   // S^T, dP^T: [key, query], K-major operands
       constexpr uint32_t idesc_kv = make_idesc_bf16(128, D, false, true);     // dV, dK: A = P^T (TMEM) / dS^T (K-major), B = dO / Q (MN-major)
       constexpr uint32_t idesc_dq = make_idesc_bf16(128, D, true, true);      // dQ: A = dS^T seen as dS (MN-major), B = K (MN-major)
@@ -811,7 +811,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          if (lane == 0) tma_store_wait_read<1>();          // the reduce before the last has finished reading this buffer
+          if (elect_one()) tma_store_wait_read<1>();          // the reduce before the last has finished reading this buffer
           __syncwarp();
 #pragma unroll
           for (int u = 0; u < 8; ++u)
@@ -819,7 +819,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 make_uint4(r[h * 32 + 4 * u], r[h * 32 + 4 * u + 1], r[h * 32 + 4 * u + 2], r[h * 32 + 4 * u + 3]);
           fence_proxy_async_smem();
           __syncwarp();
-          if (lane == 0) {
+          if (elect_one()) {
             if (row0 < p.Sq) tma_reduce_add_4d(&tm_dq, stg + h * 4096, r_ * 64 + h * 32, head, row0, b);
             tma_store_commit();
           }
@@ -827,7 +827,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       }
       if (prof_on) { const long long pt2 = clock64(); pacc[0] += pt1 - pt0; pacc[1] += pt2 - pt1; }
     }
-    if (lane == 0) tma_store_wait<0>();
+    if (elect_one()) tma_store_wait<0>();
     if (prof_on) {
       atomicAdd(&p.prof[2], (unsigned long long)pacc[0]);
       atomicAdd(&p.prof[3], (unsigned long long)pacc[1]);

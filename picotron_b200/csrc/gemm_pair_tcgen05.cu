@@ -146,7 +146,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   uint8_t* smem_a = smem;
   uint8_t* smem_b = smem + STAGES * A_BYTES;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);      // (known to be the same in all lanes)
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();           // 0 = leader
   const int cluster_id = blockIdx.x >> 1;
@@ -194,7 +194,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (both CTAs)
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -239,8 +239,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       constexpr uint32_t idesc = make_idesc_bf16(2 * BM, BN, A_MN, B_MN);
+      const uint64_t a_base = make_smem_desc_sw128(smem_u32(smem_a), A_MN ? BK * 128 : 16, 1024);
+      const uint64_t b_base = make_smem_desc_sw128(smem_u32(smem_b), B_MN ? BK * 128 : 16, 1024);
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -264,16 +266,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
             break;
           }
           tcgen05_fence_after();
-          const uint32_t sa = smem_u32(smem_a + stage * A_BYTES);
-          const uint32_t sb = smem_u32(smem_b + stage * B_BYTES);
+          const uint64_t a_st = smem_desc_advance(a_base, stage * A_BYTES), b_st = smem_desc_advance(b_base, stage * B_BYTES);
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            const uint64_t a_desc = A_MN ? make_smem_desc_sw128(sa + k * (UMMA_K * 128), BK * 128, 1024)
-                                         : make_smem_desc_sw128(sa + k * (UMMA_K * 2), 16, 1024);
-            const uint64_t b_desc = B_MN ? make_smem_desc_sw128(sb + k * (UMMA_K * 128), BK * 128, 1024)
-                                         : make_smem_desc_sw128(sb + k * (UMMA_K * 2), 16, 1024);
-            umma_bf16_pair(d_tmem, a_desc, b_desc, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-          }
+          for (int k = 0; k < BK / UMMA_K; ++k)
+            umma_bf16_pair(d_tmem, smem_desc_advance(a_st, k * UMMA_K * (A_MN ? 128 : 2)), smem_desc_advance(b_st, k * UMMA_K * (B_MN ? 128 : 2)),
+                           idesc, (kb > 0 || k > 0) ? 1u : 0u);
           const uint32_t e = smem_u32(&bars.empty[stage]);
           umma_commit_pair(mapa_u32(e, 0));
           umma_commit_pair(mapa_u32(e, 1));
@@ -305,7 +302,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       // Load the second operand of chunk (tile t, c) into buffer set `set`. The previous user of that set is the chunk before
       // the current one; its TMA store, issued a moment ago, must have finished reading the buffers.
       auto issue_load = [&](int t, int c, int set) {
-        if (lane != 0) return;
+        if (!elect_one()) return;
         int m_blk, n_blk;
         tile_coords(t, num_m, num_n, ea.group_m, m_blk, n_blk);
         const int row0 = m_blk * 2 * BM + (int)rank * BM + quarter * 32;
@@ -383,7 +380,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
           }
           fence_proxy_async_smem();
           __syncwarp();
-          if (lane == 0) {
+          if (elect_one()) {
             if (row0 < M && col0 < N) {
               tma_store_2d(&tma_d, b0, col0, row0);
               if (EPI == EPI_SWIGLU_BWD) tma_store_2d(&tma_d, b0 + 4096, ea.inter + col0, row0);
@@ -395,7 +392,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&bars.tmem_empty[acc]), 0));
       }
-      if (lane == 0) tma_store_wait<0>();
+      if (elect_one()) tma_store_wait<0>();
     } else if constexpr (EPI != EPI_NONE) {
       uint8_t* stg = smem + STAGES * STAGE_BYTES + quarter * (2 * 4096);
       int buf = 0;
@@ -414,7 +411,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         const uint32_t t_row = tmem_base + (uint32_t(quarter * 32) << 16) + acc * BN;
         // 64 bf16 of this lane's row (packed in q[32]) -> swizzled staging buffer -> TMA store at (col0, row0)
         auto stage_store = [&](const uint32_t (&q)[32], const CUtensorMap* map, int col0) {
-          if (lane == 0) tma_store_wait_read<1>();        // the store issued two chunks ago has finished reading this buffer
+          if (elect_one()) tma_store_wait_read<1>();        // the store issued two chunks ago has finished reading this buffer
           __syncwarp();
           uint8_t* dst = stg + buf * 4096;
 #pragma unroll
@@ -422,7 +419,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
             *reinterpret_cast<uint4*>(dst + sw128_unit(lane, u)) = make_uint4(q[4 * u], q[4 * u + 1], q[4 * u + 2], q[4 * u + 3]);
           fence_proxy_async_smem();
           __syncwarp();
-          if (lane == 0) {
+          if (elect_one()) {
             if (row0 < M) tma_store_2d(map, dst, col0, row0);
             tma_store_commit();
           }
@@ -535,7 +532,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&bars.tmem_empty[acc]), 0));
       }
-      if (lane == 0) tma_store_wait<0>();
+      if (elect_one()) tma_store_wait<0>();
     } else if constexpr (EPI_TMA) {
       constexpr int CH_COLS = (OUT_MODE == OUT_BF16) ? 64 : 32;      // columns per 128-byte chunk row
 
@@ -569,7 +566,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
           tmem_ld_wait();
           if (c + 1 < NCH) load_chunk(c + 1, r[(c + 1) & 1]);
           const uint32_t (&v)[CH_REGS] = r[c & 1];
-          if (lane == 0) tma_store_wait_read<1>();        // the store issued two chunks ago has finished reading this buffer
+          if (elect_one()) tma_store_wait_read<1>();        // the store issued two chunks ago has finished reading this buffer
           __syncwarp();
           uint8_t* dst = stg + buf * 4096;
 #pragma unroll
@@ -587,7 +584,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
           }
           fence_proxy_async_smem();
           __syncwarp();
-          if (lane == 0) {
+          if (elect_one()) {
             const int col0 = n_blk * BN + c * CH_COLS;
             if (row0 < M && col0 < N) {
               if (OUT_MODE == OUT_F32_ACC) tma_reduce_add_2d(&tma_d, dst, col0, slice_row0 + row0);
@@ -601,7 +598,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&bars.tmem_empty[acc]), 0));
       }
-      if (lane == 0) tma_store_wait<0>();
+      if (elect_one()) tma_store_wait<0>();
     } else {
     for (int t = cluster_id; t < num_tiles && ok; t += num_clusters, ++local) {
       int m_blk, n_blk;

@@ -79,7 +79,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   uint8_t* smem_a = smem;
   uint8_t* smem_b = smem + STAGES * A_BYTES;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);      // (known to be the same in all lanes)
   const int lane = threadIdx.x & 31;
   const int num_m = (M + BM - 1) / BM;
   const int num_n = (N + BN - 1) / BN;
@@ -114,7 +114,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -153,8 +153,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = make_idesc_bf16(BM, BN, A_MN, B_MN);
+      const uint64_t a_base = make_smem_desc_sw128(smem_u32(smem_a), A_MN ? BK * 128 : 16, 1024);
+      const uint64_t b_base = make_smem_desc_sw128(smem_u32(smem_b), B_MN ? BK * 128 : 16, 1024);
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -176,16 +178,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
             break;
           }
           tcgen05_fence_after();
-          const uint32_t sa = smem_u32(smem_a + stage * A_BYTES);
-          const uint32_t sb = smem_u32(smem_b + stage * B_BYTES);
+          const uint64_t a_st = smem_desc_advance(a_base, stage * A_BYTES), b_st = smem_desc_advance(b_base, stage * B_BYTES);
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            const uint64_t a_desc = A_MN ? make_smem_desc_sw128(sa + k * (UMMA_K * 128), BK * 128, 1024)
-                                         : make_smem_desc_sw128(sa + k * (UMMA_K * 2), 16, 1024);
-            const uint64_t b_desc = B_MN ? make_smem_desc_sw128(sb + k * (UMMA_K * 128), BK * 128, 1024)
-                                         : make_smem_desc_sw128(sb + k * (UMMA_K * 2), 16, 1024);
-            umma_bf16(d_tmem, a_desc, b_desc, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-          }
+          for (int k = 0; k < BK / UMMA_K; ++k)
+            umma_bf16(d_tmem, smem_desc_advance(a_st, k * UMMA_K * (A_MN ? 128 : 2)), smem_desc_advance(b_st, k * UMMA_K * (B_MN ? 128 : 2)),
+                      idesc, (kb > 0 || k > 0) ? 1u : 0u);
           umma_commit(&bars.empty[stage]);
           if (++stage == STAGES) {
             stage = 0;
