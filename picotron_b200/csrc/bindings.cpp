@@ -19,6 +19,8 @@ int pt_gemm_bf16_fused(const void* A, const void* B, void* D, int M, int N, int 
                        int head_dim, void* status, cudaStream_t stream);
 int pt_gemm_bf16_ce(const void* A, const void* B, void* D, int M, int N, int K, long long lda, long long ldb, long long ldd,
                     const long long* targets, long long vocab_start, void* part, float* tgt, void* status, cudaStream_t stream);
+int pt_ce_finish(void* logits, const void* part, int tiles, const long long* targets, const float* tgt, float* terms, long long T,
+                 int V, long long ld, float scale, long long vocab_start, cudaStream_t st);
 int pt_ce_combine(const void* part, float* rowmax, float* sumexp, long long T, int tiles, cudaStream_t st);
 void* pt_status_word();
 void pt_attention_set_profile(unsigned long long* counters);
@@ -387,6 +389,35 @@ std::vector<Tensor> gemm_ce_stats(const Tensor& x, const Tensor& w, const Tensor
   PT_CHECK_RC(pt_ce_combine(part.data_ptr(), rowmax.data_ptr<float>(), sumexp.data_ptr<float>(), M, (int)tiles, stream()),
               "ce_combine");
   return {logits, rowmax, sumexp, tgt};
+}
+
+// LM head and cross entropy of a chunk of tokens on one GPU: loss terms (lse - target logit) -> terms[T] (fp32) and, with
+// `need_grad`, the gradient of the logits, (softmax - onehot) * scale, as the returned bf16 [T, V] tensor (without it the logits
+// are never written and the result is an empty tensor). Undefined when the fused kernel does not apply (nothing is written then).
+Tensor gemm_ce_loss(const Tensor& x, const Tensor& w, const Tensor& targets, int64_t vocab_start, double scale, Tensor& terms,
+                    bool need_grad) {
+  PT_CHECK_BF16(x); PT_CHECK_BF16(w); PT_CHECK_F32(terms);
+  TORCH_CHECK(targets.is_cuda() && targets.scalar_type() == at::kLong && targets.is_contiguous() && targets.numel() == x.size(0));
+  TORCH_CHECK(terms.is_contiguous() && terms.numel() == x.size(0), "gemm_ce_loss: terms must be a contiguous fp32 [T] tensor");
+  const long long lda = row_stride_2d(x, "x"), ldb = row_stride_2d(w, "w");
+  const int64_t M = x.size(0), K = x.size(1), N = w.size(0);
+  TORCH_CHECK(w.size(1) == K, "gemm_ce_loss: shape mismatch");
+  if (!pt_gemm_get_pair() || N % 8 != 0) return Tensor();
+  c10::cuda::CUDAGuard guard(x.device());
+  const int64_t tiles = (N + 255) / 256;
+  auto f = x.options().dtype(at::kFloat);
+  auto logits = torch::empty({need_grad ? M : 0, N}, x.options());
+  void* lp = need_grad ? logits.data_ptr() : nullptr;
+  auto part = torch::empty({M * tiles * 2 + M}, f);                      // tile pairs, then the target logits
+  float* tgt = part.data_ptr<float>() + M * tiles * 2;
+  const long long* tg = (const long long*)targets.data_ptr<int64_t>();
+  const int rc = pt_gemm_bf16_ce(x.data_ptr(), w.data_ptr(), lp, (int)M, (int)N, (int)K, lda, ldb, N, tg, vocab_start, part.data_ptr(),
+                                 tgt, pt_status_word(), stream());
+  if (rc == 1 || rc == -5) return Tensor();
+  TORCH_CHECK(rc == 0, "gemm_ce_loss failed with code ", rc);
+  PT_CHECK_RC(pt_ce_finish(lp, part.data_ptr(), (int)tiles, tg, tgt, terms.data_ptr<float>(), M, (int)N, N, (float)scale, vocab_start,
+                           stream()), "ce_finish");
+  return logits;
 }
 
 void ce_grad_(Tensor& logits, const Tensor& targets, const Tensor& lse, double scale, int64_t vocab_start) {
@@ -798,6 +829,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("embedding_fwd", &embedding_fwd);
   m.def("embedding_bwd", &embedding_bwd);
   m.def("ce_stats", &ce_stats);
+  m.def("gemm_ce_loss", &gemm_ce_loss,
+        "LM-head GEMM + cross entropy: loss terms into `terms`, gradient of the logits returned (None if not covered).");
   m.def("gemm_ce_stats", &gemm_ce_stats,
         "LM-head GEMM whose epilogue also produces the cross-entropy row statistics: [logits, rowmax, sumexp, target_logit] or [].");
   m.def("ce_grad_", &ce_grad_);

@@ -320,14 +320,57 @@ ce_stats_kernel(const bf16* __restrict__ logits, const long long* __restrict__ t
   }
 }
 
+// A row's maximum and sum of exponentials from the per-tile pairs the LM-head GEMM's epilogue left (one warp, every lane gets it).
+__device__ __forceinline__ float2 merge_tiles(const float2* __restrict__ part, int tiles) {
+  float m = -INFINITY, s = 0.f;
+  for (int t = threadIdx.x & 31; t < tiles; t += 32) {
+    const float2 p = part[t];
+    const float nm = fmaxf(m, p.x);
+    s = (nm == -INFINITY) ? 0.f : s * __expf(m - nm) + p.y * __expf(p.x - nm);
+    m = nm;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float om = __shfl_xor_sync(0xffffffffu, m, o);
+    const float os = __shfl_xor_sync(0xffffffffu, s, o);
+    const float nm = fmaxf(m, om);
+    s = (nm == -INFINITY) ? 0.f : s * __expf(m - nm) + os * __expf(om - nm);
+    m = nm;
+  }
+  return make_float2(m, s);
+}
+// log-sum-exp of a row (the logarithm in 64 bits: fast-math would take the approximate one)
+__device__ __forceinline__ float lse_of(float2 ms) { return ms.x + (float)log((double)ms.y); }
+
+// Loss terms lse - target logit from the tile pairs alone: one warp per row. A target outside [0, V) counts as logit 0, as in
+// ce_stats_kernel (the GEMM's epilogue did not write its slot).
+__global__ void __launch_bounds__(256)
+ce_loss_kernel(const float2* __restrict__ part, const long long* __restrict__ targets, const float* __restrict__ tgt,
+               float* __restrict__ terms, long long T, int tiles, int V, long long vocab_start) {
+  pdl_enter();
+  const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (row >= T) return;
+  const float z = lse_of(merge_tiles(part + row * tiles, tiles));
+  if ((threadIdx.x & 31) == 0) {
+    const long long t = targets[row] - vocab_start;
+    terms[row] = z - (t >= 0 && t < V ? tgt[row] : 0.f);
+  }
+}
+
+// In-place gradient (softmax - onehot) * scale of a row of logits per CTA; bound by reading and writing the logits. TILES: the
+// row's log-sum-exp comes straight from the tile pairs of the LM-head GEMM (each warp merges them for itself: a few hundred bytes
+// that lie in L2) and its loss term is left in `terms`, instead of from `lse`.
+template <bool TILES>
 __global__ void __launch_bounds__(CE_THREADS)
 ce_grad_kernel(bf16* __restrict__ logits, const long long* __restrict__ targets, const float* __restrict__ lse,
-               int V, long long ld, float scale, long long vocab_start) {
+               int V, long long ld, float scale, long long vocab_start, const float2* __restrict__ part, int tiles,
+               const float* __restrict__ tgt, float* __restrict__ terms) {
   pdl_enter();
   const long long row = blockIdx.x;
   bf16* l = logits + row * ld;
-  const float z = lse[row];
+  const float z = TILES ? lse_of(merge_tiles(part + row * tiles, tiles)) : lse[row];
   const long long t = targets[row] - vocab_start;
+  if (TILES && threadIdx.x == 0) terms[row] = z - (t >= 0 && t < V ? tgt[row] : 0.f);
   const int nchunk = (ld % 8 == 0) ? V / 8 : 0;
   for (int c = threadIdx.x; c < nchunk; c += CE_THREADS) {
     float v[8];
@@ -983,24 +1026,10 @@ ce_combine_kernel(const float2* __restrict__ part, float* __restrict__ rowmax, f
   const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= T) return;
-  float m = -INFINITY, s = 0.f;
-  for (int t = lane; t < tiles; t += 32) {
-    const float2 p = part[row * tiles + t];
-    const float nm = fmaxf(m, p.x);
-    s = (nm == -INFINITY) ? 0.f : s * __expf(m - nm) + p.y * __expf(p.x - nm);
-    m = nm;
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float om = __shfl_xor_sync(0xffffffffu, m, o);
-    const float os = __shfl_xor_sync(0xffffffffu, s, o);
-    const float nm = fmaxf(m, om);
-    s = (nm == -INFINITY) ? 0.f : s * __expf(m - nm) + os * __expf(om - nm);
-    m = nm;
-  }
+  const float2 ms = merge_tiles(part + row * tiles, tiles);
   if (lane == 0) {
-    rowmax[row] = m;
-    sumexp[row] = s;
+    rowmax[row] = ms.x;
+    sumexp[row] = ms.y;
   }
 }
 
@@ -1013,7 +1042,23 @@ extern "C" int pt_ce_combine(const void* part, float* rowmax, float* sumexp, lon
 extern "C" int pt_ce_grad(void* logits, const long long* targets, const float* lse, long long T, int V, long long ld,
                           float scale, long long vocab_start, cudaStream_t st) {
   if (T == 0) return 0;
-  launch_pdl(ce_grad_kernel, dim3((unsigned)T), dim3(CE_THREADS), 0, st, (bf16*)logits, targets, lse, V, ld, scale, vocab_start);
+  launch_pdl(ce_grad_kernel<false>, dim3((unsigned)T), dim3(CE_THREADS), 0, st, (bf16*)logits, targets, lse, V, ld, scale, vocab_start,
+             nullptr, 0, nullptr, nullptr);
+  return check_launch();
+}
+
+// Loss terms (lse - target logit) of T rows from the tile pairs and target logits of pt_gemm_bf16_ce; with `logits` also the in-place
+// gradient (softmax - onehot) * scale. One launch instead of the merging kernel, the logarithm, the differences, their sum and the
+// clearing of `tgt` as launches of their own.
+extern "C" int pt_ce_finish(void* logits, const void* part, int tiles, const long long* targets, const float* tgt, float* terms,
+                            long long T, int V, long long ld, float scale, long long vocab_start, cudaStream_t st) {
+  if (T == 0) return 0;
+  if (logits != nullptr)
+    launch_pdl(ce_grad_kernel<true>, dim3((unsigned)T), dim3(CE_THREADS), 0, st, (bf16*)logits, targets, nullptr, V, ld, scale,
+               vocab_start, (const float2*)part, tiles, tgt, terms);
+  else
+    launch_pdl(ce_loss_kernel, dim3((unsigned)((T + 7) / 8)), dim3(256), 0, st, (const float2*)part, targets, tgt, terms, T, tiles, V,
+               vocab_start);
   return check_launch();
 }
 

@@ -88,6 +88,7 @@ struct EpiArgs {
   const long long* ce_targets;
   long long ce_vocab_start;
   int ce_tiles;
+  int ce_store;           // 0: statistics only, the logits are not written (loss without gradient)
 };
 
 struct Barriers {
@@ -487,7 +488,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                 for (int e = 0; e < 64; ++e) tv = ((long long)(col0 + e) == tcol) ? __uint_as_float(v[e]) : tv;
                 ea.ce_tgt[row] = tv;
               }
-              stage_store(q, &tma_d, col0);
+              if (ea.ce_store) stage_store(q, &tma_d, col0);
             }
           }
           if (row < M) ea.ce_part[(long long)row * ea.ce_tiles + n_blk] = make_float2(m_run, s_run);
@@ -1034,8 +1035,9 @@ extern "C" int pt_gemm_bf16_fused(const void* A, const void* B, void* D, int M, 
 // LM-head GEMM with the cross-entropy row statistics in its epilogue: D[M, N] = A[M, K] B[N, K]^T (bf16, stored because the
 // gradient pass rewrites it in place) and, per row and per 256-column tile, (max, sum exp(logit - max)) of the stored
 // values -> part[M, tiles] (tiles = ceil(N / 256)), plus tgt[M] = logit of column targets[row] - vocab_start where that
-// column lies in [0, N) (tgt must be zero-filled by the caller: rows whose target belongs to another shard are not
-// written). Replaces the separate statistics pass over the logits. Returns 1 when the kernel does not cover the case.
+// column lies in [0, N) (rows whose target lies elsewhere are not written). Replaces the separate statistics pass over the logits.
+// D == nullptr: the statistics alone (the loss without a gradient never reads the logits again). Returns 1 when the kernel does not
+// cover the case.
 extern "C" int pt_gemm_bf16_ce(const void* A, const void* B, void* D, int M, int N, int K, long long lda, long long ldb,
                                long long ldd, const long long* targets, long long vocab_start, void* part, float* tgt,
                                void* status, cudaStream_t stream) {
@@ -1052,11 +1054,13 @@ extern "C" int pt_gemm_bf16_ce(const void* A, const void* B, void* D, int M, int
   ea.ce_targets = targets;
   ea.ce_vocab_start = vocab_start;
   ea.ce_tiles = (N + 255) / 256;
+  ea.ce_store = D != nullptr;
   CUtensorMap ma, mb, md;
   int rc;
   if ((rc = make_bf16_map_2d(&ma, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda, BK, BM))) return rc * 10 - 1;
   if ((rc = make_bf16_map_2d(&mb, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, BK, 128))) return rc * 10 - 2;
-  if ((rc = make_bf16_map_2d(&md, D, (uint64_t)N, (uint64_t)M, (uint64_t)ldd, 64, 32))) return rc * 10 - 3;
+  md = ma;                       // (not used without D)
+  if (D != nullptr && (rc = make_bf16_map_2d(&md, D, (uint64_t)N, (uint64_t)M, (uint64_t)ldd, 64, 32))) return rc * 10 - 3;
   return launch<false, false, OUT_BF16, true, EPI_CE>(ma, mb, md, D, M, N, K, ldd, reinterpret_cast<KernelStatus*>(status), stream,
                                                       &md, ea);
 }

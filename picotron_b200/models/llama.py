@@ -606,30 +606,34 @@ class LinearCrossEntropyFn(torch.autograd.Function):
             mg = getattr(weight, "main_grad", None)
             dw = None if mg is not None else torch.zeros(weight.shape, dtype=torch.float32, device=weight.device)
             acc = mg if mg is not None else dw
-        loss_sum = torch.zeros((), dtype=torch.float32, device=h.device)
         scale = float(loss_scale) / T
+        terms = torch.empty(T, dtype=torch.float32, device=h.device)       # lse - target logit of every token
         for s in range(0, T, chunk_tokens):
             e = min(T, s + chunk_tokens)
             hc, tc = h[s:e], targets[s:e]
-            logits, rowmax, sumexp, tgt = ops.linear_ce_stats(hc, weight, tc, vocab_start)   # statistics from the GEMM epilogue
-            ws = tpc.stats_workspace(tp_group, hc, rowmax.numel())
-            if ws is not None:
-                lse, tgt = ws.ce_stats_exchange(rowmax, sumexp, tgt)          # [chunk]-sized triples through peer memory
+            if tp_group is None:
+                dlogits = ops.linear_ce_loss(hc, weight, tc, vocab_start, scale, terms[s:e], need_grad)
             else:
-                if tp_group is not None:
+                dlogits, rowmax, sumexp, tgt = ops.linear_ce_stats(hc, weight, tc, vocab_start)   # statistics from the GEMM epilogue
+                ws = tpc.stats_workspace(tp_group, hc, rowmax.numel())
+                if ws is not None:
+                    lse, tgt = ws.ce_stats_exchange(rowmax, sumexp, tgt)      # [chunk]-sized triples through peer memory
+                else:
                     gmax = rowmax.clone()
                     tpc.all_reduce_(gmax, tp_group, op="max")
                     sumexp = sumexp * torch.exp(rowmax - gmax)
                     packed = torch.stack([sumexp, tgt])
                     tpc.all_reduce_(packed, tp_group)
                     sumexp, tgt, rowmax = packed[0], packed[1], gmax
-                lse = rowmax + torch.log(sumexp)
-            loss_sum += (lse - tgt).sum()
+                    lse = rowmax + torch.log(sumexp)
+                torch.sub(lse, tgt, out=terms[s:e])
+                if need_grad:
+                    ops.ce_grad_(dlogits, tc, lse, scale, vocab_start)
             if need_grad:
-                ops.ce_grad_(logits, tc, lse, scale, vocab_start)
-                ops.linear_dgrad(logits, weight, out=dh[s:e])
-                ops.linear_wgrad(logits, hc, out=acc)
-            del logits
+                ops.linear_dgrad(dlogits, weight, out=dh[s:e])
+                ops.linear_wgrad(dlogits, hc, out=acc)
+            del dlogits
+        loss_sum = terms.sum()
         if need_grad:
             if tp_group is not None:
                 tpc.all_reduce_(dh, tp_group)

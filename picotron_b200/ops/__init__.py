@@ -235,6 +235,22 @@ def linear_ce_stats(x, w, targets, vocab_start: int = 0):
     return (logits,) + tuple(ce_stats(logits, targets, vocab_start))
 
 
+def linear_ce_loss(x, w, targets, vocab_start: int, scale: float, terms, need_grad: bool):
+    """Cross entropy of ``x @ w^T`` on one GPU: writes ``lse - target_logit`` of every row to ``terms`` (fp32 ``[T]``) and returns
+    the gradient of the logits, ``(softmax - onehot) * scale``, or an empty tensor when ``need_grad`` is False.
+
+    On the GPU two kernels: the GEMM with the row statistics in its epilogue, and one pass that finishes them and rewrites the
+    logits in place; without a gradient the logits are not written at all."""
+    if _use_tc(x, w) and FUSE_GEMM_EPILOGUES:
+        r = _c().gemm_ce_loss(x, w, targets, int(vocab_start), float(scale), terms, bool(need_grad))
+        if r is not None:
+            return r
+    logits, rowmax, sumexp, tgt = linear_ce_stats(x, w, targets, vocab_start)
+    lse = rowmax + torch.log(sumexp)
+    torch.sub(lse, tgt, out=terms)
+    return ce_grad_(logits, targets, lse, scale, vocab_start) if need_grad else logits[:0]
+
+
 def ce_grad_(logits, targets, lse, scale: float, vocab_start: int = 0):
     if logits.is_cuda:
         _c().ce_grad_(logits, targets, lse, float(scale), int(vocab_start))
@@ -275,7 +291,7 @@ def merge_attention_(out, lse, block_out, block_lse):
 # ------------------------------------------------------------------ checked mode
 _CHECKED_OPS = ("rmsnorm_fwd", "add_rmsnorm_fwd", "rmsnorm_bwd", "rope_", "swiglu_fwd", "swiglu_bwd", "linear_swiglu_fwd",
                 "linear_rope_fwd", "linear_add_fwd", "linear_dgrad_swiglu_bwd", "linear_fwd", "linear_dgrad", "linear_wgrad", "attention_fwd", "attention_bwd",
-                "embedding_fwd", "embedding_bwd", "ce_stats", "linear_ce_stats", "ce_grad_", "add", "accumulate_", "scale_", "merge_attention_")
+                "embedding_fwd", "embedding_bwd", "ce_stats", "linear_ce_stats", "linear_ce_loss", "ce_grad_", "add", "accumulate_", "scale_", "merge_attention_")
 _UNCHECKED = {}
 
 

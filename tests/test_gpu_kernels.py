@@ -178,6 +178,34 @@ def test_lm_head_gemm_with_cross_entropy_statistics_epilogue(T, V, K, vocab_star
     torch.testing.assert_close(rowmax + torch.log(sumexp), lse_ref, rtol=1e-2, atol=3e-2)
 
 
+@pytest.mark.parametrize("T,V,K,vocab_start", [(1, 8, 64, 0), (300, 1000, 192, 0), (257, 8456, 128, 0), (200, 1000, 64, 1000), (64, 128256, 64, 0)])
+def test_lm_head_loss_from_two_kernels(T, V, K, vocab_start):
+    """Loss terms and in-place gradient straight from the GEMM's tile statistics (one tile, a partial last one, more tiles than lanes;
+    targets outside the shard count as logit 0), with and without the gradient, against 64-bit arithmetic on the stored logits."""
+    from picotron_b200.ops import _ext
+    C = _ext.load()
+    C.set_gemm_pair(True)
+    C.set_gemm_tma_epilogue(True)
+    x, w = bf(T, K, seed=91), bf(V, K, seed=92, scale=0.3)
+    g = torch.Generator(device="cuda").manual_seed(93)
+    targets = torch.randint(0, vocab_start + V, (T,), device="cuda", generator=g)
+    logits = C.gemm(x, w, False, False).double()
+    lse = torch.logsumexp(logits, -1)
+    col = targets - vocab_start
+    inside = (col >= 0) & (col < V)
+    hot = torch.nn.functional.one_hot(col.clamp(0, V - 1), V) * inside[:, None]
+    terms = [torch.full((T,), float("nan"), device="cuda") for _ in range(2)]
+    got = C.gemm_ce_loss(x, w, targets, vocab_start, 0.25, terms[0], True)
+    none = C.gemm_ce_loss(x, w, targets, vocab_start, 0.25, terms[1], False)
+    _status_ok(C)
+    assert none.numel() == 0 and torch.equal(terms[0], terms[1])
+    # fp32 sums of V exponentials good to 2^-22 each, and lse itself rounded to fp32: a few 1e-6 of |lse| + 1
+    want = lse - (logits * hot).sum(-1)
+    assert float(((terms[0].double() - want).abs() / (1 + lse.abs())).max()) < 5e-6
+    want = (torch.exp(logits - lse[:, None]) - hot) * 0.25
+    assert float((got.double() - want).norm() / want.norm()) < 4e-3                  # one bf16 rounding
+
+
 @pytest.mark.parametrize("T,N,K", [(256, 256, 64), (300, 328, 320), (1024, 2048, 512), (4096, 2048, 8192), (200, 72, 136)])
 def test_gemm_with_residual_add_epilogue(T, N, K):
     """Projection + residual add from one GEMM (the epilogue fetches the residual tile) against GEMM followed by the add."""
