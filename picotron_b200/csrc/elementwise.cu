@@ -237,18 +237,31 @@ __global__ void embedding_fwd_kernel(const long long* __restrict__ ids, const bf
   for (int c = threadIdx.x; c < H8; c += blockDim.x) dst[c] = ok ? src[c] : make_uint4(0, 0, 0, 0);
 }
 
-__global__ void embedding_bwd_kernel(const long long* __restrict__ ids, const bf16* __restrict__ dy,
-                                     float* __restrict__ dw, int H8, long long rows, long long vocab_start) {
+// dw[id] += dy of every token with that id. Bound by the reductions at L2 (fp32, 4 bytes a column): 16-byte ones where the destination
+// allows it. One thread per 8 columns of a token, whatever the width (a CTA per token left 184 of 256 threads idle at 576 columns).
+// 4096 x 2048 into 49152 rows: 54 us with scalar reductions, 25 us with vector ones (3.4 TB/s of the 84 MB read and reduced).
+template <bool VEC>
+__global__ void __launch_bounds__(256)
+embedding_bwd_kernel(const long long* __restrict__ ids, const bf16* __restrict__ dy, float* __restrict__ dw, long long T, int H8,
+                     long long rows, long long vocab_start) {
   pdl_enter();
-  const long long tok = blockIdx.x;
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  const long long tok = i / H8;
+  if (tok >= T) return;
+  const int c = (int)(i - tok * H8);
   const long long id = ids[tok] - vocab_start;
   if (id < 0 || id >= rows) return;
-  float* dst = dw + id * (long long)(H8 * 8);
-  for (int c = threadIdx.x; c < H8; c += blockDim.x) {
-    float v[8];
-    unpack8(*reinterpret_cast<const bf16x8*>(dy + tok * (long long)(H8 * 8) + c * 8), v);
+  float* dst = dw + (id * H8 + c) * 8;
+  float v[8];
+  unpack8(*reinterpret_cast<const bf16x8*>(dy + i * 8), v);
+  if (VEC) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) atomicAdd(dst + c * 8 + j, v[j]);
+    for (int j = 0; j < 8; j += 4)
+      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + j), "f"(v[j]), "f"(v[j + 1]), "f"(v[j + 2]), "f"(v[j + 3])
+                   : "memory");
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) atomicAdd(dst + j, v[j]);
   }
 }
 
@@ -1007,7 +1020,11 @@ extern "C" int pt_embedding_bwd(const long long* ids, const void* dy, float* dw,
                                 long long vocab_start, cudaStream_t st) {
   if (H % 8) return -10;
   if (T == 0) return 0;
-  launch_pdl(embedding_bwd_kernel, dim3((unsigned)T), dim3(256), 0, st, ids, (const bf16*)dy, dw, H / 8, rows, vocab_start);
+  const dim3 grid((unsigned)((T * (H / 8) + 255) / 256));
+  if ((reinterpret_cast<uintptr_t>(dw) & 15) == 0)
+    launch_pdl(embedding_bwd_kernel<true>, grid, dim3(256), 0, st, ids, (const bf16*)dy, dw, T, H / 8, rows, vocab_start);
+  else
+    launch_pdl(embedding_bwd_kernel<false>, grid, dim3(256), 0, st, ids, (const bf16*)dy, dw, T, H / 8, rows, vocab_start);
   return check_launch();
 }
 

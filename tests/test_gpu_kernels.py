@@ -444,6 +444,20 @@ def test_embedding_fwd_bwd_with_vocab_shard(C):
     torch.testing.assert_close(dw, want, rtol=1e-4, atol=1e-4)
 
 
+@pytest.mark.parametrize("T,H,off", [(1, 8, 0), (37, 576, 0), (300, 2056, 0), (37, 576, 1)])
+def test_embedding_backward_of_repeated_ids_and_any_alignment(C, T, H, off):
+    """Rows hit by many tokens, widths that fill no block, and a gradient that does not start on 16 bytes (scalar additions)."""
+    ids = torch.arange(T, device="cuda") % 5 * 7
+    dy = bf(T, H, seed=3)
+    dw = torch.ones(40 * H + off, device="cuda")[off:].view(40, H)
+    C.embedding_bwd(ids, dy, dw, 0)
+    want = torch.ones(40, H, device="cuda", dtype=torch.float64)
+    want.index_add_(0, ids, dy.double())
+    _status_ok(C)
+    # sums of at most 60 bf16 values of size ~1 in fp32, in any order
+    torch.testing.assert_close(dw.double(), want, rtol=0, atol=60 * 2.0 ** -20)
+
+
 @pytest.mark.parametrize("V,start", [(1000, 0), (4096, 4096), (50257, 0)])
 def test_cross_entropy_stats_and_grad(C, V, start):
     T = 64
