@@ -5,6 +5,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
+#include <algorithm>
 #include <vector>
 
 using torch::Tensor;
@@ -285,6 +286,30 @@ Tensor gemm_dgrad_swiglu_bwd(const Tensor& dy, const Tensor& w, const Tensor& gu
   return dgu;
 }
 
+// D = op(A) op(B) on raw operands (pt_gemm_bf16). Input gradients and weight gradients with few output tiles: K in parts
+// (pt_gemm_split_parts), through a workspace from the caching allocator.
+void gemm_into(const void* a, const void* b, void* d, int64_t M, int64_t N, int64_t K, long long lda, long long ldb, long long ldd,
+               bool trans_a, bool trans_b, int mode, const at::TensorOptions& on) {
+  const bool grad = (mode == 0 && !trans_a && trans_b) || (mode == 1 && trans_a && trans_b);
+  if (grad && pt_gemm_get_pair() && pt_gemm_get_tma_epilogue() && lda % 8 == 0 && ldb % 8 == 0 && ldd % (mode == 0 ? 8 : 4) == 0 &&
+      (((uintptr_t)a | (uintptr_t)b | (uintptr_t)d) & 15) == 0) {
+    const int parts = pt_gemm_split_parts((int)M, (int)N, (int)K, mode);
+    if (parts > 1) {
+      auto ws = torch::empty({pt_gemm_split_elems((int)M, (int)N, (int)K, mode, parts)}, on.dtype(at::kFloat));
+      const int rc = pt_gemm_bf16_split(a, b, d, ws.data_ptr<float>(), (int)M, (int)N, (int)K, lda, ldb, ldd, trans_a ? 1 : 0,
+                                        trans_b ? 1 : 0, mode, parts, pt_status_word(), stream());
+      if (rc != -5) {                                    // (CTA pairs cannot be scheduled: the general path below)
+        TORCH_CHECK(rc == 0, "gemm (split) failed with code ", rc);
+        return;
+      }
+    }
+  }
+  const int rc = pt_gemm_bf16(a, b, d, (int)M, (int)N, (int)K, lda, ldb, ldd, trans_a ? 1 : 0, trans_b ? 1 : 0, mode, num_sms(), stream());
+  TORCH_CHECK(rc == 0, "gemm failed with code ", rc, " (M=", M, " N=", N, " K=", K, " lda=", lda, " ldb=", ldb, " ldd=", ldd,
+              " trans_a=", trans_a, " trans_b=", trans_b, " mode=", mode, " a%16=", (uintptr_t)a % 16, " b%16=", (uintptr_t)b % 16,
+              " d%16=", (uintptr_t)d % 16, ")");
+}
+
 // D = op(a) op(b); see pt_gemm_bf16. trans_a: a is [K,M]; trans_b: b is [K,N] (else [N,K]).
 Tensor gemm(const Tensor& a, const Tensor& b, bool trans_a, bool trans_b, const c10::optional<Tensor>& out,
             bool accumulate) {
@@ -306,28 +331,7 @@ Tensor gemm(const Tensor& a, const Tensor& b, bool trans_a, bool trans_b, const 
     d = torch::empty({M, N}, a.options());
     mode = 0;
   }
-  const long long ldd = row_stride_2d(d, "out");
-  // input gradients and weight gradients with few output tiles: K in parts (pt_gemm_split_parts)
-  const bool grad = (mode == 0 && !trans_a && trans_b) || (mode == 1 && trans_a && trans_b);
-  if (grad && pt_gemm_get_pair() && pt_gemm_get_tma_epilogue() && lda % 8 == 0 && ldb % 8 == 0 && ldd % (mode == 0 ? 8 : 4) == 0 &&
-      (((uintptr_t)a.data_ptr() | (uintptr_t)b.data_ptr() | (uintptr_t)d.data_ptr()) & 15) == 0) {
-    const int parts = pt_gemm_split_parts((int)M, (int)N, (int)K, mode);
-    if (parts > 1) {
-      auto ws = torch::empty({pt_gemm_split_elems((int)M, (int)N, (int)K, mode, parts)}, a.options().dtype(at::kFloat));
-      const int rc = pt_gemm_bf16_split(a.data_ptr(), b.data_ptr(), d.data_ptr(), ws.data_ptr<float>(), (int)M, (int)N, (int)K, lda,
-                                        ldb, ldd, trans_a ? 1 : 0, trans_b ? 1 : 0, mode, parts, pt_status_word(), stream());
-      if (rc != -5) {                                    // (CTA pairs cannot be scheduled: the general path below)
-        TORCH_CHECK(rc == 0, "gemm (split) failed with code ", rc);
-        return d;
-      }
-    }
-  }
-  const int rc = pt_gemm_bf16(a.data_ptr(), b.data_ptr(), d.data_ptr(), (int)M, (int)N, (int)K, lda, ldb, ldd,
-                              trans_a ? 1 : 0, trans_b ? 1 : 0, mode, num_sms(), stream());
-  TORCH_CHECK(rc == 0, "gemm failed with code ", rc, " (M=", M, " N=", N, " K=", K, " lda=", lda, " ldb=", ldb, " ldd=", ldd,
-              " trans_a=", trans_a, " trans_b=", trans_b, " mode=", mode, " a%16=", (uintptr_t)a.data_ptr() % 16,
-              " b%16=", (uintptr_t)b.data_ptr() % 16, " d%16=", (uintptr_t)d.data_ptr() % 16, " dev=", (int)a.device().index(), " a_ptr=", (uintptr_t)a.data_ptr(),
-              " b_ptr=", (uintptr_t)b.data_ptr(), " a_storage_bytes=", (int64_t)a.storage().nbytes(), ")");
+  gemm_into(a.data_ptr(), b.data_ptr(), d.data_ptr(), M, N, K, lda, ldb, row_stride_2d(d, "out"), trans_a, trans_b, mode, a.options());
   return d;
 }
 
@@ -573,17 +577,43 @@ std::vector<Tensor> attention_bwd(const Tensor& dout, const Tensor& q, const Ten
 
 // ---------------------------------------------------------------------------------------------
 // A decoder layer's launches in one call (one GPU per layer: no tensor, sequence or context parallelism). Small models and
-// short sequences are bound by the host: from Python every launch costs 12 to 20 us, more than most of their kernels take.
-// The kernels, their order and the fallbacks are those of the layer node's Python path.
+// short sequences are bound by the host: from Python every launch costs 12 to 20 us, more than most of their kernels take, and with
+// a tensor object per operand one native call still took 75 us per layer, half of it allocations, views and tensor bookkeeping.
+// So what the backward needs lies in TWO allocations (bf16 and fp32), addressed by offsets. The kernels, their order and the
+// fallbacks are those of the layer node's Python path.
 // ---------------------------------------------------------------------------------------------
 struct LayerDims {
-  int64_t B, S, hq, hkv, d;
+  int64_t B, S, H, I, hq, hkv, d;
+  int64_t T() const { return B * S; }
+  int64_t O() const { return hq * d; }                   // columns of the attention output
+  int64_t Q() const { return (hq + 2 * hkv) * d; }       // columns of the packed qkv activation
 };
 
-std::vector<Tensor> split_qkv(const Tensor& qkv, const LayerDims& n) {
-  return {qkv.narrow(1, 0, n.hq * n.d).view({n.B, n.S, n.hq, n.d}),
-          qkv.narrow(1, n.hq * n.d, n.hkv * n.d).view({n.B, n.S, n.hkv, n.d}),
-          qkv.narrow(1, (n.hq + n.hkv) * n.d, n.hkv * n.d).view({n.B, n.S, n.hkv, n.d})};
+// Element offsets of the parts of a layer's saved activations, each on a 256-byte (bf16) boundary.
+struct LayerSaved {
+  int64_t h1, qkv, o, x_mid, h2, gu, a, total, rstd1, rstd2, lse, total32;
+  explicit LayerSaved(const LayerDims& n) {
+    int64_t at = 0;
+    auto take = [&at](int64_t elems) { const int64_t here = at; at += (elems + 127) / 128 * 128; return here; };
+    const int64_t T = n.T();
+    h1 = take(T * n.H); qkv = take(T * n.Q()); o = take(T * n.O()); x_mid = take(T * n.H); h2 = take(T * n.H); gu = take(T * 2 * n.I);
+    a = take(T * n.I); total = at;
+    at = 0;
+    rstd1 = take(T); rstd2 = take(T); lse = take(T * n.hq); total32 = at;
+  }
+};
+
+// The saved activations as tensors {rstd1, h1, qkv, o, lse, x_mid, rstd2, h2, gu, a} (views; for callers that work on tensors).
+std::vector<Tensor> decoder_layer_saved(const Tensor& s16, const Tensor& s32, int64_t B, int64_t S, int64_t H, int64_t I, int64_t hq,
+                                        int64_t hkv, int64_t d) {
+  const LayerDims n{B, S, H, I, hq, hkv, d};
+  const LayerSaved at(n);
+  TORCH_CHECK(s16.numel() == at.total && s32.numel() == at.total32, "decoder_layer_saved: sizes do not match");
+  const int64_t T = n.T();
+  auto part = [T](const Tensor& t, int64_t off, int64_t cols) { return t.narrow(0, off, T * cols).view({T, cols}); };
+  return {s32.narrow(0, at.rstd1, T), part(s16, at.h1, H), part(s16, at.qkv, n.Q()), part(s16, at.o, n.O()),
+          s32.narrow(0, at.lse, T * hq).view({B, hq, S}), part(s16, at.x_mid, H), s32.narrow(0, at.rstd2, T), part(s16, at.h2, H),
+          part(s16, at.gu, 2 * I), part(s16, at.a, I)};
 }
 
 bool all_bf16_cuda(std::initializer_list<const Tensor*> ts) {
@@ -592,78 +622,170 @@ bool all_bf16_cuda(std::initializer_list<const Tensor*> ts) {
   return true;
 }
 
-// Returns {x_out, h1, rstd1, qkv, o, lse, x_mid, rstd2, h2, gu, a}, or {} (nothing launched) for operands that are not bf16.
+// Weights and tables of a layer: shapes and layouts that the kernels rely on.
+void check_layer(const LayerDims& n, const Tensor& ln1, const Tensor& w_qkv, const Tensor& cosT, const Tensor& sinT, const Tensor& wo,
+                 const Tensor& ln2, const Tensor& w_gu, const Tensor& wd) {
+  auto matrix = [](const Tensor& t, int64_t rows, int64_t cols) {
+    return t.dim() == 2 && t.size(0) == rows && t.size(1) == cols && (cols == 1 || t.stride(1) == 1);
+  };
+  TORCH_CHECK(matrix(w_qkv, n.Q(), n.H) && matrix(wo, n.H, n.O()) && matrix(w_gu, 2 * n.I, n.H) && matrix(wd, n.H, n.I) &&
+              ln1.numel() == n.H && ln2.numel() == n.H && ln1.is_contiguous() && ln2.is_contiguous(), "decoder layer: weight shapes");
+  PT_CHECK_F32(cosT); PT_CHECK_F32(sinT);
+  TORCH_CHECK(cosT.is_contiguous() && cosT.dim() == 2 && cosT.size(0) >= n.S && cosT.size(1) == n.d / 2 && sinT.is_contiguous() &&
+              sinT.sizes() == cosT.sizes(), "decoder layer: rope tables must be fp32 [S, d/2] with S >= the sequence length");
+}
+
+using bf16_t = at::BFloat16;
+inline bf16_t* bf16_ptr(const Tensor& t) { return reinterpret_cast<bf16_t*>(t.data_ptr()); }
+inline bool fused_gemm(int rc, const char* what) {          // false: not covered, nothing launched
+  if (rc == 1 || rc == -5) return false;
+  TORCH_CHECK(rc == 0, what, " failed with code ", rc);
+  return true;
+}
+
+// Returns {x_out, saved bf16, saved fp32} (LayerSaved), or {} (nothing launched) for operands that are not bf16.
 std::vector<Tensor> decoder_layer_fwd(const Tensor& x, const Tensor& ln1, const Tensor& w_qkv, const Tensor& cosT, const Tensor& sinT,
                                       const Tensor& wo, const Tensor& ln2, const Tensor& w_gu, const Tensor& wd, double eps, int64_t B,
                                       int64_t S, int64_t hq, int64_t hkv, int64_t d, double scale) {
   if (!all_bf16_cuda({&x, &ln1, &w_qkv, &wo, &ln2, &w_gu, &wd})) return {};
-  const LayerDims n{B, S, hq, hkv, d};
-  auto n1 = rmsnorm_fwd(x, ln1, eps);
-  Tensor qkv = gemm_rope(n1[0], w_qkv, cosT, sinT, hq + hkv, d, S);
-  if (!qkv.defined()) {
-    qkv = gemm(n1[0], w_qkv, false, false, c10::nullopt, false);
-    rope_(qkv, cosT, sinT, hq + hkv, d, S, false);
+  TORCH_CHECK(x.dim() == 2 && x.is_contiguous() && x.size(0) == B * S && w_gu.dim() == 2 && hq % hkv == 0);
+  const LayerDims n{B, S, x.size(1), w_gu.size(0) / 2, hq, hkv, d};
+  check_layer(n, ln1, w_qkv, cosT, sinT, wo, ln2, w_gu, wd);
+  const LayerSaved at(n);
+  const int64_t T = n.T(), H = n.H, I = n.I, O = n.O(), Q = n.Q();
+  c10::cuda::CUDAGuard guard(x.device());
+  const auto on = x.options();
+  Tensor s16 = torch::empty({at.total}, on), s32 = torch::empty({at.total32}, on.dtype(at::kFloat)), out = torch::empty({T, H}, on);
+  bf16_t* const b = bf16_ptr(s16);
+  float* const f = s32.data_ptr<float>();
+  bf16_t *const h1 = b + at.h1, *const qkv = b + at.qkv, *const o = b + at.o, *const x_mid = b + at.x_mid, *const h2 = b + at.h2,
+         *const gu = b + at.gu, *const a = b + at.a;
+  const float *const cosp = cosT.data_ptr<float>(), *const sinp = sinT.data_ptr<float>();
+  const long long ld_qkv = row_stride_2d(w_qkv, "w_qkv"), ld_o = row_stride_2d(wo, "wo"), ld_gu = row_stride_2d(w_gu, "w_gu"),
+                  ld_d = row_stride_2d(wd, "wd");
+  const cudaStream_t st = stream();
+  const bool pair = pt_gemm_get_pair();
+  void* const status = pt_status_word();
+  PT_CHECK_RC(pt_rmsnorm_fwd(x.data_ptr(), nullptr, ln1.data_ptr(), nullptr, h1, f + at.rstd1, (int)T, (int)H, (float)eps, st), "rmsnorm_fwd");
+  if (!(pair && Q % 8 == 0 &&
+        fused_gemm(pt_gemm_bf16_fused(h1, w_qkv.data_ptr(), qkv, (int)T, (int)Q, (int)H, H, ld_qkv, Q, 2, nullptr, 0, 0, cosp, sinp, (int)S,
+                                      (int)(hq + hkv), (int)d, status, st), "gemm_rope"))) {
+    gemm_into(h1, w_qkv.data_ptr(), qkv, T, Q, H, H, ld_qkv, Q, false, false, 0, on);
+    PT_CHECK_RC(pt_rope(qkv, cosp, sinp, T, (int)(hq + hkv), (int)d, (int)S, Q, 0, st), "rope");
   }
-  auto parts = split_qkv(qkv, n);
-  auto att = attention_fwd(parts[0], parts[1], parts[2], true, scale);
-  const Tensor o2 = att[0].view({B * S, hq * d});
-  auto n2 = add_rmsnorm_fwd(x, gemm(o2, wo, false, false, c10::nullopt, false), ln2, eps);      // {x_mid, h2, rstd2}
-  auto mlp = gemm_swiglu(n2[1], w_gu);
-  if (mlp.empty()) {
-    Tensor gu = gemm(n2[1], w_gu, false, false, c10::nullopt, false);
-    mlp = {gu, swiglu_fwd(gu)};
+  PT_CHECK_RC(pt_attention_fwd(qkv, qkv + O, qkv + O + hkv * d, o, f + at.lse, (int)B, (int)S, (int)S, (int)hq, (int)hkv, (int)d, Q, Q, Q, 1,
+                               (float)scale, st), "attention_fwd");
+  gemm_into(o, wo.data_ptr(), out.data_ptr(), T, H, O, O, ld_o, H, false, false, 0, on);     // (`out` is free until the down projection)
+  PT_CHECK_RC(pt_rmsnorm_fwd(x.data_ptr(), out.data_ptr(), ln2.data_ptr(), x_mid, h2, f + at.rstd2, (int)T, (int)H, (float)eps, st),
+              "add_rmsnorm_fwd");
+  if (!(pair && I % 128 == 0 &&
+        fused_gemm(pt_gemm_bf16_fused(h2, w_gu.data_ptr(), gu, (int)T, (int)(2 * I), (int)H, H, ld_gu, 2 * I, 1, a, I, (int)I, nullptr, nullptr,
+                                      0, 0, 0, status, st), "gemm_swiglu"))) {
+    gemm_into(h2, w_gu.data_ptr(), gu, T, 2 * I, H, H, ld_gu, 2 * I, false, false, 0, on);
+    PT_CHECK_RC(pt_swiglu_fwd(gu, a, T, (int)I, st), "swiglu_fwd");
   }
-  Tensor out = gemm_add(mlp[1], wd, n2[0]);
-  if (!out.defined()) out = ::add(n2[0], gemm(mlp[1], wd, false, false, c10::nullopt, false));
-  return {out, n1[0], n1[1], qkv, o2, att[1], n2[0], n2[2], n2[1], mlp[0], mlp[1]};
+  if (!(pair && H % 8 == 0 &&
+        fused_gemm(pt_gemm_bf16_fused(a, wd.data_ptr(), out.data_ptr(), (int)T, (int)H, (int)I, I, ld_d, H, 4, x_mid, H, 0, nullptr, nullptr, 0,
+                                      0, 0, status, st), "gemm_add"))) {
+    Tensor y = torch::empty({T, H}, on);
+    gemm_into(a, wd.data_ptr(), y.data_ptr(), T, H, I, I, ld_d, H, false, false, 0, on);
+    PT_CHECK_RC(pt_add(x_mid, y.data_ptr(), out.data_ptr(), T * H, st), "add");
+  }
+  return {out, s16, s32};
 }
 
-// The fp32 regions of parameters that one GEMM accumulates into together, as one [rows, cols] tensor; undefined unless they
-// are adjacent in one storage.
-Tensor packed_region(const std::vector<Tensor>& parts) {
-  const Tensor& f = parts[0];
-  int64_t rows = 0;
-  for (const Tensor& t : parts) {
-    if (t.dim() != 2 || !t.is_contiguous() || t.size(1) != f.size(1) || t.scalar_type() != at::kFloat || !t.is_cuda() ||
-        t.storage().data() != f.storage().data() || t.storage_offset() != f.storage_offset() + rows * f.size(1))
-      return Tensor();
-    rows += t.size(0);
+// The fp32 regions of parameters that one GEMM accumulates into together, as one [rows, cols] region: its address, or nullptr unless
+// they are adjacent in one storage.
+float* packed_region(const std::vector<Tensor>& mg, int first, int count, int64_t rows, int64_t cols) {
+  const Tensor& f = mg[first];
+  int64_t seen = 0;
+  for (int i = first; i < first + count; ++i) {
+    const Tensor& t = mg[i];
+    if (t.dim() != 2 || !t.is_contiguous() || t.size(1) != cols || t.scalar_type() != at::kFloat || !t.is_cuda() ||
+        t.storage().data() != f.storage().data() || t.storage_offset() != f.storage_offset() + seen * cols)
+      return nullptr;
+    seen += t.size(0);
   }
-  return parts.size() == 1 ? f : f.as_strided({rows, f.size(1)}, {f.size(1), 1}, f.storage_offset());
+  TORCH_CHECK(seen == rows, "decoder layer: shape of a gradient region");
+  return f.data_ptr<float>();
+}
+
+// dx of an RMSNorm (+ dres); the weight gradient is added to dw (fp32 [H]).
+void rmsnorm_bwd_into(const void* dy, const void* x, const Tensor& w, const float* rstd, const void* dres, void* dx, const Tensor& dw,
+                      int64_t T, int64_t H, const at::TensorOptions& on) {
+  const int rc = pt_rmsnorm_bwd_acc(dy, x, w.data_ptr(), rstd, dres, dx, dw.data_ptr<float>(), (int)T, (int)H, num_sms(), stream());
+  if (rc == 0) return;
+  TORCH_CHECK(rc == 1, "rmsnorm_bwd failed with code ", rc);
+  auto dw_new = torch::empty({H}, on.dtype(at::kFloat));
+  auto partial = torch::empty({pt_rmsnorm_bwd_partial_rows((int)T, num_sms()), H}, on.dtype(at::kFloat));
+  PT_CHECK_RC(pt_rmsnorm_bwd(dy, x, w.data_ptr(), rstd, dres, dx, dw_new.data_ptr<float>(), partial.data_ptr<float>(), (int)T, (int)H,
+                             num_sms(), stream()), "rmsnorm_bwd");
+  PT_CHECK_RC(pt_accumulate(dw.data_ptr<float>(), dw_new.data_ptr(), H, 1, stream()), "accumulate");
 }
 
 // Backward of decoder_layer_fwd; the weight gradients are added to the fp32 regions `mg` (q, k, v, out, gate, up, down, norm 1,
-// norm 2). `saved` = {x, rstd1, h1, qkv, o, lse, x_mid, rstd2, h2, gu, a}. Returns dx, or an undefined tensor (nothing launched).
-Tensor decoder_layer_bwd(const Tensor& dout, const std::vector<Tensor>& saved, const Tensor& ln1, const Tensor& w_qkv,
+// norm 2). x and {s16, s32}: the forward's input and saved activations. Returns dx, or an undefined tensor (nothing launched).
+Tensor decoder_layer_bwd(const Tensor& dout, const Tensor& x, const Tensor& s16, const Tensor& s32, const Tensor& ln1, const Tensor& w_qkv,
                          const Tensor& cosT, const Tensor& sinT, const Tensor& wo, const Tensor& ln2, const Tensor& w_gu,
                          const Tensor& wd, const std::vector<Tensor>& mg, int64_t B, int64_t S, int64_t hq, int64_t hkv, int64_t d,
                          double scale) {
-  TORCH_CHECK(saved.size() == 11 && mg.size() == 9);
-  if (!all_bf16_cuda({&dout, &ln1, &w_qkv, &wo, &ln2, &w_gu, &wd})) return Tensor();
-  const Tensor mg_qkv = packed_region({mg[0], mg[1], mg[2]}), mg_o = packed_region({mg[3]}), mg_gu = packed_region({mg[4], mg[5]}),
-               mg_d = packed_region({mg[6]});
-  if (!mg_qkv.defined() || !mg_o.defined() || !mg_gu.defined() || !mg_d.defined()) return Tensor();
+  TORCH_CHECK(mg.size() == 9);
+  if (!all_bf16_cuda({&dout, &x, &s16, &ln1, &w_qkv, &wo, &ln2, &w_gu, &wd})) return Tensor();
+  TORCH_CHECK(x.dim() == 2 && x.is_contiguous() && x.size(0) == B * S && dout.is_contiguous() && dout.sizes() == x.sizes() &&
+              w_gu.dim() == 2 && hq % hkv == 0);
+  const LayerDims n{B, S, x.size(1), w_gu.size(0) / 2, hq, hkv, d};
+  const int64_t T = n.T(), H = n.H, I = n.I, O = n.O(), Q = n.Q();
+  float *const mg_qkv = packed_region(mg, 0, 3, Q, H), *const mg_o = packed_region(mg, 3, 1, H, O),
+        *const mg_gu = packed_region(mg, 4, 2, 2 * I, H), *const mg_d = packed_region(mg, 6, 1, H, I);
+  if (mg_qkv == nullptr || mg_o == nullptr || mg_gu == nullptr || mg_d == nullptr) return Tensor();
   for (int i = 7; i < 9; ++i)
-    if (!mg[i].is_cuda() || mg[i].scalar_type() != at::kFloat || !mg[i].is_contiguous()) return Tensor();
-  const Tensor &x = saved[0], &rstd1 = saved[1], &h1 = saved[2], &qkv = saved[3], &o2 = saved[4], &lse = saved[5], &x_mid = saved[6],
-               &rstd2 = saved[7], &h2 = saved[8], &gu = saved[9], &a = saved[10];
-  const LayerDims n{B, S, hq, hkv, d};
-  Tensor dgu = gemm_dgrad_swiglu_bwd(dout, wd, gu);
-  if (!dgu.defined()) dgu = swiglu_bwd(gu, gemm(dout, wd, false, true, c10::nullopt, false));
-  gemm(dout, a, true, true, mg_d, true);
-  Tensor dh = gemm(dgu, w_gu, false, true, c10::nullopt, false);
-  gemm(dgu, h2, true, true, mg_gu, true);
-  dgu = Tensor();
-  const Tensor dx_mid = rmsnorm_bwd(dh, x_mid, ln2, rstd2, dout, mg[8])[0];
-  dh = gemm(dx_mid, wo, false, true, c10::nullopt, false);                     // dL/d(attention output)
-  gemm(dx_mid, o2, true, true, mg_o, true);
-  auto parts = split_qkv(qkv, n);
-  Tensor dqkv = torch::empty_like(qkv);
-  attention_bwd(dh.view({B, S, hq, d}), parts[0], parts[1], parts[2], o2.view({B, S, hq, d}), lse, true, scale, c10::nullopt,
-                split_qkv(dqkv, n), cosT, sinT);
-  dh = gemm(dqkv, w_qkv, false, true, c10::nullopt, false);
-  gemm(dqkv, h1, true, true, mg_qkv, true);
-  return rmsnorm_bwd(dh, x, ln1, rstd1, dx_mid, mg[7])[0];
+    if (!mg[i].is_cuda() || mg[i].scalar_type() != at::kFloat || !mg[i].is_contiguous() || mg[i].numel() != H) return Tensor();
+  check_layer(n, ln1, w_qkv, cosT, sinT, wo, ln2, w_gu, wd);
+  const LayerSaved at(n);
+  PT_CHECK_F32(s32);
+  TORCH_CHECK(s16.is_contiguous() && s16.numel() == at.total && s32.is_contiguous() && s32.numel() == at.total32,
+              "decoder layer: saved activations of another shape");
+  c10::cuda::CUDAGuard guard(x.device());
+  const auto on = x.options();
+  const bf16_t* const b = bf16_ptr(s16);
+  const float* const f = s32.data_ptr<float>();
+  const bf16_t *const h1 = b + at.h1, *const qkv = b + at.qkv, *const o = b + at.o, *const x_mid = b + at.x_mid, *const h2 = b + at.h2,
+               *const gu = b + at.gu, *const a = b + at.a;
+  // One scratch allocation (bytes): dgu, whose place the attention's gradients take when it is done with; the normed inputs' gradients
+  // (dh); dx_mid.
+  auto up = [](int64_t bytes) { return (bytes + 255) / 256 * 256; };
+  const int64_t b_dgu = up(4 * T * I), b_do = up(2 * T * O), b_dqkv = up(2 * T * Q), b_dq = up(4 * T * O), b_delta = up(4 * T * hq), b_h = up(2 * T * H);
+  const int64_t b_first = std::max(b_dgu, b_do + b_dqkv + b_dq + b_delta);
+  Tensor scratch = torch::empty({b_first + 2 * b_h}, on.dtype(at::kByte)), dx = torch::empty({T, H}, on);
+  char* const s = reinterpret_cast<char*>(scratch.data_ptr());
+  void *const dgu = s, *const dO = s, *const dq_ws = s + b_do + b_dqkv, *const delta = s + b_do + b_dqkv + b_dq;
+  bf16_t* const dqkv = reinterpret_cast<bf16_t*>(s + b_do);
+  void *const dh = s + b_first, *const dx_mid = s + b_first + b_h;
+  const long long ld_qkv = row_stride_2d(w_qkv, "w_qkv"), ld_o = row_stride_2d(wo, "wo"), ld_gu = row_stride_2d(w_gu, "w_gu"),
+                  ld_d = row_stride_2d(wd, "wd");
+  const cudaStream_t st = stream();
+
+  if (!(pt_gemm_get_pair() && I % 64 == 0 &&
+        fused_gemm(pt_gemm_bf16_fused(dout.data_ptr(), wd.data_ptr(), dgu, (int)T, (int)I, (int)H, H, ld_d, 2 * I, 5, const_cast<bf16_t*>(gu), 2 * I,
+                                      (int)I, nullptr, nullptr, 0, 0, 0, pt_status_word(), st), "gemm_dgrad_swiglu_bwd"))) {
+    Tensor da = torch::empty({T, I}, on);
+    gemm_into(dout.data_ptr(), wd.data_ptr(), da.data_ptr(), T, I, H, H, ld_d, I, false, true, 0, on);
+    PT_CHECK_RC(pt_swiglu_bwd(gu, da.data_ptr(), dgu, T, (int)I, st), "swiglu_bwd");
+  }
+  gemm_into(dout.data_ptr(), a, mg_d, H, I, T, H, I, I, true, true, 1, on);
+  gemm_into(dgu, w_gu.data_ptr(), dh, T, H, 2 * I, 2 * I, ld_gu, H, false, true, 0, on);
+  gemm_into(dgu, h2, mg_gu, 2 * I, H, T, 2 * I, H, H, true, true, 1, on);
+  rmsnorm_bwd_into(dh, x_mid, ln2, f + at.rstd2, dout.data_ptr(), dx_mid, mg[8], T, H, on);
+  gemm_into(dx_mid, wo.data_ptr(), dO, T, O, H, H, ld_o, O, false, true, 0, on);             // dL/d(attention output)
+  gemm_into(dx_mid, o, mg_o, H, O, T, H, O, O, true, true, 1, on);
+  PT_CHECK_BWD_RC(pt_attention_bwd_rope(dO, qkv, qkv + O, qkv + O + hkv * d, o, f + at.lse, nullptr, reinterpret_cast<float*>(delta),
+                                        reinterpret_cast<float*>(dq_ws), dqkv, dqkv + O, dqkv + O + hkv * d, (int)B, (int)S, (int)S, (int)hq,
+                                        (int)hkv, (int)d, Q, Q, Q, Q, Q, Q, 1, (float)scale, cosT.data_ptr<float>(), sinT.data_ptr<float>(),
+                                        (int)S, st), "attention_bwd");
+  gemm_into(dqkv, w_qkv.data_ptr(), dh, T, H, Q, Q, ld_qkv, H, false, true, 0, on);
+  gemm_into(dqkv, h1, mg_qkv, Q, H, T, Q, H, H, true, true, 1, on);
+  rmsnorm_bwd_into(dh, x.data_ptr(), ln1, f + at.rstd1, dx_mid, dx.data_ptr(), mg[7], T, H, on);
+  return dx;
 }
 
 void allreduce_symm(std::vector<int64_t> buf_ptrs, std::vector<int64_t> flag_ptrs, int64_t mc_ptr, int64_t offset_elems,
@@ -838,6 +960,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("add", &add);
   m.def("adamw_multi_", &adamw_multi_);
   m.def("decoder_layer_fwd", &decoder_layer_fwd);
+  m.def("decoder_layer_saved", &decoder_layer_saved, "The saved activations of decoder_layer_fwd as tensors (views).");
   m.def("decoder_layer_bwd", &decoder_layer_bwd);
   m.def("scale_", &scale_);
   m.def("merge_attention_", &merge_attention_);

@@ -69,6 +69,16 @@ def pack_parameters(params: Sequence[nn.Parameter]) -> torch.Tensor:
         p0.untyped_storage(), p0.storage_offset(), (rows, cols), (cols, 1))
 
 
+def _aliases(flat: torch.Tensor, params: Sequence[nn.Parameter]) -> bool:
+    """Whether ``flat`` starts where ``params`` lie back to back."""
+    at = flat.data_ptr()
+    for p in params:
+        if p.data_ptr() != at:
+            return False
+        at += p.numel() * p.element_size()
+    return True
+
+
 def packed_main_grad(params: Sequence[nn.Parameter]) -> Optional[torch.Tensor]:
     """The fp32 gradient-bucket region covering ``params`` as one ``[rows, cols]`` tensor, or None."""
     mgs = [getattr(p, "main_grad", None) for p in params]
@@ -359,19 +369,20 @@ class DecoderLayerFn(torch.autograd.Function):
         T = B * S
         x2 = x.reshape(B * S_in, H)
 
-        w_qkv = layer.packed_qkv()
-        w_gu = layer.packed_gu()
+        w_qkv = layer.packed_qkv((wq, wk, wv))
+        w_gu = layer.packed_gu((wg, wu))
 
+        ctx.native = False
         if tp_group is None and not att.cp_enabled and ops.runs_layer_natively(x2):
             cos, sin = layer.rope(x.device)
             r = ops.decoder_layer_fwd(x2, ln1_w, w_qkv, cos, sin, wo, ln2_w, w_gu, wd, layer.eps, B, S, hq, hkv, d, layer.sm_scale)
             if r:
-                out, h1, rstd1, qkv, o2, lse, x_mid, rstd2, h2, gu, a = r
-                ctx.save_for_backward(x2, rstd1, h1, qkv, o2, lse, x_mid, rstd2, h2, gu, a)
+                ctx.save_for_backward(x2, r[1], r[2])                       # input, saved activations (bf16 and fp32)
                 ctx.layer = layer
                 ctx.dims = (B, S, H, S_in)
                 ctx.sp_group = None
-                return out.view(B, S_in, H)
+                ctx.native = True
+                return r[0].view(B, S_in, H)
 
         h1, rstd1 = ops.rmsnorm_fwd(x2, ln1_w, layer.eps)
         h1_all = tpc.gather_tokens(h1, sp_group) if sp_group is not None else h1
@@ -414,7 +425,6 @@ class DecoderLayerFn(torch.autograd.Function):
 
     @staticmethod
     def _backward(ctx, dout):
-        x2, rstd1, h1, qkv, o2, lse, x_mid, rstd2, h2, gu, a = ctx.saved_tensors
         layer = ctx.layer
         B, S, H, S_in = ctx.dims
         sp_group = ctx.sp_group
@@ -422,25 +432,30 @@ class DecoderLayerFn(torch.autograd.Function):
         hq, hkv, d = att.num_local_heads, att.num_local_kv_heads, att.head_dim
         tp_group = layer.tp_group
         ln1, ln2 = layer.input_layernorm, layer.post_attention_layernorm
-        w_qkv, w_gu = layer.packed_qkv(), layer.packed_gu()
-        wo, wd = att.out_proj.weight, mlp.down_proj.weight
+        params = (att.q_proj.weight, att.k_proj.weight, att.v_proj.weight, att.out_proj.weight, mlp.gate_proj.weight,
+                  mlp.up_proj.weight, mlp.down_proj.weight, ln1.weight, ln2.weight)
+        wo, wd = params[3], params[6]
+        w_qkv, w_gu = layer.packed_qkv(params[:3]), layer.packed_gu(params[4:6])
         dout2 = dout.reshape(B * S_in, H)
         if not dout2.is_contiguous():
             dout2 = dout2.contiguous()
         sp = sp_group is not None
-        if not sp and tp_group is None and not att.cp_enabled and pgm.get().cp_dp_world_size == 1 and ops.runs_layer_natively(dout2):
-            # (with several data-parallel replicas a bucket's all-reduce starts as soon as its last gradient is there)
-            params = (att.q_proj.weight, att.k_proj.weight, att.v_proj.weight, wo, mlp.gate_proj.weight, mlp.up_proj.weight, wd,
-                      ln1.weight, ln2.weight)
-            grads = [getattr(p, "main_grad", None) for p in params]
-            if all(g is not None for g in grads):
-                cos, sin = layer.rope(dout.device)
-                dx = ops.decoder_layer_bwd(dout2, [x2, rstd1, h1, qkv, o2, lse, x_mid, rstd2, h2, gu, a], ln1.weight, w_qkv, cos, sin,
-                                           wo, ln2.weight, w_gu, wd, grads, B, S, hq, hkv, d, layer.sm_scale)
-                if dx is not None:
-                    for p in params:
-                        notify_grad_ready(p)
-                    return dx.view(B, S_in, H), None, None, None, None, None, None, None, None, None, None
+        if ctx.native:
+            x2, saved16, saved32 = ctx.saved_tensors
+            if tp_group is None and not att.cp_enabled and pgm.get().cp_dp_world_size == 1 and ops.runs_layer_natively(dout2):
+                # (with several data-parallel replicas a bucket's all-reduce starts as soon as its last gradient is there)
+                grads = [getattr(p, "main_grad", None) for p in params]
+                if all(g is not None for g in grads):
+                    cos, sin = layer.rope(dout.device)
+                    dx = ops.decoder_layer_bwd(dout2, x2, saved16, saved32, params[7], w_qkv, cos, sin, wo, params[8], w_gu, wd, grads,
+                                               B, S, hq, hkv, d, layer.sm_scale)
+                    if dx is not None:
+                        for p in params:
+                            notify_grad_ready(p)
+                        return dx.view(B, S_in, H), None, None, None, None, None, None, None, None, None, None
+            rstd1, h1, qkv, o2, lse, x_mid, rstd2, h2, gu, a = ops.decoder_layer_saved(saved16, saved32, B, S, H, wd.shape[1], hq, hkv, d)
+        else:
+            x2, rstd1, h1, qkv, o2, lse, x_mid, rstd2, h2, gu, a = ctx.saved_tensors
         dout_all = tpc.gather_tokens(dout2, sp_group) if sp else dout2      # backward of the forward's reduce-scatter
 
         # ---- MLP
@@ -535,22 +550,22 @@ class DecoderLayer(nn.Module):
         return self.rope(self.input_layernorm.weight.device)[1]
 
     # --- packed weights -----------------------------------------------------------------------
-    def packed_qkv(self) -> torch.Tensor:
-        a = self.attention
-        ps = [a.q_proj.weight, a.k_proj.weight, a.v_proj.weight]
+    # (`ps`: the parameters, where the caller has them at hand -- looking one up through its modules costs the host a microsecond)
+    def packed_qkv(self, ps=None) -> torch.Tensor:
+        if ps is None:
+            a = self.attention
+            ps = (a.q_proj.weight, a.k_proj.weight, a.v_proj.weight)
         f = self._qkv_flat
-        if f is None or f.data_ptr() != ps[0].data_ptr() or f.dtype != ps[0].dtype or \
-                ps[1].data_ptr() != ps[0].data_ptr() + ps[0].numel() * ps[0].element_size() or \
-                ps[2].data_ptr() != ps[1].data_ptr() + ps[1].numel() * ps[1].element_size():
+        if f is None or f.dtype != ps[0].dtype or not _aliases(f, ps):
             f = self._qkv_flat = pack_parameters(ps)
         return f
 
-    def packed_gu(self) -> torch.Tensor:
-        m = self.mlp
-        ps = [m.gate_proj.weight, m.up_proj.weight]
+    def packed_gu(self, ps=None) -> torch.Tensor:
+        if ps is None:
+            m = self.mlp
+            ps = (m.gate_proj.weight, m.up_proj.weight)
         f = self._gu_flat
-        if f is None or f.data_ptr() != ps[0].data_ptr() or f.dtype != ps[0].dtype or \
-                ps[1].data_ptr() != ps[0].data_ptr() + ps[0].numel() * ps[0].element_size():
+        if f is None or f.dtype != ps[0].dtype or not _aliases(f, ps):
             f = self._gu_flat = pack_parameters(ps)
         return f
 

@@ -192,8 +192,14 @@ def runs_layer_natively(x) -> bool:
 
 
 def decoder_layer_fwd(*args):
-    """``(x_out, h1, rstd1, qkv, o, lse, x_mid, rstd2, h2, gu, a)`` of a layer on one GPU, or ``[]`` if it is not covered."""
+    """``(x_out, saved16, saved32)`` of a layer on one GPU, or ``[]`` if it is not covered. What the backward needs besides the input
+    lies in two allocations, bf16 and fp32 (:func:`decoder_layer_saved`)."""
     return _c().decoder_layer_fwd(*args)
+
+
+def decoder_layer_saved(*args):
+    """``(rstd1, h1, qkv, o, lse, x_mid, rstd2, h2, gu, a)`` as views into the saved activations of :func:`decoder_layer_fwd`."""
+    return _c().decoder_layer_saved(*args)
 
 
 def decoder_layer_bwd(*args):
