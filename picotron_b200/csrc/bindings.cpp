@@ -27,11 +27,11 @@ void* pt_status_word();
 void pt_attention_set_profile(unsigned long long* counters);
 void pt_gemm_set_group_m(int g);
 void pt_gemm_set_tile_n(int n);
-int pt_gemm_split_parts(int M, int N, int K, int out_mode);
-long long pt_gemm_split_elems(int M, int N, int K, int out_mode, int parts);
+int pt_gemm_split_parts(int M, int N, int K, int kind, int* tile_n);
+long long pt_gemm_split_elems(int M, int N, int K, int kind, int parts);
 void pt_gemm_set_split_k(int on);
 int pt_gemm_bf16_split(const void* A, const void* B, void* D, float* ws, int M, int N, int K, long long lda, long long ldb,
-                       long long ldd, int a_mn, int b_mn, int out_mode, int parts, void* status, cudaStream_t stream);
+                       long long ldd, int kind, int parts, int tile_n, const void* res, long long ldr, void* status, cudaStream_t stream);
 int pt_gemm_get_group_m();
 void pt_gemm_set_tma_epilogue(int on);
 int pt_gemm_get_tma_epilogue();
@@ -215,6 +215,24 @@ Tensor swiglu_bwd(const Tensor& gu, const Tensor& da) {
   return dgu;
 }
 
+// A GEMM with few output tiles, K in parts (pt_gemm_split_parts) through a workspace from the caching allocator; kind 0: D = A B,
+// 1: D += A^T B (fp32), 2: D = A B^T (+ res). False (nothing launched) where it would not pay or the operands do not allow it.
+bool gemm_split_into(const void* a, const void* b, void* d, int64_t M, int64_t N, int64_t K, long long lda, long long ldb, long long ldd,
+                     int kind, const void* res, long long ldr, const at::TensorOptions& on) {
+  if (!pt_gemm_get_pair() || !pt_gemm_get_tma_epilogue() || lda % 8 || ldb % 8 || ldd % (kind == 1 ? 4 : 8) || ldr % 8 ||
+      (((uintptr_t)a | (uintptr_t)b | (uintptr_t)d | (uintptr_t)res) & 15))
+    return false;
+  int tile_n = 256;
+  const int parts = pt_gemm_split_parts((int)M, (int)N, (int)K, kind, &tile_n);
+  if (parts <= 1) return false;
+  auto ws = torch::empty({pt_gemm_split_elems((int)M, (int)N, (int)K, kind, parts)}, on.dtype(at::kFloat));
+  const int rc = pt_gemm_bf16_split(a, b, d, ws.data_ptr<float>(), (int)M, (int)N, (int)K, lda, ldb, ldd, kind, parts, tile_n, res, ldr,
+                                    pt_status_word(), stream());
+  if (rc == -5) return false;                            // (CTA pairs cannot be scheduled: the general path)
+  TORCH_CHECK(rc == 0, "gemm (split) failed with code ", rc);
+  return true;
+}
+
 // gu[T, 2I] = x w_gu^T and h[T, I] = silu(gate) * up from ONE GEMM (SwiGLU epilogue). Returns {} when the fused kernel does
 // not cover the case (CTA pairs or the TMA epilogue unavailable, I % 128 != 0): the caller then runs GEMM + activation kernel.
 std::vector<Tensor> gemm_swiglu(const Tensor& x, const Tensor& w_gu) {
@@ -262,6 +280,7 @@ Tensor gemm_add(const Tensor& x, const Tensor& w, const Tensor& res) {
   if (!pt_gemm_get_pair() || N % 8 != 0) return Tensor();
   c10::cuda::CUDAGuard guard(x.device());
   auto y = torch::empty({M, N}, x.options());
+  if (gemm_split_into(x.data_ptr(), w.data_ptr(), y.data_ptr(), M, N, K, lda, ldb, N, 2, res.data_ptr(), ldh, x.options())) return y;
   const int rc = pt_gemm_bf16_fused(x.data_ptr(), w.data_ptr(), y.data_ptr(), (int)M, (int)N, (int)K, lda, ldb, N, 4,
                                     res.data_ptr(), ldh, 0, nullptr, nullptr, 0, 0, 0, pt_status_word(), stream());
   if (rc == 1 || rc == -5) return Tensor();
@@ -286,24 +305,11 @@ Tensor gemm_dgrad_swiglu_bwd(const Tensor& dy, const Tensor& w, const Tensor& gu
   return dgu;
 }
 
-// D = op(A) op(B) on raw operands (pt_gemm_bf16). Input gradients and weight gradients with few output tiles: K in parts
-// (pt_gemm_split_parts), through a workspace from the caching allocator.
+// D = op(A) op(B) on raw operands (pt_gemm_bf16).
 void gemm_into(const void* a, const void* b, void* d, int64_t M, int64_t N, int64_t K, long long lda, long long ldb, long long ldd,
                bool trans_a, bool trans_b, int mode, const at::TensorOptions& on) {
-  const bool grad = (mode == 0 && !trans_a && trans_b) || (mode == 1 && trans_a && trans_b);
-  if (grad && pt_gemm_get_pair() && pt_gemm_get_tma_epilogue() && lda % 8 == 0 && ldb % 8 == 0 && ldd % (mode == 0 ? 8 : 4) == 0 &&
-      (((uintptr_t)a | (uintptr_t)b | (uintptr_t)d) & 15) == 0) {
-    const int parts = pt_gemm_split_parts((int)M, (int)N, (int)K, mode);
-    if (parts > 1) {
-      auto ws = torch::empty({pt_gemm_split_elems((int)M, (int)N, (int)K, mode, parts)}, on.dtype(at::kFloat));
-      const int rc = pt_gemm_bf16_split(a, b, d, ws.data_ptr<float>(), (int)M, (int)N, (int)K, lda, ldb, ldd, trans_a ? 1 : 0,
-                                        trans_b ? 1 : 0, mode, parts, pt_status_word(), stream());
-      if (rc != -5) {                                    // (CTA pairs cannot be scheduled: the general path below)
-        TORCH_CHECK(rc == 0, "gemm (split) failed with code ", rc);
-        return;
-      }
-    }
-  }
+  const int kind = mode == 0 && !trans_a ? (trans_b ? 0 : 2) : (mode == 1 && trans_a && trans_b) ? 1 : -1;
+  if (kind >= 0 && gemm_split_into(a, b, d, M, N, K, lda, ldb, ldd, kind, nullptr, 0, on)) return;
   const int rc = pt_gemm_bf16(a, b, d, (int)M, (int)N, (int)K, lda, ldb, ldd, trans_a ? 1 : 0, trans_b ? 1 : 0, mode, num_sms(), stream());
   TORCH_CHECK(rc == 0, "gemm failed with code ", rc, " (M=", M, " N=", N, " K=", K, " lda=", lda, " ldb=", ldb, " ldd=", ldd,
               " trans_a=", trans_a, " trans_b=", trans_b, " mode=", mode, " a%16=", (uintptr_t)a % 16, " b%16=", (uintptr_t)b % 16,
@@ -684,7 +690,8 @@ std::vector<Tensor> decoder_layer_fwd(const Tensor& x, const Tensor& ln1, const 
     gemm_into(h2, w_gu.data_ptr(), gu, T, 2 * I, H, H, ld_gu, 2 * I, false, false, 0, on);
     PT_CHECK_RC(pt_swiglu_fwd(gu, a, T, (int)I, st), "swiglu_fwd");
   }
-  if (!(pair && H % 8 == 0 &&
+  if (!(pair && H % 8 == 0 && gemm_split_into(a, wd.data_ptr(), out.data_ptr(), T, H, I, I, ld_d, H, 2, x_mid, H, on)) &&
+      !(pair && H % 8 == 0 &&
         fused_gemm(pt_gemm_bf16_fused(a, wd.data_ptr(), out.data_ptr(), (int)T, (int)H, (int)I, I, ld_d, H, 4, x_mid, H, 0, nullptr, nullptr, 0,
                                       0, 0, status, st), "gemm_add"))) {
     Tensor y = torch::empty({T, H}, on);
@@ -978,6 +985,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         "CTA-pair GEMM tile numbering: rows of 256-row tiles per group (L2 locality of concurrently running tiles; default 8).");
   m.def("set_gemm_split_dgrad", [](bool on) { pt_gemm_set_split_k(on ? 1 : 0); },
         "input- and weight-gradient GEMMs with few output tiles: K split over idle CTA pairs (default on; for the calling thread)");
+  m.def("set_gemm_split_parts", [](int64_t n) { pt_gemm_set_split_k(n > 1 ? (int)n : 1); },
+        "GEMMs that may be split over K are always cut into n parts by this thread (tests, measurements); 0 or 1: the rule.");
   m.def("set_gemm_tile_n", [](int64_t n) { pt_gemm_set_tile_n((int)n); },
         "columns of the GEMM output tiles: 128, 256, or 0 for the choice by shape (bf16 outputs; for the calling thread)");
   m.def("get_gemm_group_m", []() { return (int64_t)pt_gemm_get_group_m(); });

@@ -136,7 +136,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                  void* __restrict__ Dptr, int M, int N, int K, long long ldd, KernelStatus* status, EpiArgs ea) {
   static_assert(EPI == EPI_NONE || (EPI_TMA && !A_MN && OUT_MODE == OUT_BF16 && B_MN == (EPI == EPI_SWIGLU_BWD)),
                 "fused epilogues: bf16 output; forward layout, except the SwiGLU backward which rides on the dgrad layout");
-  static_assert(BN == 256 || (BN == 128 && EPI_TMA && OUT_MODE == OUT_BF16 && EPI != EPI_CE), "narrow tiles: bf16 outputs");
+  static_assert(BN == 256 || (BN == 128 && EPI_TMA && EPI != EPI_CE), "narrow tiles: the epilogues through TMA, but for the statistics");
   constexpr int BN_HALF = BN / 2;                 // columns of B per CTA
   constexpr int B_BYTES = BN_HALF * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
   constexpr int STAGES = stages_of(EPI);          // shadows the namespace constant: the variants differ in their smem split
@@ -702,11 +702,12 @@ __global__ void __launch_bounds__(256) clear_f32_kernel(float4* __restrict__ x, 
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
   if (i < n4) x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
-// out[r, c] = sum over the slices (bf16), or out[r, c] += that sum (fp32, one atomic per element as the unsplit epilogue's
-// reduce-add). Bound by the workspace's bytes, which lie in L2; four columns per thread.
-template <bool TO_BF16>
+// out[r, c] = sum over the slices (+ res[r, c]) (bf16), or out[r, c] += that sum (fp32, one atomic per element as the unsplit
+// epilogue's reduce-add). Bound by the workspace's bytes, which lie in L2; four columns per thread.
+template <bool TO_BF16, bool ADD>
 __global__ void __launch_bounds__(256) sum_slices_kernel(const float* __restrict__ ws, int slices, long long slice_elems, void* __restrict__ out,
-                                                         int rows, int cols, int ws_cols, long long ldd) {
+                                                         int rows, int cols, int ws_cols, long long ldd,
+                                                         const __nv_bfloat16* __restrict__ res, long long ldr) {
   pdl_enter();
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
   const int quads = ws_cols / 4;
@@ -719,6 +720,12 @@ __global__ void __launch_bounds__(256) sum_slices_kernel(const float* __restrict
   for (int k = 1; k < slices; ++k) {
     const float4 u = *reinterpret_cast<const float4*>(src + k * slice_elems);
     v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+  }
+  if (ADD) {
+    const uint2 q = *reinterpret_cast<const uint2*>(res + r * ldr + c);
+    const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&q.x));
+    const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&q.y));
+    v.x += lo.x; v.y += lo.y; v.z += hi.x; v.w += hi.y;
   }
   if (TO_BF16) {
     *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(out) + r * ldd + c) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
@@ -745,20 +752,32 @@ static int num_pairs() {
 }
 
 // Switches for tests and measurements, of the calling thread only: other threads' launches keep the rules.
-static thread_local int g_split_k = 1;
+static thread_local int g_split_k = 1;   // 0: never, 1: by pt_gemm_split_parts' rule, n > 1: always n parts
 static thread_local int g_tile_n = 0;    // 0: by the rule below, 128 / 256: as given (tests, measurements)
 
-// Columns of an output tile (bf16 outputs). A 256 x 256 tile moves the fewest operand bytes per product, but a few hundred
-// tokens or a few hundred columns give only a handful of them for 74 CTA pairs, and then their epilogue, 256 columns one after
-// the other, is a good part of the time. Tiles of 128 columns halve it, at the same time per k-block, wherever they still fit
-// in one wave. Measured with 256 / 128 columns (us): RoPE 256 x 960 x 576: 14.8 / 11.2, SwiGLU 256 x 3072 x 576: 11.2 / 9.7,
-// SwiGLU backward 256 x 3072 x 576: 15.9 / 12.3, residual add 256 x 576 x 1536: 15.6 / 13.8; beyond one wave they lose (RoPE
-// 512 x 6144 x 2048: 24.1 / 27.9, SwiGLU 1024 x 3072 x 576: 11.8 / 13.3), and beyond K = 8192 the epilogue no longer shows.
-static int tile_columns(int M, int n_cols, int K) {
+// Microseconds of a GEMM as far as they depend on the width of its tiles and on the parts K is split into: waves of units over the
+// CTA pairs, each its k-blocks and what of its epilogue shows, and for a split the summing kernel and its slices' traffic.
+// A 64-deep k-block of a 256 x 256 tile takes the MMA's 512 cycles; one of a 256 x 128 tile half of that, until the pairs share
+// L2's bandwidth (three quarters of the operand bytes for half of the products). Constants fitted to 211 shapes (weight and input
+// gradients, forward with and without residual; widths of 20M to 1.7B models, 256 to 8,192 tokens; both widths, 1 to 32 parts): 7 %
+// off, and the choice it makes 0.5 % slower than the best measured one. Measured 256 / 128 columns / 128 split (us): forward 256 x 576 x
+// 576: 7.1 / 5.3; 1024 x 2048 x 2048: 14.9 / 10.2; 8192 x 2048 x 2048: 47.0 / 50.4; weight gradient 576 x 576, 512 tokens: 8.6 / 6.2;
+// 2048 x 576 x 3072: 18.0 / 11.3; with residual 256 x 2048 x 8192: 43.0 / 24.5 / 12.8; input gradient 512 x 2048 x 16384: 78 / 54 /
+// 35.5 (31.5 with 256 columns).
+static double gemm_us(int M, int n_cols, int K, int bn, int parts, bool f32) {
+  const int pairs = num_pairs(), kb = (K + BK - 1) / BK, kb_part = (kb + parts - 1) / parts;
+  const long long units = (long long)((M + 2 * BM - 1) / (2 * BM)) * ((n_cols + bn - 1) / bn) * ((kb + kb_part - 1) / kb_part);
+  const double load = units < pairs ? (double)units / pairs : 1.0, waves = (double)((units + pairs - 1) / pairs);
+  const bool slices = parts > 1;
+  const double unit = bn == 256 ? kb_part * (0.29 + 0.026 * load) + 1.6 + (f32 || slices ? 0.8 : 0)
+                                : kb_part * (0.149 + 0.04 * load) + 0.85 + (f32 || slices ? 0.55 : 0);
+  return waves * unit + (slices ? 1.0 + 0.147 * parts * M * n_cols * 4e-6 : 0.0);
+}
+
+// Columns of an output tile.
+static int tile_columns(int M, int n_cols, int K, bool f32) {
   if (g_tile_n) return g_tile_n;
-  const int pairs = num_pairs();
-  const long long rows = (M + 2 * BM - 1) / (2 * BM);
-  return rows * ((n_cols + 127) / 128) <= pairs && K <= 8192 ? 128 : 256;
+  return gemm_us(M, n_cols, K, 128, 1, f32) < gemm_us(M, n_cols, K, 256, 1, f32) ? 128 : 256;
 }
 
 template <bool A_MN, bool B_MN, int OUT_MODE, bool EPI_TMA, int EPI = EPI_NONE, int BN = 256>
@@ -816,20 +835,23 @@ extern "C" void pt_gemm_set_split_k(int on) { pt::gemm_pair::g_split_k = on; }
 
 namespace pt {
 namespace gemm_pair {
+// GEMMs that may be split: dY W, dY^T X into an fp32 destination, X W^T
+enum SplitKind { SPLIT_DGRAD = 0, SPLIT_WGRAD = 1, SPLIT_FWD = 2 };
 struct SplitPlan {
-  int parts, kb_per_part, slices, shift, slice_rows, ws_cols;
+  int parts, kb_per_part, slices, shift, slice_rows, ws_cols, bn;
 };
 // Two parts add to a slice of an input gradient's workspace (a sum of two is the same in either order); the parts of a weight
-// gradient, whose result has to be read and written anyway, each store a slice of their own.
-static SplitPlan split_plan(int M, int N, int K, int out_mode, int parts) {
+// gradient, whose result has to be read and written anyway, and those of a forward GEMM each store a slice of their own.
+static SplitPlan split_plan(int M, int N, int K, int kind, int parts, int bn) {
   SplitPlan s;
   const int kb = (K + BK - 1) / BK;
   s.kb_per_part = (kb + parts - 1) / parts;
   s.parts = (kb + s.kb_per_part - 1) / s.kb_per_part;
-  s.shift = out_mode == OUT_BF16 ? 1 : 0;
+  s.shift = kind == SPLIT_DGRAD ? 1 : 0;
   s.slices = (s.parts + s.shift) >> s.shift;
   s.slice_rows = (M + 31) / 32 * 32;        // the epilogue writes 32 rows at a time
   s.ws_cols = (N + 3) / 4 * 4;
+  s.bn = bn;
   return s;
 }
 static int run_pair(const void* A, const void* B, void* D, int M, int N, int K, long long lda, long long ldb, long long ldd, int a_mn,
@@ -837,72 +859,65 @@ static int run_pair(const void* A, const void* B, void* D, int M, int N, int K, 
 }  // namespace gemm_pair
 }  // namespace pt
 
-// How many parts K is split into when D[M, N] has few tiles behind a long K; 1: not at all. In k-blocks of 0.33 us, a wave of tiles
-// takes its k-blocks plus a constant, and a split adds its further kernels and the workspace's traffic. Measured without / with it (us):
-// weight gradients (out_mode OUT_F32_ACC; K is the number of tokens; constants fitted to a sweep of 1 to 32 parts over the shapes
-// of 20M to 1.7B models and 256 to 32,768 tokens, 3 % off; a split has to give 5 %): 576 x 576, 8192 tokens: 45.7 / 16.2; 3072 x
-// 576, 4096 tokens: 27.3 / 21.2; 512 x 512, 512 tokens: 8.4 / 8.1 (not split); 2048 x 2048, 4096 tokens: 29.4 / 36.4 (not split).
-// Input gradients (OUT_BF16; the constants are on the safe side, so that it is split where it gives about a quarter): 2048 x 576 x
-// 49152 (LM head of the 135M shape): 241 / 103; 512 x 2048 x 16384: 84.7 / 35.4; 256 x 4096 x 4096: 25.0 / 18.7; 512 x 512 x 2048:
-// 13.8 / 11.4 (not split); 2048 x 2048 x 49152: 282 / 300 (not split).
-// (Weight gradients with every part added to the destination by itself needed 3 us less, but their results changed from run to run
-// and were rounded once per part. The forward GEMMs are not split.)
-extern "C" int pt_gemm_split_parts(int M, int N, int K, int out_mode) {
+// How many parts K is split into (1: not at all) and the columns of a tile then, by gemm_us; adding the weight gradient to what is
+// there costs 0.08 us a megabyte more in the GEMM's epilogue than in the summing kernel; an input gradient clears its slices first. A
+// split has to give 3 %.
+extern "C" int pt_gemm_split_parts(int M, int N, int K, int kind, int* tile_n) {
   using namespace pt::gemm_pair;
-  const bool wgrad = out_mode == OUT_F32_ACC;
+  *tile_n = g_tile_n ? g_tile_n : 256;
+  const bool wgrad = kind == SPLIT_WGRAD;
   if (M <= 0 || N <= 0 || K <= 0 || !g_split_k || (!wgrad && N % 8)) return 1;
-  const int pairs = num_pairs(), kb = (K + BK - 1) / BK;
-  const int tiles = ((M + 2 * BM - 1) / (2 * BM)) * ((N + 255) / 256);
-  if (tiles >= pairs) return 1;
-  constexpr int MIN_KB = 4, MAX_PARTS = 32;
-  const double mbytes = (double)M * N * 4e-6;
-  const int wave_kb = wgrad ? 3 : 12, other_kb = wgrad ? 16 : 0;      // other_kb: launches, split or not
-  auto cost = [&](const SplitPlan& p, bool whole) {
-    double c = other_kb + (double)((tiles * p.parts + pairs - 1) / pairs) * (p.kb_per_part + wave_kb);
-    if (whole) c += wgrad ? 2 + 0.27 * mbytes * (2 * p.slices + 2) : 24 + 0.6 * mbytes * (2 + p.parts);
-    return c;
-  };
-  // input gradients: the parts with the shortest waves first, then whether they pay (their traffic is a fraction of the tiles' time)
-  int best = 1;
-  double best_cost = other_kb + kb + wave_kb;
-  for (int parts = 2; parts <= MAX_PARTS && kb / parts >= MIN_KB; ++parts) {
-    const double c = cost(split_plan(M, N, K, out_mode, parts), wgrad);
-    if (c < best_cost) {
-      best = parts;
-      best_cost = c;
+  const int kb = (K + BK - 1) / BK;
+  if (g_split_k > 1) return g_split_k < kb ? g_split_k : kb;
+  if (g_tile_n) return 1;                  // (a width given for a measurement: of whole tiles)
+  double best = 0.97 * (gemm_us(M, N, K, tile_columns(M, N, K, wgrad), 1, wgrad) + (wgrad ? 0.08 * M * N * 4e-6 : 0.0));
+  int best_parts = 1;
+  for (const int parts : {2, 3, 4, 5, 6, 8, 10, 12, 16, 20, 24, 32}) {
+    if (kb / parts < 2) break;
+    for (const int bn : {128, 256}) {
+      const double t = gemm_us(M, N, K, bn, parts, true) + (kind == SPLIT_DGRAD ? 2.0 : 0.0);
+      if (t < best) {
+        best = t;
+        best_parts = parts;
+        *tile_n = bn;
+      }
     }
   }
-  if (best == 1) return 1;
-  const double gain = wgrad ? 0.95 : 1 / 1.125;
-  return cost(split_plan(M, N, K, out_mode, best), true) < gain * (other_kb + kb + wave_kb) ? best : 1;
+  return best_parts;
 }
 
 // Floats of workspace for pt_gemm_bf16_split with `parts` parts.
-extern "C" long long pt_gemm_split_elems(int M, int N, int K, int out_mode, int parts) {
-  const pt::gemm_pair::SplitPlan p = pt::gemm_pair::split_plan(M, N, K, out_mode, parts);
+extern "C" long long pt_gemm_split_elems(int M, int N, int K, int kind, int parts) {
+  const pt::gemm_pair::SplitPlan p = pt::gemm_pair::split_plan(M, N, K, kind, parts, 256);
   return (long long)p.slices * p.slice_rows * p.ws_cols;
 }
 
 // GEMM with K in `parts` parts, each computed by CTA pairs of its own, through the fp32 workspace ws (pt_gemm_split_elems floats,
-// 16-byte aligned). out_mode OUT_BF16: D = op(A) op(B), rounded once (N % 8 == 0, ldd % 8 == 0); OUT_F32_ACC: D += op(A) op(B) with
-// one addition per element (ldd % 4 == 0). The result does not depend on the order in which the parts finish.
+// 16-byte aligned). Kind 0: D = A B, 2: D = A B^T (+ res, a bf16 [M, N] tensor with row stride ldr % 4 == 0, or nullptr), both rounded
+// once (N % 8 == 0, ldd % 8 == 0); 1: D += A^T B in fp32 with one addition per element (ldd % 4 == 0). The result does not depend on
+// the order in which the parts finish.
 extern "C" int pt_gemm_bf16_split(const void* A, const void* B, void* D, float* ws, int M, int N, int K, long long lda, long long ldb,
-                                  long long ldd, int a_mn, int b_mn, int out_mode, int parts, void* status, cudaStream_t stream) {
+                                  long long ldd, int kind, int parts, int tile_n, const void* res, long long ldr, void* status,
+                                  cudaStream_t stream) {
   using namespace pt;
   using namespace pt::gemm_pair;
-  const SplitPlan p = split_plan(M, N, K, out_mode, parts);
+  const SplitPlan p = split_plan(M, N, K, kind, parts, tile_n);
   const long long slice_elems = (long long)p.slice_rows * p.ws_cols, n4 = p.slices * slice_elems / 4;
   if (p.shift > 0) {
     launch_pdl(clear_f32_kernel, dim3((unsigned)((n4 + 255) / 256)), dim3(256), 0, stream, reinterpret_cast<float4*>(ws), n4);
     pt_count_launches(1);
   }
-  const int rc = run_pair(A, B, ws, M, N, K, lda, ldb, p.ws_cols, a_mn, b_mn, p.shift > 0 ? OUT_F32_ACC : OUT_F32, &p, status, stream);
+  const int rc = run_pair(A, B, ws, M, N, K, lda, ldb, p.ws_cols, kind == SPLIT_WGRAD, kind != SPLIT_FWD, p.shift > 0 ? OUT_F32_ACC : OUT_F32,
+                          &p, status, stream);
   if (rc) return rc;
   const dim3 grid((unsigned)(((long long)M * (p.ws_cols / 4) + 255) / 256));
-  if (out_mode == OUT_BF16)
-    launch_pdl(sum_slices_kernel<true>, grid, dim3(256), 0, stream, (const float*)ws, p.slices, slice_elems, D, M, N, p.ws_cols, ldd);
-  else
-    launch_pdl(sum_slices_kernel<false>, grid, dim3(256), 0, stream, (const float*)ws, p.slices, slice_elems, D, M, N, p.ws_cols, ldd);
+  auto sum = [&](auto kern) {
+    launch_pdl(kern, grid, dim3(256), 0, stream, (const float*)ws, p.slices, slice_elems, D, M, N, p.ws_cols, ldd,
+               (const __nv_bfloat16*)res, ldr);
+  };
+  if (kind == SPLIT_WGRAD) sum(sum_slices_kernel<false, false>);
+  else if (res == nullptr) sum(sum_slices_kernel<true, false>);
+  else sum(sum_slices_kernel<true, true>);
   pt_count_launches(1);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
@@ -919,7 +934,10 @@ static int pt::gemm_pair::run_pair(const void* A, const void* B, void* D, int M,
                                    cudaStream_t stream) {
   using namespace pt;
   using namespace pt::gemm_pair;
-  const int bn = (out_mode == OUT_BF16 && g_tma_epilogue && !a_mn) ? tile_columns(M, N, K) : 256;
+  const bool epi_tma = g_tma_epilogue != 0;
+  // narrow tiles exist for the layouts of the model: X W^T, dY W, and dY^T X into fp32
+  const bool has_narrow = epi_tma && (out_mode == OUT_BF16 ? !a_mn : (b_mn || (!a_mn && out_mode == OUT_F32)));
+  const int bn = !has_narrow ? 256 : split ? split->bn : tile_columns(M, N, K, out_mode != OUT_BF16);
   CUtensorMap ma, mb;
   int rc;
   rc = a_mn ? make_bf16_map_2d(&ma, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, 64, BK)
@@ -929,7 +947,6 @@ static int pt::gemm_pair::run_pair(const void* A, const void* B, void* D, int M,
             : make_bf16_map_2d(&mb, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, BK, bn / 2);
   if (rc) return rc * 10 - 2;    // -22: tensor map of B could not be encoded
   CUtensorMap md = ma;           // unused by the per-thread epilogue
-  const bool epi_tma = g_tma_epilogue != 0;
   if (epi_tma) {
     uint64_t dims[2] = {(uint64_t)N, split ? (uint64_t)split->slices * split->slice_rows : (uint64_t)M};
     uint64_t strides[1] = {(uint64_t)ldd};
@@ -944,9 +961,11 @@ static int pt::gemm_pair::run_pair(const void* A, const void* B, void* D, int M,
     ea.slice_shift = split->shift;
   }
   KernelStatus* st = reinterpret_cast<KernelStatus*>(status);
-  if (bn == 128)
-    return b_mn ? launch<false, true, OUT_BF16, true, EPI_NONE, 128>(ma, mb, md, D, M, N, K, ldd, st, stream)
-                : launch<false, false, OUT_BF16, true, EPI_NONE, 128>(ma, mb, md, D, M, N, K, ldd, st, stream);
+#define PT_GEMM_NARROW(AM, BMN, OM)                                                                           \
+  if (bn == 128 && a_mn == AM && b_mn == BMN && out_mode == OM)                                               \
+    return launch<AM, BMN, OM, true, EPI_NONE, 128>(ma, mb, md, D, M, N, K, ldd, st, stream, nullptr, ea);
+  PT_GEMM_NARROW(0, 0, 0) PT_GEMM_NARROW(0, 1, 0) PT_GEMM_NARROW(0, 0, 2) PT_GEMM_NARROW(0, 1, 1) PT_GEMM_NARROW(0, 1, 2) PT_GEMM_NARROW(1, 1, 1) PT_GEMM_NARROW(1, 1, 2)
+#undef PT_GEMM_NARROW
 #define PT_GEMM_CASE(AM, BMN, OM)                                                                             \
   if (a_mn == AM && b_mn == BMN && out_mode == OM)                                                            \
     return epi_tma ? launch<AM, BMN, OM, true>(ma, mb, md, D, M, N, K, ldd, st, stream, nullptr, ea)          \
@@ -1004,7 +1023,7 @@ extern "C" int pt_gemm_bf16_fused(const void* A, const void* B, void* D, int M, 
     return -11;
   }
   if (M <= 0 || n_out <= 0 || K <= 0) return 0;
-  const int bn = tile_columns(M, epi == EPI_SWIGLU_BWD ? inter : n_out, K);
+  const int bn = tile_columns(M, epi == EPI_SWIGLU_BWD ? inter : n_out, K, false);
   CUtensorMap ma, mb, md, mh;
   int rc;
   if ((rc = make_bf16_map_2d(&ma, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda, BK, BM))) return rc * 10 - 1;

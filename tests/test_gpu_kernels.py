@@ -120,6 +120,37 @@ def test_gemm_weight_gradient_parts_are_repeatable_and_rounded_once(C, M, N, K):
     assert err <= 2 ** -4 + 1e-5 * float(want.abs().max()), err
 
 
+@pytest.mark.parametrize("tile_n", [128, 256])
+@pytest.mark.parametrize("parts", [1, 2, 7])
+@pytest.mark.parametrize("M,N,K", [(8, 8, 1024), (264, 520, 448), (600, 584, 1000), (256, 128, 512), (1000, 72, 640)])
+def test_gemm_tile_widths_and_parts_of_every_layout(tile_n, parts, M, N, K):
+    """Both tile widths, unsplit and with K in parts (uneven ones, a last k-block of 8 to 40 rows, tiles beyond the matrix), for the
+    forward layout with and without a residual, input gradients and fp32 accumulation."""
+    from picotron_b200.ops import _ext
+    C = _ext.load()
+    C.set_gemm_pair(True)
+    C.set_gemm_tma_epilogue(True)
+    x, w, wt, res, xt = bf(M, K, seed=1), bf(N, K, seed=2), bf(K, N, seed=3), bf(M, N, seed=4), bf(K, M, seed=5)
+    acc = torch.full((M, N), 0.5, device="cuda")
+    try:
+        C.set_gemm_tile_n(tile_n)
+        if parts > 1:
+            C.set_gemm_split_parts(parts)
+        else:
+            C.set_gemm_split_dgrad(False)
+        C.gemm(xt, wt, True, True, acc, True)
+        got = [C.gemm(x, w, False, False), C.gemm_add(x, w, res), C.gemm(x, wt, False, True)]
+    finally:
+        C.set_gemm_tile_n(0)
+        C.set_gemm_split_parts(0)
+    _status_ok(C)
+    y = x.double() @ w.double().t()
+    for g, want in zip(got, [y, y + res.double(), x.double() @ wt.double()]):
+        assert _rel(g.double(), want) < 4e-3                  # one bf16 rounding of the result
+    # fp32 sums in another order (sqrt(K) * 2^-24 of their size) and 0.5 added to them
+    assert _rel(acc.double() - 0.5, xt.double().t() @ wt.double()) < 1e-5
+
+
 @pytest.mark.parametrize("T,N,K", [(64, 576, 49152), (500, 520, 16392), (300, 2048, 16384)])
 def test_gemm_input_gradient_parts_are_repeatable(C, T, N, K):
     from picotron_b200.ops import _ext
