@@ -507,14 +507,14 @@ struct BwdCfg {
   static constexpr int TILES = 2 * TILE_BYTES + (QSTAGES + OSTAGES) * TILE_BYTES + DS_BYTES + DQ_BYTES + STAT_BYTES;
   static constexpr int SMEM = TILES + 256;               // + barriers; the block starts 1024-byte aligned
   static constexpr int TMEM_COLS = 512;
-  // d = 64: everything has columns of its own. d = 128: P^T reuses the columns S^T was read from (each half of a row its own
-  // half of them) and dQ those of dP^T, so S and dP of the next step wait for dV and for the dQ drain.
+  // d = 64: everything has columns of its own. d = 128: P^T reuses the columns S^T was read from (each part of a row its own
+  // part of them) and dQ those of dP^T, so S and dP of the next step wait for dV and for the dQ drain.
   static constexpr bool SHARE = (D == 128);
   static constexpr int S_COL = 0, DP_COL = 128, DV_COL = 256, DK_COL = 256 + D;
   static constexpr int DQ_COL = SHARE ? DP_COL : 256 + 2 * D;
   static constexpr int P_COL = SHARE ? S_COL : 256 + 3 * D;
-  static constexpr int P_HALF = SHARE ? 64 : 32;         // columns between the two 64-query halves of P^T
-  static_assert(DQ_COL + D <= 512 && DK_COL + D <= 512 && P_COL + P_HALF + 32 <= 512, "TMEM budget");
+  // (the parts' P^T lie 128 / PARTS columns apart with SHARE, half of that without)
+  static_assert(DQ_COL + D <= 512 && DK_COL + D <= 512 && P_COL + (SHARE ? 128 : 64) <= 512, "TMEM budget");
   static_assert(SMEM <= 232448, "shared memory budget");
 };
 
@@ -541,11 +541,25 @@ struct BwdParams {
   unsigned long long* prof;      // optional phase counters, as AttnParams::prof
 };
 
-// warps 0-7 compute (two per TMEM lane quarter), 8-11 drain dQ, 12 TMA producer, 13 MMA issuer, 14 row statistics (15 idle)
-constexpr int BWD_THREADS = 512;
-// registers per thread: 128 at launch, then redistributed between the warpgroups (2 x compute + drain + the rest = 4 x 128)
+// A step's 128 query columns are dealt to PARTS warps per TMEM lane quarter (32 keys), W columns each: warps 0 .. 4 PARTS - 1 compute, then
+// four drain dQ, then TMA producer, MMA issuer, row statistics and an idle warp. Registers per thread are even at launch and then
+// redistributed between the warpgroups (PARTS x compute + drain + the rest).
+// Four parts for d = 64, two for d = 128. Cycles per step with two / four: d = 64, 1 x 32768, 32 / 8 heads 3,127 / 2,791, 4 x 1024, 32 heads
+// 3,620 / 3,370; us: 13,260 / 13,050 (the clock falls as the power cap is reached) and 119 / 114.5; d = 128: 1 x 8192, 32 / 8 heads 1,299 /
+// 1,420 us, 4 x 1024, 32 heads 200 / 207. With d = 64 the compute warps' latencies are the step, and twice as many of them hide more;
+// with d = 128 the MMAs are half of it, and the smaller batches of tensor-memory reads and the barriers that every MMA waits for
+// count more.
 constexpr int BWD_REGS = 128, BWD_REGS_COMPUTE = 160, BWD_REGS_DRAIN = 96, BWD_REGS_REST = 96;
-static_assert(2 * BWD_REGS_COMPUTE + BWD_REGS_DRAIN + BWD_REGS_REST <= 4 * BWD_REGS, "setmaxnreg must not ask for more than the launch gave");
+constexpr int BWD4_REGS = 80, BWD4_REGS_COMPUTE = 88, BWD4_REGS_DRAIN = 72, BWD4_REGS_REST = 56;
+template <int PARTS>
+struct BwdWarps {
+  static constexpr int W = 128 / PARTS, COMPUTE = 4 * PARTS, THREADS = 32 * (COMPUTE + 8);
+  static constexpr int REGS = PARTS == 4 ? BWD4_REGS : BWD_REGS, REGS_COMPUTE = PARTS == 4 ? BWD4_REGS_COMPUTE : BWD_REGS_COMPUTE;
+  static constexpr int REGS_DRAIN = PARTS == 4 ? BWD4_REGS_DRAIN : BWD_REGS_DRAIN, REGS_REST = PARTS == 4 ? BWD4_REGS_REST : BWD_REGS_REST;
+  static_assert(PARTS * REGS_COMPUTE + REGS_DRAIN + REGS_REST <= (PARTS + 2) * REGS, "setmaxnreg must not ask for more than the launch gave");
+  static_assert(THREADS * REGS <= 65536, "register file");
+};
+template <int D> constexpr int bwd_parts() { return D == 64 ? 4 : 2; }
 template <int N> __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
@@ -556,13 +570,14 @@ template <int N> __device__ __forceinline__ void regs_dec() { asm volatile("setm
 // dQ_i is drained by warps of their own. The scores are computed TRANSPOSED (lane = key): then P^T is written straight back to
 // tensor memory as the A operand of dV += P^T dO, and only dS^T goes through shared memory (which the MMAs read all the time).
 // Measured (us; 1 x 32768, 32 / 8 heads, d = 64; 1 x 8192, 32 / 8 heads, d = 128): 21,500 -> 16,200 and 2,160 -> 1,410.
-template <int D, bool OUT_F32, bool PROF>
-__global__ void __launch_bounds__(BWD_THREADS, 1)
-attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ KVSegs segs,
-                const __grid_constant__ CUtensorMap tm_do, const __grid_constant__ CUtensorMap tm_dq,
-                const float* __restrict__ LSE, const float* __restrict__ DELTA, void* __restrict__ dK_,
-                void* __restrict__ dV_, BwdParams p, KernelStatus* status) {
+template <int D, bool OUT_F32, bool PROF, int PARTS>
+__device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tm_q, const KVSegs& segs, const CUtensorMap& tm_do, const CUtensorMap& tm_dq,
+                                              const float* __restrict__ LSE, const float* __restrict__ DELTA, void* __restrict__ dK_,
+                                              void* __restrict__ dV_, const BwdParams& p, KernelStatus* status) {
   using Cfg = BwdCfg<D>;
+  using Warps = BwdWarps<PARTS>;
+  constexpr int W = Warps::W, CW = Warps::COMPUTE;
+  constexpr int P_PART = Cfg::SHARE ? W : W / 2;          // tensor-memory columns between the parts' P^T
   pdl_launch_dependents();
   // no static shared memory in this kernel: the dynamic block starts at the (1024-byte aligned) window base
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -604,15 +619,15 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(&bars.st_full[s], 32);
-      mbar_init(&bars.st_empty[s], 8);
+      mbar_init(&bars.st_empty[s], CW);
     }
     mbar_init(&bars.s_full, 1);
-    mbar_init(&bars.s_read, 8);        // compute -> MMA: one arrival per warp
-    mbar_init(&bars.p_ready, 8);
+    mbar_init(&bars.s_read, CW);        // compute -> MMA: one arrival per warp
+    mbar_init(&bars.p_ready, CW);
     mbar_init(&bars.p_free, 1);
     mbar_init(&bars.dp_full, 1);
-    mbar_init(&bars.dp_read, 8);
-    mbar_init(&bars.ds_ready, 8);
+    mbar_init(&bars.dp_read, CW);
+    mbar_init(&bars.ds_ready, CW);
     mbar_init(&bars.ds_free, 1);
     mbar_init(&bars.dq_full, 1);
     mbar_init(&bars.dq_read, 4);
@@ -626,7 +641,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     tma_prefetch_desc(&tm_do);
     tma_prefetch_desc(&tm_dq);
   }
-  if (warp == 13) {
+  if (warp == CW + 5) {
     tmem_alloc(&bars.tmem_base, Cfg::TMEM_COLS);
     tmem_relinquish();
   }
@@ -637,8 +652,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const uint32_t tmem_base = bars.tmem_base;
   volatile int* abort_flag = &bars.abort_flag;
 
-  if (warp >= 12) regs_dec<BWD_REGS_REST>();
-  if (warp == 12) {
+  if (warp >= CW + 4) regs_dec<Warps::REGS_REST>();
+  if (warp == CW + 4) {
     // ------------------------------------------------------------------------------ TMA producer
     if (total_steps > 0 && elect_one()) {
       mbar_expect_tx(&bars.kv_full, 2 * Cfg::TILE_BYTES);
@@ -663,7 +678,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           tma_load_4d(sdO + os * Cfg::TILE_BYTES + c * (Cfg::BM * 128), &tm_do, &bars.do_full[os], c * 64, head, q0, b);
       }
     }
-  } else if (warp == 13) {
+  } else if (warp == CW + 5) {
     // ------------------------------------------------------------------------------ MMA issuer
     if (total_steps > 0 && elect_one()) {
       constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, false, false);   // S^T, dP^T: [key, query], K-major operands
@@ -725,7 +740,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         const uint64_t do_mn = smem_desc_advance(do_mn0, (it % Cfg::OSTAGES) * Cfg::TILE_BYTES);
 #pragma unroll
         for (int kk = 0; kk < 128 / 16; ++kk)
-          umma_bf16_ts(tmem_base + Cfg::DV_COL, tmem_base + Cfg::P_COL + (kk >> 2) * Cfg::P_HALF + (kk & 3) * 8,
+          umma_bf16_ts(tmem_base + Cfg::DV_COL, tmem_base + Cfg::P_COL + kk / (W / 16) * P_PART + kk % (W / 16) * 8,
                        smem_desc_advance(do_mn, kk * 2048), idesc_kv, (it > 0 || kk > 0) ? 1u : 0u);
         umma_commit(&bars.p_free);
         umma_commit(&bars.do_empty[it % Cfg::OSTAGES]);
@@ -758,7 +773,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       }
       if (ok) umma_commit(&bars.acc_full);
     }
-  } else if (warp == 14) {
+  } else if (warp == CW + 6) {
     // ------------------------------------------------------------------------------ row statistics (lse, delta) of a step's queries
     for (int it = 0; it < total_steps; ++it) {
       const int st = it & 1;
@@ -782,14 +797,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       }
       mbar_arrive(&bars.st_full[st]);
     }
-  } else if (warp >= 8 && warp < 12) {
+  } else if (warp >= CW && warp < CW + 4) {
     // ------------------------------------------------------------------------------ dQ of every step -> fp32 workspace
     // Warp w owns 32 query rows: it stages 32 columns at a time in one of its two buffers and hands them to TMA reduce-adds.
-    regs_dec<BWD_REGS_DRAIN>();
+    regs_dec<Warps::REGS_DRAIN>();
     const int quarter = warp & 3;
     const uint32_t t_lane = tmem_base + (uint32_t(quarter * 32) << 16) + Cfg::DQ_COL;
     uint8_t* stg = sDQ + quarter * 8192;
-    const bool prof_on = PROF && p.prof != nullptr && threadIdx.x == 256;
+    const bool prof_on = PROF && p.prof != nullptr && threadIdx.x == CW * 32;
     long long pacc[2] = {0, 0};
     for (int it = 0; it < total_steps; ++it) {
       const int head = kv_head * group + it / steps_per_head;
@@ -798,29 +813,31 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       if (!mbar_wait(&bars.dq_full, it & 1, abort_flag)) { if (lane == 0) report_error(status, KID_BWD, 9); break; }
       tcgen05_fence_after();
       const long long pt1 = prof_clock(prof_on);
+      constexpr int DR = PARTS == 4 ? 32 : 64;              // columns read at a time: what the registers hold
 #pragma unroll
-      for (int r_ = 0; r_ < D / 64; ++r_) {
-        uint32_t r[64];
-        tmem_ld_32x32b_x32_at(t_lane + r_ * 64, r, 0);
-        tmem_ld_32x32b_x32_at(t_lane + r_ * 64 + 32, r, 32);
+      for (int r_ = 0; r_ < D / DR; ++r_) {
+        uint32_t r[DR];
+#pragma unroll
+        for (int h = 0; h < DR / 32; ++h) tmem_ld_32x32b_x32_at(t_lane + r_ * DR + h * 32, r, h * 32);
         tmem_ld_wait();
-        if (r_ == D / 64 - 1) {
+        if (r_ == D / DR - 1) {
           tcgen05_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(&bars.dq_read);
         }
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
+        for (int h = 0; h < DR / 32; ++h) {
+          uint8_t* const buf = stg + ((r_ * (DR / 32) + h) & 1) * 4096;
           if (elect_one()) tma_store_wait_read<1>();          // the reduce before the last has finished reading this buffer
           __syncwarp();
 #pragma unroll
           for (int u = 0; u < 8; ++u)
-            *reinterpret_cast<uint4*>(stg + h * 4096 + sw128_offset(lane, u)) =
+            *reinterpret_cast<uint4*>(buf + sw128_offset(lane, u)) =
                 make_uint4(r[h * 32 + 4 * u], r[h * 32 + 4 * u + 1], r[h * 32 + 4 * u + 2], r[h * 32 + 4 * u + 3]);
           fence_proxy_async_smem();
           __syncwarp();
           if (elect_one()) {
-            if (row0 < p.Sq) tma_reduce_add_4d(&tm_dq, stg + h * 4096, r_ * 64 + h * 32, head, row0, b);
+            if (row0 < p.Sq) tma_reduce_add_4d(&tm_dq, buf, r_ * DR + h * 32, head, row0, b);
             tma_store_commit();
           }
         }
@@ -832,13 +849,17 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       atomicAdd(&p.prof[2], (unsigned long long)pacc[0]);
       atomicAdd(&p.prof[3], (unsigned long long)pacc[1]);
     }
-  } else if (warp < 8) {
-    // ------------------------------------------------------------------------------ compute threads (warps 0..7)
-    regs_inc<BWD_REGS_COMPUTE>();
-    // Thread pair (t, t + 128) shares key k0 + t (TMEM lane t): `half` 0 owns query columns 0..63 of a step and
-    // the dV output, `half` 1 the rest and dK. Nothing has to be exchanged between the two.
+  } else if (warp < CW) {
+    // ------------------------------------------------------------------------------ compute threads (warps 0 .. 4 PARTS - 1)
+    regs_inc<Warps::REGS_COMPUTE>();
+    // The PARTS threads t, t + 128, ... share key k0 + t (TMEM lane t): part i owns query columns i W .. (i + 1) W - 1 of a step; the
+    // first half of the parts writes dV, the other dK (SUBS threads per row). Nothing has to be exchanged between them.
+    constexpr int SUBS = PARTS / 2;
     const int t = threadIdx.x & 127;
-    const int half = threadIdx.x >> 7;
+    const int part = threadIdx.x >> 7;
+    const int which = part / SUBS, sub = part % SUBS;      // 0: dV, 1: dK
+    // dS^T of this thread: W / 8 16-byte units of row t, the first at ds_off, the others an exclusive-or of their number away
+    const uint32_t ds_off = ((unsigned)(part * W) >> 6) * (128 * 128) + sw128_offset(t, ((unsigned)(part * W) & 63u) >> 3);
     const int quarter = warp & 3;
     const uint32_t t_lane = tmem_base + (uint32_t(quarter * 32) << 16);
     const uint64_t sl2_2 = pair_of(p.scale * LOG2E, p.scale * LOG2E), scale_2 = pair_of(p.scale, p.scale);
@@ -850,30 +871,30 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     for (int it = 0; it < total_steps; ++it) {
       const long long pt0 = prof_clock(prof_on);
       const uint32_t par = it & 1;
-      const int qcol0 = (qb_first + it % steps_per_head) * Cfg::BM + half * 64;     // first query of this thread's columns
+      const int qcol0 = (qb_first + it % steps_per_head) * Cfg::BM + part * W;     // first query of this thread's columns
       const bool need_mask = (diag && k0 + Cfg::BN - 1 > qcol0) || (k0 + Cfg::BN > p.Sk);
-      const int hidden = key >= p.Sk ? 64 : (diag ? key - qcol0 : 0);              // columns [0, hidden) do not see this key
-      const float* st_l = sStat + par * 2 * Cfg::BM + half * 64;
+      const int hidden = key >= p.Sk ? W : (diag ? key - qcol0 : 0);              // columns [0, hidden) do not see this key
+      const float* st_l = sStat + par * 2 * Cfg::BM + part * W;
       const float* st_d = st_l + Cfg::BM;
       if (!mbar_wait(&bars.st_full[par], (it >> 1) & 1, abort_flag)) { if (lane == 0) report_error(status, KID_BWD, 18); ok = false; break; }
       if (!mbar_wait(&bars.s_full, par, abort_flag)) { if (lane == 0) report_error(status, KID_BWD, 7); ok = false; break; }
       tcgen05_fence_after();
       const long long pt1 = prof_clock(prof_on);
-      uint32_t s[64];
-      tmem_ld_32x32b_x32_at(t_lane + Cfg::S_COL + half * 64, s, 0);
-      tmem_ld_32x32b_x32_at(t_lane + Cfg::S_COL + half * 64 + 32, s, 32);
+      uint32_t s[W];
+#pragma unroll
+      for (int h = 0; h < W / 32; ++h) tmem_ld_32x32b_x32_at(t_lane + Cfg::S_COL + part * W + h * 32, s, h * 32);
       tmem_ld_wait();
       if (!Cfg::SHARE) {
         tcgen05_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars.s_read);
       }
-      uint32_t pk[32];                        // P^T of this thread's 64 queries, bf16 pairs
+      uint32_t pk[W / 2];                     // P^T of this thread's queries, bf16 pairs
       // The masked and the plain form are separate code: a test of need_mask inside the loop costs a branch per element group,
       // which took the scheduler's freedom away (d = 64, 32768 keys: 26.7 ms with it, 17.2 without).
       auto exponentials = [&](auto masked) {
 #pragma unroll
-        for (int e = 0; e < 64; e += 4) {
+        for (int e = 0; e < W; e += 4) {
           const float4 lv = *reinterpret_cast<const float4*>(st_l + e);
           const uint64_t x0 = fma2(pair_of(__uint_as_float(s[e]), __uint_as_float(s[e + 1])), sl2_2, pair_of(lv.x, lv.y));
           const uint64_t x1 = fma2(pair_of(__uint_as_float(s[e + 2]), __uint_as_float(s[e + 3])), sl2_2, pair_of(lv.z, lv.w));
@@ -894,7 +915,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         if (!mbar_wait(&bars.p_free, par ^ 1, abort_flag)) { if (lane == 0) report_error(status, KID_BWD, 19); ok = false; break; }
         tcgen05_fence_after();
       }
-      tmem_st_32x32b_x32(t_lane + Cfg::P_COL + half * Cfg::P_HALF, pk);
+      if constexpr (W == 64) tmem_st_32x32b_x32(t_lane + Cfg::P_COL + part * P_PART, pk);
+      else tmem_st_32x32b_x16(t_lane + Cfg::P_COL + part * P_PART, pk);
       tmem_st_wait();
       tcgen05_fence_before();
       __syncwarp();
@@ -903,9 +925,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       if (!mbar_wait(&bars.dp_full, par, abort_flag)) { if (lane == 0) report_error(status, KID_BWD, 8); ok = false; break; }
       tcgen05_fence_after();
       const long long pt5 = prof_clock(prof_on);
-      uint32_t dp[64];
-      tmem_ld_32x32b_x32_at(t_lane + Cfg::DP_COL + half * 64, dp, 0);
-      tmem_ld_32x32b_x32_at(t_lane + Cfg::DP_COL + half * 64 + 32, dp, 32);
+      uint32_t dp[W];
+#pragma unroll
+      for (int h = 0; h < W / 32; ++h) tmem_ld_32x32b_x32_at(t_lane + Cfg::DP_COL + part * W + h * 32, dp, h * 32);
       tmem_ld_wait();
       if (!Cfg::SHARE) {
         tcgen05_fence_before();
@@ -913,7 +935,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         if (lane == 0) mbar_arrive(&bars.dp_read);
       }
 #pragma unroll
-      for (int e = 0; e < 64; e += 4) {
+      for (int e = 0; e < W; e += 4) {
         const float4 dv = *reinterpret_cast<const float4*>(st_d + e);
         const uint64_t d0 = mul2(pair_of(__uint_as_float(s[e]), __uint_as_float(s[e + 1])),
                                  fma2(pair_of(__uint_as_float(dp[e]), __uint_as_float(dp[e + 1])), scale_2, pair_of(dv.x, dv.y)));
@@ -925,8 +947,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       // the dQ and dK MMAs of the previous step have read its dS
       if (it > 0 && !mbar_wait(&bars.ds_free, par ^ 1, abort_flag)) { if (lane == 0) report_error(status, KID_BWD, 20); ok = false; break; }
 #pragma unroll
-      for (int u = 0; u < 8; ++u)
-        *reinterpret_cast<uint4*>(sdS + half * (128 * 128) + sw128_offset(t, u)) =
+      for (int u = 0; u < W / 8; ++u)
+        *reinterpret_cast<uint4*>(sdS + (ds_off ^ (uint32_t)(u << 4))) =
             make_uint4(pk[4 * u], pk[4 * u + 1], pk[4 * u + 2], pk[4 * u + 3]);
       tcgen05_fence_before();                 // (also orders the reads of dP before the dQ MMA that may reuse its columns)
       fence_proxy_async_smem();
@@ -950,9 +972,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     // dK, dV of this key block (thread t <-> key k0 + t); fp32 when they are partials of a multi-rank reduction
     const long long seg_off = (long long)seg * p.seg_stride;
     if (total_steps == 0) {
-      if (key < p.Sk) {
+      if (key < p.Sk && sub == 0) {
         {
-          const int which = half;                  // half 0 writes dV, half 1 writes dK
           const long long rs_ = which == 0 ? p.dv_row : p.dk_row;
           const long long off = seg_off + ((long long)b * p.Sk + key) * rs_ + (long long)kv_head * D;
           if (OUT_F32) {
@@ -966,44 +987,50 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       }
     } else if (ok && mbar_wait(&bars.acc_full, 0, abort_flag)) {
       tcgen05_fence_after();
-      if (!OUT_F32 && half == 1 && p.cosT != nullptr) {
-        // dK with the inverse rotation: the whole row (D columns) in registers, pairs j <-> j + D/2
-        uint32_t r[D];
+      if (!OUT_F32 && which == 1 && p.cosT != nullptr) {
+        // dK with the inverse rotation: pairs j <-> j + D/2, 16 columns of each half of the row at a time
+        const int row = key < p.Sk ? key : 0, pos = row % p.rope_seq;
+        const float* cos_row = p.cosT + (long long)pos * (D / 2);
+        const float* sin_row = p.sinT + (long long)pos * (D / 2);
+        bf16* orow = reinterpret_cast<bf16*>(dK_) + seg_off + ((long long)b * p.Sk + row) * p.dk_row + (long long)kv_head * D;
+        auto store16 = [](bf16* dst, const uint32_t (&r)[16]) {
 #pragma unroll
-        for (int c = 0; c < D / 32; ++c) tmem_ld_32x32b_x32_at(t_lane + Cfg::DK_COL + c * 32, r, c * 32);
-        tmem_ld_wait();
-        if (key < p.Sk) {
-          const int pos = key % p.rope_seq;
-          const float* cos_row = p.cosT + (long long)pos * (D / 2);
-          const float* sin_row = p.sinT + (long long)pos * (D / 2);
-#pragma unroll
-          for (int j = 0; j < D / 2; j += 4) {
-            const float4 cs = __ldg(reinterpret_cast<const float4*>(cos_row + j));
-            const float4 sn = __ldg(reinterpret_cast<const float4*>(sin_row + j));
-            const float csv[4] = {cs.x, cs.y, cs.z, cs.w}, snv[4] = {sn.x, sn.y, sn.z, sn.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const float a = __uint_as_float(r[j + i]), b = __uint_as_float(r[j + i + D / 2]);
-              r[j + i] = __float_as_uint(a * csv[i] + b * snv[i]);
-              r[j + i + D / 2] = __float_as_uint(b * csv[i] - a * snv[i]);
-            }
-          }
-          bf16* orow = reinterpret_cast<bf16*>(dK_) + seg_off + ((long long)b * p.Sk + key) * p.dk_row + (long long)kv_head * D;
-#pragma unroll
-          for (int u = 0; u < D / 8; ++u)
-            reinterpret_cast<uint4*>(orow)[u] =
+          for (int u = 0; u < 2; ++u)
+            reinterpret_cast<uint4*>(dst)[u] =
                 make_uint4(pack_bf16(__uint_as_float(r[8 * u]), __uint_as_float(r[8 * u + 1])),
                            pack_bf16(__uint_as_float(r[8 * u + 2]), __uint_as_float(r[8 * u + 3])),
                            pack_bf16(__uint_as_float(r[8 * u + 4]), __uint_as_float(r[8 * u + 5])),
                            pack_bf16(__uint_as_float(r[8 * u + 6]), __uint_as_float(r[8 * u + 7])));
+        };
+#pragma unroll 1
+        for (int c = sub; c < D / 32; c += SUBS) {
+          uint32_t lo[16], hi[16];
+          tmem_ld_32x32b_x16(t_lane + Cfg::DK_COL + c * 16, lo);
+          tmem_ld_32x32b_x16(t_lane + Cfg::DK_COL + D / 2 + c * 16, hi);
+          tmem_ld_wait();
+          if (key < p.Sk) {
+#pragma unroll
+            for (int j = 0; j < 16; j += 4) {
+              const float4 cs = __ldg(reinterpret_cast<const float4*>(cos_row + c * 16 + j));
+              const float4 sn = __ldg(reinterpret_cast<const float4*>(sin_row + c * 16 + j));
+              const float csv[4] = {cs.x, cs.y, cs.z, cs.w}, snv[4] = {sn.x, sn.y, sn.z, sn.w};
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const float a = __uint_as_float(lo[j + i]), b = __uint_as_float(hi[j + i]);
+                lo[j + i] = __float_as_uint(a * csv[i] + b * snv[i]);
+                hi[j + i] = __float_as_uint(b * csv[i] - a * snv[i]);
+              }
+            }
+            store16(orow + c * 16, lo);
+            store16(orow + D / 2 + c * 16, hi);
+          }
         }
       } else {
-        const int which = half;                    // half 0 writes dV, half 1 writes dK
         const long long rs_ = which == 0 ? p.dv_row : p.dk_row;
         const int col_base = which == 0 ? Cfg::DV_COL : Cfg::DK_COL;
         const long long off = seg_off + ((long long)b * p.Sk + (key < p.Sk ? key : 0)) * rs_ + (long long)kv_head * D;
 #pragma unroll 1
-        for (int c = 0; c < D / 32; ++c) {
+        for (int c = sub; c < D / 32; c += SUBS) {
           uint32_t r[32];
           tmem_ld_32x32b_x32(t_lane + col_base + c * 32, r);
           tmem_ld_wait();
@@ -1039,11 +1066,26 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     for (int i = 0; i < 2000; ++i) __nanosleep(1000);
     __syncthreads();
   }
-  if (warp == 13) {
+  if (warp == CW + 5) {
     tcgen05_fence_after();
     tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
   }
 }
+
+#define PT_BWD_PARAMS                                                                                                           \
+  const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ KVSegs segs, const __grid_constant__ CUtensorMap tm_do,      \
+      const __grid_constant__ CUtensorMap tm_dq, const float* __restrict__ LSE, const float* __restrict__ DELTA,                 \
+      void* __restrict__ dK_, void* __restrict__ dV_, const __grid_constant__ BwdParams p, KernelStatus* status
+// (two kernels, because the build checks their register counts by name)
+template <int D, bool OUT_F32, bool PROF>
+__global__ void __launch_bounds__(BwdWarps<2>::THREADS, 1) attn_bwd_kernel(PT_BWD_PARAMS) {
+  attn_bwd_body<D, OUT_F32, PROF, 2>(tm_q, segs, tm_do, tm_dq, LSE, DELTA, dK_, dV_, p, status);
+}
+template <int D, bool OUT_F32, bool PROF>
+__global__ void __launch_bounds__(BwdWarps<4>::THREADS, 1) attn_bwd_parts4_kernel(PT_BWD_PARAMS) {
+  attn_bwd_body<D, OUT_F32, PROF, 4>(tm_q, segs, tm_do, tm_dq, LSE, DELTA, dK_, dV_, p, status);
+}
+#undef PT_BWD_PARAMS
 
 // ---------------------------------------------------------------------------------------------------------
 // host side
@@ -1080,20 +1122,24 @@ static int launch_bwd(const CUtensorMap& mq, const KVSegs& segs, const CUtensorM
                       const float* delta, void* dk, void* dv, const BwdParams& p, KernelStatus* st, cudaStream_t stream) {
   if (!PROF && p.prof != nullptr)
     return launch_bwd<D, OUT_F32, true>(mq, segs, mdo, mdq, lse, delta, dk, dv, p, st, stream);
-  auto kern = attn_bwd_kernel<D, OUT_F32, PROF>;
+  using Warps = BwdWarps<bwd_parts<D>()>;
+  auto kern = [] {
+    if constexpr (bwd_parts<D>() == 4) return attn_bwd_parts4_kernel<D, OUT_F32, PROF>;
+    else return attn_bwd_kernel<D, OUT_F32, PROF>;
+  }();
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdCfg<D>::SMEM) != cudaSuccess) return -3;
     cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    // the warpgroups share out BWD_REGS registers per thread; with fewer at launch setmaxnreg.inc would wait forever (the build
+    // the warpgroups share out Warps::REGS registers per thread; with fewer at launch setmaxnreg.inc would wait forever (the build
     // fails for another count, build.py: FIXED_REGISTERS)
     cudaFuncAttributes fa;
-    if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess || fa.numRegs != BWD_REGS) return -6;
+    if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess || fa.numRegs != Warps::REGS) return -6;
     configured = true;
   }
   const int num_kb = ((p.Sk + 127) / 128) * p.n_segs;
   const long long grid = (long long)num_kb * p.hkv * p.B;
-  launch_pdl(kern, dim3((unsigned)grid), dim3(BWD_THREADS), BwdCfg<D>::SMEM, stream, mq, segs, mdo, mdq, lse, delta, dk, dv, p, st);
+  launch_pdl(kern, dim3((unsigned)grid), dim3(Warps::THREADS), BwdCfg<D>::SMEM, stream, mq, segs, mdo, mdq, lse, delta, dk, dv, p, st);
   pt_count_launches(1);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
