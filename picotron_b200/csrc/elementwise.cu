@@ -622,6 +622,9 @@ static inline int check_launch(int n = 1) {
 // and now, us, launch included: forward / with add / backward of 8192 x 576: 15.2 -> 11.3 / 17.5 -> 15.0 / 27.6 -> 17.5;
 // 4096 x 960: 12.3 -> 10.2 / 14.4 / 20.6 -> 16.4; 4096 x 2048: 14.3 / 20.5 -> 18.5 / 24.6 -> 22.6; wide rows gain nothing: 4096 x
 // 4096: 20.5 -> 21.4 / 30.7 / 41.9 -> 43.0, 32768 x 2048: 56.3 -> 59.4 / 95.1 -> 94.2 / 110.6 -> 104.4.)
+// The backward's next rows travel through shared memory while one is reduced (its rows were one load latency after the other): without /
+// with, inputs not in L2: 8192 x 576: 11.5 -> 10.5, 4096 x 960: 10.6 -> 9.3, 4096 x 2048: 16.3 -> 15.4, 8192 x 4096: 58.1 -> 52.5, 32768 x
+// 2048: 95.1 -> 83.0 (6.5 TB/s); few rows (512 x 2048: 5.1 -> 5.0) have nothing to fetch ahead.
 // ---------------------------------------------------------------------------------------------
 constexpr int ROWS_THREADS = 256;
 
@@ -730,6 +733,17 @@ rmsnorm_fwd_rows_kernel(const bf16* __restrict__ x, const bf16* __restrict__ del
   }
 }
 
+// Backward: a team has the next rows' operands on their way into shared memory (cp.async, every thread the chunks it will use itself, so
+// no barrier is needed) while it works on one. Rows in flight per team, and the bytes that takes per CTA.
+template <int NC> __host__ __device__ constexpr int bwd_stages() { return NC <= 1 ? 4 : NC == 2 ? 3 : 2; }
+template <int TEAM, int NC> __host__ __device__ constexpr int bwd_smem() {
+  const int pipe = bwd_stages<NC>() * 3 * NC * ROWS_THREADS * 16, comb = TEAM < ROWS_THREADS ? ROWS_THREADS * NC * 32 : 0;
+  return pipe > comb ? pipe : comb;
+}
+__device__ __forceinline__ void cp_async16(void* smem, const void* g) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem)), "l"(g) : "memory");
+}
+
 template <int TEAM, int NC>
 __global__ void __launch_bounds__(ROWS_THREADS, NC <= 2 ? 3 : 2)
 rmsnorm_bwd_rows_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, const bf16* __restrict__ w,
@@ -737,7 +751,8 @@ rmsnorm_bwd_rows_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x,
                         float* __restrict__ dw_acc, int T, int H) {
   constexpr int TEAMS = ROWS_THREADS / TEAM;
   __shared__ __align__(16) float red[2 * TEAMS * 8];
-  __shared__ __align__(16) float comb[TEAMS > 1 ? TEAMS * TEAM * NC * 8 : 4];
+  constexpr int STAGES = bwd_stages<NC>();
+  extern __shared__ __align__(16) uint4 pipe[];      // [stage][x, dy, dres][chunk][thread]; after the rows the teams' sums
   pdl_enter();
   const int nchunk = H / 8, tid = threadIdx.x % TEAM, team = threadIdx.x / TEAM;
   bf16x8 wv[NC];
@@ -749,27 +764,49 @@ rmsnorm_bwd_rows_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x,
 #pragma unroll
     for (int j = 0; j < 8; ++j) dwacc[i][j] = 0.f;
   }
-  int it = 0;
-  for (long long row = (long long)blockIdx.x * TEAMS + team; row < T; row += (long long)gridDim.x * TEAMS, ++it) {
-    bf16x8 px[NC], pdy[NC], pr[NC];
-    const float rstd = rstd_in[row];
+  const long long step = (long long)gridDim.x * TEAMS;
+  auto fetch = [&](long long row, int stage) {
+    if (row < T) {
 #pragma unroll
-    for (int i = 0; i < NC; ++i) {
-      const int c = tid + i * TEAM;
-      if (c < nchunk) {
-        px[i] = *reinterpret_cast<const bf16x8*>(x + row * H + c * 8);
-        pdy[i] = *reinterpret_cast<const bf16x8*>(dy + row * H + c * 8);
-        if (dres != nullptr) pr[i] = *reinterpret_cast<const bf16x8*>(dres + row * H + c * 8);
+      for (int i = 0; i < NC; ++i) {
+        const int c = tid + i * TEAM;
+        if (c < nchunk) {
+          uint4* const q = pipe + (stage * 3 * NC + i) * ROWS_THREADS + threadIdx.x;
+          cp_async16(q, x + row * H + c * 8);
+          cp_async16(q + NC * ROWS_THREADS, dy + row * H + c * 8);
+          if (dres != nullptr) cp_async16(q + 2 * NC * ROWS_THREADS, dres + row * H + c * 8);
+        }
       }
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  long long row = (long long)blockIdx.x * TEAMS + team;
+#pragma unroll
+  for (int st = 0; st + 1 < STAGES; ++st) fetch(row + st * step, st);
+  float rstd_next = row < T ? rstd_in[row] : 0.f;
+  int stage = 0;
+  for (int it = 0; row < T; row += step, ++it) {
+    fetch(row + (STAGES - 1) * step, stage == 0 ? STAGES - 1 : stage - 1);
+    const float rstd = rstd_next;
+    if (row + step < T) rstd_next = rstd_in[row + step];
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
+    // (read again for the second pass, instead of held in registers)
+    const uint4* const cur = pipe + stage * 3 * NC * ROWS_THREADS + threadIdx.x;
+    auto operand = [&](int which, int i) {
+      uint4 v;
+      asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                   : "r"(smem_u32(cur + (which * NC + i) * ROWS_THREADS)) : "memory");
+      return *reinterpret_cast<const bf16x8*>(&v);
+    };
+    stage = stage + 1 == STAGES ? 0 : stage + 1;
     float dot[accs<TEAM, NC>()] = {};
 #pragma unroll
     for (int i = 0; i < NC; ++i) {
       const int c = tid + i * TEAM;
       if (c < nchunk) {
         float xv[8], dv[8], ww[8];
-        unpack8(px[i], xv);
-        unpack8(pdy[i], dv);
+        unpack8(operand(0, i), xv);
+        unpack8(operand(1, i), dv);
         unpack8(wv[i], ww);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -785,14 +822,14 @@ rmsnorm_bwd_rows_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x,
       const int c = tid + i * TEAM;
       if (c < nchunk) {
         float xv[8], dv[8], ww[8], o[8];
-        unpack8(px[i], xv);
-        unpack8(pdy[i], dv);
+        unpack8(operand(0, i), xv);
+        unpack8(operand(1, i), dv);
         unpack8(wv[i], ww);
 #pragma unroll
         for (int j = 0; j < 8; ++j) o[j] = (dv[j] * ww[j] - xv[j] * rstd * cmean) * rstd;
         if (dres != nullptr) {
           float rr[8];
-          unpack8(pr[i], rr);
+          unpack8(operand(2, i), rr);
 #pragma unroll
           for (int j = 0; j < 8; ++j) o[j] += rr[j];
         }
@@ -813,6 +850,9 @@ rmsnorm_bwd_rows_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x,
       }
     }
   } else {
+    float* const comb = reinterpret_cast<float*>(pipe);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
 #pragma unroll
     for (int i = 0; i < NC; ++i) {
       float4* q = reinterpret_cast<float4*>(comb + (team * TEAM * NC + tid + i * TEAM) * 8);
@@ -931,12 +971,21 @@ extern "C" int pt_rmsnorm_bwd_acc(const void* dy, const void* x, const void* w, 
                                   void* dx, float* dw_acc, int T, int H, int num_sms, cudaStream_t st) {
   if (H % 8 || H > 8 * ROWS_THREADS * 4 || (reinterpret_cast<uintptr_t>(dw_acc) & 15)) return 1;
   if (T == 0) return 0;
+  bool failed = false;
   with_backward_team(H, [&](auto team, auto nc) {
     constexpr int TEAM = decltype(team)::value, NC = decltype(nc)::value, ROWS = ROWS_THREADS / TEAM;
     const int want = (T + ROWS - 1) / ROWS, cap = (NC <= 2 ? 3 : 2) * num_sms;
-    launch_pdl(rmsnorm_bwd_rows_kernel<TEAM, NC>, dim3((unsigned)(want < cap ? want : cap)), dim3(ROWS_THREADS), 0, st,
+    auto kern = rmsnorm_bwd_rows_kernel<TEAM, NC>;
+    constexpr int SMEM = bwd_smem<TEAM, NC>();
+    static const cudaError_t configured = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    if (configured != cudaSuccess) {
+      failed = true;
+      return;
+    }
+    launch_pdl(kern, dim3((unsigned)(want < cap ? want : cap)), dim3(ROWS_THREADS), SMEM, st,
                (const bf16*)dy, (const bf16*)x, (const bf16*)w, rstd, (const bf16*)dres, (bf16*)dx, dw_acc, T, H);
   });
+  if (failed) return -3;
   return check_launch();
 }
 

@@ -370,6 +370,23 @@ def test_rmsnorm_at_the_edges_of_its_team_sizes(C, T, H):
     torch.testing.assert_close(acc - 0.5, dw_ref, rtol=1e-4, atol=1e-5 * T ** 0.5 * 16)
 
 
+@pytest.mark.parametrize("residual", [True, False])
+@pytest.mark.parametrize("T,H", [(9001, 256), (9001, 576), (9001, 960), (4000, 1032), (3000, 4104)])
+def test_rmsnorm_backward_with_rows_fetched_ahead(C, T, H, residual):
+    """Enough rows for every team to go round its ring of fetched rows more than once, the last round partly filled."""
+    x, dy = bf(T, H, seed=1), bf(T, H, seed=2)
+    dres = bf(T, H, seed=3) if residual else None
+    w = (1 + 0.1 * bf(H, seed=4).float()).to(torch.bfloat16)
+    rstd = 0.5 + torch.rand(T, device="cuda", generator=torch.Generator(device="cuda").manual_seed(5))
+    acc = torch.full((H,), 0.5, device="cuda")
+    dx, _ = C.rmsnorm_bwd(dy, x, w, rstd, dres, acc)
+    _status_ok(C)
+    dx_ref, dw_ref = ref.rmsnorm_bwd(dy, x, w, rstd, dres)
+    # fp32 terms of size up to 1.5 |dy| + |dres|, rounded once to bf16; T terms of size 1.5 |dy x| in fp32, in any order
+    torch.testing.assert_close(dx.float(), dx_ref.float(), rtol=2 ** -7, atol=4e-3)
+    torch.testing.assert_close(acc - 0.5, dw_ref, rtol=1e-4, atol=2e-5 * T ** 0.5 * 16)
+
+
 def _row_sum_in_kernel_order(terms):
     """Sum over the last dimension of an fp32 CPU tensor in the RMSNorm kernels' order: running sums over the 8-element chunks
     c, c + 256, ..., a butterfly over 32 neighbouring ones, then the eight warp sums."""
