@@ -861,7 +861,7 @@ static int run_pair(const void* A, const void* B, void* D, int M, int N, int K, 
 
 // How many parts K is split into (1: not at all) and the columns of a tile then, by gemm_us; adding the weight gradient to what is
 // there costs 0.08 us a megabyte more in the GEMM's epilogue than in the summing kernel; an input gradient clears its slices first. A
-// split has to give 3 %.
+// split has to give 3 %, or 15 % (2048 x 2048 x 49152 on 64 whole tiles: 282 us, in parts 300).
 extern "C" int pt_gemm_split_parts(int M, int N, int K, int kind, int* tile_n) {
   using namespace pt::gemm_pair;
   *tile_n = g_tile_n ? g_tile_n : 256;
@@ -870,7 +870,9 @@ extern "C" int pt_gemm_split_parts(int M, int N, int K, int kind, int* tile_n) {
   const int kb = (K + BK - 1) / BK;
   if (g_split_k > 1) return g_split_k < kb ? g_split_k : kb;
   if (g_tile_n) return 1;                  // (a width given for a measurement: of whole tiles)
-  double best = 0.97 * (gemm_us(M, N, K, tile_columns(M, N, K, wgrad), 1, wgrad) + (wgrad ? 0.08 * M * N * 4e-6 : 0.0));
+  // (where whole tiles fill more than half of the pairs, what is left to gain is less than what parts at different K cost in L2 reuse)
+  const bool few = 2LL * ((M + 2 * BM - 1) / (2 * BM)) * ((N + 255) / 256) <= num_pairs();
+  double best = (few ? 0.97 : 0.85) * (gemm_us(M, N, K, tile_columns(M, N, K, wgrad), 1, wgrad) + (wgrad ? 0.08 * M * N * 4e-6 : 0.0));
   int best_parts = 1;
   for (const int parts : {2, 3, 4, 5, 6, 8, 10, 12, 16, 20, 24, 32}) {
     if (kb / parts < 2) break;
