@@ -23,7 +23,8 @@
 // this key block, pipelined over the steps (attn_bwd_kernel):
 //   S^T = K Q^T and dP^T = V dO^T into TMEM; threads (one key each) form P^T = exp2(S^T*c - lse), stored as bf16 into TMEM, and
 //   dS^T = P^T*(dP^T - delta)*scale, stored as bf16 into swizzled shared memory; then dV += P^T dO, dK += dS^T Q (TMEM
-//   accumulators that live for the whole CTA) and dQ = dS K, which four warps add to an fp32 workspace with TMA reduce-adds.
+//   accumulators that live for the whole CTA) and dQ = dS K, which four warps add to an fp32 workspace with TMA reduce-adds. Eight
+//   (d = 128) or sixteen (d = 64) warps compute.
 //   A small kernel computes delta = rowsum(dO*O) beforehand and another converts the fp32 dQ to bf16.
 #include "common.cuh"
 #include "tensormap.cuh"

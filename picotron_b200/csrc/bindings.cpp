@@ -585,7 +585,7 @@ std::vector<Tensor> attention_bwd(const Tensor& dout, const Tensor& q, const Ten
 // A decoder layer's launches in one call (one GPU per layer: no tensor, sequence or context parallelism). Small models and
 // short sequences are bound by the host: from Python every launch costs 12 to 20 us, more than most of their kernels take, and with
 // a tensor object per operand one native call still took 75 us per layer, half of it allocations, views and tensor bookkeeping.
-// So what the backward needs lies in TWO allocations (bf16 and fp32), addressed by offsets. The kernels, their order and the
+// (43 us of it in the native call, 26 as it is now.) So what the backward needs lies in TWO allocations (bf16 and fp32), addressed by offsets. The kernels, their order and the
 // fallbacks are those of the layer node's Python path.
 // ---------------------------------------------------------------------------------------------
 struct LayerDims {

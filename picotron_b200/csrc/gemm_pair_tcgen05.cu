@@ -1,7 +1,7 @@
 // bf16 GEMM for sm_100a on CTA pairs (tcgen05 cta_group::2): D[M,N] = op(A) * op(B), fp32 accumulate in TMEM.
 //
 // Same contract and operand layouts as gemm_tcgen05.cu, but two CTAs (a cluster of 2 on neighbouring SMs)
-// cooperate on one 256x256 output tile (256x128 where such tiles still give one wave): each CTA loads its own 128 rows of A
+// cooperate on one 256x256 or 256x128 output tile (see gemm_us for which): each CTA loads its own 128 rows of A
 // and its own half of the columns of
 // B -- with plain, non-multicast TMA loads -- and one thread of the leader CTA issues a 256-row MMA that
 // reads both CTAs' shared memory and writes both CTAs' tensor memory. Per output element this moves a
@@ -22,7 +22,7 @@
 // warp) and one lane hands it to TMA: a tiled store for bf16 / fp32 outputs, a tiled reduce-add for the
 // "accumulate into an fp32 destination" mode, so the weight-gradient GEMMs never read their destination into
 // the SM. TMA clips rows and columns beyond M and N. The older epilogue (each thread storing its own row with
-// 16-byte stores, read-modify-write for the accumulate mode) is kept as a template variant. Gradient GEMMs of few tiles split K
+// 16-byte stores, read-modify-write for the accumulate mode) is kept as a template variant. GEMMs of few tiles split K
 // over several CTA pairs, which write slices of a workspace that a small kernel sums (pt_gemm_bf16_split).
 //
 // Fused epilogues (forward GEMMs X W^T with bf16 output only):
@@ -45,6 +45,7 @@
 #include "common.cuh"
 #include "tensormap.cuh"
 
+#include <algorithm>
 #include <type_traits>
 
 extern "C" void pt_count_launches(int n);
@@ -861,7 +862,9 @@ static int run_pair(const void* A, const void* B, void* D, int M, int N, int K, 
 
 // How many parts K is split into (1: not at all) and the columns of a tile then, by gemm_us; adding the weight gradient to what is
 // there costs 0.08 us a megabyte more in the GEMM's epilogue than in the summing kernel; an input gradient clears its slices first. A
-// split has to give 3 %, or 15 % (2048 x 2048 x 49152 on 64 whole tiles: 282 us, in parts 300).
+// split has to give 3 %, or 15 % (2048 x 2048 x 128256 on 64 whole tiles: 724 us, in parts 760), and a forward GEMM 2 us more: its second
+// launch costs the host 3.5, and passes of small forward GEMMs are bound by the host (256 x 576 x 1536 is 8.7 us whole and 7.6 in five
+// parts; the forward pass of the 135M shape on 256 tokens, with 30 of them, took 1,590 us with whole ones and 1,740 with parts).
 extern "C" int pt_gemm_split_parts(int M, int N, int K, int kind, int* tile_n) {
   using namespace pt::gemm_pair;
   *tile_n = g_tile_n ? g_tile_n : 256;
@@ -872,7 +875,8 @@ extern "C" int pt_gemm_split_parts(int M, int N, int K, int kind, int* tile_n) {
   if (g_tile_n) return 1;                  // (a width given for a measurement: of whole tiles)
   // (where whole tiles fill more than half of the pairs, what is left to gain is less than what parts at different K cost in L2 reuse)
   const bool few = 2LL * ((M + 2 * BM - 1) / (2 * BM)) * ((N + 255) / 256) <= num_pairs();
-  double best = (few ? 0.97 : 0.85) * (gemm_us(M, N, K, tile_columns(M, N, K, wgrad), 1, wgrad) + (wgrad ? 0.08 * M * N * 4e-6 : 0.0));
+  const double whole = gemm_us(M, N, K, tile_columns(M, N, K, wgrad), 1, wgrad) + (wgrad ? 0.08 * M * N * 4e-6 : 0.0);
+  double best = (few ? 0.97 : 0.85) * whole - (kind == SPLIT_FWD ? 2.0 : 0.0);
   int best_parts = 1;
   for (const int parts : {2, 3, 4, 5, 6, 8, 10, 12, 16, 20, 24, 32}) {
     if (kb / parts < 2) break;
