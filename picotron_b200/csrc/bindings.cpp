@@ -988,7 +988,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("set_gemm_split_parts", [](int64_t n) { pt_gemm_set_split_k(n > 1 ? (int)n : 1); },
         "GEMMs that may be split over K are always cut into n parts by this thread (tests, measurements); 0 or 1: the rule.");
   m.def("set_gemm_tile_n", [](int64_t n) { pt_gemm_set_tile_n((int)n); },
-        "columns of the GEMM output tiles: 128, 256, or 0 for the choice by shape (bf16 outputs; for the calling thread)");
+        "columns of the GEMM output tiles: 128, 192 (where the epilogue has it), 256, or 0 for the choice by shape (for the calling thread)");
   m.def("get_gemm_group_m", []() { return (int64_t)pt_gemm_get_group_m(); });
   m.def("attention_set_profile", [](const c10::optional<Tensor>& counters) {
           if (!counters.has_value()) { pt_attention_set_profile(nullptr); return; }

@@ -68,8 +68,10 @@ enum Epilogue { EPI_NONE = 0, EPI_SWIGLU = 1, EPI_ROPE64 = 2, EPI_ROPE128 = 3, E
 __host__ __device__ constexpr int stages_of(int epi) { return epi == EPI_SWIGLU_BWD ? 5 : 6; }
 __host__ __device__ constexpr int staging_bufs_of(int epi) { return epi == EPI_SWIGLU_BWD ? 4 : 2; }
 // a stage holds BM x BK of A and bn / 2 x BK of B; four epilogue warps stage [32 rows][128 B] per buffer
+// (MN-major operands come in boxes of 64 columns: 192-column tiles fetch 128 columns per CTA and use 96)
+__host__ __device__ constexpr int b_bytes_of(int bn) { return (bn / 2 + 63) / 64 * 64 * BK * 2; }
 __host__ __device__ constexpr int smem_bytes_of(int epi, int bn) {
-  return stages_of(epi) * (A_BYTES + bn / 2 * BK * 2) + 4 * staging_bufs_of(epi) * 4096 + 1024;
+  return stages_of(epi) * (A_BYTES + b_bytes_of(bn)) + 4 * staging_bufs_of(epi) * 4096 + 1024;
 }
 
 struct EpiArgs {
@@ -137,9 +139,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                  void* __restrict__ Dptr, int M, int N, int K, long long ldd, KernelStatus* status, EpiArgs ea) {
   static_assert(EPI == EPI_NONE || (EPI_TMA && !A_MN && OUT_MODE == OUT_BF16 && B_MN == (EPI == EPI_SWIGLU_BWD)),
                 "fused epilogues: bf16 output; forward layout, except the SwiGLU backward which rides on the dgrad layout");
-  static_assert(BN == 256 || (BN == 128 && EPI_TMA && EPI != EPI_CE), "narrow tiles: the epilogues through TMA, but for the statistics");
+  static_assert(BN == 256 || (BN == 128 && EPI_TMA && EPI != EPI_CE) ||
+                    (BN == 192 && EPI_TMA && (EPI == EPI_NONE || EPI == EPI_ADD || EPI == EPI_SWIGLU_BWD)),
+                "narrow tiles: the epilogues through TMA, but for the statistics; 192 columns: where 64-column chunks are independent");
   constexpr int BN_HALF = BN / 2;                 // columns of B per CTA
-  constexpr int B_BYTES = BN_HALF * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
+  constexpr int B_BYTES = b_bytes_of(BN), STAGE_BYTES = A_BYTES + B_BYTES;
+  constexpr int LOAD_BYTES = A_BYTES + (B_MN ? B_BYTES : BN_HALF * BK * 2);      // what the loads of a stage bring
   constexpr int STAGES = stages_of(EPI);          // shadows the namespace constant: the variants differ in their smem split
   pdl_launch_dependents();
   extern __shared__ uint8_t smem_raw[];
@@ -215,7 +220,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
             break;
           }
           const uint32_t full_leader = mapa_u32(smem_u32(&bars.full[stage]), 0);
-          if (rank == 0) mbar_expect_tx(&bars.full[stage], 2 * STAGE_BYTES);
+          if (rank == 0) mbar_expect_tx(&bars.full[stage], 2 * LOAD_BYTES);
           uint8_t* sa = smem_a + stage * A_BYTES;
           uint8_t* sb = smem_b + stage * B_BYTES;
           if (!A_MN) {
@@ -229,7 +234,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
             tma_load_2d_pair(sb, &tma_b, full_leader, kb * BK, col0);
           } else {
 #pragma unroll
-            for (int c = 0; c < BN_HALF / 64; ++c)
+            for (int c = 0; c < B_BYTES / (BK * 128); ++c)
               tma_load_2d_pair(sb + c * (BK * 128), &tma_b, full_leader, col0 + c * 64, kb * BK);
           }
           if (++stage == STAGES) {
@@ -754,7 +759,7 @@ static int num_pairs() {
 
 // Switches for tests and measurements, of the calling thread only: other threads' launches keep the rules.
 static thread_local int g_split_k = 1;   // 0: never, 1: by pt_gemm_split_parts' rule, n > 1: always n parts
-static thread_local int g_tile_n = 0;    // 0: by the rule below, 128 / 256: as given (tests, measurements)
+static thread_local int g_tile_n = 0;    // 0: by the rule below, 128 / 192 / 256: as given (tests, measurements)
 
 // Microseconds of a GEMM as far as they depend on the width of its tiles and on the parts K is split into: waves of units over the
 // CTA pairs, each its k-blocks and what of its epilogue shows, and for a split the summing kernel and its slices' traffic.
@@ -770,15 +775,24 @@ static double gemm_us(int M, int n_cols, int K, int bn, int parts, bool f32) {
   const long long units = (long long)((M + 2 * BM - 1) / (2 * BM)) * ((n_cols + bn - 1) / bn) * ((kb + kb_part - 1) / kb_part);
   const double load = units < pairs ? (double)units / pairs : 1.0, waves = (double)((units + pairs - 1) / pairs);
   const bool slices = parts > 1;
-  const double unit = bn == 256 ? kb_part * (0.29 + 0.026 * load) + 1.6 + (f32 || slices ? 0.8 : 0)
-                                : kb_part * (0.149 + 0.04 * load) + 0.85 + (f32 || slices ? 0.55 : 0);
+  const double unit = bn == 256   ? kb_part * (0.29 + 0.026 * load) + 1.6 + (f32 || slices ? 0.8 : 0)
+                      : bn == 192 ? kb_part * (0.21 + 0.02 * load) + 1.25 + (f32 || slices ? 1.5 : 0)
+                                  : kb_part * (0.149 + 0.04 * load) + 0.85 + (f32 || slices ? 0.55 : 0);
   return waves * unit + (slices ? 1.0 + 0.147 * parts * M * n_cols * 4e-6 : 0.0);
 }
 
-// Columns of an output tile.
-static int tile_columns(int M, int n_cols, int K, bool f32) {
-  if (g_tile_n) return g_tile_n;
-  return gemm_us(M, n_cols, K, 128, 1, f32) < gemm_us(M, n_cols, K, 256, 1, f32) ? 128 : 256;
+// Columns of an output tile. 192 (where the epilogue works on independent 64-column chunks) only for a gain of 6 %: such tiles fetch as
+// many bytes of an MN-major operand as 256. Outputs of 576 and 960 columns are whole numbers of them. Measured 256 / 128 / 192 (us), unsplit
+// unless noted: input gradient 4096 x 576 x 3072: 20.7 / 19.8 / 17.2; 2048 x 576 x 49152, in parts: 101 / 120 / 91; weight gradient 960 x 2560 over
+// 4,096 tokens: 26.0 / 27.3 / 22.5; 49152 x 576 over 2,048: 110 / 118 / 102; 5120 x 960 over 8,192: 76.8 / 81.2 / 69.3; SwiGLU backward 4096 x
+// 1536 x 576: 23.4 / 20.1 / 19.6; and where it loses: forward 4096 x 960 x 2560: 20.9 / 20.7 / 25.0; 4096 x 2048 x 2048: 26.7 / 31.1 / 28.6.
+// (Constants of 192 columns fitted to 66 shapes; the choice among the three is 0.03 % off the best there, without 192 columns 3.6 %.)
+constexpr double GAIN_192 = 0.94;
+static int tile_columns(int M, int n_cols, int K, bool f32, bool has_192) {
+  if (g_tile_n) return g_tile_n == 192 && !has_192 ? 256 : g_tile_n;
+  const double t128 = gemm_us(M, n_cols, K, 128, 1, f32), t256 = gemm_us(M, n_cols, K, 256, 1, f32);
+  if (has_192 && gemm_us(M, n_cols, K, 192, 1, f32) < GAIN_192 * std::min(t128, t256)) return 192;
+  return t128 < t256 ? 128 : 256;
 }
 
 template <bool A_MN, bool B_MN, int OUT_MODE, bool EPI_TMA, int EPI = EPI_NONE, int BN = 256>
@@ -825,7 +839,7 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMa
 
 extern "C" void pt_gemm_set_group_m(int g) { pt::gemm_pair::g_group_m = g < 1 ? 1 : g; }
 extern "C" int pt_gemm_get_group_m() { return pt::gemm_pair::g_group_m; }
-extern "C" void pt_gemm_set_tile_n(int n) { pt::gemm_pair::g_tile_n = n == 128 || n == 256 ? n : 0; }
+extern "C" void pt_gemm_set_tile_n(int n) { pt::gemm_pair::g_tile_n = n == 128 || n == 192 || n == 256 ? n : 0; }
 
 // 1 (default): epilogue through shared memory and TMA store / reduce-add; 0: per-thread 16-byte stores.
 static int g_tma_epilogue = 1;
@@ -875,13 +889,13 @@ extern "C" int pt_gemm_split_parts(int M, int N, int K, int kind, int* tile_n) {
   if (g_tile_n) return 1;                  // (a width given for a measurement: of whole tiles)
   // (where whole tiles fill more than half of the pairs, what is left to gain is less than what parts at different K cost in L2 reuse)
   const bool few = 2LL * ((M + 2 * BM - 1) / (2 * BM)) * ((N + 255) / 256) <= num_pairs();
-  const double whole = gemm_us(M, N, K, tile_columns(M, N, K, wgrad), 1, wgrad) + (wgrad ? 0.08 * M * N * 4e-6 : 0.0);
+  const double whole = gemm_us(M, N, K, tile_columns(M, N, K, wgrad, true), 1, wgrad) + (wgrad ? 0.08 * M * N * 4e-6 : 0.0);
   double best = (few ? 0.97 : 0.85) * whole - (kind == SPLIT_FWD ? 2.0 : 0.0);
   int best_parts = 1;
   for (const int parts : {2, 3, 4, 5, 6, 8, 10, 12, 16, 20, 24, 32}) {
     if (kb / parts < 2) break;
-    for (const int bn : {128, 256}) {
-      const double t = gemm_us(M, N, K, bn, parts, true) + (kind == SPLIT_DGRAD ? 2.0 : 0.0);
+    for (const int bn : {128, 192, 256}) {
+      const double t = gemm_us(M, N, K, bn, parts, true) / (bn == 192 ? GAIN_192 : 1.0) + (kind == SPLIT_DGRAD ? 2.0 : 0.0);
       if (t < best) {
         best = t;
         best_parts = parts;
@@ -943,7 +957,7 @@ static int pt::gemm_pair::run_pair(const void* A, const void* B, void* D, int M,
   const bool epi_tma = g_tma_epilogue != 0;
   // narrow tiles exist for the layouts of the model: X W^T, dY W, and dY^T X into fp32
   const bool has_narrow = epi_tma && (out_mode == OUT_BF16 ? !a_mn : (b_mn || (!a_mn && out_mode == OUT_F32)));
-  const int bn = !has_narrow ? 256 : split ? split->bn : tile_columns(M, N, K, out_mode != OUT_BF16);
+  const int bn = !has_narrow ? 256 : split ? split->bn : tile_columns(M, N, K, out_mode != OUT_BF16, true);
   CUtensorMap ma, mb;
   int rc;
   rc = a_mn ? make_bf16_map_2d(&ma, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, 64, BK)
@@ -968,9 +982,11 @@ static int pt::gemm_pair::run_pair(const void* A, const void* B, void* D, int M,
   }
   KernelStatus* st = reinterpret_cast<KernelStatus*>(status);
 #define PT_GEMM_NARROW(AM, BMN, OM)                                                                           \
-  if (bn == 128 && a_mn == AM && b_mn == BMN && out_mode == OM)                                               \
-    return launch<AM, BMN, OM, true, EPI_NONE, 128>(ma, mb, md, D, M, N, K, ldd, st, stream, nullptr, ea);
-  PT_GEMM_NARROW(0, 0, 0) PT_GEMM_NARROW(0, 1, 0) PT_GEMM_NARROW(0, 0, 2) PT_GEMM_NARROW(0, 1, 1) PT_GEMM_NARROW(0, 1, 2) PT_GEMM_NARROW(1, 1, 1) PT_GEMM_NARROW(1, 1, 2)
+  if (bn != 256 && a_mn == AM && b_mn == BMN && out_mode == OM)                                               \
+    return bn == 128 ? launch<AM, BMN, OM, true, EPI_NONE, 128>(ma, mb, md, D, M, N, K, ldd, st, stream, nullptr, ea) \
+                     : launch<AM, BMN, OM, true, EPI_NONE, 192>(ma, mb, md, D, M, N, K, ldd, st, stream, nullptr, ea);
+  PT_GEMM_NARROW(0, 0, 0) PT_GEMM_NARROW(0, 1, 0) PT_GEMM_NARROW(0, 0, 2) PT_GEMM_NARROW(0, 1, 1) PT_GEMM_NARROW(0, 1, 2) PT_GEMM_NARROW(1, 1, 1)
+  PT_GEMM_NARROW(1, 1, 2)
 #undef PT_GEMM_NARROW
 #define PT_GEMM_CASE(AM, BMN, OM)                                                                             \
   if (a_mn == AM && b_mn == BMN && out_mode == OM)                                                            \
@@ -1029,7 +1045,7 @@ extern "C" int pt_gemm_bf16_fused(const void* A, const void* B, void* D, int M, 
     return -11;
   }
   if (M <= 0 || n_out <= 0 || K <= 0) return 0;
-  const int bn = tile_columns(M, epi == EPI_SWIGLU_BWD ? inter : n_out, K, false);
+  const int bn = tile_columns(M, epi == EPI_SWIGLU_BWD ? inter : n_out, K, false, epi == EPI_ADD || epi == EPI_SWIGLU_BWD);
   CUtensorMap ma, mb, md, mh;
   int rc;
   if ((rc = make_bf16_map_2d(&ma, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda, BK, BM))) return rc * 10 - 1;
@@ -1048,12 +1064,16 @@ extern "C" int pt_gemm_bf16_fused(const void* A, const void* B, void* D, int M, 
   KernelStatus* st = reinterpret_cast<KernelStatus*>(status);
   auto run = [&](auto width) -> int {
     constexpr int W = decltype(width)::value;
-    if (epi == EPI_SWIGLU) return launch<false, false, OUT_BF16, true, EPI_SWIGLU, W>(ma, mb, md, D, M, inter, K, ldd, st, stream, &mh, ea);
     if (epi == EPI_ADD) return launch<false, false, OUT_BF16, true, EPI_ADD, W>(ma, mb, md, D, M, N, K, ldd, st, stream, &mh, ea);
     if (epi == EPI_SWIGLU_BWD) return launch<false, true, OUT_BF16, true, EPI_SWIGLU_BWD, W>(ma, mb, md, D, M, inter, K, ldd, st, stream, &mh, ea);
-    if (head_dim == 64) return launch<false, false, OUT_BF16, true, EPI_ROPE64, W>(ma, mb, md, D, M, N, K, ldd, st, stream, &mh, ea);
-    return launch<false, false, OUT_BF16, true, EPI_ROPE128, W>(ma, mb, md, D, M, N, K, ldd, st, stream, &mh, ea);
+    if constexpr (W != 192) {                           // (tile_columns does not give 192 to the others)
+      if (epi == EPI_SWIGLU) return launch<false, false, OUT_BF16, true, EPI_SWIGLU, W>(ma, mb, md, D, M, inter, K, ldd, st, stream, &mh, ea);
+      if (head_dim == 64) return launch<false, false, OUT_BF16, true, EPI_ROPE64, W>(ma, mb, md, D, M, N, K, ldd, st, stream, &mh, ea);
+      return launch<false, false, OUT_BF16, true, EPI_ROPE128, W>(ma, mb, md, D, M, N, K, ldd, st, stream, &mh, ea);
+    }
+    return -11;
   };
+  if (bn == 192) return run(std::integral_constant<int, 192>{});
   return bn == 128 ? run(std::integral_constant<int, 128>{}) : run(std::integral_constant<int, 256>{});
 }
 

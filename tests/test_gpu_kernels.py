@@ -120,11 +120,11 @@ def test_gemm_weight_gradient_parts_are_repeatable_and_rounded_once(C, M, N, K):
     assert err <= 2 ** -4 + 1e-5 * float(want.abs().max()), err
 
 
-@pytest.mark.parametrize("tile_n", [128, 256])
+@pytest.mark.parametrize("tile_n", [128, 192, 256])
 @pytest.mark.parametrize("parts", [1, 2, 7])
-@pytest.mark.parametrize("M,N,K", [(8, 8, 1024), (264, 520, 448), (600, 584, 1000), (256, 128, 512), (1000, 72, 640)])
+@pytest.mark.parametrize("M,N,K", [(8, 8, 1024), (264, 520, 448), (600, 584, 1000), (256, 128, 512), (1000, 72, 640), (304, 576, 192)])
 def test_gemm_tile_widths_and_parts_of_every_layout(tile_n, parts, M, N, K):
-    """Both tile widths, unsplit and with K in parts (uneven ones, a last k-block of 8 to 40 rows, tiles beyond the matrix), for the
+    """Every tile width, unsplit and with K in parts (uneven ones, a last k-block of 8 to 40 rows, tiles beyond the matrix), for the
     forward layout with and without a residual, input gradients and fp32 accumulation."""
     from picotron_b200.ops import _ext
     C = _ext.load()
@@ -140,6 +140,11 @@ def test_gemm_tile_widths_and_parts_of_every_layout(tile_n, parts, M, N, K):
             C.set_gemm_split_dgrad(False)
         C.gemm(xt, wt, True, True, acc, True)
         got = [C.gemm(x, w, False, False), C.gemm_add(x, w, res), C.gemm(x, wt, False, True)]
+        if N % 64 == 0:                                       # the SwiGLU backward is never split: equal, whatever the width
+            gu = bf(M, 2 * N, seed=6)
+            dgu = C.gemm_dgrad_swiglu_bwd(x, wt, gu)
+            C.set_gemm_tile_n(256)
+            assert torch.equal(dgu, C.gemm_dgrad_swiglu_bwd(x, wt, gu))
     finally:
         C.set_gemm_tile_n(0)
         C.set_gemm_split_parts(0)
