@@ -20,6 +20,14 @@ CSRC = os.path.join(PKG, "csrc")
 OBJ = os.path.join(PKG, "csrc", "_obj")
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "--use_fast_math", "-Xcompiler", "-fPIC", "-Xptxas", "-v"]
+# Sources that need the accurate functions (logf): the rounding modes of --use_fast_math without its replacement of functions
+PRECISE = {"cross_entropy.cu"}
+
+
+def nvcc_flags(source: str) -> list:
+    if source not in PRECISE:
+        return NVCC_FLAGS
+    return [f for f in NVCC_FLAGS if f != "--use_fast_math"] + ["-ftz=true", "-prec-div=false", "-prec-sqrt=false"]
 
 
 def ext_path() -> str:
@@ -75,7 +83,7 @@ def build(verbose: bool = True) -> str:
         src, obj = os.path.join(CSRC, f), os.path.join(OBJ, f[:-3] + ".o")
         objs.append(obj)
         if _newer([src] + headers, obj):
-            jobs.append(([nvcc] + NVCC_FLAGS + ["-I", CSRC, "-c", src, "-o", obj], f[:-3] + ".nvcc.log"))
+            jobs.append(([nvcc] + nvcc_flags(f) + ["-I", CSRC, "-c", src, "-o", obj], f[:-3] + ".nvcc.log"))
     bsrc, bobj = os.path.join(CSRC, "bindings.cpp"), os.path.join(OBJ, "bindings.o")
     objs.append(bobj)
     if _newer([bsrc], bobj):

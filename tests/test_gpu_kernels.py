@@ -242,6 +242,26 @@ def test_lm_head_loss_from_two_kernels(T, V, K, vocab_start):
     assert float((got.double() - want).norm() / want.norm()) < 4e-3                  # one bf16 rounding
 
 
+@pytest.mark.parametrize("T,V,K,vocab_start", [(2048, 2048, 512, 0), (600, 1000, 192, 1000), (1024, 8456, 128, 0), (256, 128256, 64, 0)])
+def test_lm_head_loss_is_that_of_the_separate_kernels_to_the_bit(T, V, K, vocab_start):
+    """The log-sum-exp is the row maximum plus torch.log of the sum in fp32, so loss terms and gradient do not depend on whether one
+    kernel finishes the statistics or several do."""
+    from picotron_b200.ops import _ext
+    C = _ext.load()
+    C.set_gemm_pair(True)
+    C.set_gemm_tma_epilogue(True)
+    x, w = bf(T, K, seed=94), bf(V, K, seed=95, scale=0.3)
+    targets = torch.randint(0, vocab_start + V, (T,), device="cuda", generator=torch.Generator(device="cuda").manual_seed(96))
+    logits, rowmax, sumexp, tgt = C.gemm_ce_stats(x, w, targets, vocab_start)
+    lse = rowmax + torch.log(sumexp)
+    terms = torch.empty(T, device="cuda")
+    got = C.gemm_ce_loss(x, w, targets, vocab_start, 0.25, terms, True)
+    C.ce_grad_(logits, targets, lse, 0.25, vocab_start)
+    _status_ok(C)
+    assert torch.equal(terms, lse - tgt)
+    assert torch.equal(got, logits)
+
+
 @pytest.mark.parametrize("T,N,K", [(256, 256, 64), (300, 328, 320), (1024, 2048, 512), (4096, 2048, 8192), (200, 72, 136)])
 def test_gemm_with_residual_add_epilogue(T, N, K):
     """Projection + residual add from one GEMM (the epilogue fetches the residual tile) against GEMM followed by the add."""
