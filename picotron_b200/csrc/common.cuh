@@ -12,10 +12,18 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "per_device.h"
+
 namespace pt {
 
+inline int current_device() {
+  int dev = -1;
+  cudaGetDevice(&dev);
+  return dev;
+}
+
 // ---------------------------------------------------------------------------------------------
-// status word: one per process, in managed-free plain device memory, read by the host on demand.
+// status word: one per device, in managed-free plain device memory, read by the host on demand.
 // code 0 = ok. Non-zero: (kernel_id << 24) | (site << 16) | (blockIdx.x & 0xffff)
 // ---------------------------------------------------------------------------------------------
 struct KernelStatus {

@@ -812,8 +812,13 @@ extern "C" int pt_rmsnorm_bwd_acc(const void* dy, const void* x, const void* w, 
     const int want = (T + ROWS - 1) / ROWS, cap = (NC <= 2 ? 3 : 2) * num_sms;
     auto kern = rmsnorm_bwd_rows_kernel<TEAM, NC>;
     constexpr int SMEM = bwd_smem<TEAM, NC>();
-    static const cudaError_t configured = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-    if (configured != cudaSuccess) {
+    static PerDevice opted_in;
+    const int rc = opted_in.get(current_device(), [&] {
+      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) == cudaSuccess) return 1;
+      cudaGetLastError();
+      return -3;
+    });
+    if (rc <= 0) {
       failed = true;
       return;
     }

@@ -17,6 +17,19 @@ def _run(tp=1, cp=1, pp=1, dp=1, engine="1f1b", grad_acc=2, layers=4, graph=Fals
     H.check(res, tp, cp, pp, dp, grad_acc, layers, gpu=True)
 
 
+def test_rmsnorm_backward_on_a_second_device_of_the_process():
+    """Its shared memory has to be opted into on each device."""
+    from picotron_b200 import ops
+    from picotron_b200.ops import reference as ref
+    for dev in ("cuda:0", "cuda:1"):
+        g = torch.Generator(device=dev).manual_seed(1)
+        x, dy = (torch.randn(64, 2048, device=dev, generator=g).to(torch.bfloat16) for _ in range(2))
+        w, rstd, acc = x[0].contiguous(), torch.ones(64, device=dev), torch.zeros(2048, device=dev)
+        dx, _ = ops.rmsnorm_bwd(dy, x, w, rstd, None, acc)
+        want, _ = ref.rmsnorm_bwd(dy, x, w, rstd, None)
+        torch.testing.assert_close(dx.float(), want.float(), rtol=2 ** -7, atol=1e-2)      # one bf16 rounding of fp32 terms
+
+
 def test_dp2():
     _run(dp=2)
 

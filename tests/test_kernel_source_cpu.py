@@ -1,7 +1,10 @@
 """What the memory model asks of the kernels and no run can be relied on to show, read from their sources."""
+import ctypes
 import glob
 import os
 import re
+import shutil
+import subprocess
 
 import pytest
 
@@ -64,3 +67,41 @@ def test_a_build_with_other_register_counts_than_a_kernel_depends_on_fails():
         build.check_registers(log.format(126))
     with open(os.path.join(CSRC, "attention_tcgen05.cu")) as f:
         assert f"BWD_REGS = {build.FIXED_REGISTERS['attn_bwd_kernel']}," in f.read()
+
+
+PER_DEVICE_PROBE = r"""
+#include "per_device.h"
+static pt::PerDevice state;
+extern "C" int get(int device, int result, int* calls) {
+  return state.get(device, [&] { ++*calls; return result; });
+}
+"""
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="needs a host compiler")
+def test_launcher_state_is_found_once_on_every_device_and_a_failure_is_not_kept(tmp_path):
+    src, lib = tmp_path / "probe.cpp", tmp_path / "probe.so"
+    src.write_text(PER_DEVICE_PROBE)
+    subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-I", CSRC, str(src), "-o", str(lib)], check=True)
+    probe, calls = ctypes.CDLL(str(lib)), ctypes.c_int(0)
+
+    def get(device, result):
+        return probe.get(device, result, ctypes.byref(calls)), calls.value
+
+    assert get(0, 7) == (7, 1) and get(0, 9) == (7, 1)           # kept
+    assert get(1, -3) == (-3, 2) and get(1, 5) == (5, 3) and get(1, 6) == (5, 3)
+    assert get(63, 1) == (1, 4) and get(0, 9) == (7, 4)
+    assert get(64, 2) == (2, 5) and get(-1, 2) == (2, 6)         # beyond the table: found at every call
+
+
+@pytest.mark.parametrize("name", ["elementwise.cu"])
+def test_kernel_attributes_are_set_on_every_device(name):
+    """What remembers that a kernel's attribute was set is kept per device: the attribute is that of the current device alone."""
+    with open(os.path.join(CSRC, name)) as f:
+        src = re.sub(r"//[^\n]*", "", f.read())
+    keeper = None
+    for m in re.finditer(r"static (?:const )?(\w+) \w+(?: =|;)|cudaFuncSetAttribute", src):
+        if m.group(0) == "cudaFuncSetAttribute":
+            assert keeper == "PerDevice", src[m.start() - 200:m.start() + 100]
+        else:
+            keeper = m.group(1)
