@@ -1104,13 +1104,14 @@ static int launch_fwd(const CUtensorMap& mq, const KVSegs& segs, void* o, float*
                       KernelStatus* st, cudaStream_t stream) {
   if (!PROF && p.prof != nullptr) return launch_fwd<D, BN, true>(mq, segs, o, lse, p, st, stream);
   auto kern = attn_fwd_kernel<D, BN, PROF>;
-  static bool configured = false;
-  if (!configured) {
+  static PerDevice configured;
+  const int rc = configured.get(current_device(), [&] {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdCfg<D, BN>::SMEM) != cudaSuccess) return -3;
     // two CTAs per SM need the largest shared-memory carve-out
     cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    configured = true;
-  }
+    return 1;
+  });
+  if (rc <= 0) return rc;
   const int num_qb = (p.Sq + 127) / 128;
   const long long grid = (long long)num_qb * p.hq * p.B;
   launch_pdl(kern, dim3((unsigned)grid), dim3(192), FwdCfg<D, BN>::SMEM, stream, mq, segs, (bf16*)o, lse, p, st);
@@ -1128,16 +1129,17 @@ static int launch_bwd(const CUtensorMap& mq, const KVSegs& segs, const CUtensorM
     if constexpr (bwd_parts<D>() == 4) return attn_bwd_parts4_kernel<D, OUT_F32, PROF>;
     else return attn_bwd_kernel<D, OUT_F32, PROF>;
   }();
-  static bool configured = false;
-  if (!configured) {
+  static PerDevice configured;
+  const int rc = configured.get(current_device(), [&] {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdCfg<D>::SMEM) != cudaSuccess) return -3;
     cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     // the warpgroups share out Warps::REGS registers per thread; with fewer at launch setmaxnreg.inc would wait forever (the build
     // fails for another count, build.py: FIXED_REGISTERS)
     cudaFuncAttributes fa;
     if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess || fa.numRegs != Warps::REGS) return -6;
-    configured = true;
-  }
+    return 1;
+  });
+  if (rc <= 0) return rc;
   const int num_kb = ((p.Sk + 127) / 128) * p.n_segs;
   const long long grid = (long long)num_kb * p.hkv * p.B;
   launch_pdl(kern, dim3((unsigned)grid), dim3(Warps::THREADS), BwdCfg<D>::SMEM, stream, mq, segs, mdo, mdq, lse, delta, dk, dv, p, st);

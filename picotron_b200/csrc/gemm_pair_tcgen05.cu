@@ -800,8 +800,8 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMa
                   long long ldd, KernelStatus* status, cudaStream_t stream, const CUtensorMap* mh = nullptr,
                   EpiArgs ea = EpiArgs{}) {
   auto kern = gemm_pair_kernel<A_MN, B_MN, OUT_MODE, EPI_TMA, EPI, BN>;
-  static int max_clusters = 0;
-  if (max_clusters == 0) {
+  static PerDevice clusters_that_fit;
+  const int max_clusters = clusters_that_fit.get(current_device(), [&] {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes_of(EPI, BN)) != cudaSuccess) return -3;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2, 1, 1);
@@ -819,8 +819,9 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMa
       cudaGetLastError();
       return -5;
     }
-    max_clusters = n;
-  }
+    return n;
+  });
+  if (max_clusters <= 0) return max_clusters;
   const int n_tiles = (EPI == EPI_SWIGLU) ? (N + BN / 2 - 1) / (BN / 2) : (N + BN - 1) / BN;
   const int tiles = ((M + 2 * BM - 1) / (2 * BM)) * n_tiles;
   const int num_kb = (K + BK - 1) / BK;

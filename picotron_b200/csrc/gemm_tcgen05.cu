@@ -314,11 +314,11 @@ template <bool A_MN, bool B_MN, int OUT_MODE>
 static int launch(const CUtensorMap& ma, const CUtensorMap& mb, void* D, int M, int N, int K, long long ldd,
                   int num_sms, cudaStream_t stream) {
   auto kern = gemm_bf16_kernel<A_MN, B_MN, OUT_MODE>;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess) return -3;
-    configured = true;
-  }
+  static PerDevice opted_in;
+  const int rc = opted_in.get(current_device(), [&] {
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) == cudaSuccess ? 1 : -3;
+  });
+  if (rc <= 0) return rc;
   const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
   const int grid = tiles < num_sms ? tiles : num_sms;
   const cudaError_t err = launch_pdl(kern, dim3(grid), dim3(NUM_THREADS), SMEM_BYTES, stream, ma, mb, D, M, N, K, ldd, status_word());

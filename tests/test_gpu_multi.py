@@ -17,17 +17,25 @@ def _run(tp=1, cp=1, pp=1, dp=1, engine="1f1b", grad_acc=2, layers=4, graph=Fals
     H.check(res, tp, cp, pp, dp, grad_acc, layers, gpu=True)
 
 
-def test_rmsnorm_backward_on_a_second_device_of_the_process():
-    """Its shared memory has to be opted into on each device."""
+def test_ops_on_a_second_device_of_the_process():
+    """Large shared memory has to be opted into on each device."""
     from picotron_b200 import ops
     from picotron_b200.ops import reference as ref
     for dev in ("cuda:0", "cuda:1"):
         g = torch.Generator(device=dev).manual_seed(1)
-        x, dy = (torch.randn(64, 2048, device=dev, generator=g).to(torch.bfloat16) for _ in range(2))
-        w, rstd, acc = x[0].contiguous(), torch.ones(64, device=dev), torch.zeros(2048, device=dev)
+        x, dy = (torch.randn(256, 2048, device=dev, generator=g).to(torch.bfloat16) for _ in range(2))
+        w, rstd, acc = x[0].contiguous(), torch.ones(256, device=dev), torch.zeros(2048, device=dev)
         dx, _ = ops.rmsnorm_bwd(dy, x, w, rstd, None, acc)
         want, _ = ref.rmsnorm_bwd(dy, x, w, rstd, None)
         torch.testing.assert_close(dx.float(), want.float(), rtol=2 ** -7, atol=1e-2)      # one bf16 rounding of fp32 terms
+        y, want = ops.linear_fwd(x, dy).double(), x.double() @ dy.double().t()
+        assert float((y - want).norm() / want.norm()) < 4e-3                               # one bf16 rounding
+        q, do = x.view(1, 256, 32, 64), dy.view(1, 256, 32, 64)
+        o, lse = ops.attention_fwd(q, q, q, True)
+        o_ref, lse_ref = ref.attention_fwd(q, q, q, True, 0.125)
+        torch.testing.assert_close(o.float(), o_ref.float(), rtol=2e-2, atol=2e-2)
+        for got, want in zip(ops.attention_bwd(do, q, q, q, o, lse, True), ref.attention_bwd(do, q, q, q, o_ref, lse_ref, True, 0.125)):
+            assert float((got.float() - want.float()).norm() / want.float().norm()) < 2e-2
 
 
 def test_dp2():

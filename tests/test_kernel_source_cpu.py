@@ -94,7 +94,7 @@ def test_launcher_state_is_found_once_on_every_device_and_a_failure_is_not_kept(
     assert get(64, 2) == (2, 5) and get(-1, 2) == (2, 6)         # beyond the table: found at every call
 
 
-@pytest.mark.parametrize("name", ["elementwise.cu"])
+@pytest.mark.parametrize("name", ["elementwise.cu", "gemm_tcgen05.cu", "gemm_pair_tcgen05.cu", "gemm_allreduce_tcgen05.cu", "attention_tcgen05.cu"])
 def test_kernel_attributes_are_set_on_every_device(name):
     """What remembers that a kernel's attribute was set is kept per device: the attribute is that of the current device alone."""
     with open(os.path.join(CSRC, name)) as f:
