@@ -609,7 +609,8 @@ struct LayerSaved {
   }
 };
 
-// The saved activations as tensors {rstd1, h1, qkv, o, lse, x_mid, rstd2, h2, gu, a} (views; for callers that work on tensors).
+// The saved activations of decoder_layer_fwd_packed as tensors {rstd1, h1, qkv, o, lse, x_mid, rstd2, h2, gu, a} (views; for callers that
+// work on tensors).
 std::vector<Tensor> decoder_layer_saved(const Tensor& s16, const Tensor& s32, int64_t B, int64_t S, int64_t H, int64_t I, int64_t hq,
                                         int64_t hkv, int64_t d) {
   const LayerDims n{B, S, H, I, hq, hkv, d};
@@ -650,9 +651,9 @@ inline bool fused_gemm(int rc, const char* what) {          // false: not covere
 }
 
 // Returns {x_out, saved bf16, saved fp32} (LayerSaved), or {} (nothing launched) for operands that are not bf16.
-std::vector<Tensor> decoder_layer_fwd(const Tensor& x, const Tensor& ln1, const Tensor& w_qkv, const Tensor& cosT, const Tensor& sinT,
-                                      const Tensor& wo, const Tensor& ln2, const Tensor& w_gu, const Tensor& wd, double eps, int64_t B,
-                                      int64_t S, int64_t hq, int64_t hkv, int64_t d, double scale) {
+std::vector<Tensor> decoder_layer_fwd_packed(const Tensor& x, const Tensor& ln1, const Tensor& w_qkv, const Tensor& cosT, const Tensor& sinT,
+                                             const Tensor& wo, const Tensor& ln2, const Tensor& w_gu, const Tensor& wd, double eps, int64_t B,
+                                             int64_t S, int64_t hq, int64_t hkv, int64_t d, double scale) {
   if (!all_bf16_cuda({&x, &ln1, &w_qkv, &wo, &ln2, &w_gu, &wd})) return {};
   TORCH_CHECK(x.dim() == 2 && x.is_contiguous() && x.size(0) == B * S && w_gu.dim() == 2 && hq % hkv == 0);
   const LayerDims n{B, S, x.size(1), w_gu.size(0) / 2, hq, hkv, d};
@@ -701,6 +702,16 @@ std::vector<Tensor> decoder_layer_fwd(const Tensor& x, const Tensor& ln1, const 
   return {out, s16, s32};
 }
 
+// The same with the activations as tensors of their own (views): {x_out, h1, rstd1, qkv, o, lse, x_mid, rstd2, h2, gu, a}, or {}.
+std::vector<Tensor> decoder_layer_fwd(const Tensor& x, const Tensor& ln1, const Tensor& w_qkv, const Tensor& cosT, const Tensor& sinT,
+                                      const Tensor& wo, const Tensor& ln2, const Tensor& w_gu, const Tensor& wd, double eps, int64_t B,
+                                      int64_t S, int64_t hq, int64_t hkv, int64_t d, double scale) {
+  auto r = decoder_layer_fwd_packed(x, ln1, w_qkv, cosT, sinT, wo, ln2, w_gu, wd, eps, B, S, hq, hkv, d, scale);
+  if (r.empty()) return {};
+  auto v = decoder_layer_saved(r[1], r[2], B, S, x.size(1), w_gu.size(0) / 2, hq, hkv, d);
+  return {r[0], v[1], v[0], v[2], v[3], v[4], v[5], v[6], v[7], v[8], v[9]};
+}
+
 // The fp32 regions of parameters that one GEMM accumulates into together, as one [rows, cols] region: its address, or nullptr unless
 // they are adjacent in one storage.
 float* packed_region(const std::vector<Tensor>& mg, int first, int count, int64_t rows, int64_t cols) {
@@ -730,14 +741,21 @@ void rmsnorm_bwd_into(const void* dy, const void* x, const Tensor& w, const floa
   PT_CHECK_RC(pt_accumulate(dw.data_ptr<float>(), dw_new.data_ptr(), H, 1, stream()), "accumulate");
 }
 
-// Backward of decoder_layer_fwd; the weight gradients are added to the fp32 regions `mg` (q, k, v, out, gate, up, down, norm 1,
-// norm 2). x and {s16, s32}: the forward's input and saved activations. Returns dx, or an undefined tensor (nothing launched).
-Tensor decoder_layer_bwd(const Tensor& dout, const Tensor& x, const Tensor& s16, const Tensor& s32, const Tensor& ln1, const Tensor& w_qkv,
-                         const Tensor& cosT, const Tensor& sinT, const Tensor& wo, const Tensor& ln2, const Tensor& w_gu,
-                         const Tensor& wd, const std::vector<Tensor>& mg, int64_t B, int64_t S, int64_t hq, int64_t hkv, int64_t d,
-                         double scale) {
+// What a layer's backward reads of its forward.
+struct LayerActivations {
+  const bf16_t *h1, *qkv, *o, *x_mid, *h2, *gu, *a;
+  const float *rstd1, *rstd2, *lse;
+};
+
+// Backward of a layer; the weight gradients are added to the fp32 regions `mg` (q, k, v, out, gate, up, down, norm 1, norm 2). x: the
+// forward's input; `saved_by(dims)` gives its activations once the dimensions are known. Returns dx, or an undefined tensor (nothing
+// launched).
+template <class SavedBy>
+Tensor layer_bwd(const Tensor& dout, const Tensor& x, SavedBy saved_by, const Tensor& ln1, const Tensor& w_qkv, const Tensor& cosT,
+                 const Tensor& sinT, const Tensor& wo, const Tensor& ln2, const Tensor& w_gu, const Tensor& wd, const std::vector<Tensor>& mg,
+                 int64_t B, int64_t S, int64_t hq, int64_t hkv, int64_t d, double scale) {
   TORCH_CHECK(mg.size() == 9);
-  if (!all_bf16_cuda({&dout, &x, &s16, &ln1, &w_qkv, &wo, &ln2, &w_gu, &wd})) return Tensor();
+  if (!all_bf16_cuda({&dout, &x, &ln1, &w_qkv, &wo, &ln2, &w_gu, &wd})) return Tensor();
   TORCH_CHECK(x.dim() == 2 && x.is_contiguous() && x.size(0) == B * S && dout.is_contiguous() && dout.sizes() == x.sizes() &&
               w_gu.dim() == 2 && hq % hkv == 0);
   const LayerDims n{B, S, x.size(1), w_gu.size(0) / 2, hq, hkv, d};
@@ -748,16 +766,11 @@ Tensor decoder_layer_bwd(const Tensor& dout, const Tensor& x, const Tensor& s16,
   for (int i = 7; i < 9; ++i)
     if (!mg[i].is_cuda() || mg[i].scalar_type() != at::kFloat || !mg[i].is_contiguous() || mg[i].numel() != H) return Tensor();
   check_layer(n, ln1, w_qkv, cosT, sinT, wo, ln2, w_gu, wd);
-  const LayerSaved at(n);
-  PT_CHECK_F32(s32);
-  TORCH_CHECK(s16.is_contiguous() && s16.numel() == at.total && s32.is_contiguous() && s32.numel() == at.total32,
-              "decoder layer: saved activations of another shape");
+  const LayerActivations acts = saved_by(n);
   c10::cuda::CUDAGuard guard(x.device());
   const auto on = x.options();
-  const bf16_t* const b = bf16_ptr(s16);
-  const float* const f = s32.data_ptr<float>();
-  const bf16_t *const h1 = b + at.h1, *const qkv = b + at.qkv, *const o = b + at.o, *const x_mid = b + at.x_mid, *const h2 = b + at.h2,
-               *const gu = b + at.gu, *const a = b + at.a;
+  const bf16_t *const h1 = acts.h1, *const qkv = acts.qkv, *const o = acts.o, *const x_mid = acts.x_mid, *const h2 = acts.h2,
+               *const gu = acts.gu, *const a = acts.a;
   // One scratch allocation (bytes): dgu, whose place the attention's gradients take when it is done with; the normed inputs' gradients
   // (dh); dx_mid.
   auto up = [](int64_t bytes) { return (bytes + 255) / 256 * 256; };
@@ -782,17 +795,57 @@ Tensor decoder_layer_bwd(const Tensor& dout, const Tensor& x, const Tensor& s16,
   gemm_into(dout.data_ptr(), a, mg_d, H, I, T, H, I, I, true, true, 1, on);
   gemm_into(dgu, w_gu.data_ptr(), dh, T, H, 2 * I, 2 * I, ld_gu, H, false, true, 0, on);
   gemm_into(dgu, h2, mg_gu, 2 * I, H, T, 2 * I, H, H, true, true, 1, on);
-  rmsnorm_bwd_into(dh, x_mid, ln2, f + at.rstd2, dout.data_ptr(), dx_mid, mg[8], T, H, on);
+  rmsnorm_bwd_into(dh, x_mid, ln2, acts.rstd2, dout.data_ptr(), dx_mid, mg[8], T, H, on);
   gemm_into(dx_mid, wo.data_ptr(), dO, T, O, H, H, ld_o, O, false, true, 0, on);             // dL/d(attention output)
   gemm_into(dx_mid, o, mg_o, H, O, T, H, O, O, true, true, 1, on);
-  PT_CHECK_BWD_RC(pt_attention_bwd_rope(dO, qkv, qkv + O, qkv + O + hkv * d, o, f + at.lse, nullptr, reinterpret_cast<float*>(delta),
+  PT_CHECK_BWD_RC(pt_attention_bwd_rope(dO, qkv, qkv + O, qkv + O + hkv * d, o, acts.lse, nullptr, reinterpret_cast<float*>(delta),
                                         reinterpret_cast<float*>(dq_ws), dqkv, dqkv + O, dqkv + O + hkv * d, (int)B, (int)S, (int)S, (int)hq,
                                         (int)hkv, (int)d, Q, Q, Q, Q, Q, Q, 1, (float)scale, cosT.data_ptr<float>(), sinT.data_ptr<float>(),
                                         (int)S, st), "attention_bwd");
   gemm_into(dqkv, w_qkv.data_ptr(), dh, T, H, Q, Q, ld_qkv, H, false, true, 0, on);
   gemm_into(dqkv, h1, mg_qkv, Q, H, T, Q, H, H, true, true, 1, on);
-  rmsnorm_bwd_into(dh, x.data_ptr(), ln1, f + at.rstd1, dx_mid, dx.data_ptr(), mg[7], T, H, on);
+  rmsnorm_bwd_into(dh, x.data_ptr(), ln1, acts.rstd1, dx_mid, dx.data_ptr(), mg[7], T, H, on);
   return dx;
+}
+
+// `s16`, `s32`: what decoder_layer_fwd_packed saved.
+Tensor decoder_layer_bwd_packed(const Tensor& dout, const Tensor& x, const Tensor& s16, const Tensor& s32, const Tensor& ln1, const Tensor& w_qkv,
+                                const Tensor& cosT, const Tensor& sinT, const Tensor& wo, const Tensor& ln2, const Tensor& w_gu,
+                                const Tensor& wd, const std::vector<Tensor>& mg, int64_t B, int64_t S, int64_t hq, int64_t hkv, int64_t d,
+                                double scale) {
+  if (!all_bf16_cuda({&s16})) return Tensor();
+  auto saved_by = [&](const LayerDims& n) {
+    const LayerSaved at(n);
+    PT_CHECK_F32(s32);
+    TORCH_CHECK(s16.is_contiguous() && s16.numel() == at.total && s32.is_contiguous() && s32.numel() == at.total32,
+                "decoder layer: saved activations of another shape");
+    const bf16_t* const b = bf16_ptr(s16);
+    const float* const f = s32.data_ptr<float>();
+    return LayerActivations{b + at.h1, b + at.qkv, b + at.o, b + at.x_mid, b + at.h2, b + at.gu, b + at.a, f + at.rstd1, f + at.rstd2, f + at.lse};
+  };
+  return layer_bwd(dout, x, saved_by, ln1, w_qkv, cosT, sinT, wo, ln2, w_gu, wd, mg, B, S, hq, hkv, d, scale);
+}
+
+// `saved` = {x, rstd1, h1, qkv, o, lse, x_mid, rstd2, h2, gu, a}, tensors wherever they lie.
+Tensor decoder_layer_bwd(const Tensor& dout, const std::vector<Tensor>& saved, const Tensor& ln1, const Tensor& w_qkv, const Tensor& cosT,
+                         const Tensor& sinT, const Tensor& wo, const Tensor& ln2, const Tensor& w_gu, const Tensor& wd,
+                         const std::vector<Tensor>& mg, int64_t B, int64_t S, int64_t hq, int64_t hkv, int64_t d, double scale) {
+  TORCH_CHECK(saved.size() == 11);
+  auto saved_by = [&](const LayerDims& n) {
+    auto bf16 = [&](int i, int64_t cols) {
+      PT_CHECK_BF16(saved[i]);
+      TORCH_CHECK(saved[i].is_contiguous() && saved[i].numel() == n.T() * cols, "decoder layer: saved activation ", i, " of another shape");
+      return (const bf16_t*)bf16_ptr(saved[i]);
+    };
+    auto f32 = [&](int i, int64_t cols) {
+      PT_CHECK_F32(saved[i]);
+      TORCH_CHECK(saved[i].is_contiguous() && saved[i].numel() == n.T() * cols, "decoder layer: saved statistic ", i, " of another shape");
+      return (const float*)saved[i].data_ptr<float>();
+    };
+    return LayerActivations{bf16(2, n.H), bf16(3, n.Q()), bf16(4, n.O()), bf16(6, n.H), bf16(8, n.H), bf16(9, 2 * n.I), bf16(10, n.I),
+                            f32(1, 1), f32(7, 1), f32(5, n.hq)};
+  };
+  return layer_bwd(dout, saved[0], saved_by, ln1, w_qkv, cosT, sinT, wo, ln2, w_gu, wd, mg, B, S, hq, hkv, d, scale);
 }
 
 void allreduce_symm(std::vector<int64_t> buf_ptrs, std::vector<int64_t> flag_ptrs, int64_t mc_ptr, int64_t offset_elems,
@@ -967,8 +1020,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("add", &add);
   m.def("adamw_multi_", &adamw_multi_);
   m.def("decoder_layer_fwd", &decoder_layer_fwd);
-  m.def("decoder_layer_saved", &decoder_layer_saved, "The saved activations of decoder_layer_fwd as tensors (views).");
   m.def("decoder_layer_bwd", &decoder_layer_bwd);
+  m.def("decoder_layer_fwd_packed", &decoder_layer_fwd_packed, "decoder_layer_fwd with the saved activations in two allocations.");
+  m.def("decoder_layer_saved", &decoder_layer_saved, "The saved activations of decoder_layer_fwd_packed as tensors (views).");
+  m.def("decoder_layer_bwd_packed", &decoder_layer_bwd_packed);
   m.def("scale_", &scale_);
   m.def("merge_attention_", &merge_attention_);
   m.def("attention_fwd", &attention_fwd);

@@ -375,7 +375,7 @@ class DecoderLayerFn(torch.autograd.Function):
         ctx.native = False
         if tp_group is None and not att.cp_enabled and ops.runs_layer_natively(x2):
             cos, sin = layer.rope(x.device)
-            r = ops.decoder_layer_fwd(x2, ln1_w, w_qkv, cos, sin, wo, ln2_w, w_gu, wd, layer.eps, B, S, hq, hkv, d, layer.sm_scale)
+            r = ops.decoder_layer_fwd_packed(x2, ln1_w, w_qkv, cos, sin, wo, ln2_w, w_gu, wd, layer.eps, B, S, hq, hkv, d, layer.sm_scale)
             if r:
                 ctx.save_for_backward(x2, r[1], r[2])                       # input, saved activations (bf16 and fp32)
                 ctx.layer = layer
@@ -447,8 +447,8 @@ class DecoderLayerFn(torch.autograd.Function):
                 grads = [getattr(p, "main_grad", None) for p in params]
                 if all(g is not None for g in grads):
                     cos, sin = layer.rope(dout.device)
-                    dx = ops.decoder_layer_bwd(dout2, x2, saved16, saved32, params[7], w_qkv, cos, sin, wo, params[8], w_gu, wd, grads,
-                                               B, S, hq, hkv, d, layer.sm_scale)
+                    dx = ops.decoder_layer_bwd_packed(dout2, x2, saved16, saved32, params[7], w_qkv, cos, sin, wo, params[8], w_gu, wd,
+                                                      grads, B, S, hq, hkv, d, layer.sm_scale)
                     if dx is not None:
                         for p in params:
                             notify_grad_ready(p)

@@ -192,19 +192,30 @@ def runs_layer_natively(x) -> bool:
 
 
 def decoder_layer_fwd(*args):
-    """``(x_out, saved16, saved32)`` of a layer on one GPU, or ``[]`` if it is not covered. What the backward needs besides the input
-    lies in two allocations, bf16 and fp32 (:func:`decoder_layer_saved`)."""
+    """``(x_out, h1, rstd1, qkv, o, lse, x_mid, rstd2, h2, gu, a)`` of a layer on one GPU, or ``[]`` if it is not covered."""
     return _c().decoder_layer_fwd(*args)
-
-
-def decoder_layer_saved(*args):
-    """``(rstd1, h1, qkv, o, lse, x_mid, rstd2, h2, gu, a)`` as views into the saved activations of :func:`decoder_layer_fwd`."""
-    return _c().decoder_layer_saved(*args)
 
 
 def decoder_layer_bwd(*args):
     """``dx`` of a layer whose weight gradients go into fp32 regions, or None (and nothing launched) if it is not covered."""
     return _c().decoder_layer_bwd(*args)
+
+
+def decoder_layer_fwd_packed(*args):
+    """:func:`decoder_layer_fwd` with what the backward needs besides the input in two allocations, bf16 and fp32:
+    ``(x_out, saved16, saved32)``, or ``[]``. A layer call of a small model is bound by the host, and a tensor object per activation
+    was half of its time."""
+    return _c().decoder_layer_fwd_packed(*args)
+
+
+def decoder_layer_saved(*args):
+    """``(rstd1, h1, qkv, o, lse, x_mid, rstd2, h2, gu, a)`` as views into what :func:`decoder_layer_fwd_packed` saved."""
+    return _c().decoder_layer_saved(*args)
+
+
+def decoder_layer_bwd_packed(*args):
+    """:func:`decoder_layer_bwd` from the input and the two allocations of :func:`decoder_layer_fwd_packed`."""
+    return _c().decoder_layer_bwd_packed(*args)
 
 
 # ------------------------------------------------------------------ embedding

@@ -79,3 +79,41 @@ def test_native_layer_matches_the_separate_calls(monkeypatch, hq, hkv, d, inter,
     for x, y in zip(ga, gb):
         # dQ is summed in fp32 in any order and rounded to bf16: neighbours (2^-8) in places, carried through two layers
         assert float((x - y).norm()) <= 4 * 2 ** -8 * float(y.norm()) + 1e-6
+
+
+@pytest.mark.parametrize("hq,hkv,d,inter,B,S", [(4, 2, 64, 320, 2, 97), (2, 1, 128, 200, 1, 64)])
+def test_layer_ops_with_a_tensor_per_activation(hq, hkv, d, inter, B, S):
+    """``ops.decoder_layer_fwd`` hands every activation out, and ``ops.decoder_layer_bwd`` takes such a list, wherever its tensors
+    lie; both equal the calls that keep them in two allocations."""
+    from picotron_b200 import ops
+    H, Q, T = hq * d, (hq + 2 * hkv) * d, B * S
+    g = torch.Generator(device="cuda").manual_seed(3)
+    bf = lambda *s: (0.05 * torch.randn(*s, device="cuda", generator=g)).to(torch.bfloat16)
+    x, dout, ln1, ln2 = 20 * bf(T, H), 20 * bf(T, H), 1 + bf(H), 1 + bf(H)
+    w_qkv, wo, w_gu, wd = bf(Q, H), bf(H, H), bf(2 * inter, H), bf(H, inter)
+    angles = torch.rand(S, d // 2, device="cuda", generator=g)
+    cos, sin, scale = angles.cos(), angles.sin(), d ** -0.5
+    fwd = (x, ln1, w_qkv, cos, sin, wo, ln2, w_gu, wd, 1e-5, B, S, hq, hkv, d, scale)
+    out, h1, rstd1, qkv, o, lse, x_mid, rstd2, h2, gu, a = ops.decoder_layer_fwd(*fwd)
+    packed = ops.decoder_layer_fwd_packed(*fwd)
+    saved = [x, rstd1, h1, qkv, o, lse, x_mid, rstd2, h2, gu, a]
+    assert torch.equal(out, packed[0])
+    for mine, theirs in zip(saved[1:], ops.decoder_layer_saved(packed[1], packed[2], B, S, H, inter, hq, hkv, d)):
+        assert mine.shape == theirs.shape and torch.equal(mine, theirs)
+    assert [tuple(t.shape) for t in saved] == [(T, H), (T,), (T, H), (T, Q), (T, H), (B, hq, S), (T, H), (T,), (T, H), (T, 2 * inter), (T, inter)]
+
+    def regions():
+        flat = torch.zeros(Q * H + H * H + 3 * inter * H + 2 * H, device="cuda")
+        shapes = [(hq * d, H), (hkv * d, H), (hkv * d, H), (H, H), (inter, H), (inter, H), (H, inter), (H,), (H,)]
+        return list(t.view(s) for t, s in zip(flat.split([torch.Size(s).numel() for s in shapes]), shapes)), flat
+
+    rest = (ln1, w_qkv, cos, sin, wo, ln2, w_gu, wd)
+    mg, flat = regions()
+    dx = ops.decoder_layer_bwd_packed(dout, x, packed[1], packed[2], *rest, mg, B, S, hq, hkv, d, scale)
+    mg2, flat2 = regions()
+    dx2 = ops.decoder_layer_bwd(dout, [t.clone() for t in saved], *rest, mg2, B, S, hq, hkv, d, scale)
+    # one key block: dQ is not added up in any order; the norm weights' gradients are, over T rows in fp32
+    assert torch.equal(dx, dx2)
+    torch.testing.assert_close(flat, flat2, rtol=1e-4, atol=1e-5)
+    with pytest.raises(RuntimeError):
+        ops.decoder_layer_bwd(dout, [t.clone() for t in saved[:9]] + [gu[:, 1:], a], *rest, mg2, B, S, hq, hkv, d, scale)
