@@ -309,6 +309,8 @@ def merge_attention_(out, lse, block_out, block_lse):
 _CHECKED_OPS = ("rmsnorm_fwd", "add_rmsnorm_fwd", "rmsnorm_bwd", "rope_", "swiglu_fwd", "swiglu_bwd", "linear_swiglu_fwd",
                 "linear_rope_fwd", "linear_add_fwd", "linear_dgrad_swiglu_bwd", "linear_fwd", "linear_dgrad", "linear_wgrad", "attention_fwd", "attention_bwd",
                 "embedding_fwd", "embedding_bwd", "ce_stats", "linear_ce_stats", "linear_ce_loss", "ce_grad_", "add", "accumulate_", "scale_", "merge_attention_")
+# results that an op writes into an argument and does not return: position, name
+_RESULT_ARGS = {"linear_ce_loss": (5, "terms")}
 _UNCHECKED = {}
 
 
@@ -347,7 +349,11 @@ def enable_checked_mode(on: bool = True, check_finite: bool = True) -> None:
                     raise RuntimeError(f"ops.{name}: a kernel gave up a bounded wait (status {status:#x}: kernel id "
                                        f"{status >> 24}, site {(status >> 16) & 0xff}, block {status & 0xffff})")
             if check_finite:
-                for t in _tensors_of(out):
+                results = [out]
+                if name in _RESULT_ARGS:
+                    at, arg = _RESULT_ARGS[name]
+                    results.append(kwargs[arg] if arg in kwargs else args[at])
+                for t in _tensors_of(results):
                     if t.is_floating_point() and t.numel() and not bool(torch.isfinite(t).all()):
                         raise FloatingPointError(f"ops.{name}: non-finite values in a result of shape {tuple(t.shape)}")
             return out

@@ -117,3 +117,17 @@ def test_layer_ops_with_a_tensor_per_activation(hq, hkv, d, inter, B, S):
     torch.testing.assert_close(flat, flat2, rtol=1e-4, atol=1e-5)
     with pytest.raises(RuntimeError):
         ops.decoder_layer_bwd(dout, [t.clone() for t in saved[:9]] + [gu[:, 1:], a], *rest, mg2, B, S, hq, hkv, d, scale)
+
+
+def test_checked_mode_sees_a_loss_that_is_not_finite_without_a_gradient():
+    from picotron_b200 import ops
+    x, w = torch.ones(3, 64, device="cuda", dtype=torch.bfloat16), torch.ones(16, 64, device="cuda", dtype=torch.bfloat16)
+    targets, terms = torch.zeros(3, device="cuda", dtype=torch.long), torch.empty(3, device="cuda")
+    ops.enable_checked_mode(True)
+    try:
+        ops.linear_ce_loss(x, w, targets, 0, 1.0, terms, False)
+        x[1, 2] = float("nan")
+        with pytest.raises(FloatingPointError, match="linear_ce_loss"):
+            ops.linear_ce_loss(x, w, targets, 0, 1.0, terms, False)
+    finally:
+        ops.enable_checked_mode(False)

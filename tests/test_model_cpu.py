@@ -1,3 +1,4 @@
+import pytest
 import torch
 
 from picotron_b200.config import ModelConfig
@@ -118,6 +119,33 @@ def test_checked_mode_names_the_op_that_produced_non_finite_values():
     finally:
         ops.enable_checked_mode(False)
     assert torch.isnan(ops.linear_fwd(x, bad)).any()                 # unchecked again
+
+
+@pytest.mark.parametrize("by_name", [True, False])
+def test_checked_mode_looks_at_the_loss_terms_that_the_fused_head_leaves_in_its_argument(monkeypatch, by_name):
+    """Without a gradient the terms are all there is: the logits are not written."""
+    from picotron_b200 import ops
+
+    class Fused:
+        @staticmethod
+        def gemm_ce_loss(x, w, targets, vocab_start, scale, terms, need_grad):
+            terms.fill_(value)
+            return x.new_empty(0)
+
+    monkeypatch.setattr(ops, "_use_tc", lambda *ts: True)
+    monkeypatch.setattr(ops, "_c", lambda: Fused)
+    x, w, targets, terms = torch.ones(2, 4), torch.ones(3, 4), torch.zeros(2, dtype=torch.long), torch.empty(2)
+    rest = {"terms": terms, "need_grad": False} if by_name else {}
+    call = lambda: ops.linear_ce_loss(x, w, targets, 0, 1.0, *([] if by_name else [terms, False]), **rest)
+    ops.enable_checked_mode(True)
+    try:
+        value = 1.0
+        assert call().numel() == 0
+        value = float("nan")
+        with pytest.raises(FloatingPointError, match="linear_ce_loss"):
+            call()
+    finally:
+        ops.enable_checked_mode(False)
 
 
 def test_reference_named_model_symbols_exist_and_agree():
