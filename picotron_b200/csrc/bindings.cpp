@@ -27,6 +27,7 @@ void* pt_status_word();
 void pt_attention_set_profile(unsigned long long* counters);
 void pt_gemm_set_group_m(int g);
 void pt_gemm_set_tile_n(int n);
+int pt_gemm_tile_columns(int M, int n_cols, int K, int f32, int b_mn, int has_192);
 int pt_gemm_split_parts(int M, int N, int K, int kind, int* tile_n);
 long long pt_gemm_split_elems(int M, int N, int K, int kind, int parts);
 void pt_gemm_set_split_k(int on);
@@ -1042,6 +1043,16 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         "input- and weight-gradient GEMMs with few output tiles: K split over idle CTA pairs (default on; for the calling thread)");
   m.def("set_gemm_split_parts", [](int64_t n) { pt_gemm_set_split_k(n > 1 ? (int)n : 1); },
         "GEMMs that may be split over K are always cut into n parts by this thread (tests, measurements); 0 or 1: the rule.");
+  m.def("gemm_plan", [](const std::string& kind, int64_t M, int64_t N, int64_t K) {
+          const int splits = kind == "dgrad" ? 0 : kind == "wgrad" ? 1 : kind == "fwd" || kind == "add" ? 2 : -1;
+          TORCH_CHECK(splits >= 0 || kind == "rope" || kind == "swiglu" || kind == "swiglu_bwd", "gemm_plan: ", kind);
+          int tile_n = 256;
+          const int parts = splits >= 0 ? pt_gemm_split_parts((int)M, (int)N, (int)K, splits, &tile_n) : 1;
+          if (parts <= 1) tile_n = pt_gemm_tile_columns((int)M, (int)N, (int)K, splits == 1, splits == 0 || splits == 1 || kind == "swiglu_bwd",
+                                                       splits >= 0 || kind == "swiglu_bwd");
+          return std::pair<int64_t, int64_t>(tile_n, parts);
+        }, "(columns of a tile, parts of K) that the rule gives a GEMM with output [M, N]: kind fwd, add, dgrad, wgrad, rope, swiglu (N = 2I) or\n"
+           "swiglu_bwd (N = I).");
   m.def("set_gemm_tile_n", [](int64_t n) { pt_gemm_set_tile_n((int)n); },
         "columns of the GEMM output tiles: 128, 192 (where the epilogue has it), 256, or 0 for the choice by shape (for the calling thread)");
   m.def("get_gemm_group_m", []() { return (int64_t)pt_gemm_get_group_m(); });

@@ -1,9 +1,9 @@
 // bf16 GEMM for sm_100a on CTA pairs (tcgen05 cta_group::2): D[M,N] = op(A) * op(B), fp32 accumulate in TMEM.
 //
 // Same contract and operand layouts as gemm_tcgen05.cu, but two CTAs (a cluster of 2 on neighbouring SMs)
-// cooperate on one 256x256 or 256x128 output tile (see gemm_us for which): each CTA loads its own 128 rows of A
-// and its own half of the columns of
-// B -- with plain, non-multicast TMA loads -- and one thread of the leader CTA issues a 256-row MMA that
+// cooperate on one output tile of 256 rows and 256, 192 or 128 columns (see choice_us for which): each CTA loads
+// its own 128 rows of A and its own half of the columns of B -- with plain, non-multicast TMA loads -- and one
+// thread of the leader CTA issues a 256-row MMA that
 // reads both CTAs' shared memory and writes both CTAs' tensor memory. Per output element this moves a
 // third less operand data from L2 into shared memory than the single-CTA 128x256 tile (each B half is
 // fetched once per pair instead of once per CTA), which is what the single-CTA kernel is limited by.
@@ -781,18 +781,44 @@ static double gemm_us(int M, int n_cols, int K, int bn, int parts, bool f32) {
   return waves * unit + (slices ? 1.0 + 0.147 * parts * M * n_cols * 4e-6 : 0.0);
 }
 
-// Columns of an output tile. 192 (where the epilogue works on independent 64-column chunks) only for a gain of 6 %: such tiles fetch as
-// many bytes of an MN-major operand as 256. Outputs of 576 and 960 columns are whole numbers of them. Measured 256 / 128 / 192 (us), unsplit
-// unless noted: input gradient 4096 x 576 x 3072: 20.7 / 19.8 / 17.2; 2048 x 576 x 49152, in parts: 101 / 120 / 91; weight gradient 960 x 2560 over
-// 4,096 tokens: 26.0 / 27.3 / 22.5; 49152 x 576 over 2,048: 110 / 118 / 102; 5120 x 960 over 8,192: 76.8 / 81.2 / 69.3; SwiGLU backward 4096 x
-// 1536 x 576: 23.4 / 20.1 / 19.6; and where it loses: forward 4096 x 960 x 2560: 20.9 / 20.7 / 25.0; 4096 x 2048 x 2048: 26.7 / 31.1 / 28.6.
-// (Constants of 192 columns fitted to 66 shapes; the choice among the three is 0.03 % off the best there, without 192 columns 3.6 %.)
-constexpr double GAIN_192 = 0.94;
-static int tile_columns(int M, int n_cols, int K, bool f32, bool has_192) {
+// gemm_us over the gain that tiles of bn columns have to promise. Narrower tiles fetch more operand bytes per product (192 columns as
+// many bytes of an MN-major B as 256), and where these come from HBM or L2's bandwidth is short, that takes what gemm_us sees them give. So 192
+// columns need a gain of 6 %, of 12 % for an MN-major B from K = 2048 on; 128 columns in more than one wave 7 %, from K = 4096 on 12 %, and
+// 20 % beyond K = 8192 whatever the waves; and among parts, those of 128 columns 5 %. Fitted to 864 shapes (widths of a 20M to an 8B model, 64 to
+// 8,192 tokens, operands not in L2; every layout and epilogue with 128 and 256 columns, RoPE and SwiGLU forward without, the others with 192): 3 of
+// them are more than 3 % slower than with 256 columns wherever 128 give several waves (22 without these gains, by up to 17 %), and the choice is
+// 0.5 % off the best one on average (RoPE 0.15, SwiGLU 0.0, its backward 0.1, forward 1.0, with residual 2.1, input gradients 0.4, weight gradients 0.4 %).
+// Measured 256 / 128 columns (us): SwiGLU backward 1024 x 11008 x 4096: 86.1 / 101.0; 768 x 14336 x 4096: 88.1 / 102.4; SwiGLU 512 x 22016 x 4096:
+// 81.9 / 92.6; RoPE 512 x 12288 x 4096: 55.3 / 59.5; input gradient 1024 x 2048 x 16384: 60.4 in two parts / 65.8; weight gradient 2048 x 512 over
+// 8,192 tokens: 27.6 in four parts / 29.6 in two. 256 / 192: SwiGLU backward 2048 x 8192 x 2048: 69.7 / 73.7.
+// Where narrow ones win, 256 / 128 / 192: input gradient 4096 x 576 x 3072: 20.7 / 19.8 / 17.2; 2048 x 576 x 49152, in parts: 101 / 120 / 91; weight
+// gradient 960 x 2560 over 4,096 tokens: 26.0 / 27.3 / 22.5; 49152 x 576 over 2,048: 110 / 118 / 102; 5120 x 960 over 8,192: 76.8 / 81.2 / 69.3.
+static double choice_us(int M, int n_cols, int K, int bn, int parts, bool f32, bool b_mn) {
+  double gain = 1.0;
+  if (bn == 192) gain = b_mn && parts == 1 && K >= 2048 ? 0.88 : 0.94;
+  if (bn == 128) {
+    const long long units = (long long)((M + 2 * BM - 1) / (2 * BM)) * ((n_cols + bn - 1) / bn);
+    if (parts > 1) gain = 0.95;
+    else if (K > 8192) gain = 0.8;
+    else if (units > num_pairs()) gain = K < 4096 ? 0.93 : 0.88;
+  }
+  return gemm_us(M, n_cols, K, bn, parts, f32) / gain;
+}
+
+// Columns of an output tile; 192 where the epilogue works on independent 64-column chunks.
+static int tile_columns(int M, int n_cols, int K, bool f32, bool b_mn, bool has_192) {
   if (g_tile_n) return g_tile_n == 192 && !has_192 ? 256 : g_tile_n;
-  const double t128 = gemm_us(M, n_cols, K, 128, 1, f32), t256 = gemm_us(M, n_cols, K, 256, 1, f32);
-  if (has_192 && gemm_us(M, n_cols, K, 192, 1, f32) < GAIN_192 * std::min(t128, t256)) return 192;
-  return t128 < t256 ? 128 : 256;
+  int best = 256;
+  double best_us = choice_us(M, n_cols, K, 256, 1, f32, b_mn);
+  for (const int bn : {192, 128}) {
+    if (bn == 192 && !has_192) continue;
+    const double us = choice_us(M, n_cols, K, bn, 1, f32, b_mn);
+    if (us < best_us) {
+      best = bn;
+      best_us = us;
+    }
+  }
+  return best;
 }
 
 template <bool A_MN, bool B_MN, int OUT_MODE, bool EPI_TMA, int EPI = EPI_NONE, int BN = 256>
@@ -875,7 +901,12 @@ static int run_pair(const void* A, const void* B, void* D, int M, int N, int K, 
 }  // namespace gemm_pair
 }  // namespace pt
 
-// How many parts K is split into (1: not at all) and the columns of a tile then, by gemm_us; adding the weight gradient to what is
+// Columns of the tiles of an unsplit GEMM with n_cols output columns (fp32 or bf16 results; B MN-major or not; 192 columns allowed or not).
+extern "C" int pt_gemm_tile_columns(int M, int n_cols, int K, int f32, int b_mn, int has_192) {
+  return pt::gemm_pair::tile_columns(M, n_cols, K, f32 != 0, b_mn != 0, has_192 != 0);
+}
+
+// How many parts K is split into (1: not at all) and the columns of a tile then, by choice_us; adding the weight gradient to what is
 // there costs 0.08 us a megabyte more in the GEMM's epilogue than in the summing kernel; an input gradient clears its slices first. A
 // split has to give 3 %, or 15 % (2048 x 2048 x 128256 on 64 whole tiles: 724 us, in parts 760), and a forward GEMM 2 us more: its second
 // launch costs the host 3.5, and passes of small forward GEMMs are bound by the host (256 x 576 x 1536 is 8.7 us whole and 7.6 in five
@@ -883,27 +914,31 @@ static int run_pair(const void* A, const void* B, void* D, int M, int N, int K, 
 extern "C" int pt_gemm_split_parts(int M, int N, int K, int kind, int* tile_n) {
   using namespace pt::gemm_pair;
   *tile_n = g_tile_n ? g_tile_n : 256;
-  const bool wgrad = kind == SPLIT_WGRAD;
+  const bool wgrad = kind == SPLIT_WGRAD, b_mn = kind != SPLIT_FWD;
   if (M <= 0 || N <= 0 || K <= 0 || !g_split_k || (!wgrad && N % 8)) return 1;
   const int kb = (K + BK - 1) / BK;
   if (g_split_k > 1) return g_split_k < kb ? g_split_k : kb;
   if (g_tile_n) return 1;                  // (a width given for a measurement: of whole tiles)
   // (where whole tiles fill more than half of the pairs, what is left to gain is less than what parts at different K cost in L2 reuse)
   const bool few = 2LL * ((M + 2 * BM - 1) / (2 * BM)) * ((N + 255) / 256) <= num_pairs();
-  const double whole = gemm_us(M, N, K, tile_columns(M, N, K, wgrad, true), 1, wgrad) + (wgrad ? 0.08 * M * N * 4e-6 : 0.0);
-  double best = (few ? 0.97 : 0.85) * whole - (kind == SPLIT_FWD ? 2.0 : 0.0);
-  int best_parts = 1;
+  const double whole = choice_us(M, N, K, tile_columns(M, N, K, wgrad, b_mn, true), 1, wgrad, b_mn) + (wgrad ? 0.08 * M * N * 4e-6 : 0.0);
+  double best = 1e30;
+  int best_parts = 1, best_bn = 256;
   for (const int parts : {2, 3, 4, 5, 6, 8, 10, 12, 16, 20, 24, 32}) {
     if (kb / parts < 2) break;
     for (const int bn : {128, 192, 256}) {
-      const double t = gemm_us(M, N, K, bn, parts, true) / (bn == 192 ? GAIN_192 : 1.0) + (kind == SPLIT_DGRAD ? 2.0 : 0.0);
+      const double t = choice_us(M, N, K, bn, parts, true, b_mn);
       if (t < best) {
         best = t;
         best_parts = parts;
-        *tile_n = bn;
+        best_bn = bn;
       }
     }
   }
+  if (best_parts == 1) return 1;
+  const double split = gemm_us(M, N, K, best_bn, best_parts, true) + (kind == SPLIT_DGRAD ? 2.0 : 0.0);
+  if (split >= (few ? 0.97 : 0.85) * whole - (kind == SPLIT_FWD ? 2.0 : 0.0)) return 1;
+  *tile_n = best_bn;
   return best_parts;
 }
 
@@ -958,7 +993,7 @@ static int pt::gemm_pair::run_pair(const void* A, const void* B, void* D, int M,
   const bool epi_tma = g_tma_epilogue != 0;
   // narrow tiles exist for the layouts of the model: X W^T, dY W, and dY^T X into fp32
   const bool has_narrow = epi_tma && (out_mode == OUT_BF16 ? !a_mn : (b_mn || (!a_mn && out_mode == OUT_F32)));
-  const int bn = !has_narrow ? 256 : split ? split->bn : tile_columns(M, N, K, out_mode != OUT_BF16, true);
+  const int bn = !has_narrow ? 256 : split ? split->bn : tile_columns(M, N, K, out_mode != OUT_BF16, b_mn != 0, true);
   CUtensorMap ma, mb;
   int rc;
   rc = a_mn ? make_bf16_map_2d(&ma, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, 64, BK)
@@ -1046,7 +1081,7 @@ extern "C" int pt_gemm_bf16_fused(const void* A, const void* B, void* D, int M, 
     return -11;
   }
   if (M <= 0 || n_out <= 0 || K <= 0) return 0;
-  const int bn = tile_columns(M, epi == EPI_SWIGLU_BWD ? inter : n_out, K, false, epi == EPI_ADD || epi == EPI_SWIGLU_BWD);
+  const int bn = tile_columns(M, epi == EPI_SWIGLU_BWD ? inter : n_out, K, false, epi == EPI_SWIGLU_BWD, epi == EPI_ADD || epi == EPI_SWIGLU_BWD);
   CUtensorMap ma, mb, md, mh;
   int rc;
   if ((rc = make_bf16_map_2d(&ma, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda, BK, BM))) return rc * 10 - 1;

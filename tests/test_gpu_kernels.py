@@ -156,6 +156,36 @@ def test_gemm_tile_widths_and_parts_of_every_layout(tile_n, parts, M, N, K):
     assert _rel(acc.double() - 0.5, xt.double().t() @ wt.double()) < 1e-5
 
 
+# us by (columns of a tile, parts), each the middle of ten runs with operands not in L2
+MEASURED_PLANS = [
+    ("swiglu_bwd", 1024, 11008, 4096, {(128, 1): 101.0, (192, 1): 98.2, (256, 1): 86.1}),
+    ("swiglu_bwd", 768, 14336, 4096, {(128, 1): 102.4, (256, 1): 88.1}),
+    ("swiglu_bwd", 2048, 8192, 2048, {(128, 1): 81.9, (192, 1): 73.7, (256, 1): 69.7}),
+    ("swiglu", 512, 22016, 4096, {(128, 1): 92.6, (256, 1): 81.9}),
+    ("rope", 512, 12288, 4096, {(128, 1): 59.5, (256, 1): 55.3}),
+    ("dgrad", 1024, 2048, 16384, {(128, 1): 65.8, (256, 2): 60.4}),
+    ("dgrad", 512, 4096, 12288, {(128, 1): 57.3, (256, 2): 52.9}),
+    ("wgrad", 2048, 512, 8192, {(128, 2): 29.6, (256, 4): 27.6, (192, 3): 27.6}),
+    ("fwd", 128, 4096, 4096, {(128, 2): 23.5, (128, 1): 26.2}),
+    ("dgrad", 4096, 576, 3072, {(256, 1): 20.7, (128, 1): 19.8, (192, 1): 17.2}),
+    ("wgrad", 49152, 576, 2048, {(256, 1): 110.0, (128, 1): 118.0, (192, 1): 102.0}),
+    ("fwd", 256, 576, 576, {(256, 1): 7.1, (128, 1): 5.3}),
+]
+
+
+@pytest.mark.parametrize("kind,M,N,K,us", MEASURED_PLANS)
+def test_gemm_tiles_and_parts_are_the_fastest_measured(kind, M, N, K, us):
+    """The rule's choice among plans that were measured (3 %: what runs of one plan differ by)."""
+    from picotron_b200.ops import _ext
+    C = _ext.load()
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("measured on 148 SMs")
+    C.set_gemm_pair(True)
+    C.set_gemm_tma_epilogue(True)
+    plan = tuple(C.gemm_plan(kind, M, N, K))
+    assert plan in us and us[plan] <= 1.03 * min(us.values()), plan
+
+
 @pytest.mark.parametrize("T,N,K", [(64, 576, 49152), (500, 520, 16392), (300, 2048, 16384)])
 def test_gemm_input_gradient_parts_are_repeatable(C, T, N, K):
     from picotron_b200.ops import _ext
