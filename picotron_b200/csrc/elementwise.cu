@@ -457,9 +457,10 @@ using namespace pt;
 // and now, us, launch included: forward / with add / backward of 8192 x 576: 15.2 -> 11.3 / 17.5 -> 15.0 / 27.6 -> 17.5;
 // 4096 x 960: 12.3 -> 10.2 / 14.4 / 20.6 -> 16.4; 4096 x 2048: 14.3 / 20.5 -> 18.5 / 24.6 -> 22.6; wide rows gain nothing: 4096 x
 // 4096: 20.5 -> 21.4 / 30.7 / 41.9 -> 43.0, 32768 x 2048: 56.3 -> 59.4 / 95.1 -> 94.2 / 110.6 -> 104.4.)
-// The backward's next rows travel through shared memory while one is reduced (its rows were one load latency after the other): without /
-// with, inputs not in L2: 8192 x 576: 11.5 -> 10.5, 4096 x 960: 10.6 -> 9.3, 4096 x 2048: 16.3 -> 15.4, 8192 x 4096: 58.1 -> 52.5, 32768 x
-// 2048: 95.1 -> 83.0 (6.5 TB/s); few rows (512 x 2048: 5.1 -> 5.0) have nothing to fetch ahead.
+// The backward's next rows travel through shared memory while one is reduced (its rows were one load latency after the other). Without /
+// with, us, inputs not in L2: 8192 x 256: 7.3 -> 6.8, 8192 x 512: 9.9 -> 9.3, 8192 x 576: 12.1 -> 10.6, 8192 x 960: 17.9 -> 14.3, 2048 x 2048: 10.6 -> 9.6,
+// 32768 x 2048: 96.8 -> 81.1 (6.6 TB/s), 8192 x 4096: 60.1 -> 54.4, 8192 x 8192: 107.8 -> 93.4; few rows have nothing to fetch ahead (512 x 2048:
+// 5.7 -> 5.2, 512 x 264: 2.7 -> 2.8).
 // ---------------------------------------------------------------------------------------------
 constexpr int ROWS_THREADS = 256;
 
@@ -569,10 +570,12 @@ rmsnorm_fwd_rows_kernel(const bf16* __restrict__ x, const bf16* __restrict__ del
 }
 
 // Backward: a team has the next rows' operands on their way into shared memory (cp.async, every thread the chunks it will use itself, so
-// no barrier is needed) while it works on one. Rows in flight per team, and the bytes that takes per CTA.
-template <int NC> __host__ __device__ constexpr int bwd_stages() { return NC <= 1 ? 4 : NC == 2 ? 3 : 2; }
+// no barrier is needed) while it works on one. Rows in flight per team, and the bytes that takes per CTA. Two are enough where three CTAs
+// of several teams share an SM; a third would take 221 of its 228 KB (three / two, us: 8192 x 512: 10.6 / 9.3, 32768 x 264: 23.2 / 21.8, 2048 x 2048: 11.0 / 9.6);
+// a CTA that is one team wants three (8192 x 4096: 54.4 / 58.4), rows of one chunk a thread four (8192 x 64: 4.8 / 5.4 with two).
+template <int TEAM, int NC> __host__ __device__ constexpr int bwd_stages() { return NC <= 1 ? 4 : NC == 2 && TEAM == ROWS_THREADS ? 3 : 2; }
 template <int TEAM, int NC> __host__ __device__ constexpr int bwd_smem() {
-  const int pipe = bwd_stages<NC>() * 3 * NC * ROWS_THREADS * 16, comb = TEAM < ROWS_THREADS ? ROWS_THREADS * NC * 32 : 0;
+  const int pipe = bwd_stages<TEAM, NC>() * 3 * NC * ROWS_THREADS * 16, comb = TEAM < ROWS_THREADS ? ROWS_THREADS * NC * 32 : 0;
   return pipe > comb ? pipe : comb;
 }
 __device__ __forceinline__ void cp_async16(void* smem, const void* g) {
@@ -586,7 +589,7 @@ rmsnorm_bwd_rows_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x,
                         float* __restrict__ dw_acc, int T, int H) {
   constexpr int TEAMS = ROWS_THREADS / TEAM;
   __shared__ __align__(16) float red[2 * TEAMS * 8];
-  constexpr int STAGES = bwd_stages<NC>();
+  constexpr int STAGES = bwd_stages<TEAM, NC>();
   extern __shared__ __align__(16) uint4 pipe[];      // [stage][x, dy, dres][chunk][thread]; after the rows the teams' sums
   pdl_enter();
   const int nchunk = H / 8, tid = threadIdx.x % TEAM, team = threadIdx.x / TEAM;
