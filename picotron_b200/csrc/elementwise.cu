@@ -911,7 +911,7 @@ extern "C" int pt_embedding_fwd(const long long* ids, const void* w, void* out, 
 extern "C" int pt_embedding_bwd(const long long* ids, const void* dy, float* dw, long long T, int H, long long rows,
                                 long long vocab_start, cudaStream_t st) {
   if (H % 8) return -10;
-  if (T == 0) return 0;
+  if (T == 0 || H == 0) return 0;
   const dim3 grid((unsigned)((T * (H / 8) + 255) / 256));
   if ((reinterpret_cast<uintptr_t>(dw) & 15) == 0)
     launch_pdl(embedding_bwd_kernel<true>, grid, dim3(256), 0, st, ids, (const bf16*)dy, dw, T, H / 8, rows, vocab_start);

@@ -561,6 +561,12 @@ def test_embedding_backward_of_repeated_ids_and_any_alignment(C, T, H, off):
     torch.testing.assert_close(dw.double(), want, rtol=0, atol=60 * 2.0 ** -20)
 
 
+def test_embedding_backward_without_columns_does_nothing(C):
+    ids = torch.zeros(5, device="cuda", dtype=torch.long)
+    C.embedding_bwd(ids, torch.empty(5, 0, device="cuda", dtype=torch.bfloat16), torch.empty(3, 0, device="cuda"), 0)
+    _status_ok(C)
+
+
 @pytest.mark.parametrize("V,start", [(1000, 0), (4096, 4096), (50257, 0)])
 def test_cross_entropy_stats_and_grad(C, V, start):
     T = 64
