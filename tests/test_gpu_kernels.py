@@ -425,10 +425,14 @@ def test_rmsnorm_at_the_edges_of_its_team_sizes(C, T, H):
     torch.testing.assert_close(acc - 0.5, dw_ref, rtol=1e-4, atol=1e-5 * T ** 0.5 * 16)
 
 
+# one width per variant of the kernel: rows a CTA works on at a time, its CTAs per SM, rows in flight per team (with_backward_team, bwd_stages)
 @pytest.mark.parametrize("residual", [True, False])
-@pytest.mark.parametrize("T,H", [(9001, 256), (9001, 576), (9001, 960), (4000, 1032), (3000, 4104)])
-def test_rmsnorm_backward_with_rows_fetched_ahead(C, T, H, residual):
-    """Enough rows for every team to go round its ring of fetched rows more than once, the last round partly filled."""
+@pytest.mark.parametrize("H,rows,ctas,slots", [(256, 8, 3, 4), (264, 8, 3, 2), (512, 8, 3, 2), (576, 8, 2, 2), (960, 8, 2, 2), (1032, 2, 3, 2),
+                                               (2056, 1, 3, 3), (4104, 1, 2, 2)])
+def test_rmsnorm_backward_with_rows_fetched_ahead(C, H, rows, ctas, slots, residual):
+    """Every team goes round its ring of fetched rows more than twice, some a row further than the others."""
+    teams = rows * ctas * torch.cuda.get_device_properties(0).multi_processor_count
+    T = 2 * slots * teams + teams // 2 + 1
     x, dy = bf(T, H, seed=1), bf(T, H, seed=2)
     dres = bf(T, H, seed=3) if residual else None
     w = (1 + 0.1 * bf(H, seed=4).float()).to(torch.bfloat16)
