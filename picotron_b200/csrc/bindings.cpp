@@ -338,6 +338,7 @@ Tensor gemm(const Tensor& a, const Tensor& b, bool trans_a, bool trans_b, const 
     d = torch::empty({M, N}, a.options());
     mode = 0;
   }
+  if (K == 0) return mode == 1 ? d : d.zero_();          // (the weight gradient of no tokens: the GEMM writes nothing)
   gemm_into(a.data_ptr(), b.data_ptr(), d.data_ptr(), M, N, K, lda, ldb, row_stride_2d(d, "out"), trans_a, trans_b, mode, a.options());
   return d;
 }

@@ -156,6 +156,18 @@ def test_gemm_tile_widths_and_parts_of_every_layout(tile_n, parts, M, N, K):
     assert _rel(acc.double() - 0.5, xt.double().t() @ wt.double()) < 1e-5
 
 
+def test_gemm_over_nothing_is_zero(C):
+    """The weight gradient of an empty batch: zeros, or what the destination holds where it is added to."""
+    dy, x = bf(0, 72), bf(0, 136)
+    stale = [torch.full((72, 136), float("nan"), device="cuda", dtype=torch.bfloat16) for _ in range(4)]
+    del stale                                                 # (the allocator hands the same memory out again)
+    assert torch.count_nonzero(C.gemm(dy, x, True, True)) == 0
+    acc = torch.full((72, 136), 0.5, device="cuda")
+    assert C.gemm(dy, x, True, True, acc, True).eq(0.5).all()
+    assert C.gemm(dy, x, True, True, acc, False).eq(0.0).all()
+    assert C.gemm(x, bf(200, 136), False, False).shape == (0, 200)
+
+
 # us by (columns of a tile, parts), each the middle of ten runs with operands not in L2
 MEASURED_PLANS = [
     ("swiglu_bwd", 1024, 11008, 4096, {(128, 1): 101.0, (192, 1): 98.2, (256, 1): 86.1}),
