@@ -1,7 +1,7 @@
 // bf16 GEMM for sm_100a on CTA pairs (tcgen05 cta_group::2): D[M,N] = op(A) * op(B), fp32 accumulate in TMEM.
 //
 // Same contract and operand layouts as gemm_tcgen05.cu, but two CTAs (a cluster of 2 on neighbouring SMs)
-// cooperate on one output tile of 256 rows and 256, 192 or 128 columns (see choice_us for which): each CTA loads
+// cooperate on one output tile of 256 rows and 256, 192 or 128 columns (see gain_asked for which): each CTA loads
 // its own 128 rows of A and its own half of the columns of B -- with plain, non-multicast TMA loads -- and one
 // thread of the leader CTA issues a 256-row MMA that
 // reads both CTAs' shared memory and writes both CTAs' tensor memory. Per output element this moves a
@@ -770,18 +770,25 @@ static thread_local int g_tile_n = 0;    // 0: by the rule below, 128 / 192 / 25
 // 576: 7.1 / 5.3; 1024 x 2048 x 2048: 14.9 / 10.2; 8192 x 2048 x 2048: 47.0 / 50.4; weight gradient 576 x 576, 512 tokens: 8.6 / 6.2;
 // 2048 x 576 x 3072: 18.0 / 11.3; with residual 256 x 2048 x 8192: 43.0 / 24.5 / 12.8; input gradient 512 x 2048 x 16384: 78 / 54 /
 // 35.5 (31.5 with 256 columns).
-static double gemm_us(int M, int n_cols, int K, int bn, int parts, bool f32) {
-  const int pairs = num_pairs(), kb = (K + BK - 1) / BK, kb_part = (kb + parts - 1) / parts;
-  const long long units = (long long)((M + 2 * BM - 1) / (2 * BM)) * ((n_cols + bn - 1) / bn) * ((kb + kb_part - 1) / kb_part);
-  const double load = units < pairs ? (double)units / pairs : 1.0, waves = (double)((units + pairs - 1) / pairs);
-  const bool slices = parts > 1;
+// (asked: the parts K is to be split into; parts, kb_part: how many k-blocks of at most kb_part each that gives.)
+struct GemmShape {
+  int M, n_cols, K, kb;
+  GemmShape(int M_, int n_cols_, int K_) : M(M_), n_cols(n_cols_), K(K_), kb((K_ + BK - 1) / BK) {}
+  long long tiles(int bn) const { return (long long)((M + 2 * BM - 1) / (2 * BM)) * ((n_cols + bn - 1) / bn); }
+  double mbytes32() const { return (double)M * n_cols * 4e-6; }
+};
+static double gemm_us(const GemmShape& g, int bn, int asked, int parts, int kb_part, bool f32) {
+  const int pairs = num_pairs();
+  const long long units = g.tiles(bn) * parts;
+  const double load = units < pairs ? (double)units / pairs : 1.0, waves = units <= pairs ? 1.0 : (double)((units + pairs - 1) / pairs);
+  const bool slices = asked > 1;
   const double unit = bn == 256   ? kb_part * (0.29 + 0.026 * load) + 1.6 + (f32 || slices ? 0.8 : 0)
                       : bn == 192 ? kb_part * (0.21 + 0.02 * load) + 1.25 + (f32 || slices ? 1.5 : 0)
                                   : kb_part * (0.149 + 0.04 * load) + 0.85 + (f32 || slices ? 0.55 : 0);
-  return waves * unit + (slices ? 1.0 + 0.147 * parts * M * n_cols * 4e-6 : 0.0);
+  return waves * unit + (slices ? 1.0 + 0.147 * asked * g.mbytes32() : 0.0);
 }
 
-// gemm_us over the gain that tiles of bn columns have to promise. Narrower tiles fetch more operand bytes per product (192 columns as
+// The gain that tiles of bn columns have to promise over wider ones. Narrower tiles fetch more operand bytes per product (192 columns as
 // many bytes of an MN-major B as 256), and where these come from HBM or L2's bandwidth is short, that takes what gemm_us sees them give. So 192
 // columns need a gain of 6 %, of 12 % for an MN-major B from K = 2048 on; 128 columns in more than one wave 7 %, from K = 4096 on 12 %, and
 // 20 % beyond K = 8192 whatever the waves; and among parts, those of 128 columns 5 %. Fitted to 864 shapes (widths of a 20M to an 8B model, 64 to
@@ -793,26 +800,24 @@ static double gemm_us(int M, int n_cols, int K, int bn, int parts, bool f32) {
 // 8,192 tokens: 27.6 in four parts / 29.6 in two. 256 / 192: SwiGLU backward 2048 x 8192 x 2048: 69.7 / 73.7.
 // Where narrow ones win, 256 / 128 / 192: input gradient 4096 x 576 x 3072: 20.7 / 19.8 / 17.2; 2048 x 576 x 49152, in parts: 101 / 120 / 91; weight
 // gradient 960 x 2560 over 4,096 tokens: 26.0 / 27.3 / 22.5; 49152 x 576 over 2,048: 110 / 118 / 102; 5120 x 960 over 8,192: 76.8 / 81.2 / 69.3.
-static double choice_us(int M, int n_cols, int K, int bn, int parts, bool f32, bool b_mn) {
-  double gain = 1.0;
-  if (bn == 192) gain = b_mn && parts == 1 && K >= 2048 ? 0.88 : 0.94;
-  if (bn == 128) {
-    const long long units = (long long)((M + 2 * BM - 1) / (2 * BM)) * ((n_cols + bn - 1) / bn);
-    if (parts > 1) gain = 0.95;
-    else if (K > 8192) gain = 0.8;
-    else if (units > num_pairs()) gain = K < 4096 ? 0.93 : 0.88;
-  }
-  return gemm_us(M, n_cols, K, bn, parts, f32) / gain;
+static double gain_asked(const GemmShape& g, int bn, int parts, bool b_mn) {
+  if (bn == 192) return b_mn && parts == 1 && g.K >= 2048 ? 0.88 : 0.94;
+  if (bn == 256) return 1.0;
+  if (parts > 1) return 0.95;
+  if (g.K > 8192) return 0.8;
+  return g.tiles(128) <= num_pairs() ? 1.0 : g.K < 4096 ? 0.93 : 0.88;
 }
+static double whole_us(const GemmShape& g, int bn, bool f32, bool b_mn) { return gemm_us(g, bn, 1, 1, g.kb, f32) / gain_asked(g, bn, 1, b_mn); }
 
 // Columns of an output tile; 192 where the epilogue works on independent 64-column chunks.
 static int tile_columns(int M, int n_cols, int K, bool f32, bool b_mn, bool has_192) {
   if (g_tile_n) return g_tile_n == 192 && !has_192 ? 256 : g_tile_n;
+  const GemmShape g(M, n_cols, K);
   int best = 256;
-  double best_us = choice_us(M, n_cols, K, 256, 1, f32, b_mn);
+  double best_us = whole_us(g, 256, f32, b_mn);
   for (const int bn : {192, 128}) {
     if (bn == 192 && !has_192) continue;
-    const double us = choice_us(M, n_cols, K, bn, 1, f32, b_mn);
+    const double us = whole_us(g, bn, f32, b_mn);
     if (us < best_us) {
       best = bn;
       best_us = us;
@@ -906,7 +911,7 @@ extern "C" int pt_gemm_tile_columns(int M, int n_cols, int K, int f32, int b_mn,
   return pt::gemm_pair::tile_columns(M, n_cols, K, f32 != 0, b_mn != 0, has_192 != 0);
 }
 
-// How many parts K is split into (1: not at all) and the columns of a tile then, by choice_us; adding the weight gradient to what is
+// How many parts K is split into (1: not at all) and the columns of a tile then, by gemm_us and gain_asked; adding the weight gradient to what is
 // there costs 0.08 us a megabyte more in the GEMM's epilogue than in the summing kernel; an input gradient clears its slices first. A
 // split has to give 3 %, or 15 % (2048 x 2048 x 128256 on 64 whole tiles: 724 us, in parts 760), and a forward GEMM 2 us more: its second
 // launch costs the host 3.5, and passes of small forward GEMMs are bound by the host (256 x 576 x 1536 is 8.7 us whole and 7.6 in five
@@ -916,27 +921,29 @@ extern "C" int pt_gemm_split_parts(int M, int N, int K, int kind, int* tile_n) {
   *tile_n = g_tile_n ? g_tile_n : 256;
   const bool wgrad = kind == SPLIT_WGRAD, b_mn = kind != SPLIT_FWD;
   if (M <= 0 || N <= 0 || K <= 0 || !g_split_k || (!wgrad && N % 8)) return 1;
-  const int kb = (K + BK - 1) / BK;
-  if (g_split_k > 1) return g_split_k < kb ? g_split_k : kb;
+  const GemmShape g(M, N, K);
+  if (g_split_k > 1) return g_split_k < g.kb ? g_split_k : g.kb;
   if (g_tile_n) return 1;                  // (a width given for a measurement: of whole tiles)
   // (where whole tiles fill more than half of the pairs, what is left to gain is less than what parts at different K cost in L2 reuse)
-  const bool few = 2LL * ((M + 2 * BM - 1) / (2 * BM)) * ((N + 255) / 256) <= num_pairs();
-  const double whole = choice_us(M, N, K, tile_columns(M, N, K, wgrad, b_mn, true), 1, wgrad, b_mn) + (wgrad ? 0.08 * M * N * 4e-6 : 0.0);
-  double best = 1e30;
+  const bool few = 2 * g.tiles(256) <= num_pairs();
+  const double whole = whole_us(g, tile_columns(M, N, K, wgrad, b_mn, true), wgrad, b_mn) + (wgrad ? 0.08 * g.mbytes32() : 0.0);
+  double best = 1e30, best_us = 0;
   int best_parts = 1, best_bn = 256;
-  for (const int parts : {2, 3, 4, 5, 6, 8, 10, 12, 16, 20, 24, 32}) {
-    if (kb / parts < 2) break;
+  for (const int asked : {2, 3, 4, 5, 6, 8, 10, 12, 16, 20, 24, 32}) {
+    if (g.kb < 2 * asked) break;
+    const int kb_part = (g.kb + asked - 1) / asked, parts = (g.kb + kb_part - 1) / kb_part;
     for (const int bn : {128, 192, 256}) {
-      const double t = choice_us(M, N, K, bn, parts, true, b_mn);
+      const double us = gemm_us(g, bn, asked, parts, kb_part, true), t = us / gain_asked(g, bn, asked, b_mn);
       if (t < best) {
         best = t;
-        best_parts = parts;
+        best_us = us;
+        best_parts = asked;
         best_bn = bn;
       }
     }
   }
   if (best_parts == 1) return 1;
-  const double split = gemm_us(M, N, K, best_bn, best_parts, true) + (kind == SPLIT_DGRAD ? 2.0 : 0.0);
+  const double split = best_us + (kind == SPLIT_DGRAD ? 2.0 : 0.0);
   if (split >= (few ? 0.97 : 0.85) * whole - (kind == SPLIT_FWD ? 2.0 : 0.0)) return 1;
   *tile_n = best_bn;
   return best_parts;
