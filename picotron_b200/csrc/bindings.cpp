@@ -585,10 +585,10 @@ std::vector<Tensor> attention_bwd(const Tensor& dout, const Tensor& q, const Ten
 
 // ---------------------------------------------------------------------------------------------
 // A decoder layer's launches in one call (one GPU per layer: no tensor, sequence or context parallelism). Small models and
-// short sequences are bound by the host: from Python every launch costs 12 to 20 us, more than most of their kernels take, and with
-// a tensor object per operand one native call still took 75 us per layer, half of it allocations, views and tensor bookkeeping.
-// (43 us of it in the native call, 26 as it is now.) So what the backward needs lies in TWO allocations (bf16 and fp32), addressed by offsets. The kernels, their order and the
-// fallbacks are those of the layer node's Python path.
+// short sequences are bound by the host: from Python every launch costs 12 to 20 us, more than most of their kernels take, and a
+// tensor object per operand costs again: the native call of a forward layer took 43 us with one and takes 26 as it is. So what the
+// backward needs lies in TWO allocations (bf16 and fp32), addressed by offsets. The kernels, their order and the fallbacks are those of
+// the layer node's Python path.
 // ---------------------------------------------------------------------------------------------
 struct LayerDims {
   int64_t B, S, H, I, hq, hkv, d;
@@ -1041,7 +1041,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("set_gemm_group_m", [](int64_t g) { pt_gemm_set_group_m((int)g); },
         "CTA-pair GEMM tile numbering: rows of 256-row tiles per group (L2 locality of concurrently running tiles; default 8).");
   m.def("set_gemm_split_dgrad", [](bool on) { pt_gemm_set_split_k(on ? 1 : 0); },
-        "input- and weight-gradient GEMMs with few output tiles: K split over idle CTA pairs (default on; for the calling thread)");
+        "GEMMs with few output tiles (forward, with a residual, input and weight gradients): K split over idle CTA pairs (default on; for the "
+         "calling thread)");
   m.def("set_gemm_split_parts", [](int64_t n) { pt_gemm_set_split_k(n > 1 ? (int)n : 1); },
         "GEMMs that may be split over K are always cut into n parts by this thread (tests, measurements); 0 or 1: the rule.");
   m.def("gemm_plan", [](const std::string& kind, int64_t M, int64_t N, int64_t K) {
@@ -1055,7 +1056,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         }, "(columns of a tile, parts of K) that the rule gives a GEMM with output [M, N]: kind fwd, add, dgrad, wgrad, rope, swiglu (N = 2I) or\n"
            "swiglu_bwd (N = I).");
   m.def("set_gemm_tile_n", [](int64_t n) { pt_gemm_set_tile_n((int)n); },
-        "columns of the GEMM output tiles: 128, 192 (where the epilogue has it), 256, or 0 for the choice by shape (for the calling thread)");
+        "columns of the GEMM output tiles: 128, 192 (where the epilogue has it), 256, or 0 for the choice by shape (for the calling thread). "
+         "With a given width K is not split, unless set_gemm_split_parts says so.");
   m.def("get_gemm_group_m", []() { return (int64_t)pt_gemm_get_group_m(); });
   m.def("attention_set_profile", [](const c10::optional<Tensor>& counters) {
           if (!counters.has_value()) { pt_attention_set_profile(nullptr); return; }

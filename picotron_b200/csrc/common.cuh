@@ -90,8 +90,8 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-// True in one lane of a full, converged warp, always the same one. Single-thread roles (TMA producer, MMA issuer, TMA stores) branch
-// on this, not on `lane == 0`: tcgen05.mma, tcgen05.commit and the TMA instructions take their operands from uniform registers, and
+// True in one lane of a full, converged warp, always the same one. The single-thread roles of the GEMM and attention kernels (TMA producer,
+// MMA issuer, TMA stores; not yet those of the GEMM with all-reduce) branch on this, not on `lane == 0`: tcgen05.mma, tcgen05.commit and the TMA instructions take their operands from uniform registers, and
 // only for elect.sync does the compiler know that one lane is active; after `lane == 0` an MMA issuer's 64-deep k-block (4 MMAs, 2
 // commits) took 0.305 us whatever the tile, after elect.sync 0.138 us with 256 x 128 tiles and 0.278 us (the MMA's own time) with
 // 256 x 256. Measured before / after (us): 512 x 2048 x 8192: 44.9 / 22.7; 256 x 576 x 1536: 10.8 / 7.1; attention backward of 1 x 32768,

@@ -115,8 +115,11 @@ ce_loss_kernel(const float2* __restrict__ part, const long long* __restrict__ ta
 }
 
 // In-place gradient (softmax - onehot) * scale of a row of logits per CTA; bound by reading and writing the logits. TILES: the
-// row's log-sum-exp comes straight from the tile pairs of the LM-head GEMM (each warp merges them for itself: a few hundred bytes
-// that lie in L2) and its loss term is left in `terms`, instead of from `lse`.
+// row's log-sum-exp comes straight from the tile pairs of the LM-head GEMM and its loss term is left in `terms`, instead of from `lse`. Every
+// warp of the CTA merges the pairs for itself (8 bytes per 256 columns, 1.5 KB a row of 49152 and 4 KB of 128256, from L2 but for the first).
+// Measured, us, 2048 x 49152 / 2048 x 128256 behind a GEMM with K = 64: GEMM and this kernel 186 / 479; GEMM, clearing and merging kernel and the
+// gradient from a given lse 182 / 461 (the gradient alone 69.5 / 180, at the copy rate 62 / 163), without the logarithm, the differences and their
+// sum, which were launches of their own.
 template <bool TILES>
 __global__ void __launch_bounds__(CE_THREADS)
 ce_grad_kernel(bf16* __restrict__ logits, const long long* __restrict__ targets, const float* __restrict__ lse,

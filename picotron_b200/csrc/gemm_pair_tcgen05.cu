@@ -766,11 +766,11 @@ static thread_local int g_tile_n = 0;    // 0: by the rule below, 128 / 192 / 25
 // A 64-deep k-block of a 256 x 256 tile takes the MMA's 512 cycles; one of a 256 x 128 tile half of that, until the pairs share
 // L2's bandwidth (three quarters of the operand bytes for half of the products). Constants fitted to 211 shapes (weight and input
 // gradients, forward with and without residual; widths of 20M to 1.7B models, 256 to 8,192 tokens; both widths, 1 to 32 parts): 7 %
-// off, and the choice it makes 0.5 % slower than the best measured one. Measured 256 / 128 columns / 128 split (us): forward 256 x 576 x
-// 576: 7.1 / 5.3; 1024 x 2048 x 2048: 14.9 / 10.2; 8192 x 2048 x 2048: 47.0 / 50.4; weight gradient 576 x 576, 512 tokens: 8.6 / 6.2;
+// off, and the choice it makes 0.5 % slower than the best measured one; those of 192 columns to 66 shapes. Measured 256 / 128 columns /
+// 128 split (us): forward 256 x 576 x 576: 7.1 / 5.3; 1024 x 2048 x 2048: 14.9 / 10.2; 8192 x 2048 x 2048: 47.0 / 50.4; weight gradient 576 x 576, 512 tokens: 8.6 / 6.2;
 // 2048 x 576 x 3072: 18.0 / 11.3; with residual 256 x 2048 x 8192: 43.0 / 24.5 / 12.8; input gradient 512 x 2048 x 16384: 78 / 54 /
 // 35.5 (31.5 with 256 columns).
-// (asked: the parts K is to be split into; parts, kb_part: how many k-blocks of at most kb_part each that gives.)
+// (asked: the parts K is to be split into; that gives `parts` of at most kb_part k-blocks.)
 struct GemmShape {
   int M, n_cols, K, kb;
   GemmShape(int M_, int n_cols_, int K_) : M(M_), n_cols(n_cols_), K(K_), kb((K_ + BK - 1) / BK) {}

@@ -168,7 +168,7 @@ def test_gemm_over_nothing_is_zero(C):
     assert C.gemm(x, bf(200, 136), False, False).shape == (0, 200)
 
 
-# us by (columns of a tile, parts), each the middle of ten runs with operands not in L2
+# us by (columns of a tile, parts), operands not in L2
 MEASURED_PLANS = [
     ("swiglu_bwd", 1024, 11008, 4096, {(128, 1): 101.0, (192, 1): 98.2, (256, 1): 86.1}),
     ("swiglu_bwd", 768, 14336, 4096, {(128, 1): 102.4, (256, 1): 88.1}),
