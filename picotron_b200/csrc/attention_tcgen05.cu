@@ -52,29 +52,6 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
-// Two fp32 operations per instruction (each rounded as its scalar form): the softmax warps are short of issue slots. Measured (us):
-// forward 32768, d = 64: 6,040 -> 5,970; 4 x 1024, 32 heads, d = 64: forward 62 -> 56, backward 159 -> 147.
-__device__ __forceinline__ uint64_t pair_of(float lo, float hi) {
-  return (uint64_t)__float_as_uint(lo) | ((uint64_t)__float_as_uint(hi) << 32);
-}
-__device__ __forceinline__ float lo_of(uint64_t v) { return __uint_as_float((uint32_t)v); }
-__device__ __forceinline__ float hi_of(uint64_t v) { return __uint_as_float((uint32_t)(v >> 32)); }
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t d;
-  asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-
 // byte offset of the 16-byte unit holding columns [8u, 8u+8) of row r inside one [rows][64] bf16 chunk
 // stored with the 128-byte swizzle (what TMA writes and UMMA descriptors of layout type SWIZZLE_128B read)
 __device__ __forceinline__ uint32_t sw128_offset(int r, int u) { return (uint32_t)(r * 128 + ((u ^ (r & 7)) << 4)); }
