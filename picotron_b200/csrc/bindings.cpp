@@ -652,6 +652,55 @@ inline bool fused_gemm(int rc, const char* what) {          // false: not covere
   return true;
 }
 
+// A layer's weights and tables as the launches take them; q|k|v and gate|up are one matrix each.
+struct LayerPointers {
+  const void *ln1, *w_qkv, *wo, *ln2, *w_gu, *wd;
+  long long ld_qkv, ld_o, ld_gu, ld_d;
+  const float *cosp, *sinp;
+};
+LayerPointers layer_pointers(const Tensor& ln1, const Tensor& w_qkv, const Tensor& cosT, const Tensor& sinT, const Tensor& wo, const Tensor& ln2,
+                             const Tensor& w_gu, const Tensor& wd) {
+  return {ln1.data_ptr(), w_qkv.data_ptr(), wo.data_ptr(), ln2.data_ptr(), w_gu.data_ptr(), wd.data_ptr(), row_stride_2d(w_qkv, "w_qkv"),
+          row_stride_2d(wo, "wo"), row_stride_2d(w_gu, "w_gu"), row_stride_2d(wd, "wd"), cosT.data_ptr<float>(), sinT.data_ptr<float>()};
+}
+
+// The launches of a layer's forward: x [T, H] -> out [T, H], the activations to `b` and `f` (LayerSaved).
+void layer_fwd(const LayerDims& n, const void* x, const LayerPointers& w, double eps, double scale, bf16_t* const b, float* const f, void* out,
+               const at::TensorOptions& on) {
+  const LayerSaved at(n);
+  const int64_t T = n.T(), H = n.H, I = n.I, O = n.O(), Q = n.Q(), B = n.B, S = n.S, hq = n.hq, hkv = n.hkv, d = n.d;
+  bf16_t *const h1 = b + at.h1, *const qkv = b + at.qkv, *const o = b + at.o, *const x_mid = b + at.x_mid, *const h2 = b + at.h2,
+         *const gu = b + at.gu, *const a = b + at.a;
+  const cudaStream_t st = stream();
+  const bool pair = pt_gemm_get_pair();
+  void* const status = pt_status_word();
+  PT_CHECK_RC(pt_rmsnorm_fwd(x, nullptr, w.ln1, nullptr, h1, f + at.rstd1, (int)T, (int)H, (float)eps, st), "rmsnorm_fwd");
+  if (!(pair && Q % 8 == 0 &&
+        fused_gemm(pt_gemm_bf16_fused(h1, w.w_qkv, qkv, (int)T, (int)Q, (int)H, H, w.ld_qkv, Q, 2, nullptr, 0, 0, w.cosp, w.sinp, (int)S,
+                                      (int)(hq + hkv), (int)d, status, st), "gemm_rope"))) {
+    gemm_into(h1, w.w_qkv, qkv, T, Q, H, H, w.ld_qkv, Q, false, false, 0, on);
+    PT_CHECK_RC(pt_rope(qkv, w.cosp, w.sinp, T, (int)(hq + hkv), (int)d, (int)S, Q, 0, st), "rope");
+  }
+  PT_CHECK_RC(pt_attention_fwd(qkv, qkv + O, qkv + O + hkv * d, o, f + at.lse, (int)B, (int)S, (int)S, (int)hq, (int)hkv, (int)d, Q, Q, Q, 1,
+                               (float)scale, st), "attention_fwd");
+  gemm_into(o, w.wo, out, T, H, O, O, w.ld_o, H, false, false, 0, on);     // (`out` is free until the down projection)
+  PT_CHECK_RC(pt_rmsnorm_fwd(x, out, w.ln2, x_mid, h2, f + at.rstd2, (int)T, (int)H, (float)eps, st), "add_rmsnorm_fwd");
+  if (!(pair && I % 128 == 0 &&
+        fused_gemm(pt_gemm_bf16_fused(h2, w.w_gu, gu, (int)T, (int)(2 * I), (int)H, H, w.ld_gu, 2 * I, 1, a, I, (int)I, nullptr, nullptr,
+                                      0, 0, 0, status, st), "gemm_swiglu"))) {
+    gemm_into(h2, w.w_gu, gu, T, 2 * I, H, H, w.ld_gu, 2 * I, false, false, 0, on);
+    PT_CHECK_RC(pt_swiglu_fwd(gu, a, T, (int)I, st), "swiglu_fwd");
+  }
+  if (!(pair && H % 8 == 0 && gemm_split_into(a, w.wd, out, T, H, I, I, w.ld_d, H, 2, x_mid, H, on)) &&
+      !(pair && H % 8 == 0 &&
+        fused_gemm(pt_gemm_bf16_fused(a, w.wd, out, (int)T, (int)H, (int)I, I, w.ld_d, H, 4, x_mid, H, 0, nullptr, nullptr, 0,
+                                      0, 0, status, st), "gemm_add"))) {
+    Tensor y = torch::empty({T, H}, on);
+    gemm_into(a, w.wd, y.data_ptr(), T, H, I, I, w.ld_d, H, false, false, 0, on);
+    PT_CHECK_RC(pt_add(x_mid, y.data_ptr(), out, T * H, st), "add");
+  }
+}
+
 // Returns {x_out, saved bf16, saved fp32} (LayerSaved), or {} (nothing launched) for operands that are not bf16.
 std::vector<Tensor> decoder_layer_fwd_packed(const Tensor& x, const Tensor& ln1, const Tensor& w_qkv, const Tensor& cosT, const Tensor& sinT,
                                              const Tensor& wo, const Tensor& ln2, const Tensor& w_gu, const Tensor& wd, double eps, int64_t B,
@@ -661,47 +710,100 @@ std::vector<Tensor> decoder_layer_fwd_packed(const Tensor& x, const Tensor& ln1,
   const LayerDims n{B, S, x.size(1), w_gu.size(0) / 2, hq, hkv, d};
   check_layer(n, ln1, w_qkv, cosT, sinT, wo, ln2, w_gu, wd);
   const LayerSaved at(n);
-  const int64_t T = n.T(), H = n.H, I = n.I, O = n.O(), Q = n.Q();
   c10::cuda::CUDAGuard guard(x.device());
   const auto on = x.options();
-  Tensor s16 = torch::empty({at.total}, on), s32 = torch::empty({at.total32}, on.dtype(at::kFloat)), out = torch::empty({T, H}, on);
-  bf16_t* const b = bf16_ptr(s16);
-  float* const f = s32.data_ptr<float>();
-  bf16_t *const h1 = b + at.h1, *const qkv = b + at.qkv, *const o = b + at.o, *const x_mid = b + at.x_mid, *const h2 = b + at.h2,
-         *const gu = b + at.gu, *const a = b + at.a;
-  const float *const cosp = cosT.data_ptr<float>(), *const sinp = sinT.data_ptr<float>();
-  const long long ld_qkv = row_stride_2d(w_qkv, "w_qkv"), ld_o = row_stride_2d(wo, "wo"), ld_gu = row_stride_2d(w_gu, "w_gu"),
-                  ld_d = row_stride_2d(wd, "wd");
-  const cudaStream_t st = stream();
-  const bool pair = pt_gemm_get_pair();
-  void* const status = pt_status_word();
-  PT_CHECK_RC(pt_rmsnorm_fwd(x.data_ptr(), nullptr, ln1.data_ptr(), nullptr, h1, f + at.rstd1, (int)T, (int)H, (float)eps, st), "rmsnorm_fwd");
-  if (!(pair && Q % 8 == 0 &&
-        fused_gemm(pt_gemm_bf16_fused(h1, w_qkv.data_ptr(), qkv, (int)T, (int)Q, (int)H, H, ld_qkv, Q, 2, nullptr, 0, 0, cosp, sinp, (int)S,
-                                      (int)(hq + hkv), (int)d, status, st), "gemm_rope"))) {
-    gemm_into(h1, w_qkv.data_ptr(), qkv, T, Q, H, H, ld_qkv, Q, false, false, 0, on);
-    PT_CHECK_RC(pt_rope(qkv, cosp, sinp, T, (int)(hq + hkv), (int)d, (int)S, Q, 0, st), "rope");
-  }
-  PT_CHECK_RC(pt_attention_fwd(qkv, qkv + O, qkv + O + hkv * d, o, f + at.lse, (int)B, (int)S, (int)S, (int)hq, (int)hkv, (int)d, Q, Q, Q, 1,
-                               (float)scale, st), "attention_fwd");
-  gemm_into(o, wo.data_ptr(), out.data_ptr(), T, H, O, O, ld_o, H, false, false, 0, on);     // (`out` is free until the down projection)
-  PT_CHECK_RC(pt_rmsnorm_fwd(x.data_ptr(), out.data_ptr(), ln2.data_ptr(), x_mid, h2, f + at.rstd2, (int)T, (int)H, (float)eps, st),
-              "add_rmsnorm_fwd");
-  if (!(pair && I % 128 == 0 &&
-        fused_gemm(pt_gemm_bf16_fused(h2, w_gu.data_ptr(), gu, (int)T, (int)(2 * I), (int)H, H, ld_gu, 2 * I, 1, a, I, (int)I, nullptr, nullptr,
-                                      0, 0, 0, status, st), "gemm_swiglu"))) {
-    gemm_into(h2, w_gu.data_ptr(), gu, T, 2 * I, H, H, ld_gu, 2 * I, false, false, 0, on);
-    PT_CHECK_RC(pt_swiglu_fwd(gu, a, T, (int)I, st), "swiglu_fwd");
-  }
-  if (!(pair && H % 8 == 0 && gemm_split_into(a, wd.data_ptr(), out.data_ptr(), T, H, I, I, ld_d, H, 2, x_mid, H, on)) &&
-      !(pair && H % 8 == 0 &&
-        fused_gemm(pt_gemm_bf16_fused(a, wd.data_ptr(), out.data_ptr(), (int)T, (int)H, (int)I, I, ld_d, H, 4, x_mid, H, 0, nullptr, nullptr, 0,
-                                      0, 0, status, st), "gemm_add"))) {
-    Tensor y = torch::empty({T, H}, on);
-    gemm_into(a, wd.data_ptr(), y.data_ptr(), T, H, I, I, ld_d, H, false, false, 0, on);
-    PT_CHECK_RC(pt_add(x_mid, y.data_ptr(), out.data_ptr(), T * H, st), "add");
-  }
+  Tensor s16 = torch::empty({at.total}, on), s32 = torch::empty({at.total32}, on.dtype(at::kFloat)), out = torch::empty({n.T(), n.H}, on);
+  layer_fwd(n, x.data_ptr(), layer_pointers(ln1, w_qkv, cosT, sinT, wo, ln2, w_gu, wd), eps, scale, bf16_ptr(s16), s32.data_ptr<float>(),
+            out.data_ptr(), on);
   return {out, s16, s32};
+}
+
+// ---------------------------------------------------------------------------------------------
+// All layers of a model in one call each way. A layer of its own costs the host 25 us (forward) and 85 (backward) in Python and autograd on top
+// of its launches, which small models and short prompts do not hide. `params`: nine tensors a layer (q, k, v, out, gate, up, down, norm 1,
+// norm 2), `tables`: two (cosines, sines).
+// ---------------------------------------------------------------------------------------------
+constexpr int LAYER_PARAMS = 9;
+
+// Matrices that lie back to back in one storage, [rows, cols] together: their address, or nullptr.
+const void* adjacent(const std::vector<Tensor>& ts, size_t first, int count, int64_t rows, int64_t cols) {
+  int64_t seen = 0;
+  const char* const base = reinterpret_cast<const char*>(ts[first].data_ptr());
+  for (size_t i = first; i < first + count; ++i) {
+    const Tensor& t = ts[i];
+    if (t.dim() != 2 || t.size(1) != cols || !t.is_contiguous() || base + seen * cols * 2 != t.data_ptr() ||
+        t.storage().data() != ts[first].storage().data())
+      return nullptr;
+    seen += t.size(0);
+  }
+  return seen == rows ? base : nullptr;
+}
+
+// The layers' operands, or {} where one is not a contiguous bf16 tensor of the expected shape on x's device or its q|k|v or gate|up do not lie
+// back to back (the single layers' calls say what is wrong, or put them together).
+std::vector<LayerPointers> stack_pointers(const LayerDims& n, const Tensor& x, const std::vector<Tensor>& params, const std::vector<Tensor>& tables) {
+  const size_t layers = tables.size() / 2;
+  if (layers == 0 || params.size() != layers * LAYER_PARAMS || tables.size() != 2 * layers) return {};
+  std::vector<LayerPointers> out(layers);
+  for (const Tensor& t : params)
+    if (t.scalar_type() != at::kBFloat16 || !t.is_contiguous() || t.device() != x.device()) return {};
+  for (const Tensor& t : tables)
+    if (t.scalar_type() != at::kFloat || !t.is_contiguous() || t.device() != x.device() || t.dim() != 2 || t.size(0) < n.S || t.size(1) != n.d / 2)
+      return {};
+  for (size_t i = 0; i < layers; ++i) {
+    const size_t p = i * LAYER_PARAMS;
+    LayerPointers& w = out[i];
+    w.w_qkv = adjacent(params, p, 3, n.Q(), n.H);
+    w.wo = adjacent(params, p + 3, 1, n.H, n.O());
+    w.w_gu = adjacent(params, p + 4, 2, 2 * n.I, n.H);
+    w.wd = adjacent(params, p + 6, 1, n.H, n.I);
+    if (!w.w_qkv || !w.wo || !w.w_gu || !w.wd || params[p + 7].numel() != n.H || params[p + 8].numel() != n.H) return {};
+    w.ln1 = params[p + 7].data_ptr();
+    w.ln2 = params[p + 8].data_ptr();
+    w.ld_qkv = w.ld_gu = n.H;
+    w.ld_o = n.O();
+    w.ld_d = n.I;
+    w.cosp = tables[2 * i].data_ptr<float>();
+    w.sinp = tables[2 * i + 1].data_ptr<float>();
+  }
+  return out;
+}
+LayerDims stack_dims(const Tensor& x, const std::vector<Tensor>& params, int64_t B, int64_t S, int64_t hq, int64_t hkv, int64_t d) {
+  return LayerDims{B, S, x.size(1), params.size() < LAYER_PARAMS || params[6].dim() != 2 ? 0 : params[6].size(1), hq, hkv, d};
+}
+
+// x [T, H] through all layers: {x_out, then per layer its saved bf16, saved fp32 and output} (LayerSaved; the output of the last one is
+// x_out), or with save = false {x_out} alone, the activations of all layers in one place. {} (nothing launched) where an operand is not as
+// stack_pointers wants it.
+std::vector<Tensor> decoder_stack_fwd(const Tensor& x, const std::vector<Tensor>& params, const std::vector<Tensor>& tables, double eps, int64_t B,
+                                      int64_t S, int64_t hq, int64_t hkv, int64_t d, double scale, bool save) {
+  if (!all_bf16_cuda({&x}) || x.dim() != 2 || !x.is_contiguous() || x.size(0) != B * S || x.size(0) == 0 || hq % hkv) return {};
+  const LayerDims n = stack_dims(x, params, B, S, hq, hkv, d);
+  const auto w = stack_pointers(n, x, params, tables);
+  if (w.empty()) return {};
+  const LayerSaved at(n);
+  c10::cuda::CUDAGuard guard(x.device());
+  const auto on = x.options();
+  std::vector<Tensor> r(1);
+  Tensor in = x, s16, s32, free;
+  for (size_t i = 0; i < w.size(); ++i) {
+    if (save || i == 0) {
+      s16 = torch::empty({at.total}, on);
+      s32 = torch::empty({at.total32}, on.dtype(at::kFloat));
+    }
+    // (without saving, two outputs are used in turn; the caller's x is not one of them)
+    Tensor out = !save && i >= 2 ? free : torch::empty({n.T(), n.H}, on);
+    layer_fwd(n, in.data_ptr(), w[i], eps, scale, bf16_ptr(s16), s32.data_ptr<float>(), out.data_ptr(), on);
+    if (save) {
+      r.push_back(s16);
+      r.push_back(s32);
+      r.push_back(out);
+    }
+    free = in;
+    in = out;
+  }
+  r[0] = in;
+  return r;
 }
 
 // The same with the activations as tensors of their own (views): {x_out, h1, rstd1, qkv, o, lse, x_mid, rstd2, h2, gu, a}, or {}.
@@ -749,6 +851,81 @@ struct LayerActivations {
   const float *rstd1, *rstd2, *lse;
 };
 
+// Where a layer's weight gradients are added (fp32).
+struct LayerGrads {
+  float *qkv, *o, *gu, *d;
+  const Tensor *ln1, *ln2;
+};
+// The regions of the nine parameters from mg[first] on; false unless they are as the launches take them.
+bool layer_grads(const LayerDims& n, const std::vector<Tensor>& mg, size_t first, LayerGrads& g) {
+  g.qkv = packed_region(mg, (int)first, 3, n.Q(), n.H);
+  g.o = packed_region(mg, (int)first + 3, 1, n.H, n.O());
+  g.gu = packed_region(mg, (int)first + 4, 2, 2 * n.I, n.H);
+  g.d = packed_region(mg, (int)first + 6, 1, n.H, n.I);
+  if (g.qkv == nullptr || g.o == nullptr || g.gu == nullptr || g.d == nullptr) return false;
+  for (size_t i = first + 7; i < first + 9; ++i)
+    if (!mg[i].is_cuda() || mg[i].scalar_type() != at::kFloat || !mg[i].is_contiguous() || mg[i].numel() != n.H) return false;
+  g.ln1 = &mg[first + 7];
+  g.ln2 = &mg[first + 8];
+  return true;
+}
+
+// Scratch of a layer's backward (bytes): dgu, whose place the attention's gradients take when it is done with; the normed inputs' gradients
+// (dh); dx_mid.
+struct LayerScratch {
+  int64_t dqkv, dq, delta, dh, dx_mid, total;
+  explicit LayerScratch(const LayerDims& n) {
+    auto up = [](int64_t bytes) { return (bytes + 255) / 256 * 256; };
+    const int64_t T = n.T(), b_h = up(2 * T * n.H);
+    dqkv = up(2 * T * n.O());
+    dq = dqkv + up(2 * T * n.Q());
+    delta = dq + up(4 * T * n.O());
+    dh = std::max(up(4 * T * n.I), delta + up(4 * T * n.hq));
+    dx_mid = dh + b_h;
+    total = dx_mid + b_h;
+  }
+};
+
+// The launches of a layer's backward. x: the forward's input; ln1, ln2: the norms' weights; s: LayerScratch bytes.
+void layer_bwd_launches(const LayerDims& n, const void* dout, const void* x, const LayerActivations& acts, const LayerPointers& w, const Tensor& ln1,
+                        const Tensor& ln2, const LayerGrads& g, char* const s, void* dx, double scale, const at::TensorOptions& on) {
+  const LayerScratch at(n);
+  const int64_t T = n.T(), H = n.H, I = n.I, O = n.O(), Q = n.Q(), B = n.B, S = n.S, hq = n.hq, hkv = n.hkv, d = n.d;
+  const bf16_t *const h1 = acts.h1, *const qkv = acts.qkv, *const o = acts.o, *const x_mid = acts.x_mid, *const h2 = acts.h2,
+               *const gu = acts.gu, *const a = acts.a;
+  void *const dgu = s, *const dO = s, *const dq_ws = s + at.dq, *const delta = s + at.delta;
+  bf16_t* const dqkv = reinterpret_cast<bf16_t*>(s + at.dqkv);
+  void *const dh = s + at.dh, *const dx_mid = s + at.dx_mid;
+  const cudaStream_t st = stream();
+
+  if (!(pt_gemm_get_pair() && I % 64 == 0 &&
+        fused_gemm(pt_gemm_bf16_fused(dout, w.wd, dgu, (int)T, (int)I, (int)H, H, w.ld_d, 2 * I, 5, const_cast<bf16_t*>(gu), 2 * I,
+                                      (int)I, nullptr, nullptr, 0, 0, 0, pt_status_word(), st), "gemm_dgrad_swiglu_bwd"))) {
+    Tensor da = torch::empty({T, I}, on);
+    gemm_into(dout, w.wd, da.data_ptr(), T, I, H, H, w.ld_d, I, false, true, 0, on);
+    PT_CHECK_RC(pt_swiglu_bwd(gu, da.data_ptr(), dgu, T, (int)I, st), "swiglu_bwd");
+  }
+  gemm_into(dout, a, g.d, H, I, T, H, I, I, true, true, 1, on);
+  gemm_into(dgu, w.w_gu, dh, T, H, 2 * I, 2 * I, w.ld_gu, H, false, true, 0, on);
+  gemm_into(dgu, h2, g.gu, 2 * I, H, T, 2 * I, H, H, true, true, 1, on);
+  rmsnorm_bwd_into(dh, x_mid, ln2, acts.rstd2, dout, dx_mid, *g.ln2, T, H, on);
+  gemm_into(dx_mid, w.wo, dO, T, O, H, H, w.ld_o, O, false, true, 0, on);             // dL/d(attention output)
+  gemm_into(dx_mid, o, g.o, H, O, T, H, O, O, true, true, 1, on);
+  PT_CHECK_BWD_RC(pt_attention_bwd_rope(dO, qkv, qkv + O, qkv + O + hkv * d, o, acts.lse, nullptr, reinterpret_cast<float*>(delta),
+                                        reinterpret_cast<float*>(dq_ws), dqkv, dqkv + O, dqkv + O + hkv * d, (int)B, (int)S, (int)S, (int)hq,
+                                        (int)hkv, (int)d, Q, Q, Q, Q, Q, Q, 1, (float)scale, w.cosp, w.sinp, (int)S, st), "attention_bwd");
+  gemm_into(dqkv, w.w_qkv, dh, T, H, Q, Q, w.ld_qkv, H, false, true, 0, on);
+  gemm_into(dqkv, h1, g.qkv, Q, H, T, Q, H, H, true, true, 1, on);
+  rmsnorm_bwd_into(dh, x, ln1, acts.rstd1, dx_mid, dx, *g.ln1, T, H, on);
+}
+
+LayerActivations saved_activations(const LayerDims& n, const Tensor& s16, const Tensor& s32) {
+  const LayerSaved at(n);
+  const bf16_t* const b = bf16_ptr(s16);
+  const float* const f = s32.data_ptr<float>();
+  return LayerActivations{b + at.h1, b + at.qkv, b + at.o, b + at.x_mid, b + at.h2, b + at.gu, b + at.a, f + at.rstd1, f + at.rstd2, f + at.lse};
+}
+
 // Backward of a layer; the weight gradients are added to the fp32 regions `mg` (q, k, v, out, gate, up, down, norm 1, norm 2). x: the
 // forward's input; `saved_by(dims)` gives its activations once the dimensions are known. Returns dx, or an undefined tensor (nothing
 // launched).
@@ -761,53 +938,48 @@ Tensor layer_bwd(const Tensor& dout, const Tensor& x, SavedBy saved_by, const Te
   TORCH_CHECK(x.dim() == 2 && x.is_contiguous() && x.size(0) == B * S && dout.is_contiguous() && dout.sizes() == x.sizes() &&
               w_gu.dim() == 2 && hq % hkv == 0);
   const LayerDims n{B, S, x.size(1), w_gu.size(0) / 2, hq, hkv, d};
-  const int64_t T = n.T(), H = n.H, I = n.I, O = n.O(), Q = n.Q();
-  float *const mg_qkv = packed_region(mg, 0, 3, Q, H), *const mg_o = packed_region(mg, 3, 1, H, O),
-        *const mg_gu = packed_region(mg, 4, 2, 2 * I, H), *const mg_d = packed_region(mg, 6, 1, H, I);
-  if (mg_qkv == nullptr || mg_o == nullptr || mg_gu == nullptr || mg_d == nullptr) return Tensor();
-  for (int i = 7; i < 9; ++i)
-    if (!mg[i].is_cuda() || mg[i].scalar_type() != at::kFloat || !mg[i].is_contiguous() || mg[i].numel() != H) return Tensor();
+  LayerGrads g;
+  if (!layer_grads(n, mg, 0, g)) return Tensor();
   check_layer(n, ln1, w_qkv, cosT, sinT, wo, ln2, w_gu, wd);
   const LayerActivations acts = saved_by(n);
   c10::cuda::CUDAGuard guard(x.device());
   const auto on = x.options();
-  const bf16_t *const h1 = acts.h1, *const qkv = acts.qkv, *const o = acts.o, *const x_mid = acts.x_mid, *const h2 = acts.h2,
-               *const gu = acts.gu, *const a = acts.a;
-  // One scratch allocation (bytes): dgu, whose place the attention's gradients take when it is done with; the normed inputs' gradients
-  // (dh); dx_mid.
-  auto up = [](int64_t bytes) { return (bytes + 255) / 256 * 256; };
-  const int64_t b_dgu = up(4 * T * I), b_do = up(2 * T * O), b_dqkv = up(2 * T * Q), b_dq = up(4 * T * O), b_delta = up(4 * T * hq), b_h = up(2 * T * H);
-  const int64_t b_first = std::max(b_dgu, b_do + b_dqkv + b_dq + b_delta);
-  Tensor scratch = torch::empty({b_first + 2 * b_h}, on.dtype(at::kByte)), dx = torch::empty({T, H}, on);
-  char* const s = reinterpret_cast<char*>(scratch.data_ptr());
-  void *const dgu = s, *const dO = s, *const dq_ws = s + b_do + b_dqkv, *const delta = s + b_do + b_dqkv + b_dq;
-  bf16_t* const dqkv = reinterpret_cast<bf16_t*>(s + b_do);
-  void *const dh = s + b_first, *const dx_mid = s + b_first + b_h;
-  const long long ld_qkv = row_stride_2d(w_qkv, "w_qkv"), ld_o = row_stride_2d(wo, "wo"), ld_gu = row_stride_2d(w_gu, "w_gu"),
-                  ld_d = row_stride_2d(wd, "wd");
-  const cudaStream_t st = stream();
-
-  if (!(pt_gemm_get_pair() && I % 64 == 0 &&
-        fused_gemm(pt_gemm_bf16_fused(dout.data_ptr(), wd.data_ptr(), dgu, (int)T, (int)I, (int)H, H, ld_d, 2 * I, 5, const_cast<bf16_t*>(gu), 2 * I,
-                                      (int)I, nullptr, nullptr, 0, 0, 0, pt_status_word(), st), "gemm_dgrad_swiglu_bwd"))) {
-    Tensor da = torch::empty({T, I}, on);
-    gemm_into(dout.data_ptr(), wd.data_ptr(), da.data_ptr(), T, I, H, H, ld_d, I, false, true, 0, on);
-    PT_CHECK_RC(pt_swiglu_bwd(gu, da.data_ptr(), dgu, T, (int)I, st), "swiglu_bwd");
-  }
-  gemm_into(dout.data_ptr(), a, mg_d, H, I, T, H, I, I, true, true, 1, on);
-  gemm_into(dgu, w_gu.data_ptr(), dh, T, H, 2 * I, 2 * I, ld_gu, H, false, true, 0, on);
-  gemm_into(dgu, h2, mg_gu, 2 * I, H, T, 2 * I, H, H, true, true, 1, on);
-  rmsnorm_bwd_into(dh, x_mid, ln2, acts.rstd2, dout.data_ptr(), dx_mid, mg[8], T, H, on);
-  gemm_into(dx_mid, wo.data_ptr(), dO, T, O, H, H, ld_o, O, false, true, 0, on);             // dL/d(attention output)
-  gemm_into(dx_mid, o, mg_o, H, O, T, H, O, O, true, true, 1, on);
-  PT_CHECK_BWD_RC(pt_attention_bwd_rope(dO, qkv, qkv + O, qkv + O + hkv * d, o, acts.lse, nullptr, reinterpret_cast<float*>(delta),
-                                        reinterpret_cast<float*>(dq_ws), dqkv, dqkv + O, dqkv + O + hkv * d, (int)B, (int)S, (int)S, (int)hq,
-                                        (int)hkv, (int)d, Q, Q, Q, Q, Q, Q, 1, (float)scale, cosT.data_ptr<float>(), sinT.data_ptr<float>(),
-                                        (int)S, st), "attention_bwd");
-  gemm_into(dqkv, w_qkv.data_ptr(), dh, T, H, Q, Q, ld_qkv, H, false, true, 0, on);
-  gemm_into(dqkv, h1, mg_qkv, Q, H, T, Q, H, H, true, true, 1, on);
-  rmsnorm_bwd_into(dh, x.data_ptr(), ln1, acts.rstd1, dx_mid, dx.data_ptr(), mg[7], T, H, on);
+  Tensor scratch = torch::empty({LayerScratch(n).total}, on.dtype(at::kByte)), dx = torch::empty({n.T(), n.H}, on);
+  layer_bwd_launches(n, dout.data_ptr(), x.data_ptr(), acts, layer_pointers(ln1, w_qkv, cosT, sinT, wo, ln2, w_gu, wd), ln1, ln2, g,
+                     reinterpret_cast<char*>(scratch.data_ptr()), dx.data_ptr(), scale, on);
   return dx;
+}
+
+// Backward of decoder_stack_fwd (with save): xs, s16, s32 are the layers' inputs and saved activations, mg the fp32 regions of `params`.
+// Returns dx, or an undefined tensor (nothing launched).
+Tensor decoder_stack_bwd(const Tensor& dout, const std::vector<Tensor>& xs, const std::vector<Tensor>& s16, const std::vector<Tensor>& s32,
+                         const std::vector<Tensor>& params, const std::vector<Tensor>& tables, const std::vector<Tensor>& mg, int64_t B, int64_t S,
+                         int64_t hq, int64_t hkv, int64_t d, double scale) {
+  const size_t layers = xs.size();
+  if (layers == 0 || !all_bf16_cuda({&dout}) || dout.dim() != 2 || !dout.is_contiguous() || dout.size(0) != B * S || dout.size(0) == 0 || hq % hkv ||
+      s16.size() != layers || s32.size() != layers || mg.size() != params.size())
+    return Tensor();
+  const LayerDims n = stack_dims(dout, params, B, S, hq, hkv, d);
+  const auto w = stack_pointers(n, dout, params, tables);
+  if (w.size() != layers) return Tensor();
+  const LayerSaved at(n);
+  std::vector<LayerGrads> g(layers);
+  for (size_t i = 0; i < layers; ++i) {
+    if (!layer_grads(n, mg, i * LAYER_PARAMS, g[i])) return Tensor();
+    for (const Tensor* t : {&xs[i], &s16[i], &s32[i]})
+      if (t->device() != dout.device() || !t->is_contiguous() || t->scalar_type() != (t == &s32[i] ? at::kFloat : at::kBFloat16)) return Tensor();
+    if (xs[i].sizes() != dout.sizes() || s16[i].numel() != at.total || s32[i].numel() != at.total32) return Tensor();
+  }
+  c10::cuda::CUDAGuard guard(dout.device());
+  const auto on = dout.options();
+  Tensor scratch = torch::empty({LayerScratch(n).total}, on.dtype(at::kByte)), grad = dout;
+  for (size_t i = layers; i-- > 0;) {
+    Tensor dx = torch::empty({n.T(), n.H}, on);
+    layer_bwd_launches(n, grad.data_ptr(), xs[i].data_ptr(), saved_activations(n, s16[i], s32[i]), w[i], params[i * LAYER_PARAMS + 7],
+                       params[i * LAYER_PARAMS + 8], g[i], reinterpret_cast<char*>(scratch.data_ptr()), dx.data_ptr(), scale, on);
+    grad = dx;
+  }
+  return grad;
 }
 
 // `s16`, `s32`: what decoder_layer_fwd_packed saved.
@@ -821,9 +993,7 @@ Tensor decoder_layer_bwd_packed(const Tensor& dout, const Tensor& x, const Tenso
     PT_CHECK_F32(s32);
     TORCH_CHECK(s16.is_contiguous() && s16.numel() == at.total && s32.is_contiguous() && s32.numel() == at.total32,
                 "decoder layer: saved activations of another shape");
-    const bf16_t* const b = bf16_ptr(s16);
-    const float* const f = s32.data_ptr<float>();
-    return LayerActivations{b + at.h1, b + at.qkv, b + at.o, b + at.x_mid, b + at.h2, b + at.gu, b + at.a, f + at.rstd1, f + at.rstd2, f + at.lse};
+    return saved_activations(n, s16, s32);
   };
   return layer_bwd(dout, x, saved_by, ln1, w_qkv, cosT, sinT, wo, ln2, w_gu, wd, mg, B, S, hq, hkv, d, scale);
 }
@@ -1026,6 +1196,13 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("decoder_layer_fwd_packed", &decoder_layer_fwd_packed, "decoder_layer_fwd with the saved activations in two allocations.");
   m.def("decoder_layer_saved", &decoder_layer_saved, "The saved activations of decoder_layer_fwd_packed as tensors (views).");
   m.def("decoder_layer_bwd_packed", &decoder_layer_bwd_packed);
+  m.def("decoder_stack_fwd", &decoder_stack_fwd, "All layers' forward in one call; [] where an operand is not as it has to be.");
+  m.def("decoder_stack_bwd", [](const Tensor& dout, const std::vector<Tensor>& xs, const std::vector<Tensor>& s16, const std::vector<Tensor>& s32,
+                                const std::vector<Tensor>& params, const std::vector<Tensor>& tables, const std::vector<Tensor>& mg, int64_t B,
+                                int64_t S, int64_t hq, int64_t hkv, int64_t d, double scale) -> c10::optional<Tensor> {
+    Tensor dx = decoder_stack_bwd(dout, xs, s16, s32, params, tables, mg, B, S, hq, hkv, d, scale);
+    return dx.defined() ? c10::optional<Tensor>(dx) : c10::nullopt;
+  }, "All layers' backward in one call; None where an operand is not as it has to be.");
   m.def("scale_", &scale_);
   m.def("merge_attention_", &merge_attention_);
   m.def("attention_fwd", &attention_fwd);

@@ -31,7 +31,7 @@ import torch.nn as nn
 from .. import ops
 from .. import process_group_manager as pgm
 from ..parallel import tp_communications as tpc
-from ..utils.tracing import nvtx_range
+from ..utils.tracing import nvtx_enabled, nvtx_range
 
 
 # ----------------------------------------------------------------------------------------------
@@ -503,6 +503,133 @@ class DecoderLayerFn(torch.autograd.Function):
         return dx.view(B, S_in, H), g_ln1, g_ln2, g_wq, g_wk, g_wv, g_wo[0], g_wg, g_wu, g_wd[0], None
 
 
+class _NotCovered(Exception):
+    """The native call takes these operands layer by layer only (nothing was launched)."""
+
+
+class DecoderStackFn(torch.autograd.Function):
+    """All decoder layers as one node with one native call each way, for one GPU without tensor, sequence or context parallelism.
+
+    A node per layer costs the host 25 us forward and 85 us backward beside the layer's launches, which small models and short prompts do
+    not hide. What is saved is what the layers' own nodes save.
+    """
+
+    @staticmethod
+    def forward(ctx, x, layers, dims, tables, *params):
+        B, S, H = x.shape
+        hq, hkv, d, eps, sm_scale = dims
+        x2 = x.reshape(B * S, H)
+        r = ops.decoder_stack_fwd(x2, list(params), tables, eps, B, S, hq, hkv, d, sm_scale, True)
+        if not r:
+            raise _NotCovered
+        ctx.save_for_backward(x2, *r[1:-1])          # input, then (saved bf16, saved fp32, next layer's input) per layer
+        ctx.layers, ctx.dims, ctx.tables = layers, dims, tables
+        return r[0].view(B, S, H)
+
+    @staticmethod
+    def backward(ctx, dout):
+        layers, (hq, hkv, d, _, sm_scale) = ctx.layers, ctx.dims
+        saved = ctx.saved_tensors
+        xs, s16, s32 = saved[0::3], saved[1::3], saved[2::3]
+        B, S, H = dout.shape
+        none = (None,) * (4 + 9 * len(layers))
+        if ops.runs_layer_natively(dout) and not nvtx_enabled() and pgm.get().cp_dp_world_size == 1:
+            stack = [layer_parameters(layer) for layer in layers]
+            if all(ps is not None for ps in stack) and not any(layer.tp_group is not None or layer._modules["attention"].cp_enabled for layer in layers):
+                params = [p for ps in stack for p in ps]
+                grads = [getattr(p, "main_grad", None) for p in params]
+                if all(g is not None for g in grads):
+                    dx = ops.decoder_stack_bwd(dout.reshape(B * S, H).contiguous(), xs, s16, s32, params, ctx.tables, grads, B, S, hq, hkv, d,
+                                               sm_scale)
+                    if dx is not None:
+                        for ps in reversed(stack):
+                            for p in ps:
+                                notify_grad_ready(p)
+                        return (dx.view(B, S, H),) + none[1:]
+        # the layers' own backward, one after the other
+        out = list(none)
+        for i in range(len(layers) - 1, -1, -1):
+            r = DecoderLayerFn.backward(_SavedLayer(layers[i], (B, S, H, S), (xs[i], s16[i], s32[i])), dout)
+            dout, g_ln1, g_ln2, *g = r[:10]
+            out[4 + 9 * i: 13 + 9 * i] = [*g, g_ln1, g_ln2]
+        out[0] = dout
+        return tuple(out)
+
+
+class _SavedLayer:
+    """What :class:`DecoderLayerFn`'s backward reads of its context, for a layer that ran in a stack."""
+
+    def __init__(self, layer, dims, saved):
+        self.layer, self.dims, self.saved_tensors = layer, dims, saved
+        self.sp_group, self.native = None, True
+
+
+def layer_parameters(layer):
+    """``(q, k, v, out, gate, up, down, norm 1, norm 2)`` weights of a decoder layer, or None where one is not a plain parameter of its
+    module (looking them up through ``nn.Module`` costs five times as much)."""
+    try:
+        m = layer._modules
+        a, f = m["attention"]._modules, m["mlp"]._modules
+        ps = (a["q_proj"]._parameters["weight"], a["k_proj"]._parameters["weight"], a["v_proj"]._parameters["weight"],
+              a["out_proj"]._parameters["weight"], f["gate_proj"]._parameters["weight"], f["up_proj"]._parameters["weight"],
+              f["down_proj"]._parameters["weight"], m["input_layernorm"]._parameters["weight"],
+              m["post_attention_layernorm"]._parameters["weight"])
+    except KeyError:
+        return None
+    return None if any(p is None for p in ps) else ps
+
+
+_GLOBAL_HOOKS = [getattr(nn.modules.module, name) for name in ("_global_forward_hooks", "_global_forward_pre_hooks", "_global_backward_hooks",
+                                                               "_global_backward_pre_hooks")]
+
+
+def run_layers(layers, x: torch.Tensor) -> torch.Tensor:
+    """``x`` through the decoder layers: in one native call where they are plain layers of one shape on one GPU that nobody observes
+    (hooks, NVTX ranges, tracing, checked mode), else layer by layer."""
+    y = _run_stack(layers, x)
+    if y is None:
+        for layer in layers:
+            x = layer(x)
+        return x
+    return y
+
+
+def _run_stack(layers, x):
+    if not ops.runs_layer_natively(x) or nvtx_enabled() or x.dim() != 3 or x.numel() == 0 or len(layers) == 0 or any(_GLOBAL_HOOKS):
+        return None
+    if torch.jit.is_tracing() or torch.compiler.is_compiling():
+        return None
+    g = pgm.get()
+    if g.tp_world_size > 1 or g.cp_dp_world_size > 1 or tpc.sequence_parallel_group() is not None:
+        return None
+    first = layers[0]
+    tables, params, dims = [], [], None
+    for layer in layers:
+        if type(layer) is not DecoderLayer or "forward" in layer.__dict__ or layer._forward_hooks or layer._forward_pre_hooks or \
+                layer._backward_hooks or layer._backward_pre_hooks:
+            return None
+        ps = layer_parameters(layer)
+        att = layer._modules["attention"]
+        here = (att.num_local_heads, att.num_local_kv_heads, att.head_dim, layer.eps, layer.sm_scale)
+        if ps is None or att.cp_enabled or here != (dims or here):
+            return None
+        dims = here
+        params += ps
+        tables += layer.rope(x.device, first)
+    if torch.is_grad_enabled() and (x.requires_grad or any(p.requires_grad for p in params)):
+        # (without gradient buckets the layers' own nodes give back their activations as the backward pass goes)
+        if any(getattr(p, "main_grad", None) is None for p in params):
+            return None
+        try:
+            return DecoderStackFn.apply(x, tuple(layers), dims, tables, *params)
+        except _NotCovered:
+            return None
+    B, S, H = x.shape
+    hq, hkv, d, eps, sm_scale = dims
+    r = ops.decoder_stack_fwd(x.reshape(B * S, H), params, tables, eps, B, S, hq, hkv, d, sm_scale, False)
+    return r[0].view(B, S, H) if r else None
+
+
 class DecoderLayer(nn.Module):
     """Pre-norm residual block (``model.py:214-235``) executed as :class:`DecoderLayerFn`."""
 
@@ -531,9 +658,14 @@ class DecoderLayer(nn.Module):
         return g.tp_group if g.tp_world_size > 1 else None
 
     # --- rope tables: fp32, built once per device, sliced for this CP rank ----------------
-    def rope(self, device):
+    def rope(self, device, like=None):
+        """``(cos, sin)``; those of the layer ``like`` where it has the same positions and frequencies (a table takes 0.2 ms to make)."""
         key = str(device)
         if key not in self._rope_cache:
+            if like is not None and like is not self and (self.max_position_embeddings, self.head_dim, self.rope_theta, self.rope_scaling) == \
+                    (like.max_position_embeddings, like.head_dim, like.rope_theta, like.rope_scaling):
+                self._rope_cache[key] = like.rope(device)
+                return self._rope_cache[key]
             cos, sin = ops.rope_tables(self.max_position_embeddings, self.head_dim, self.rope_theta,
                                        scaling=self.rope_scaling)
             from ..parallel.context_parallel import update_rope_for_context_parallel
@@ -711,9 +843,7 @@ class Llama(nn.Module):
 
     def forward(self, input_ids, attention_mask=None, position_ids=None, target_ids=None, loss_scale: float = 1.0):
         """Logits ``[B,S,V]`` (reference signature, ``model.py:291-298``), or the fused loss when ``target_ids`` is given."""
-        x = self.embedding(input_ids)
-        for layer in self.decoder_layers:
-            x = layer(x)
+        x = run_layers(self.decoder_layers, self.embedding(input_ids))
         x = gather_tokens_for_head(self.final_norm(x))
         if target_ids is None:
             return self.final_proj(x)

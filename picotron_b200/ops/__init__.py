@@ -218,6 +218,17 @@ def decoder_layer_bwd_packed(*args):
     return _c().decoder_layer_bwd_packed(*args)
 
 
+def decoder_stack_fwd(*args):
+    """:func:`decoder_layer_fwd_packed` for all layers of a model in one call: ``[x_out]`` and, with ``save``, per layer its saved bf16,
+    saved fp32 and output; ``[]`` (nothing launched) where an operand is not as the launches take it."""
+    return _c().decoder_stack_fwd(*args)
+
+
+def decoder_stack_bwd(*args):
+    """The backward of :func:`decoder_stack_fwd`: dx, or None (nothing launched)."""
+    return _c().decoder_stack_bwd(*args)
+
+
 # ------------------------------------------------------------------ embedding
 def embedding_fwd(ids, w, vocab_start: int = 0):
     if w.is_cuda:

@@ -131,3 +131,75 @@ def test_checked_mode_sees_a_loss_that_is_not_finite_without_a_gradient():
             ops.linear_ce_loss(x, w, targets, 0, 1.0, terms, False)
     finally:
         ops.enable_checked_mode(False)
+
+
+@pytest.mark.parametrize("layers,hq,hkv,d,inter,B,S", [(1, 2, 1, 64, 192, 1, 1), (3, 3, 1, 64, 320, 2, 97), (2, 2, 2, 128, 200, 1, 130)])
+def test_layers_in_one_native_call_equal_the_layers_one_by_one(layers, hq, hkv, d, inter, B, S):
+    """The same launches: outputs, losses and logits equal to the bit, gradients up to the order of atomic additions; a hook on a layer is still
+    called (and its layers run one by one); weights that do not lie side by side, saved-tensor hooks are no matter;
+    another layer's norm weight swapped for the call is used."""
+    from picotron_b200.models import llama as M
+    torch.manual_seed(2)
+    cfg = ModelConfig(hidden_size=hq * d, intermediate_size=inter, num_hidden_layers=layers, num_attention_heads=hq,
+                      num_key_value_heads=hkv, vocab_size=256, max_position_embeddings=S + 3)
+    model = Llama(cfg, init="normal").to(torch.bfloat16).cuda()
+    w = model.decoder_layers[-1].mlp.up_proj.weight
+    w.data = w.data.clone()                                     # no longer behind its gate projection
+    ids = torch.randint(0, cfg.vocab_size, (B, S), device="cuda")
+    stacks = []
+    one_call = M._run_stack
+
+    def watched(*a):
+        y = one_call(*a)
+        stacks.append(y is not None)
+        return y
+
+    def passes(**swap):
+        call = lambda **kw: torch.func.functional_call(model, swap, (ids,), kw) if swap else model(ids, **kw)   # noqa: E731
+        out = []
+        with torch.no_grad():
+            out += [call(), call(target_ids=ids)]
+        with torch.inference_mode():
+            out.append(call())
+        return out
+
+    M._run_stack = watched
+    try:
+        passes()                                                # (the layers put their packed weights together)
+        stacks.clear()
+        together, swapped = passes(), passes(**{"final_norm.weight": model.final_norm.weight * 2,
+                                                "decoder_layers.0.input_layernorm.weight": model.decoder_layers[0].input_layernorm.weight * 2})
+        assert stacks == [True] * 6
+        model.embedding.weight.requires_grad_(layers != 2)      # once with an input that needs no gradient
+        wrapped = DataParallelBucket(model)
+
+        def grads(hooked):
+            wrapped.reset()
+            stacks.clear()
+            calls = []
+            handle = model.decoder_layers[0].register_forward_hook(lambda *a: calls.append(1)) if hooked else None
+            with torch.autograd.graph.save_on_cpu():
+                loss = wrapped(ids, target_ids=ids)
+            loss.backward()
+            if hooked:
+                handle.remove()
+            assert stacks == [not hooked] and len(calls) == hooked
+            return [loss.detach().clone()] + [p.main_grad.clone() for p in model.parameters() if p.requires_grad]
+
+        many, each = grads(False), grads(True)
+        handles = [layer.register_forward_pre_hook(lambda *a: None) for layer in model.decoder_layers]
+        stacks.clear()
+        single, single_swapped = passes(), passes(**{"final_norm.weight": model.final_norm.weight * 2,
+                                                     "decoder_layers.0.input_layernorm.weight": model.decoder_layers[0].input_layernorm.weight * 2})
+        assert stacks == [False] * 6
+        for h in handles:
+            h.remove()
+    finally:
+        M._run_stack = one_call
+    for x, y in zip(together + swapped, single + single_swapped):
+        assert torch.equal(x, y)
+    assert not torch.equal(together[0], swapped[0])
+    assert torch.equal(many[0], each[0])
+    for x, y in zip(many[1:], each[1:]):
+        # (dQ of more than two key blocks and the norm and embedding gradients add in any order: fp32 sums, rounded to bf16 once)
+        assert float((x - y).norm()) <= 4e-3 * float(y.norm()) + 1e-12
