@@ -516,6 +516,7 @@ struct BwdParams {
   const float* cosT;
   const float* sinT;
   int rope_seq;
+  int tma_out;                   // dk and dv are stored through their tensor maps (bf16, one segment)
   unsigned long long* prof;      // optional phase counters, as AttnParams::prof
 };
 
@@ -537,6 +538,27 @@ struct BwdWarps {
   static_assert(PARTS * REGS_COMPUTE + REGS_DRAIN + REGS_REST <= (PARTS + 2) * REGS, "setmaxnreg must not ask for more than the launch gave");
   static_assert(THREADS * REGS <= 65536, "register file");
 };
+// What a CTA works on: a key block of a key/value head, with the query heads of its group and the query blocks that see it.
+struct BwdWork {
+  int seg, k0, kv_head, b, qb_first, steps_per_head, steps;
+  bool diag;
+};
+__device__ __forceinline__ BwdWork bwd_work(const BwdParams& p, int BM, int BN, unsigned cta) {
+  const unsigned bps = (unsigned)(p.Sk + BN - 1) / BN;    // key blocks per segment
+  const unsigned num_kb = bps * p.n_segs, heads = (unsigned)(p.hkv * p.B);
+  // causal: the first (heaviest) key blocks of all heads first, full attention: head by head (see the forward)
+  const unsigned kbg = p.causal ? cta / heads : cta % num_kb, bh = p.causal ? cta % heads : cta / num_kb;
+  BwdWork w;
+  w.seg = (int)(kbg / bps);
+  w.k0 = (int)(kbg - w.seg * bps) * BN;
+  w.diag = p.causal && w.seg == p.n_segs - 1;             // the causal diagonal runs through the last segment only
+  w.kv_head = (int)(bh % (unsigned)p.hkv);
+  w.b = (int)(bh / (unsigned)p.hkv);
+  w.qb_first = w.diag ? w.k0 / BM : 0;                    // first query block that sees key k0
+  w.steps_per_head = (p.Sq + BM - 1) / BM - w.qb_first;
+  w.steps = w.steps_per_head > 0 ? w.steps_per_head * (p.hq / p.hkv) : 0;
+  return w;
+}
 template <int D> constexpr int bwd_parts() { return D == 64 ? 4 : 2; }
 template <int N> __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
@@ -550,6 +572,7 @@ template <int N> __device__ __forceinline__ void regs_dec() { asm volatile("setm
 // Measured (us; 1 x 32768, 32 / 8 heads, d = 64; 1 x 8192, 32 / 8 heads, d = 128): 21,500 -> 16,200 and 2,160 -> 1,410.
 template <int D, bool OUT_F32, bool PROF, int PARTS>
 __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tm_q, const KVSegs& segs, const CUtensorMap& tm_do, const CUtensorMap& tm_dq,
+                                              const CUtensorMap& tm_dk, const CUtensorMap& tm_dv,
                                               const float* __restrict__ LSE, const float* __restrict__ DELTA, void* __restrict__ dK_,
                                               void* __restrict__ dV_, const BwdParams& p, KernelStatus* status) {
   using Cfg = BwdCfg<D>;
@@ -569,25 +592,28 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tm_q, const KVS
   float* sStat = reinterpret_cast<float*>(sDQ + Cfg::DQ_BYTES);       // [stage][-lse * log2(e) | -delta * scale][128]
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-  const int bps = (p.Sk + Cfg::BN - 1) / Cfg::BN;         // key blocks per segment
-  const int num_kb = bps * p.n_segs;
-  // causal: the first (heaviest) key blocks of all heads first, full attention: head by head (see the forward)
-  const unsigned bh_count = (unsigned)(p.hkv * p.B);
-  const int kbg = (int)(p.causal ? blockIdx.x / bh_count : blockIdx.x % (unsigned)num_kb);
-  const unsigned bh = p.causal ? blockIdx.x % bh_count : blockIdx.x / (unsigned)num_kb;
-  const int seg = kbg / bps;
-  const int kb = kbg - seg * bps;
-  const bool diag = p.causal && seg == p.n_segs - 1;      // the causal diagonal runs through the last segment only
-  const int kv_head = (int)(bh % (unsigned)p.hkv);
-  const int b = (int)(bh / (unsigned)p.hkv);
   const int group = p.hq / p.hkv;
-  const int k0 = kb * Cfg::BN;
-  const int num_qb = (p.Sq + Cfg::BM - 1) / Cfg::BM;
-  const int qb_first = diag ? (k0 / Cfg::BM) : 0;              // first query block that sees key k0
-  const int steps_per_head = num_qb - qb_first;
-  const int total_steps = steps_per_head > 0 ? steps_per_head * group : 0;
+  const BwdWork work = bwd_work(p, Cfg::BM, Cfg::BN, blockIdx.x);
+  const int seg = work.seg, kv_head = work.kv_head, b = work.b, k0 = work.k0, qb_first = work.qb_first, steps_per_head = work.steps_per_head,
+            total_steps = work.steps;
+  const bool diag = work.diag;
+  const bool tm_out = !OUT_F32 && p.tma_out;
+  auto load_q = [&](int it, int head, int q0) {
+    const int qs = it % Cfg::QSTAGES;
+    mbar_expect_tx(&bars.q_full[qs], Cfg::TILE_BYTES);
+#pragma unroll
+    for (int c = 0; c < Cfg::DCH; ++c)
+      tma_load_4d(sQ + qs * Cfg::TILE_BYTES + c * (Cfg::BM * 128), &tm_q, &bars.q_full[qs], c * 64, head, q0, b);
+  };
+  auto load_do = [&](int it, int head, int q0) {
+    const int os = it % Cfg::OSTAGES;
+    mbar_expect_tx(&bars.do_full[os], Cfg::TILE_BYTES);
+#pragma unroll
+    for (int c = 0; c < Cfg::DCH; ++c)
+      tma_load_4d(sdO + os * Cfg::TILE_BYTES + c * (Cfg::BM * 128), &tm_do, &bars.do_full[os], c * 64, head, q0, b);
+  };
 
-  if (threadIdx.x == 0) {
+  if (warp == CW + 4 && elect_one()) {
     mbar_init(&bars.kv_full, 1);
     for (int s = 0; s < 3; ++s) {
       mbar_init(&bars.q_full[s], 1);
@@ -618,6 +644,22 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tm_q, const KVS
     tma_prefetch_desc(&segs.v[seg]);
     tma_prefetch_desc(&tm_do);
     tma_prefetch_desc(&tm_dq);
+      if (tm_out) {
+      tma_prefetch_desc(&tm_dk);
+      tma_prefetch_desc(&tm_dv);
+    }
+    // The first loads leave before the other warps are let go: they travel under the tensor-memory allocation and the first barrier.
+    pdl_wait();
+    if (total_steps > 0) {
+      mbar_expect_tx(&bars.kv_full, 2 * Cfg::TILE_BYTES);
+#pragma unroll
+      for (int c = 0; c < Cfg::DCH; ++c) {
+        tma_load_4d(sK + c * (Cfg::BN * 128), &segs.k[seg], &bars.kv_full, c * 64, kv_head, k0, b);
+        tma_load_4d(sV + c * (Cfg::BN * 128), &segs.v[seg], &bars.kv_full, c * 64, kv_head, k0, b);
+      }
+      load_q(0, kv_head * group, qb_first * Cfg::BM);
+      load_do(0, kv_head * group, qb_first * Cfg::BM);
+    }
   }
   if (warp == CW + 5) {
     tmem_alloc(&bars.tmem_base, Cfg::TMEM_COLS);
@@ -634,26 +676,12 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tm_q, const KVS
   if (warp == CW + 4) {
     // ------------------------------------------------------------------------------ TMA producer
     if (total_steps > 0 && elect_one()) {
-      mbar_expect_tx(&bars.kv_full, 2 * Cfg::TILE_BYTES);
-#pragma unroll
-      for (int c = 0; c < Cfg::DCH; ++c) {
-        tma_load_4d(sK + c * (Cfg::BN * 128), &segs.k[seg], &bars.kv_full, c * 64, kv_head, k0, b);
-        tma_load_4d(sV + c * (Cfg::BN * 128), &segs.v[seg], &bars.kv_full, c * 64, kv_head, k0, b);
-      }
-      for (int it = 0; it < total_steps; ++it) {
-        const int head = kv_head * group + it / steps_per_head;
-        const int q0 = (qb_first + it % steps_per_head) * Cfg::BM;
-        const int qs = it % Cfg::QSTAGES, os = it % Cfg::OSTAGES;
-        if (!mbar_wait(&bars.q_empty[qs], ((it / Cfg::QSTAGES) & 1) ^ 1, abort_flag)) { report_error(status, KID_BWD, 1); break; }
-        mbar_expect_tx(&bars.q_full[qs], Cfg::TILE_BYTES);
-#pragma unroll
-        for (int c = 0; c < Cfg::DCH; ++c)
-          tma_load_4d(sQ + qs * Cfg::TILE_BYTES + c * (Cfg::BM * 128), &tm_q, &bars.q_full[qs], c * 64, head, q0, b);
-        if (!mbar_wait(&bars.do_empty[os], ((it / Cfg::OSTAGES) & 1) ^ 1, abort_flag)) { report_error(status, KID_BWD, 11); break; }
-        mbar_expect_tx(&bars.do_full[os], Cfg::TILE_BYTES);
-#pragma unroll
-        for (int c = 0; c < Cfg::DCH; ++c)
-          tma_load_4d(sdO + os * Cfg::TILE_BYTES + c * (Cfg::BM * 128), &tm_do, &bars.do_full[os], c * 64, head, q0, b);
+      for (int it = 1; it < total_steps; ++it) {           // (the first step's and K, V: above)
+        const int head = kv_head * group + it / steps_per_head, q0 = (qb_first + it % steps_per_head) * Cfg::BM;
+        if (!mbar_wait(&bars.q_empty[it % Cfg::QSTAGES], ((it / Cfg::QSTAGES) & 1) ^ 1, abort_flag)) { report_error(status, KID_BWD, 1); break; }
+        load_q(it, head, q0);
+        if (!mbar_wait(&bars.do_empty[it % Cfg::OSTAGES], ((it / Cfg::OSTAGES) & 1) ^ 1, abort_flag)) { report_error(status, KID_BWD, 11); break; }
+        load_do(it, head, q0);
       }
     }
   } else if (warp == CW + 5) {
@@ -835,7 +863,6 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tm_q, const KVS
     constexpr int SUBS = PARTS / 2;
     const int t = threadIdx.x & 127;
     const int part = threadIdx.x >> 7;
-    const int which = part / SUBS, sub = part % SUBS;      // 0: dV, 1: dK
     // dS^T of this thread: W / 8 16-byte units of row t, the first at ds_off, the others an exclusive-or of their number away
     const uint32_t ds_off = ((unsigned)(part * W) >> 6) * (128 * 128) + sw128_offset(t, ((unsigned)(part * W) & 63u) >> 3);
     const int quarter = warp & 3;
@@ -947,7 +974,18 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tm_q, const KVS
       atomicAdd(&p.prof[5], (unsigned long long)(clock64() - pstart));
       atomicAdd(&p.prof[6], 1ull);
     }
+    {
     // dK, dV of this key block (thread t <-> key k0 + t); fp32 when they are partials of a multi-rank reduction
+    // (The block and thread are read anew: what is kept from before the loop over the steps takes registers there, and with the stores below
+    // its compute warps executed 8 % more instructions, 14.0 -> 14.6 ms at 32,768 tokens.)
+    unsigned cta, thread;
+    asm volatile("mov.u32 %0, %%ctaid.x;" : "=r"(cta));
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(thread));
+    const BwdWork work = bwd_work(p, Cfg::BM, Cfg::BN, cta);
+    const int kv_head = work.kv_head, b = work.b, k0 = work.k0, seg = work.seg, total_steps = work.steps;
+    const int lane = thread & 31, quarter = (thread >> 5) & 3, part = thread >> 7, which = part / SUBS, sub = part % SUBS, key = k0 + (int)(thread & 127);
+    const uint32_t t_lane = tmem_base + (uint32_t(quarter * 32) << 16);
+    const bool tm_out = !OUT_F32 && p.tma_out;
     const long long seg_off = (long long)seg * p.seg_stride;
     if (total_steps == 0) {
       if (key < p.Sk && sub == 0) {
@@ -963,78 +1001,90 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tm_q, const KVS
           }
         }
       }
-    } else if (ok && mbar_wait(&bars.acc_full, 0, abort_flag)) {
+    } else if (ok && (which == 0 ? mbar_wait(&bars.p_free, (total_steps - 1) & 1, abort_flag) : mbar_wait(&bars.acc_full, 0, abort_flag))) {
+      // dV is complete with its last MMA, half a step before dK. Rows of 16 columns (32 bytes) of each warp's 32 keys go to TMA through the
+      // place of V, which the last dP was the last to read, and of K: stored by every thread for itself they were 16-byte pieces of 32 rows an
+      // instruction, and the end of a CTA took 3,600 (d = 64) and 7,600 cycles (d = 128) of the 20,900 and 34,000 that one of 4 x 1024,
+      // 32 heads lives.
       tcgen05_fence_after();
+      const long long rs_ = which == 0 ? p.dv_row : p.dk_row;
+      const long long off = seg_off + ((long long)b * p.Sk + (key < p.Sk ? key : 0)) * rs_ + (long long)kv_head * D;
+      uint8_t* const stg = (which == 0 ? sV : sK) + (sub * 4 + quarter) * (D / SUBS * 64);
+      int pieces = 0;
+      auto put16 = [&](int col, const uint32_t* r) {        // 16 columns of this thread's row from `col` on
+        const uint4 lo = make_uint4(pack_bf16(__uint_as_float(r[0]), __uint_as_float(r[1])), pack_bf16(__uint_as_float(r[2]), __uint_as_float(r[3])),
+                                    pack_bf16(__uint_as_float(r[4]), __uint_as_float(r[5])), pack_bf16(__uint_as_float(r[6]), __uint_as_float(r[7])));
+        const uint4 hi = make_uint4(pack_bf16(__uint_as_float(r[8]), __uint_as_float(r[9])), pack_bf16(__uint_as_float(r[10]), __uint_as_float(r[11])),
+                                    pack_bf16(__uint_as_float(r[12]), __uint_as_float(r[13])), pack_bf16(__uint_as_float(r[14]), __uint_as_float(r[15])));
+        if (tm_out) {
+          uint4* const q = reinterpret_cast<uint4*>(stg + pieces * 1024 + lane * 32);
+          q[0] = lo;
+          q[1] = hi;
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (elect_one()) {
+            const int row0 = k0 + quarter * 32;
+            if (row0 < p.Sk) tma_store_4d(which == 0 ? &tm_dv : &tm_dk, stg + pieces * 1024, col, kv_head, row0, b);
+            tma_store_commit();
+          }
+          ++pieces;
+        } else if (key < p.Sk) {
+          uint4* const q = reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(which == 0 ? dV_ : dK_) + off + col);
+          q[0] = lo;
+          q[1] = hi;
+        }
+      };
       if (!OUT_F32 && which == 1 && p.cosT != nullptr) {
         // dK with the inverse rotation: pairs j <-> j + D/2, 16 columns of each half of the row at a time
-        const int row = key < p.Sk ? key : 0, pos = row % p.rope_seq;
+        const int pos = (key < p.Sk ? key : 0) % p.rope_seq;
         const float* cos_row = p.cosT + (long long)pos * (D / 2);
         const float* sin_row = p.sinT + (long long)pos * (D / 2);
-        bf16* orow = reinterpret_cast<bf16*>(dK_) + seg_off + ((long long)b * p.Sk + row) * p.dk_row + (long long)kv_head * D;
-        auto store16 = [](bf16* dst, const uint32_t (&r)[16]) {
-#pragma unroll
-          for (int u = 0; u < 2; ++u)
-            reinterpret_cast<uint4*>(dst)[u] =
-                make_uint4(pack_bf16(__uint_as_float(r[8 * u]), __uint_as_float(r[8 * u + 1])),
-                           pack_bf16(__uint_as_float(r[8 * u + 2]), __uint_as_float(r[8 * u + 3])),
-                           pack_bf16(__uint_as_float(r[8 * u + 4]), __uint_as_float(r[8 * u + 5])),
-                           pack_bf16(__uint_as_float(r[8 * u + 6]), __uint_as_float(r[8 * u + 7])));
-        };
 #pragma unroll 1
         for (int c = sub; c < D / 32; c += SUBS) {
           uint32_t lo[16], hi[16];
           tmem_ld_32x32b_x16(t_lane + Cfg::DK_COL + c * 16, lo);
           tmem_ld_32x32b_x16(t_lane + Cfg::DK_COL + D / 2 + c * 16, hi);
           tmem_ld_wait();
-          if (key < p.Sk) {
 #pragma unroll
-            for (int j = 0; j < 16; j += 4) {
-              const float4 cs = __ldg(reinterpret_cast<const float4*>(cos_row + c * 16 + j));
-              const float4 sn = __ldg(reinterpret_cast<const float4*>(sin_row + c * 16 + j));
-              const float csv[4] = {cs.x, cs.y, cs.z, cs.w}, snv[4] = {sn.x, sn.y, sn.z, sn.w};
+          for (int j = 0; j < 16; j += 4) {
+            const float4 cs = __ldg(reinterpret_cast<const float4*>(cos_row + c * 16 + j));
+            const float4 sn = __ldg(reinterpret_cast<const float4*>(sin_row + c * 16 + j));
+            const float csv[4] = {cs.x, cs.y, cs.z, cs.w}, snv[4] = {sn.x, sn.y, sn.z, sn.w};
 #pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                const float a = __uint_as_float(lo[j + i]), b = __uint_as_float(hi[j + i]);
-                lo[j + i] = __float_as_uint(a * csv[i] + b * snv[i]);
-                hi[j + i] = __float_as_uint(b * csv[i] - a * snv[i]);
-              }
+            for (int i = 0; i < 4; ++i) {
+              const float a = __uint_as_float(lo[j + i]), b_ = __uint_as_float(hi[j + i]);
+              lo[j + i] = __float_as_uint(a * csv[i] + b_ * snv[i]);
+              hi[j + i] = __float_as_uint(b_ * csv[i] - a * snv[i]);
             }
-            store16(orow + c * 16, lo);
-            store16(orow + D / 2 + c * 16, hi);
           }
+          put16(c * 16, lo);
+          put16(D / 2 + c * 16, hi);
         }
       } else {
-        const long long rs_ = which == 0 ? p.dv_row : p.dk_row;
         const int col_base = which == 0 ? Cfg::DV_COL : Cfg::DK_COL;
-        const long long off = seg_off + ((long long)b * p.Sk + (key < p.Sk ? key : 0)) * rs_ + (long long)kv_head * D;
 #pragma unroll 1
         for (int c = sub; c < D / 32; c += SUBS) {
           uint32_t r[32];
           tmem_ld_32x32b_x32(t_lane + col_base + c * 32, r);
           tmem_ld_wait();
-          if (key < p.Sk) {
-            if (OUT_F32) {
+          if (OUT_F32) {
+            if (key < p.Sk) {
               float* orow = reinterpret_cast<float*>(which == 0 ? dV_ : dK_) + off + c * 32;
 #pragma unroll
               for (int u = 0; u < 8; ++u)
                 reinterpret_cast<float4*>(orow)[u] = make_float4(__uint_as_float(r[4 * u]), __uint_as_float(r[4 * u + 1]),
                                                                  __uint_as_float(r[4 * u + 2]), __uint_as_float(r[4 * u + 3]));
-            } else {
-              bf16* orow = reinterpret_cast<bf16*>(which == 0 ? dV_ : dK_) + off + c * 32;
-#pragma unroll
-              for (int u = 0; u < 4; ++u) {
-                uint4 v = make_uint4(pack_bf16(__uint_as_float(r[8 * u]), __uint_as_float(r[8 * u + 1])),
-                                     pack_bf16(__uint_as_float(r[8 * u + 2]), __uint_as_float(r[8 * u + 3])),
-                                     pack_bf16(__uint_as_float(r[8 * u + 4]), __uint_as_float(r[8 * u + 5])),
-                                     pack_bf16(__uint_as_float(r[8 * u + 6]), __uint_as_float(r[8 * u + 7])));
-                reinterpret_cast<uint4*>(orow)[u] = v;
-              }
             }
+          } else {
+            put16(c * 32, r);
+            put16(c * 32 + 16, r + 16);
           }
         }
       }
+      if (tm_out && elect_one()) tma_store_wait<0>();
     } else if (ok && lane == 0) {
       report_error(status, KID_BWD, 10);
+    }
     }
   }
 
@@ -1052,16 +1102,17 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tm_q, const KVS
 
 #define PT_BWD_PARAMS                                                                                                           \
   const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ KVSegs segs, const __grid_constant__ CUtensorMap tm_do,      \
-      const __grid_constant__ CUtensorMap tm_dq, const float* __restrict__ LSE, const float* __restrict__ DELTA,                 \
+      const __grid_constant__ CUtensorMap tm_dq, const __grid_constant__ CUtensorMap tm_dk,                                     \
+      const __grid_constant__ CUtensorMap tm_dv, const float* __restrict__ LSE, const float* __restrict__ DELTA,                 \
       void* __restrict__ dK_, void* __restrict__ dV_, const __grid_constant__ BwdParams p, KernelStatus* status
 // (two kernels, because the build checks their register counts by name)
 template <int D, bool OUT_F32, bool PROF>
 __global__ void __launch_bounds__(BwdWarps<2>::THREADS, 1) attn_bwd_kernel(PT_BWD_PARAMS) {
-  attn_bwd_body<D, OUT_F32, PROF, 2>(tm_q, segs, tm_do, tm_dq, LSE, DELTA, dK_, dV_, p, status);
+  attn_bwd_body<D, OUT_F32, PROF, 2>(tm_q, segs, tm_do, tm_dq, tm_dk, tm_dv, LSE, DELTA, dK_, dV_, p, status);
 }
 template <int D, bool OUT_F32, bool PROF>
 __global__ void __launch_bounds__(BwdWarps<4>::THREADS, 1) attn_bwd_parts4_kernel(PT_BWD_PARAMS) {
-  attn_bwd_body<D, OUT_F32, PROF, 4>(tm_q, segs, tm_do, tm_dq, LSE, DELTA, dK_, dV_, p, status);
+  attn_bwd_body<D, OUT_F32, PROF, 4>(tm_q, segs, tm_do, tm_dq, tm_dk, tm_dv, LSE, DELTA, dK_, dV_, p, status);
 }
 #undef PT_BWD_PARAMS
 
@@ -1097,10 +1148,11 @@ static int launch_fwd(const CUtensorMap& mq, const KVSegs& segs, void* o, float*
 }
 
 template <int D, bool OUT_F32, bool PROF = false>
-static int launch_bwd(const CUtensorMap& mq, const KVSegs& segs, const CUtensorMap& mdo, const CUtensorMap& mdq, const float* lse,
+static int launch_bwd(const CUtensorMap& mq, const KVSegs& segs, const CUtensorMap& mdo, const CUtensorMap& mdq, const CUtensorMap& mdk,
+                      const CUtensorMap& mdv, const float* lse,
                       const float* delta, void* dk, void* dv, const BwdParams& p, KernelStatus* st, cudaStream_t stream) {
   if (!PROF && p.prof != nullptr)
-    return launch_bwd<D, OUT_F32, true>(mq, segs, mdo, mdq, lse, delta, dk, dv, p, st, stream);
+    return launch_bwd<D, OUT_F32, true>(mq, segs, mdo, mdq, mdk, mdv, lse, delta, dk, dv, p, st, stream);
   using Warps = BwdWarps<bwd_parts<D>()>;
   auto kern = [] {
     if constexpr (bwd_parts<D>() == 4) return attn_bwd_parts4_kernel<D, OUT_F32, PROF>;
@@ -1119,7 +1171,7 @@ static int launch_bwd(const CUtensorMap& mq, const KVSegs& segs, const CUtensorM
   if (rc <= 0) return rc;
   const int num_kb = ((p.Sk + 127) / 128) * p.n_segs;
   const long long grid = (long long)num_kb * p.hkv * p.B;
-  launch_pdl(kern, dim3((unsigned)grid), dim3(Warps::THREADS), BwdCfg<D>::SMEM, stream, mq, segs, mdo, mdq, lse, delta, dk, dv, p, st);
+  launch_pdl(kern, dim3((unsigned)grid), dim3(Warps::THREADS), BwdCfg<D>::SMEM, stream, mq, segs, mdo, mdq, mdk, mdv, lse, delta, dk, dv, p, st);
   pt_count_launches(1);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
@@ -1205,12 +1257,24 @@ static int attention_bwd_impl(const void* dout, const void* q, const void* const
   if (cosT != nullptr && (n_segs != 1 || out_f32 || sinT == nullptr || rope_seq <= 0 || (reinterpret_cast<uintptr_t>(cosT) & 15) ||
                           (reinterpret_cast<uintptr_t>(sinT) & 15)))
     return -12;
-  BwdParams p{B, Sq, Sk, hq, hkv, causal, scale, dk_row, dv_row, n_segs, seg_stride, cosT, sinT, rope_seq, g_attn_prof};
+  // dk, dv through TMA: pieces of 16 columns and 32 keys
+  CUtensorMap mdk = mq, mdv = mq;
+  int tma_out = 0;
+  if (!out_f32 && n_segs == 1) {
+    auto piece_map = [&](CUtensorMap* m, const void* base, long long row) {
+      uint64_t dims[4] = {(uint64_t)d, (uint64_t)hkv, (uint64_t)Sk, (uint64_t)B};
+      uint64_t strides[3] = {(uint64_t)d, (uint64_t)row, (uint64_t)row * (uint64_t)Sk};
+      uint32_t box[4] = {16, 1, 32, 1};
+      return make_bf16_map(m, base, 4, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE) == 0;
+    };
+    tma_out = piece_map(&mdk, dk, dk_row) && piece_map(&mdv, dv, dv_row);
+  }
+  BwdParams p{B, Sq, Sk, hq, hkv, causal, scale, dk_row, dv_row, n_segs, seg_stride, cosT, sinT, rope_seq, tma_out, g_attn_prof};
   KernelStatus* sw = status_word_attn();
-  if (d == 64) rc = out_f32 ? launch_bwd<64, true>(mq, segs, mdo, mdq, lse, delta, dk, dv, p, sw, st)
-                            : launch_bwd<64, false>(mq, segs, mdo, mdq, lse, delta, dk, dv, p, sw, st);
-  else rc = out_f32 ? launch_bwd<128, true>(mq, segs, mdo, mdq, lse, delta, dk, dv, p, sw, st)
-                    : launch_bwd<128, false>(mq, segs, mdo, mdq, lse, delta, dk, dv, p, sw, st);
+  if (d == 64) rc = out_f32 ? launch_bwd<64, true>(mq, segs, mdo, mdq, mdk, mdv, lse, delta, dk, dv, p, sw, st)
+                            : launch_bwd<64, false>(mq, segs, mdo, mdq, mdk, mdv, lse, delta, dk, dv, p, sw, st);
+  else rc = out_f32 ? launch_bwd<128, true>(mq, segs, mdo, mdq, mdk, mdv, lse, delta, dk, dv, p, sw, st)
+                    : launch_bwd<128, false>(mq, segs, mdo, mdq, mdk, mdv, lse, delta, dk, dv, p, sw, st);
   if (rc) return rc;
   if (dq != nullptr) {
     const long long n = (long long)B * Sq * hq * d;

@@ -23,10 +23,10 @@ inline EncodeTiledFn tensormap_encode_fn() {
   return fn;
 }
 
-// bf16 tensor map of rank `rank` (<= 4), 128-byte swizzle, zero fill out of bounds.
+// bf16 tensor map of rank `rank` (<= 4), 128-byte swizzle unless told otherwise, zero fill out of bounds.
 // dims[0] is the contiguous dimension; strides_elems[i] is the stride of dimension i+1 in elements.
 inline int make_bf16_map(CUtensorMap* map, const void* base, int rank, const uint64_t* dims,
-                         const uint64_t* strides_elems, const uint32_t* box) {
+                         const uint64_t* strides_elems, const uint32_t* box, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
   EncodeTiledFn fn = tensormap_encode_fn();
   if (fn == nullptr) return -1;
   // The driver call needs a context bound to the calling thread. A fresh thread (an autograd worker whose first
@@ -41,7 +41,7 @@ inline int make_bf16_map(CUtensorMap* map, const void* base, int rank, const uin
   for (int i = 0; i < rank; ++i) { d[i] = dims[i]; b[i] = box[i]; }
   for (int i = 0; i + 1 < rank; ++i) s[i] = strides_elems[i] * 2;
   CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(base), d, s, b, e,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : -2;
 }
