@@ -29,6 +29,7 @@
 #include "common.cuh"
 #include "tensormap.cuh"
 
+#include <algorithm>
 #include <type_traits>
 
 extern "C" void pt_count_launches(int n);
@@ -517,6 +518,7 @@ struct BwdParams {
   const float* sinT;
   int rope_seq;
   int tma_out;                   // dk and dv are stored through their tensor maps (bf16, one segment)
+  int parts;                     // CTAs (of one cluster) that share a key block's query heads, see bwd_head_parts
   unsigned long long* prof;      // optional phase counters, as AttnParams::prof
 };
 
@@ -540,10 +542,12 @@ struct BwdWarps {
 };
 // What a CTA works on: a key block of a key/value head, with the query heads of its group and the query blocks that see it.
 struct BwdWork {
-  int seg, k0, kv_head, b, qb_first, steps_per_head, steps;
+  int seg, k0, kv_head, b, part, head0, qb_first, steps_per_head, steps;       // part: of the key block's CTAs; head0: its first query head
   bool diag;
 };
-__device__ __forceinline__ BwdWork bwd_work(const BwdParams& p, int BM, int BN, unsigned cta) {
+template <bool SPLIT>
+__device__ __forceinline__ BwdWork bwd_work(const BwdParams& p, int BM, int BN, unsigned block) {
+  const unsigned parts = SPLIT ? p.parts : 1, cta = block / parts;
   const unsigned bps = (unsigned)(p.Sk + BN - 1) / BN;    // key blocks per segment
   const unsigned num_kb = bps * p.n_segs, heads = (unsigned)(p.hkv * p.B);
   // causal: the first (heaviest) key blocks of all heads first, full attention: head by head (see the forward)
@@ -556,12 +560,39 @@ __device__ __forceinline__ BwdWork bwd_work(const BwdParams& p, int BM, int BN, 
   w.b = (int)(bh / (unsigned)p.hkv);
   w.qb_first = w.diag ? w.k0 / BM : 0;                    // first query block that sees key k0
   w.steps_per_head = (p.Sq + BM - 1) / BM - w.qb_first;
-  w.steps = w.steps_per_head > 0 ? w.steps_per_head * (p.hq / p.hkv) : 0;
+  const int heads_here = p.hq / p.hkv / (int)parts;
+  w.part = (int)(block % parts);
+  w.head0 = (w.kv_head * (int)parts + w.part) * heads_here;
+  w.steps = w.steps_per_head > 0 ? w.steps_per_head * heads_here : 0;
   return w;
 }
 template <int D> constexpr int bwd_parts() { return D == 64 ? 4 : 2; }
 template <int N> __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+
+// Bytes of one CTA's dV and dK sums (fp32) on their way to the first CTA of the cluster: [dV, dK][4 columns][128 keys][4].
+template <int D> constexpr int BWD_SUM_BYTES = 2 * 128 * D * 4;
+// A compute thread's share of them to `to` (shared::cluster address).
+template <int D, int PARTS>
+__device__ __forceinline__ void bwd_send_sums(uint32_t tmem_base, uint32_t to) {
+  using Cfg = BwdCfg<D>;
+  constexpr int SUBS = PARTS / 2;
+  unsigned thread;
+  asm volatile("mov.u32 %0, %%tid.x;" : "=r"(thread));
+  const int part = thread >> 7, which = part / SUBS, sub = part % SUBS;
+  const uint32_t from = tmem_base + (((thread >> 5) & 3) * 32 << 16) + (which == 0 ? Cfg::DV_COL : Cfg::DK_COL);
+#pragma unroll 1
+  for (int c = sub; c < D / 32; c += SUBS) {
+    uint32_t r[32];
+    tmem_ld_32x32b_x32(from + c * 32, r);
+    tmem_ld_wait();
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(to + ((which * (D / 4) + c * 8 + u) * 128 + (thread & 127)) * 16),
+                   "r"(r[4 * u]), "r"(r[4 * u + 1]), "r"(r[4 * u + 2]), "r"(r[4 * u + 3])
+                   : "memory");
+  }
+}
 
 // What bounds it: a step (128 keys x 128 queries) is a chain S -> exp -> dP -> dS -> dQ -> drain of hand-offs between the
 // tensor core and the compute warps, each of a few hundred cycles; run one after the other they cost 5,400 (d = 64) and
@@ -570,7 +601,7 @@ template <int N> __device__ __forceinline__ void regs_dec() { asm volatile("setm
 // dQ_i is drained by warps of their own. The scores are computed TRANSPOSED (lane = key): then P^T is written straight back to
 // tensor memory as the A operand of dV += P^T dO, and only dS^T goes through shared memory (which the MMAs read all the time).
 // Measured (us; 1 x 32768, 32 / 8 heads, d = 64; 1 x 8192, 32 / 8 heads, d = 128): 21,500 -> 16,200 and 2,160 -> 1,410.
-template <int D, bool OUT_F32, bool PROF, int PARTS>
+template <int D, bool OUT_F32, bool PROF, bool SPLIT, int PARTS>
 __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tm_q, const KVSegs& segs, const CUtensorMap& tm_do, const CUtensorMap& tm_dq,
                                               const CUtensorMap& tm_dk, const CUtensorMap& tm_dv,
                                               const float* __restrict__ LSE, const float* __restrict__ DELTA, void* __restrict__ dK_,
@@ -592,9 +623,8 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tm_q, const KVS
   float* sStat = reinterpret_cast<float*>(sDQ + Cfg::DQ_BYTES);       // [stage][-lse * log2(e) | -delta * scale][128]
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-  const int group = p.hq / p.hkv;
-  const BwdWork work = bwd_work(p, Cfg::BM, Cfg::BN, blockIdx.x);
-  const int seg = work.seg, kv_head = work.kv_head, b = work.b, k0 = work.k0, qb_first = work.qb_first, steps_per_head = work.steps_per_head,
+  const BwdWork work = bwd_work<SPLIT>(p, Cfg::BM, Cfg::BN, blockIdx.x);
+  const int seg = work.seg, kv_head = work.kv_head, head0 = work.head0, b = work.b, k0 = work.k0, qb_first = work.qb_first, steps_per_head = work.steps_per_head,
             total_steps = work.steps;
   const bool diag = work.diag;
   const bool tm_out = !OUT_F32 && p.tma_out;
@@ -657,8 +687,8 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tm_q, const KVS
         tma_load_4d(sK + c * (Cfg::BN * 128), &segs.k[seg], &bars.kv_full, c * 64, kv_head, k0, b);
         tma_load_4d(sV + c * (Cfg::BN * 128), &segs.v[seg], &bars.kv_full, c * 64, kv_head, k0, b);
       }
-      load_q(0, kv_head * group, qb_first * Cfg::BM);
-      load_do(0, kv_head * group, qb_first * Cfg::BM);
+      load_q(0, head0, qb_first * Cfg::BM);
+      load_do(0, head0, qb_first * Cfg::BM);
     }
   }
   if (warp == CW + 5) {
@@ -677,7 +707,7 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tm_q, const KVS
     // ------------------------------------------------------------------------------ TMA producer
     if (total_steps > 0 && elect_one()) {
       for (int it = 1; it < total_steps; ++it) {           // (the first step's and K, V: above)
-        const int head = kv_head * group + it / steps_per_head, q0 = (qb_first + it % steps_per_head) * Cfg::BM;
+        const int head = head0 + it / steps_per_head, q0 = (qb_first + it % steps_per_head) * Cfg::BM;
         if (!mbar_wait(&bars.q_empty[it % Cfg::QSTAGES], ((it / Cfg::QSTAGES) & 1) ^ 1, abort_flag)) { report_error(status, KID_BWD, 1); break; }
         load_q(it, head, q0);
         if (!mbar_wait(&bars.do_empty[it % Cfg::OSTAGES], ((it / Cfg::OSTAGES) & 1) ^ 1, abort_flag)) { report_error(status, KID_BWD, 11); break; }
@@ -783,7 +813,7 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tm_q, const KVS
     // ------------------------------------------------------------------------------ row statistics (lse, delta) of a step's queries
     for (int it = 0; it < total_steps; ++it) {
       const int st = it & 1;
-      const int head = kv_head * group + it / steps_per_head;
+      const int head = head0 + it / steps_per_head;
       const int q0 = (qb_first + it % steps_per_head) * Cfg::BM;
       const long long base = ((long long)b * p.hq + head) * p.Sq;
       float l[4], dl[4];
@@ -813,7 +843,7 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tm_q, const KVS
     const bool prof_on = PROF && p.prof != nullptr && threadIdx.x == CW * 32;
     long long pacc[2] = {0, 0};
     for (int it = 0; it < total_steps; ++it) {
-      const int head = kv_head * group + it / steps_per_head;
+      const int head = head0 + it / steps_per_head;
       const int row0 = (qb_first + it % steps_per_head) * Cfg::BM + quarter * 32;
       const long long pt0 = prof_clock(prof_on);
       if (!mbar_wait(&bars.dq_full, it & 1, abort_flag)) { if (lane == 0) report_error(status, KID_BWD, 9); break; }
@@ -972,22 +1002,39 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tm_q, const KVS
       for (int i = 0; i < 2; ++i) atomicAdd(&p.prof[i], (unsigned long long)pacc[i]);
       atomicAdd(&p.prof[4], (unsigned long long)total_steps);
       atomicAdd(&p.prof[5], (unsigned long long)(clock64() - pstart));
-      atomicAdd(&p.prof[6], 1ull);
+      atomicAdd(&p.prof[6], work.part == 0 ? 1ull : 0ull);
     }
     {
+    if constexpr (SPLIT) {
+      // The other CTAs' sums come to the first one's shared memory, in the place of the operand rings and dS, when everybody's MMAs are done.
+      if (ok && !mbar_wait(&bars.acc_full, 0, abort_flag)) {
+        if (lane == 0) report_error(status, KID_BWD, 10);
+        ok = false;
+      }
+      __syncwarp();
+      cluster_arrive();
+      cluster_wait();
+      tcgen05_fence_after();
+      if (ok && cluster_ctarank() > 0) bwd_send_sums<D, PARTS>(tmem_base, mapa_u32(smem_u32(sQ), 0) + (cluster_ctarank() - 1) * BWD_SUM_BYTES<D>);
+      __syncwarp();
+      cluster_arrive();
+      cluster_wait();
+    }
     // dK, dV of this key block (thread t <-> key k0 + t); fp32 when they are partials of a multi-rank reduction
     // (The block and thread are read anew: what is kept from before the loop over the steps takes registers there, and with the stores below
     // its compute warps executed 8 % more instructions, 14.0 -> 14.6 ms at 32,768 tokens.)
     unsigned cta, thread;
     asm volatile("mov.u32 %0, %%ctaid.x;" : "=r"(cta));
     asm volatile("mov.u32 %0, %%tid.x;" : "=r"(thread));
-    const BwdWork work = bwd_work(p, Cfg::BM, Cfg::BN, cta);
+    const BwdWork work = bwd_work<SPLIT>(p, Cfg::BM, Cfg::BN, cta);
     const int kv_head = work.kv_head, b = work.b, k0 = work.k0, seg = work.seg, total_steps = work.steps;
+    constexpr int SUBS = PARTS / 2;
     const int lane = thread & 31, quarter = (thread >> 5) & 3, part = thread >> 7, which = part / SUBS, sub = part % SUBS, key = k0 + (int)(thread & 127);
     const uint32_t t_lane = tmem_base + (uint32_t(quarter * 32) << 16);
     const bool tm_out = !OUT_F32 && p.tma_out;
     const long long seg_off = (long long)seg * p.seg_stride;
-    if (total_steps == 0) {
+    if (SPLIT && work.part > 0) {            // (its sums are with the first)
+    } else if (total_steps == 0) {
       if (key < p.Sk && sub == 0) {
         {
           const long long rs_ = which == 0 ? p.dv_row : p.dk_row;
@@ -1001,7 +1048,7 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tm_q, const KVS
           }
         }
       }
-    } else if (ok && (which == 0 ? mbar_wait(&bars.p_free, (total_steps - 1) & 1, abort_flag) : mbar_wait(&bars.acc_full, 0, abort_flag))) {
+    } else if (ok && (SPLIT || (which == 0 ? mbar_wait(&bars.p_free, (total_steps - 1) & 1, abort_flag) : mbar_wait(&bars.acc_full, 0, abort_flag)))) {
       // dV is complete with its last MMA, half a step before dK. Rows of 16 columns (32 bytes) of each warp's 32 keys go to TMA through the
       // place of V, which the last dP was the last to read, and of K: stored by every thread for itself they were 16-byte pieces of 32 rows an
       // instruction, and the end of a CTA took 3,600 (d = 64) and 7,600 cycles (d = 128) of the 20,900 and 34,000 that one of 4 x 1024,
@@ -1011,6 +1058,21 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tm_q, const KVS
       const long long off = seg_off + ((long long)b * p.Sk + (key < p.Sk ? key : 0)) * rs_ + (long long)kv_head * D;
       uint8_t* const stg = (which == 0 ? sV : sK) + (sub * 4 + quarter) * (D / SUBS * 64);
       int pieces = 0;
+      // 4 x N columns of this row from `col` on, of the other CTAs, in their order
+      auto add_parts = [&](int col, uint32_t* r, int quads) {
+        for (int o = 1; SPLIT && o < p.parts; ++o) {
+          const float4* const q = reinterpret_cast<const float4*>(sQ + (o - 1) * BWD_SUM_BYTES<D>) + (which * (D / 4) + col / 4) * 128 + (thread & 127);
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+            if (u < quads) {
+              const float4 v = q[u * 128];
+              r[4 * u] = __float_as_uint(__uint_as_float(r[4 * u]) + v.x);
+              r[4 * u + 1] = __float_as_uint(__uint_as_float(r[4 * u + 1]) + v.y);
+              r[4 * u + 2] = __float_as_uint(__uint_as_float(r[4 * u + 2]) + v.z);
+              r[4 * u + 3] = __float_as_uint(__uint_as_float(r[4 * u + 3]) + v.w);
+            }
+        }
+      };
       auto put16 = [&](int col, const uint32_t* r) {        // 16 columns of this thread's row from `col` on
         const uint4 lo = make_uint4(pack_bf16(__uint_as_float(r[0]), __uint_as_float(r[1])), pack_bf16(__uint_as_float(r[2]), __uint_as_float(r[3])),
                                     pack_bf16(__uint_as_float(r[4]), __uint_as_float(r[5])), pack_bf16(__uint_as_float(r[6]), __uint_as_float(r[7])));
@@ -1045,6 +1107,8 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tm_q, const KVS
           tmem_ld_32x32b_x16(t_lane + Cfg::DK_COL + c * 16, lo);
           tmem_ld_32x32b_x16(t_lane + Cfg::DK_COL + D / 2 + c * 16, hi);
           tmem_ld_wait();
+          add_parts(c * 16, lo, 4);
+          add_parts(D / 2 + c * 16, hi, 4);
 #pragma unroll
           for (int j = 0; j < 16; j += 4) {
             const float4 cs = __ldg(reinterpret_cast<const float4*>(cos_row + c * 16 + j));
@@ -1067,6 +1131,7 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tm_q, const KVS
           uint32_t r[32];
           tmem_ld_32x32b_x32(t_lane + col_base + c * 32, r);
           tmem_ld_wait();
+          add_parts(c * 32, r, 8);
           if (OUT_F32) {
             if (key < p.Sk) {
               float* orow = reinterpret_cast<float*>(which == 0 ? dV_ : dK_) + off + c * 32;
@@ -1085,6 +1150,15 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tm_q, const KVS
     } else if (ok && lane == 0) {
       report_error(status, KID_BWD, 10);
     }
+    }
+  }
+  if constexpr (SPLIT) {
+    if (warp >= CW) {                  // (the compute warps' two)
+      for (int i = 0; i < 2; ++i) {
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+      }
     }
   }
 
@@ -1106,13 +1180,13 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tm_q, const KVS
       const __grid_constant__ CUtensorMap tm_dv, const float* __restrict__ LSE, const float* __restrict__ DELTA,                 \
       void* __restrict__ dK_, void* __restrict__ dV_, const __grid_constant__ BwdParams p, KernelStatus* status
 // (two kernels, because the build checks their register counts by name)
-template <int D, bool OUT_F32, bool PROF>
+template <int D, bool OUT_F32, bool PROF, bool SPLIT>
 __global__ void __launch_bounds__(BwdWarps<2>::THREADS, 1) attn_bwd_kernel(PT_BWD_PARAMS) {
-  attn_bwd_body<D, OUT_F32, PROF, 2>(tm_q, segs, tm_do, tm_dq, tm_dk, tm_dv, LSE, DELTA, dK_, dV_, p, status);
+  attn_bwd_body<D, OUT_F32, PROF, SPLIT, 2>(tm_q, segs, tm_do, tm_dq, tm_dk, tm_dv, LSE, DELTA, dK_, dV_, p, status);
 }
-template <int D, bool OUT_F32, bool PROF>
+template <int D, bool OUT_F32, bool PROF, bool SPLIT>
 __global__ void __launch_bounds__(BwdWarps<4>::THREADS, 1) attn_bwd_parts4_kernel(PT_BWD_PARAMS) {
-  attn_bwd_body<D, OUT_F32, PROF, 4>(tm_q, segs, tm_do, tm_dq, tm_dk, tm_dv, LSE, DELTA, dK_, dV_, p, status);
+  attn_bwd_body<D, OUT_F32, PROF, SPLIT, 4>(tm_q, segs, tm_do, tm_dq, tm_dk, tm_dv, LSE, DELTA, dK_, dV_, p, status);
 }
 #undef PT_BWD_PARAMS
 
@@ -1147,33 +1221,52 @@ static int launch_fwd(const CUtensorMap& mq, const KVSegs& segs, void* o, float*
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 
-template <int D, bool OUT_F32, bool PROF = false>
+// CTAs that share the query heads of a key block (`ctas` of them): where all parts still have an SM each and the longest CTA gets four steps shorter at
+// least, as far as the parts' sums fit beside each other (3 parts for d = 64, 2 for d = 128). 3 x 601, 9 / 3 heads are 45 key blocks of up to
+// 15 steps: 36.9 us, in three parts 29.9; 2 x 256, 8 / 4 heads, 16 of up to 4: 16.4, in two 17.8. Beyond one wave the CTAs' starts and ends and the
+// clusters' (of CTAs that fill an SM) waiting for neighbouring SMs cost more than evenness gives: 8 x 1024, 9 / 3 heads 57 us, in three 98.
+static int bwd_head_parts(const BwdParams& p, int d, long long ctas, int sms) {
+  const long long group = p.hq / p.hkv, steps = (p.Sq + 127) / 128 * group;
+  for (int parts = d == 64 ? 3 : 2; parts > 1; --parts)
+    if (group % parts == 0 && ctas * parts <= sms && steps - steps / parts >= 4) return parts;
+  return 1;
+}
+
+template <int D, bool OUT_F32, bool PROF = false, bool SPLIT = false>
 static int launch_bwd(const CUtensorMap& mq, const KVSegs& segs, const CUtensorMap& mdo, const CUtensorMap& mdq, const CUtensorMap& mdk,
-                      const CUtensorMap& mdv, const float* lse,
-                      const float* delta, void* dk, void* dv, const BwdParams& p, KernelStatus* st, cudaStream_t stream) {
+                      const CUtensorMap& mdv, const float* lse, const float* delta, void* dk, void* dv, BwdParams p, KernelStatus* st,
+                      cudaStream_t stream) {
   if (!PROF && p.prof != nullptr)
     return launch_bwd<D, OUT_F32, true>(mq, segs, mdo, mdq, mdk, mdv, lse, delta, dk, dv, p, st, stream);
   using Warps = BwdWarps<bwd_parts<D>()>;
   auto kern = [] {
-    if constexpr (bwd_parts<D>() == 4) return attn_bwd_parts4_kernel<D, OUT_F32, PROF>;
-    else return attn_bwd_kernel<D, OUT_F32, PROF>;
+    if constexpr (bwd_parts<D>() == 4) return attn_bwd_parts4_kernel<D, OUT_F32, PROF, SPLIT>;
+    else return attn_bwd_kernel<D, OUT_F32, PROF, SPLIT>;
   }();
   static PerDevice configured;
-  const int rc = configured.get(current_device(), [&] {
+  const int sms = configured.get(current_device(), [&] {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdCfg<D>::SMEM) != cudaSuccess) return -3;
     cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     // the warpgroups share out Warps::REGS registers per thread; with fewer at launch setmaxnreg.inc would wait forever (the build
     // fails for another count, build.py: FIXED_REGISTERS)
     cudaFuncAttributes fa;
     if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess || fa.numRegs != Warps::REGS) return -6;
-    return 1;
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -3;
+    return n;
   });
-  if (rc <= 0) return rc;
-  const int num_kb = ((p.Sk + 127) / 128) * p.n_segs;
-  const long long grid = (long long)num_kb * p.hkv * p.B;
-  launch_pdl(kern, dim3((unsigned)grid), dim3(Warps::THREADS), BwdCfg<D>::SMEM, stream, mq, segs, mdo, mdq, mdk, mdv, lse, delta, dk, dv, p, st);
+  if (sms <= 0) return sms;
+  const long long ctas = (long long)((p.Sk + 127) / 128) * p.n_segs * p.hkv * p.B;
+  if constexpr (!SPLIT) {
+    p.parts = bwd_head_parts(p, D, ctas, sms);
+    if (p.parts > 1) return launch_bwd<D, OUT_F32, PROF, true>(mq, segs, mdo, mdq, mdk, mdv, lse, delta, dk, dv, p, st, stream);
+  }
+  static_assert((D == 64 ? 2 : 1) * BWD_SUM_BYTES<D> <= (BwdCfg<D>::QSTAGES + BwdCfg<D>::OSTAGES) * BwdCfg<D>::TILE_BYTES + BwdCfg<D>::DS_BYTES,
+                "the parts' sums take the place of the rings and dS");
+  const cudaError_t err = launch_pdl_cluster(kern, dim3((unsigned)(ctas * p.parts)), dim3(Warps::THREADS), BwdCfg<D>::SMEM, stream, p.parts, mq, segs,
+                                             mdo, mdq, mdk, mdv, lse, delta, dk, dv, p, st);
   pt_count_launches(1);
-  return cudaGetLastError() == cudaSuccess ? 0 : -4;
+  return err == cudaSuccess && cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 
 }  // namespace attn
@@ -1269,7 +1362,7 @@ static int attention_bwd_impl(const void* dout, const void* q, const void* const
     };
     tma_out = piece_map(&mdk, dk, dk_row) && piece_map(&mdv, dv, dv_row);
   }
-  BwdParams p{B, Sq, Sk, hq, hkv, causal, scale, dk_row, dv_row, n_segs, seg_stride, cosT, sinT, rope_seq, tma_out, g_attn_prof};
+  BwdParams p{B, Sq, Sk, hq, hkv, causal, scale, dk_row, dv_row, n_segs, seg_stride, cosT, sinT, rope_seq, tma_out, 1, g_attn_prof};
   KernelStatus* sw = status_word_attn();
   if (d == 64) rc = out_f32 ? launch_bwd<64, true>(mq, segs, mdo, mdq, mdk, mdv, lse, delta, dk, dv, p, sw, st)
                             : launch_bwd<64, false>(mq, segs, mdo, mdq, mdk, mdv, lse, delta, dk, dv, p, sw, st);

@@ -136,6 +136,33 @@ def test_attention_backward_at_tile_and_ring_edges(C, Sq, Sk, group, causal, d):
         assert err <= 1e-2 * float(w.norm()) + 2e-3 * w.numel() ** 0.5, f"{name}: {err} of {float(w.norm())}"
 
 
+@pytest.mark.parametrize("d,Sq,Sk,group,causal", [(64, 300, 300, 3, True), (64, 130, 400, 4, True), (64, 257, 129, 6, False), (64, 700, 700, 8, True),
+                                                  (128, 520, 520, 2, True), (128, 260, 300, 4, False), (64, 300, 300, 5, True)])
+@pytest.mark.parametrize("rope", [False, True])
+def test_attention_backward_of_few_key_blocks_with_long_groups(C, d, Sq, Sk, group, causal, rope):
+    """Key blocks whose query heads are shared by the CTAs of a cluster (groups of 3, 4, 6, 8 and 2), one whose group cannot be cut (5), and keys no
+    query sees; dK and dV repeat to the bit (their sums have an order)."""
+    if rope and Sq != Sk:
+        pytest.skip("the fused rotation is that of self-attention")
+    q, k, v = rnd(2, Sq, 2 * group, d, seed=1), rnd(2, Sk, 2, d, seed=2), rnd(2, Sk, 2, d, seed=3)
+    do = rnd(2, Sq, 2 * group, d, seed=4)
+    scale = 1.0 / math.sqrt(d)
+    o_ref, lse_ref = ref.attention_fwd(q, k, v, causal, scale)
+    want = list(ref.attention_bwd(do, q, k, v, o_ref, lse_ref, causal, scale))
+    tables = ref.rope_tables(Sk, d, 10000.0, device="cuda") if rope else (None, None)
+    if rope:
+        for i, h in ((0, 2 * group), (1, 2)):
+            want[i] = ref.rope_(want[i].reshape(2 * Sk, h * d).clone(), *tables, h, d, Sk, True).view(2, Sk, h, d)
+    got = C.attention_bwd(do, q, k, v, o_ref, lse_ref, causal, scale, None, None, *tables)
+    again = C.attention_bwd(do, q, k, v, o_ref, lse_ref, causal, scale, None, None, *tables)
+    torch.cuda.synchronize()
+    assert C.kernel_status() == 0
+    assert torch.equal(got[1], again[1]) and torch.equal(got[2], again[2])
+    for name, g, w in zip(("dq", "dk", "dv"), got, want):          # (bounds as above)
+        err = float((g.float() - w.float()).norm())
+        assert err <= 1e-2 * float(w.float().norm()) + 2e-3 * w.numel() ** 0.5, f"{name}: {err} of {float(w.float().norm())}"
+
+
 @pytest.mark.parametrize("B,S,hq,hkv,d", [(2, 256, 4, 2, 64), (1, 300, 4, 4, 64), (2, 256, 2, 1, 128), (3, 128, 2, 2, 64)])
 def test_attention_backward_with_inverse_rope_on_dq_dk(C, B, S, hq, hkv, d):
     """dq / dk un-rotated inside the backward (dq in the fp32->bf16 conversion, dk in the epilogue) vs the RoPE kernel."""
