@@ -108,7 +108,7 @@ __device__ __forceinline__ long long prof_clock(bool on) { return on ? clock64()
 
 template <int D, int BN, bool PROF>
 __global__ void __launch_bounds__(192, 2)
-attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ KVSegs segs, bf16* __restrict__ O,
+attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ KVSegs segs, const __grid_constant__ CUtensorMap tm_o,
                 float* __restrict__ LSE, AttnParams p, KernelStatus* status) {
   using Cfg = FwdCfg<D, BN>;
   pdl_launch_dependents();
@@ -137,7 +137,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const int last_end = p.causal ? min(p.Sk, q0 + Cfg::BM) : p.Sk;    // keys of the last segment this tile can see
   const int nblk = (p.n_segs - 1) * bps + (last_end + BN - 1) / BN;
 
-  if (threadIdx.x == 0) {
+  auto load_kv = [&](int st, uint8_t* ring, const CUtensorMap& map, uint64_t* bar, int kv0) {
+    mbar_expect_tx(bar, Cfg::KV_BYTES);
+#pragma unroll
+    for (int c = 0; c < Cfg::DCH; ++c) tma_load_4d(ring + st * Cfg::KV_BYTES + c * (BN * 128), &map, bar, c * 64, kv_head, kv0, b);
+  };
+
+  if (warp == 4 && elect_one()) {
     mbar_init(&bars.q_full, 1);
     for (int s = 0; s < 2; ++s) {
       mbar_init(&bars.k_full[s], 1);
@@ -155,6 +161,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     tma_prefetch_desc(&tm_q);
     tma_prefetch_desc(&segs.k[0]);
     tma_prefetch_desc(&segs.v[0]);
+      tma_prefetch_desc(&tm_o);
+    // The first loads leave before the other warps are let go: they travel under the tensor-memory allocation and the first barrier.
+    pdl_wait();
+    mbar_expect_tx(&bars.q_full, Cfg::Q_BYTES);
+#pragma unroll
+    for (int c = 0; c < Cfg::DCH; ++c) tma_load_4d(sQ + c * (Cfg::BM * 128), &tm_q, &bars.q_full, c * 64, head, q0, b);
+    if (nblk > 0) {
+      load_kv(0, sK, segs.k[0], &bars.k_full[0], 0);
+      load_kv(0, sV, segs.v[0], &bars.v_full[0], 0);
+    }
   }
   if (warp == 5) {
     tmem_alloc(&bars.tmem_base, Cfg::TMEM_COLS);
@@ -170,23 +186,18 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   if (warp == 4) {
     // ------------------------------------------------------------------------------ TMA producer
     if (elect_one()) {
-      mbar_expect_tx(&bars.q_full, Cfg::Q_BYTES);
-#pragma unroll
-      for (int c = 0; c < Cfg::DCH; ++c) tma_load_4d(sQ + c * (Cfg::BM * 128), &tm_q, &bars.q_full, c * 64, head, q0, b);
-      for (int j = 0; j < nblk; ++j) {
+      int seg = 0, kv0 = 0;                          // (the first block's: above)
+      for (int j = 1; j < nblk; ++j) {
         const int st = j & 1;
         const uint32_t ph = (j >> 1) & 1;
-        const int seg = j / bps, kv0 = (j - seg * bps) * BN;
+        if ((kv0 += BN) >= p.Sk) {
+          kv0 = 0;
+          ++seg;
+        }
         if (!mbar_wait(&bars.k_empty[st], ph ^ 1, abort_flag)) { report_error(status, KID_FWD, 1); break; }
-        mbar_expect_tx(&bars.k_full[st], Cfg::KV_BYTES);
-#pragma unroll
-        for (int c = 0; c < Cfg::DCH; ++c)
-          tma_load_4d(sK + st * Cfg::KV_BYTES + c * (BN * 128), &segs.k[seg], &bars.k_full[st], c * 64, kv_head, kv0, b);
+        load_kv(st, sK, segs.k[seg], &bars.k_full[st], kv0);
         if (!mbar_wait(&bars.v_empty[st], ph ^ 1, abort_flag)) { report_error(status, KID_FWD, 2); break; }
-        mbar_expect_tx(&bars.v_full[st], Cfg::KV_BYTES);
-#pragma unroll
-        for (int c = 0; c < Cfg::DCH; ++c)
-          tma_load_4d(sV + st * Cfg::KV_BYTES + c * (BN * 128), &segs.v[seg], &bars.v_full[st], c * 64, kv_head, kv0, b);
+        load_kv(st, sV, segs.v[seg], &bars.v_full[st], kv0);
       }
     }
   } else if (warp == 5) {
@@ -248,6 +259,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     const bool prof_on = PROF && p.prof != nullptr && threadIdx.x == 0;
     long long pacc[4] = {0, 0, 0, 0};
     const long long pstart = prof_clock(prof_on);
+    int seg = 0, col0 = 0;                           // the block's segment and first key in it
     for (int j = 0; j < nblk; ++j) {
       const long long pt0 = prof_clock(prof_on);
       if (!mbar_wait(&bars.s_full, j & 1, abort_flag)) { if (lane == 0) report_error(status, KID_FWD, 7); ok = false; break; }
@@ -260,8 +272,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       tcgen05_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars.s_free);                   // S_j is in registers: the next S may overwrite it
-      const int seg = j / bps;
-      const int col0 = (j - seg * bps) * BN;                      // key index inside its segment
       const bool diag = p.causal && seg == p.n_segs - 1;
       const bool need_mask = (diag && col0 + BN - 1 > q0) || (col0 + BN > p.Sk);
       // four independent running maxima / sums: a single one is a 128-deep chain of dependent instructions
@@ -276,6 +286,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       } else {
 #pragma unroll
         for (int e = 0; e < BN; ++e) mx4[e & 3] = fmaxf(mx4[e & 3], __uint_as_float(s[e]));
+      }
+      if ((col0 += BN) >= p.Sk) {                                 // (the next block's)
+        col0 = 0;
+        ++seg;
       }
       const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
       const float m_blk = mx * sl2;
@@ -347,25 +361,34 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     if (ok && mbar_wait(&bars.o_full, (nblk - 1) & 1, abort_flag)) {
       tcgen05_fence_after();
       const float inv_l = l > 0.f ? 1.f / l : 0.f;
-      bf16* orow = O + (((long long)b * p.Sq + (row < p.Sq ? row : 0)) * p.hq + head) * D;
+      // O goes to TMA through the place of Q, which the last S was the last to read: 32 rows of 64 columns (128 bytes, swizzled) a piece.
+      // (Stored by every thread for itself, they were 16-byte pieces of 32 rows an instruction.)
 #pragma unroll
-      for (int c = 0; c < D / 32; ++c) {
-        uint32_t r[32];
-        tmem_ld_32x32b_x32(t_lane + Cfg::O_COL + c * 32, r);
-        tmem_ld_wait();
-        if (row < p.Sq) {
+      for (int c = 0; c < D / 64; ++c) {
+        uint8_t* const stg = sQ + (warp * (D / 64) + c) * 4096;
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            uint4 v = make_uint4(pack_bf16(__uint_as_float(r[8 * u]) * inv_l, __uint_as_float(r[8 * u + 1]) * inv_l),
-                                 pack_bf16(__uint_as_float(r[8 * u + 2]) * inv_l, __uint_as_float(r[8 * u + 3]) * inv_l),
-                                 pack_bf16(__uint_as_float(r[8 * u + 4]) * inv_l, __uint_as_float(r[8 * u + 5]) * inv_l),
-                                 pack_bf16(__uint_as_float(r[8 * u + 6]) * inv_l, __uint_as_float(r[8 * u + 7]) * inv_l));
-            reinterpret_cast<uint4*>(orow + c * 32)[u] = v;
-          }
+        for (int h = 0; h < 2; ++h) {
+          uint32_t r[32];
+          tmem_ld_32x32b_x32(t_lane + Cfg::O_COL + c * 64 + h * 32, r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            *reinterpret_cast<uint4*>(stg + sw128_offset(lane, h * 4 + u)) =
+                make_uint4(pack_bf16(__uint_as_float(r[8 * u]) * inv_l, __uint_as_float(r[8 * u + 1]) * inv_l),
+                           pack_bf16(__uint_as_float(r[8 * u + 2]) * inv_l, __uint_as_float(r[8 * u + 3]) * inv_l),
+                           pack_bf16(__uint_as_float(r[8 * u + 4]) * inv_l, __uint_as_float(r[8 * u + 5]) * inv_l),
+                           pack_bf16(__uint_as_float(r[8 * u + 6]) * inv_l, __uint_as_float(r[8 * u + 7]) * inv_l));
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (elect_one()) {
+          if (q0 + warp * 32 < p.Sq) tma_store_4d(&tm_o, stg, c * 64, head, q0 + warp * 32, b);
+          tma_store_commit();
         }
       }
       if (row < p.Sq)
         LSE[((long long)b * p.hq + head) * p.Sq + row] = (l > 0.f) ? (m_ref * LN2 + __logf(l)) : -INFINITY;
+      if (elect_one()) tma_store_wait<0>();
     } else if (ok && lane == 0) {
       report_error(status, KID_FWD, 9);
     }
@@ -811,11 +834,15 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tm_q, const KVS
     }
   } else if (warp == CW + 6) {
     // ------------------------------------------------------------------------------ row statistics (lse, delta) of a step's queries
+    int q_at = qb_first * Cfg::BM, head = head0;
     for (int it = 0; it < total_steps; ++it) {
       const int st = it & 1;
-      const int head = head0 + it / steps_per_head;
-      const int q0 = (qb_first + it % steps_per_head) * Cfg::BM;
+      const int q0 = q_at;
       const long long base = ((long long)b * p.hq + head) * p.Sq;
+      if ((q_at += Cfg::BM) >= p.Sq) {
+        q_at = qb_first * Cfg::BM;
+        ++head;
+      }
       float l[4], dl[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -842,9 +869,13 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tm_q, const KVS
     uint8_t* stg = sDQ + quarter * 8192;
     const bool prof_on = PROF && p.prof != nullptr && threadIdx.x == CW * 32;
     long long pacc[2] = {0, 0};
+    int q_at = qb_first * Cfg::BM, head = head0;
     for (int it = 0; it < total_steps; ++it) {
-      const int head = head0 + it / steps_per_head;
-      const int row0 = (qb_first + it % steps_per_head) * Cfg::BM + quarter * 32;
+      const int row0 = q_at + quarter * 32, head_here = head;
+      if ((q_at += Cfg::BM) >= p.Sq) {
+        q_at = qb_first * Cfg::BM;
+        ++head;
+      }
       const long long pt0 = prof_clock(prof_on);
       if (!mbar_wait(&bars.dq_full, it & 1, abort_flag)) { if (lane == 0) report_error(status, KID_BWD, 9); break; }
       tcgen05_fence_after();
@@ -873,7 +904,7 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tm_q, const KVS
           fence_proxy_async_smem();
           __syncwarp();
           if (elect_one()) {
-            if (row0 < p.Sq) tma_reduce_add_4d(&tm_dq, buf, r_ * DR + h * 32, head, row0, b);
+            if (row0 < p.Sq) tma_reduce_add_4d(&tm_dq, buf, r_ * DR + h * 32, head_here, row0, b);
             tma_store_commit();
           }
         }
@@ -903,10 +934,13 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tm_q, const KVS
     const bool prof_on = PROF && p.prof != nullptr && threadIdx.x == 0;
     long long pacc[2] = {0, 0};
     const long long pstart = prof_clock(prof_on);
+    int q_at = qb_first * Cfg::BM;                         // first query of the step (the steps go through them once per head)
     for (int it = 0; it < total_steps; ++it) {
       const long long pt0 = prof_clock(prof_on);
       const uint32_t par = it & 1;
-      const int qcol0 = (qb_first + it % steps_per_head) * Cfg::BM + part * W;     // first query of this thread's columns
+      // first query of this thread's columns (a division a step is slower, but four parts have no register for the counter)
+      const int qcol0 = (PARTS == 4 ? (qb_first + it % steps_per_head) * Cfg::BM : q_at) + part * W;
+      if (PARTS != 4 && (q_at += Cfg::BM) >= p.Sq) q_at = qb_first * Cfg::BM;
       const bool need_mask = (diag && k0 + Cfg::BN - 1 > qcol0) || (k0 + Cfg::BN > p.Sk);
       const int hidden = key >= p.Sk ? W : (diag ? key - qcol0 : 0);              // columns [0, hidden) do not see this key
       const float* st_l = sStat + par * 2 * Cfg::BM + part * W;
@@ -1202,9 +1236,9 @@ static int make_attn_map(CUtensorMap* m, const void* base, int B, int S, int h, 
 }
 
 template <int D, int BN, bool PROF = false>
-static int launch_fwd(const CUtensorMap& mq, const KVSegs& segs, void* o, float* lse, const AttnParams& p,
+static int launch_fwd(const CUtensorMap& mq, const KVSegs& segs, const CUtensorMap& mo, float* lse, const AttnParams& p,
                       KernelStatus* st, cudaStream_t stream) {
-  if (!PROF && p.prof != nullptr) return launch_fwd<D, BN, true>(mq, segs, o, lse, p, st, stream);
+  if (!PROF && p.prof != nullptr) return launch_fwd<D, BN, true>(mq, segs, mo, lse, p, st, stream);
   auto kern = attn_fwd_kernel<D, BN, PROF>;
   static PerDevice configured;
   const int rc = configured.get(current_device(), [&] {
@@ -1216,7 +1250,7 @@ static int launch_fwd(const CUtensorMap& mq, const KVSegs& segs, void* o, float*
   if (rc <= 0) return rc;
   const int num_qb = (p.Sq + 127) / 128;
   const long long grid = (long long)num_qb * p.hq * p.B;
-  launch_pdl(kern, dim3((unsigned)grid), dim3(192), FwdCfg<D, BN>::SMEM, stream, mq, segs, (bf16*)o, lse, p, st);
+  launch_pdl(kern, dim3((unsigned)grid), dim3(192), FwdCfg<D, BN>::SMEM, stream, mq, segs, mo, lse, p, st);
   pt_count_launches(1);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
@@ -1283,19 +1317,20 @@ extern "C" int pt_attention_fwd_segs(const void* q, const void* const* k_ptrs, c
   if (B <= 0 || Sq <= 0 || Sk <= 0) return 0;
   if ((d != 64 && d != 128) || hq % hkv || (q_row % 8) || (k_row % 8) || (v_row % 8) || n_segs < 1 || n_segs > MAX_SEGS)
     return -10;
-  CUtensorMap mq;
+  CUtensorMap mq, mo;
   KVSegs segs;
   const int bn = d == 64 ? 128 : 64;
   int rc;
   if ((rc = make_attn_map(&mq, q, B, Sq, hq, d, q_row, 128))) return rc;
+  if ((rc = make_attn_map(&mo, o, B, Sq, hq, d, (long long)hq * d, 32))) return rc;
   for (int i = 0; i < n_segs; ++i) {
     if ((rc = make_attn_map(&segs.k[i], k_ptrs[i], B, Sk, hkv, d, k_row, bn))) return rc;
     if ((rc = make_attn_map(&segs.v[i], v_ptrs[i], B, Sk, hkv, d, v_row, bn))) return rc;
   }
   for (int i = n_segs; i < MAX_SEGS; ++i) { segs.k[i] = segs.k[0]; segs.v[i] = segs.v[0]; }
   AttnParams p{B, Sq, Sk, hq, hkv, causal, scale, n_segs, g_attn_prof};
-  if (d == 64) return launch_fwd<64, 128>(mq, segs, o, lse, p, status_word_attn(), st);
-  return launch_fwd<128, 64>(mq, segs, o, lse, p, status_word_attn(), st);
+  if (d == 64) return launch_fwd<64, 128>(mq, segs, mo, lse, p, status_word_attn(), st);
+  return launch_fwd<128, 64>(mq, segs, mo, lse, p, status_word_attn(), st);
 }
 
 extern "C" int pt_attention_fwd(const void* q, const void* k, const void* v, void* o, float* lse, int B, int Sq, int Sk,
