@@ -71,6 +71,8 @@ int pt_allreduce_symm(void* const* buf_ptrs, void* const* flag_ptrs, void* mc_pt
 void pt_set_wait_limit_ns(unsigned long long ns);
 int pt_pdl_enabled();
 void pt_set_pdl(int on);
+void pt_chain_begin();
+void pt_chain_end();
 unsigned long long pt_get_wait_limit_ns();
 int pt_gemm_allreduce_bf16(const void* A, const void* B, void* const* buf_ptrs, void* const* flag_ptrs, void* mc_ptr,
                            long long d_offset,
@@ -724,6 +726,12 @@ std::vector<Tensor> decoder_layer_fwd_packed(const Tensor& x, const Tensor& ln1,
 // norm 2), `tables`: two (cosines, sines).
 // ---------------------------------------------------------------------------------------------
 constexpr int LAYER_PARAMS = 9;
+// The layers' launches are a chain (pt_chain_begin): the GEMMs' B operands are weights and, in the backward, activations of the forward, none of
+// which it writes; nor the second operand of the SwiGLU backward.
+struct Chain {
+  Chain() { pt_chain_begin(); }
+  ~Chain() { pt_chain_end(); }
+};
 
 // Matrices that lie back to back in one storage, [rows, cols] together: their address, or nullptr.
 const void* adjacent(const std::vector<Tensor>& ts, size_t first, int count, int64_t rows, int64_t cols) {
@@ -786,6 +794,7 @@ std::vector<Tensor> decoder_stack_fwd(const Tensor& x, const std::vector<Tensor>
   const auto on = x.options();
   std::vector<Tensor> r(1);
   Tensor in = x, s16, s32, free;
+  const Chain chain;
   for (size_t i = 0; i < w.size(); ++i) {
     if (save || i == 0) {
       s16 = torch::empty({at.total}, on);
@@ -973,6 +982,7 @@ Tensor decoder_stack_bwd(const Tensor& dout, const std::vector<Tensor>& xs, cons
   c10::cuda::CUDAGuard guard(dout.device());
   const auto on = dout.options();
   Tensor scratch = torch::empty({LayerScratch(n).total}, on.dtype(at::kByte)), grad = dout;
+  const Chain chain;
   for (size_t i = layers; i-- > 0;) {
     Tensor dx = torch::empty({n.T(), n.H}, on);
     layer_bwd_launches(n, grad.data_ptr(), xs[i].data_ptr(), saved_activations(n, s16[i], s32[i]), w[i], params[i * LAYER_PARAMS + 7],

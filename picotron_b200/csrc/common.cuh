@@ -63,7 +63,7 @@ __device__ __forceinline__ void pdl_enter() {
 
 }  // namespace pt
 
-extern "C" int pt_pdl_enabled();
+extern "C" int pt_pdl_next();
 
 namespace pt {
 
@@ -77,7 +77,7 @@ inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, siz
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = pt_pdl_enabled() ? 1 : 0;
+  attr[0].val.programmaticStreamSerializationAllowed = pt_pdl_next() ? 1 : 0;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
@@ -93,7 +93,7 @@ inline cudaError_t launch_pdl_cluster(void (*kern)(KArgs...), dim3 grid, dim3 bl
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = pt_pdl_enabled() ? 1 : 0;
+  attr[0].val.programmaticStreamSerializationAllowed = pt_pdl_next() ? 1 : 0;
   attr[1].id = cudaLaunchAttributeClusterDimension;
   attr[1].val.clusterDim.x = (unsigned)size;
   attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;

@@ -49,6 +49,7 @@
 #include <type_traits>
 
 extern "C" void pt_count_launches(int n);
+extern "C" int pt_chain_early();
 
 namespace pt {
 namespace gemm_pair {
@@ -80,6 +81,7 @@ struct EpiArgs {
   const float* sinT;
   int seq;                // RoPE: row r is at position r % seq
   int rot_cols;           // RoPE: columns [0, rot_cols) are rotated (rotated heads x d)
+  int early;              // what was written before this chain of launches: B and, of the SwiGLU backward, the second operand (pt_chain_begin)
   int group_m;            // tile numbering: rows of tiles per group (all epilogues)
   // K split into parts (fp32 outputs without a fused epilogue, pt_gemm_bf16_split): k-blocks per part, rows between the slices of
   // the destination, and which slice a part goes to (part >> slice_shift). Unsplit: one part with all k-blocks.
@@ -208,7 +210,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   cluster_arrive();
   cluster_wait();
   tcgen05_fence_after();
-  pdl_wait();                      // the prologue above ran under the predecessor's tail; its results are needed from here on
   const uint32_t tmem_base = bars.tmem_base;
   volatile int* abort_flag = &bars.abort_flag;
 
@@ -218,13 +219,40 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
+      // This CTA's part of B. In a chain the first stages' travel under the predecessor's tail, the rest of the prologue's way: a small GEMM is
+      // little more than the latency of its first loads, and weights come from HBM (forward of the 135M shape on 256 tokens, 120 of them: 1,418 us
+      // a pass without, 1,368 with).
+      auto load_b = [&](int st, int kb, int col0) {
+        const uint32_t full_leader = mapa_u32(smem_u32(&bars.full[st]), 0);
+        if (rank == 0) mbar_expect_tx(&bars.full[st], 2 * LOAD_BYTES);
+        uint8_t* sb = smem_b + st * B_BYTES;
+        if (!B_MN) {
+          tma_load_2d_pair(sb, &tma_b, full_leader, kb * BK, col0);
+        } else {
+#pragma unroll
+          for (int c = 0; c < B_BYTES / (BK * 128); ++c)
+            tma_load_2d_pair(sb + c * (BK * 128), &tma_b, full_leader, col0 + c * 64, kb * BK);
+        }
+      };
+      auto first_col = [&](int n_blk) {              // (SwiGLU: gate rows for the leader, the up rows of the same units for its partner)
+        return (EPI == EPI_SWIGLU) ? n_blk * BN_HALF + (int)rank * ea.inter : n_blk * BN + (int)rank * BN_HALF;
+      };
+      int early = 0;
+      if (ea.early && cluster_id < num_tiles) {
+        int m_blk, n_blk;
+        const int part = PARTS ? cluster_id / tiles : 0;
+        tile_coords(cluster_id - part * tiles, num_m, num_n, ea.group_m, m_blk, n_blk);
+        const int col0 = first_col(n_blk), kb0 = part * kbs;
+        early = min(STAGES, min(num_kb - kb0, kbs));
+        for (int i = 0; i < early; ++i) load_b(i, kb0 + i, col0);
+      }
+      pdl_wait();                    // what the predecessor wrote is needed from here on
       for (int t = cluster_id; t < num_tiles && ok; t += num_clusters) {
         int m_blk, n_blk;
         const int part = PARTS ? t / tiles : 0;
         tile_coords(t - part * tiles, num_m, num_n, ea.group_m, m_blk, n_blk);
         const int row0 = m_blk * 2 * BM + (int)rank * BM;          // this CTA's rows of A
-        // this CTA's columns of B (SwiGLU: gate rows for the leader, the up rows of the same units for its partner)
-        const int col0 = (EPI == EPI_SWIGLU) ? n_blk * BN_HALF + (int)rank * ea.inter : n_blk * BN + (int)rank * BN_HALF;
+        const int col0 = first_col(n_blk);
         const int kb_end = min(num_kb, (part + 1) * kbs);
         for (int kb = part * kbs; kb < kb_end; ++kb) {
           if (!mbar_wait(&bars.empty[stage], phase ^ 1, abort_flag)) {
@@ -232,23 +260,16 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
             ok = false;
             break;
           }
+          if (early > 0) --early;
+          else load_b(stage, kb, col0);
           const uint32_t full_leader = mapa_u32(smem_u32(&bars.full[stage]), 0);
-          if (rank == 0) mbar_expect_tx(&bars.full[stage], 2 * LOAD_BYTES);
           uint8_t* sa = smem_a + stage * A_BYTES;
-          uint8_t* sb = smem_b + stage * B_BYTES;
           if (!A_MN) {
             tma_load_2d_pair(sa, &tma_a, full_leader, kb * BK, row0);
           } else {
 #pragma unroll
             for (int c = 0; c < BM / 64; ++c)
               tma_load_2d_pair(sa + c * (BK * 128), &tma_a, full_leader, row0 + c * 64, kb * BK);
-          }
-          if (!B_MN) {
-            tma_load_2d_pair(sb, &tma_b, full_leader, kb * BK, col0);
-          } else {
-#pragma unroll
-            for (int c = 0; c < B_BYTES / (BK * 128); ++c)
-              tma_load_2d_pair(sb + c * (BK * 128), &tma_b, full_leader, col0 + c * 64, kb * BK);
           }
           if (++stage == STAGES) {
             stage = 0;
@@ -311,6 +332,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     const int quarter = warp & 3;
     bool ok = true;
     int local = 0;
+    if (EPI != EPI_SWIGLU_BWD) pdl_wait();
     if constexpr (EPI == EPI_ADD || EPI == EPI_SWIGLU_BWD) {
       // ---- epilogues with a second operand: chunk c of a tile = 64 accumulator columns of this warp's 32 rows
       constexpr int PER = EPI == EPI_SWIGLU_BWD ? 2 : 1;      // buffers of a chunk: the residual, or (gate, up)
@@ -348,7 +370,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
           load_t += num_clusters;
         }
       };
+      if (EPI == EPI_SWIGLU_BWD && !ea.early) pdl_wait();
       for (int i = 0; i + 1 < SETS; ++i) issue_load();
+      if (EPI == EPI_SWIGLU_BWD && ea.early) pdl_wait();
       int set = 0;
       uint32_t ld_phase = 0;
       for (int t = cluster_id; t < num_tiles && ok; t += num_clusters, ++local) {
@@ -936,6 +960,7 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMa
   const int tiles = ((M + 2 * BM - 1) / (2 * BM)) * n_tiles;
   const int num_kb = (K + BK - 1) / BK;
   ea.group_m = g_group_m;
+  ea.early = pt_chain_early();
   if (ea.kb_per_part <= 0) ea.kb_per_part = num_kb;
   const int units = tiles * ((num_kb + ea.kb_per_part - 1) / ea.kb_per_part);
   const int clusters = units < max_clusters ? units : max_clusters;

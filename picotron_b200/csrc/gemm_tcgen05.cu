@@ -387,6 +387,22 @@ extern "C" int pt_pdl_enabled() {
 }
 extern "C" void pt_set_pdl(int on) { g_pdl = on ? 1 : 0; }
 
+// A chain of launches by this thread on one stream, from pt_chain_begin to pt_chain_end: its first kernel starts when everything before it in the
+// stream is done, so what was written before the chain (weights, saved activations) may be read by all others ahead of griddepcontrol.wait, which
+// orders them only against the kernels of the chain itself. The GEMMs ask (pt_chain_early) and fetch their B operand that soon: callers
+// open a chain only where no B operand is written in it.
+static thread_local int t_chain_head = 0, t_chain = 0;
+extern "C" void pt_chain_begin() { t_chain_head = t_chain = 1; }
+extern "C" void pt_chain_end() { t_chain_head = t_chain = 0; }
+extern "C" int pt_chain_early() { return t_chain; }
+extern "C" int pt_pdl_next() {                     // for the launch that is about to be made
+  if (t_chain_head) {
+    t_chain_head = 0;
+    return 0;
+  }
+  return pt_pdl_enabled();
+}
+
 // Reads and clears the per-device kernel status word. 0 = no kernel reported a timed-out wait.
 extern "C" unsigned int pt_kernel_status_fetch_and_clear() {
   pt::KernelStatus* p = pt::gemm::status_word();

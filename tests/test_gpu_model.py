@@ -203,3 +203,44 @@ def test_layers_in_one_native_call_equal_the_layers_one_by_one(layers, hq, hkv, 
     for x, y in zip(many[1:], each[1:]):
         # (dQ of more than two key blocks and the norm and embedding gradients add in any order: fp32 sums, rounded to bf16 once)
         assert float((x - y).norm()) <= 4e-3 * float(y.norm()) + 1e-12
+
+
+@pytest.mark.parametrize("layers,T", [(1, 64), (4, 64), (4, 700)])
+def test_weights_changed_just_before_a_pass_are_those_it_uses(layers, T):
+    """The layers' GEMMs fetch weights and saved activations ahead of the kernel before them; what an optimizer step or a copy wrote right before
+    the pass has to be seen, and a backward pass reads its own forward's activations: every pass equals the same one layer by layer."""
+    torch.manual_seed(3)
+    cfg = ModelConfig(hidden_size=192, intermediate_size=384, num_hidden_layers=layers, num_attention_heads=3, num_key_value_heads=1,
+                      vocab_size=256, max_position_embeddings=T)
+    model = Llama(cfg, init="normal").to(torch.bfloat16).cuda()
+    wrapped = DataParallelBucket(model)
+    opt = FusedAdamW(wrapped.parameters(), lr=2e-2)
+    ids = torch.randint(0, cfg.vocab_size, (1, T), device="cuda")
+    model(ids, target_ids=ids)                                  # (the layers put their packed weights together)
+    start = [p.detach().clone() for p in model.parameters()]
+
+    def train(hooked):
+        with torch.no_grad():
+            for p, q in zip(model.parameters(), start):
+                p.copy_(q)
+        opt.state.clear()
+        wrapped.reset()
+        handles = [layer.register_forward_pre_hook(lambda *a: None) for layer in model.decoder_layers] if hooked else []
+        out = []
+        for _ in range(4):
+            loss = wrapped(ids, target_ids=ids)
+            loss.backward()
+            out += [loss.detach()] + [p.main_grad.clone() for p in model.decoder_layers[0].attention.parameters()]
+            opt.step()
+            wrapped.reset()
+            with torch.no_grad():
+                out.append(model(ids))                          # logits with the weights of this moment
+        for h in handles:
+            h.remove()
+        return out
+
+    together, single = train(False), train(True)
+    assert float((together[-1] - together[5]).float().norm()) > 0.1 * float(together[5].float().norm()), "the weights hardly moved"
+    for x, y in zip(together, single):
+        # (gradients are summed in any order in places, and AdamW moves weights by what is left of them)
+        assert float((x.float() - y.float()).norm()) <= 3e-2 * float(y.float().norm()) + 1e-12
