@@ -73,6 +73,7 @@ int pt_pdl_enabled();
 void pt_set_pdl(int on);
 void pt_chain_begin();
 void pt_chain_end();
+void pt_next_launch_waits();
 unsigned long long pt_get_wait_limit_ns();
 int pt_gemm_allreduce_bf16(const void* A, const void* B, void* const* buf_ptrs, void* const* flag_ptrs, void* mc_ptr,
                            long long d_offset,
@@ -860,6 +861,57 @@ struct LayerActivations {
   const float *rstd1, *rstd2, *lse;
 };
 
+// A second stream beside the current one. It goes on (`go`) from where the current one was at the last `mark`; `done` notes how far it has got and
+// `join` makes the current stream wait for that (two notes, so that one may be a layer old). One per thread and device (a stream that two threads
+// use could be drawn into the graph capture of either), made at the first use and given back with the thread. The allocator keeps
+// memory that is allocated on it apart.
+struct SideStream {
+  c10::cuda::CUDAStream stream;
+  cudaEvent_t marked, noted[2];
+  void mark(cudaStream_t at) { C10_CUDA_CHECK(cudaEventRecord(marked, at)); }
+  void go() {
+    C10_CUDA_CHECK(cudaStreamWaitEvent(stream, marked, 0));
+    pt_next_launch_waits();
+  }
+  void done(int i) { C10_CUDA_CHECK(cudaEventRecord(noted[i & 1], stream)); }
+  void join(cudaStream_t waits, int i) {
+    C10_CUDA_CHECK(cudaStreamWaitEvent(waits, noted[i & 1], 0));
+    pt_next_launch_waits();
+  }
+};
+// That of the current device, or nullptr where none can be made.
+SideStream* side_stream() {
+  struct Streams {
+    std::vector<std::unique_ptr<SideStream>> of;
+    ~Streams() {
+      for (auto& s : of)
+        if (s) {                                     // (errors: the process may be past its CUDA context)
+          for (cudaEvent_t e : {s->marked, s->noted[0], s->noted[1]}) cudaEventDestroy(e);
+          cudaStreamDestroy(s->stream);
+        }
+    }
+  };
+  static thread_local Streams streams;
+  const int device = c10::cuda::current_device();
+  if ((size_t)device >= streams.of.size()) streams.of.resize(device + 1);
+  auto& s = streams.of[device];
+  if (!s) {
+    cudaStream_t raw = nullptr;
+    cudaEvent_t e[3] = {};
+    bool made = cudaStreamCreateWithFlags(&raw, cudaStreamNonBlocking) == cudaSuccess;
+    for (cudaEvent_t& ev : e) made = made && cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) == cudaSuccess;
+    if (!made) {
+      for (cudaEvent_t ev : e)
+        if (ev != nullptr) cudaEventDestroy(ev);
+      if (raw != nullptr) cudaStreamDestroy(raw);
+      cudaGetLastError();
+      return nullptr;
+    }
+    s.reset(new SideStream{c10::cuda::getStreamFromExternal(raw, (c10::DeviceIndex)device), e[0], {e[1], e[2]}});
+  }
+  return s.get();
+}
+
 // Where a layer's weight gradients are added (fp32).
 struct LayerGrads {
   float *qkv, *o, *gu, *d;
@@ -879,17 +931,18 @@ bool layer_grads(const LayerDims& n, const std::vector<Tensor>& mg, size_t first
   return true;
 }
 
-// Scratch of a layer's backward (bytes): dgu, whose place the attention's gradients take when it is done with; the normed inputs' gradients
-// (dh); dx_mid.
+// Scratch of a layer's backward (bytes): dgu, whose place the attention's gradients take when it is done with, or, beside a second stream that may
+// still read it, not; the normed inputs' gradients (dh); dx_mid.
 struct LayerScratch {
-  int64_t dqkv, dq, delta, dh, dx_mid, total;
-  explicit LayerScratch(const LayerDims& n) {
+  int64_t dO, dqkv, dq, delta, dh, dx_mid, total;
+  LayerScratch(const LayerDims& n, bool two_streams) {
     auto up = [](int64_t bytes) { return (bytes + 255) / 256 * 256; };
-    const int64_t T = n.T(), b_h = up(2 * T * n.H);
-    dqkv = up(2 * T * n.O());
+    const int64_t T = n.T(), b_h = up(2 * T * n.H), b_dgu = up(4 * T * n.I);
+    dO = two_streams ? b_dgu : 0;
+    dqkv = dO + up(2 * T * n.O());
     dq = dqkv + up(2 * T * n.Q());
     delta = dq + up(4 * T * n.O());
-    dh = std::max(up(4 * T * n.I), delta + up(4 * T * n.hq));
+    dh = std::max(b_dgu, delta + up(4 * T * n.hq));
     dx_mid = dh + b_h;
     total = dx_mid + b_h;
   }
@@ -897,16 +950,28 @@ struct LayerScratch {
 
 // The launches of a layer's backward. x: the forward's input; ln1, ln2: the norms' weights; s: LayerScratch bytes.
 void layer_bwd_launches(const LayerDims& n, const void* dout, const void* x, const LayerActivations& acts, const LayerPointers& w, const Tensor& ln1,
-                        const Tensor& ln2, const LayerGrads& g, char* const s, void* dx, double scale, const at::TensorOptions& on) {
-  const LayerScratch at(n);
+                        const Tensor& ln2, const LayerGrads& g, char* const s, void* dx, double scale, const at::TensorOptions& on, SideStream* side = nullptr) {
+  const LayerScratch at(n, side != nullptr);
   const int64_t T = n.T(), H = n.H, I = n.I, O = n.O(), Q = n.Q(), B = n.B, S = n.S, hq = n.hq, hkv = n.hkv, d = n.d;
   const bf16_t *const h1 = acts.h1, *const qkv = acts.qkv, *const o = acts.o, *const x_mid = acts.x_mid, *const h2 = acts.h2,
                *const gu = acts.gu, *const a = acts.a;
-  void *const dgu = s, *const dO = s, *const dq_ws = s + at.dq, *const delta = s + at.delta;
+  void *const dgu = s, *const dO = s + at.dO, *const dq_ws = s + at.dq, *const delta = s + at.delta;
   bf16_t* const dqkv = reinterpret_cast<bf16_t*>(s + at.dqkv);
   void *const dh = s + at.dh, *const dx_mid = s + at.dx_mid;
   const cudaStream_t st = stream();
+  // The weight gradients are nobody's input: on a stream beside the layer's own they fill the SMs that its kernels leave idle. Each is given to the
+  // device after the kernel of the layer that needs the same gradient, so that the layer's goes first.
+  auto mark = [&] {
+    if (side != nullptr) side->mark(st);
+  };
+  auto weight_grad = [&](auto launch) {
+    if (side == nullptr) return launch();
+    side->go();
+    const c10::cuda::CUDAStreamGuard on_side(side->stream);
+    launch();
+  };
 
+  mark();
   if (!(pt_gemm_get_pair() && I % 64 == 0 &&
         fused_gemm(pt_gemm_bf16_fused(dout, w.wd, dgu, (int)T, (int)I, (int)H, H, w.ld_d, 2 * I, 5, const_cast<bf16_t*>(gu), 2 * I,
                                       (int)I, nullptr, nullptr, 0, 0, 0, pt_status_word(), st), "gemm_dgrad_swiglu_bwd"))) {
@@ -914,17 +979,20 @@ void layer_bwd_launches(const LayerDims& n, const void* dout, const void* x, con
     gemm_into(dout, w.wd, da.data_ptr(), T, I, H, H, w.ld_d, I, false, true, 0, on);
     PT_CHECK_RC(pt_swiglu_bwd(gu, da.data_ptr(), dgu, T, (int)I, st), "swiglu_bwd");
   }
-  gemm_into(dout, a, g.d, H, I, T, H, I, I, true, true, 1, on);
+  weight_grad([&] { gemm_into(dout, a, g.d, H, I, T, H, I, I, true, true, 1, on); });
+  mark();
   gemm_into(dgu, w.w_gu, dh, T, H, 2 * I, 2 * I, w.ld_gu, H, false, true, 0, on);
-  gemm_into(dgu, h2, g.gu, 2 * I, H, T, 2 * I, H, H, true, true, 1, on);
+  weight_grad([&] { gemm_into(dgu, h2, g.gu, 2 * I, H, T, 2 * I, H, H, true, true, 1, on); });
   rmsnorm_bwd_into(dh, x_mid, ln2, acts.rstd2, dout, dx_mid, *g.ln2, T, H, on);
+  mark();
   gemm_into(dx_mid, w.wo, dO, T, O, H, H, w.ld_o, O, false, true, 0, on);             // dL/d(attention output)
-  gemm_into(dx_mid, o, g.o, H, O, T, H, O, O, true, true, 1, on);
   PT_CHECK_BWD_RC(pt_attention_bwd_rope(dO, qkv, qkv + O, qkv + O + hkv * d, o, acts.lse, nullptr, reinterpret_cast<float*>(delta),
                                         reinterpret_cast<float*>(dq_ws), dqkv, dqkv + O, dqkv + O + hkv * d, (int)B, (int)S, (int)S, (int)hq,
                                         (int)hkv, (int)d, Q, Q, Q, Q, Q, Q, 1, (float)scale, w.cosp, w.sinp, (int)S, st), "attention_bwd");
+  weight_grad([&] { gemm_into(dx_mid, o, g.o, H, O, T, H, O, O, true, true, 1, on); });
+  mark();
   gemm_into(dqkv, w.w_qkv, dh, T, H, Q, Q, w.ld_qkv, H, false, true, 0, on);
-  gemm_into(dqkv, h1, g.qkv, Q, H, T, Q, H, H, true, true, 1, on);
+  weight_grad([&] { gemm_into(dqkv, h1, g.qkv, Q, H, T, Q, H, H, true, true, 1, on); });
   rmsnorm_bwd_into(dh, x, ln1, acts.rstd1, dx_mid, dx, *g.ln1, T, H, on);
 }
 
@@ -953,7 +1021,7 @@ Tensor layer_bwd(const Tensor& dout, const Tensor& x, SavedBy saved_by, const Te
   const LayerActivations acts = saved_by(n);
   c10::cuda::CUDAGuard guard(x.device());
   const auto on = x.options();
-  Tensor scratch = torch::empty({LayerScratch(n).total}, on.dtype(at::kByte)), dx = torch::empty({n.T(), n.H}, on);
+  Tensor scratch = torch::empty({LayerScratch(n, false).total}, on.dtype(at::kByte)), dx = torch::empty({n.T(), n.H}, on);
   layer_bwd_launches(n, dout.data_ptr(), x.data_ptr(), acts, layer_pointers(ln1, w_qkv, cosT, sinT, wo, ln2, w_gu, wd), ln1, ln2, g,
                      reinterpret_cast<char*>(scratch.data_ptr()), dx.data_ptr(), scale, on);
   return dx;
@@ -981,12 +1049,41 @@ Tensor decoder_stack_bwd(const Tensor& dout, const std::vector<Tensor>& xs, cons
   }
   c10::cuda::CUDAGuard guard(dout.device());
   const auto on = dout.options();
-  Tensor scratch = torch::empty({LayerScratch(n).total}, on.dtype(at::kByte)), grad = dout;
+  // Two streams where a layer keeps the device busier than the host (8 us a layer for the second): at least 12 GFLOP. Measured, us a pass, one / two:
+  // 16 layers of the 135M shape, 3 x 601 tokens 3,307 / 3,099, 8 x 1024 7,957 / 7,669; 5 layers of the 1.7B shape, 2 x 4 x 128 4,679 / 4,416, 15
+  // layers, 4 x 1024 27,443 / 26,777; 4 of the 7B shape 21,094 / 21,083; 2 layers of width 512, 512 tokens 795 / 817.
+  const double gflop = 4e-9 * n.T() * (double)(n.H * (n.Q() + n.O() + 3 * n.I));
+  SideStream* const side = gflop >= 12 ? side_stream() : nullptr;
+  const cudaStream_t st = stream();
+  // The second stream may be a layer behind, so layers take two scratch areas in turn (up to 1 GB for both) and a layer's incoming gradient is kept
+  // for one layer more; a larger one is used again as soon as the second stream is done with it.
+  const int64_t bytes = LayerScratch(n, side != nullptr).total;
+  const bool late = side != nullptr && layers > 1 && bytes <= (512 << 20);
+  Tensor scratch = torch::empty({late ? 2 * bytes : bytes}, on.dtype(at::kByte)), grad = dout, kept[2];
+  struct Joined {                                                        // whatever happens, memory is not given back before it is done with
+    SideStream* side;
+    cudaStream_t st;
+    ~Joined() {
+      if (side == nullptr) return;
+      cudaEventRecord(side->noted[0], side->stream);
+      cudaStreamWaitEvent(st, side->noted[0], 0);
+    }
+  } joined{side, st};
   const Chain chain;
   for (size_t i = layers; i-- > 0;) {
+    if (late && i + 2 < layers) {
+      side->join(st, (int)i);                                            // (what layer i + 2 noted)
+      kept[i & 1] = Tensor();
+    }
     Tensor dx = torch::empty({n.T(), n.H}, on);
     layer_bwd_launches(n, grad.data_ptr(), xs[i].data_ptr(), saved_activations(n, s16[i], s32[i]), w[i], params[i * LAYER_PARAMS + 7],
-                       params[i * LAYER_PARAMS + 8], g[i], reinterpret_cast<char*>(scratch.data_ptr()), dx.data_ptr(), scale, on);
+                       params[i * LAYER_PARAMS + 8], g[i], reinterpret_cast<char*>(scratch.data_ptr()) + (late ? (int64_t)(i & 1) * bytes : 0),
+                       dx.data_ptr(), scale, on, side);
+    if (side != nullptr) {
+      side->done((int)i);
+      if (!late) side->join(st, (int)i);
+      kept[i & 1] = grad;
+    }
     grad = dx;
   }
   return grad;

@@ -395,6 +395,7 @@ static thread_local int t_chain_head = 0, t_chain = 0;
 extern "C" void pt_chain_begin() { t_chain_head = t_chain = 1; }
 extern "C" void pt_chain_end() { t_chain_head = t_chain = 0; }
 extern "C" int pt_chain_early() { return t_chain; }
+extern "C" void pt_next_launch_waits() { t_chain_head = 1; }      // the next launch waits for all before it in its stream (after a join of streams)
 extern "C" int pt_pdl_next() {                     // for the launch that is about to be made
   if (t_chain_head) {
     t_chain_head = 0;

@@ -244,3 +244,89 @@ def test_weights_changed_just_before_a_pass_are_those_it_uses(layers, T):
     for x, y in zip(together, single):
         # (gradients are summed in any order in places, and AdamW moves weights by what is left of them)
         assert float((x.float() - y.float()).norm()) <= 3e-2 * float(y.float().norm()) + 1e-12
+
+
+@pytest.mark.parametrize("layers,inter", [(1, 1024), (2, 1024), (5, 1000)])
+def test_weight_gradients_on_a_second_stream(layers, inter):
+    """Layers large enough that their weight gradients run beside their input gradients (12 GFLOP and more): the gradients of several micro-batches
+    equal those layer by layer, on the default stream, on another one, from two threads at once, with the saved tensors fetched from the
+    host, and from a captured graph that is replayed; memory that is freed right after the pass is not written by it any more."""
+    import threading
+    torch.manual_seed(4)
+    cfg = ModelConfig(hidden_size=512, intermediate_size=inter, num_hidden_layers=layers, num_attention_heads=8, num_key_value_heads=4,
+                      vocab_size=512, max_position_embeddings=1024)
+    B, S = 2, 1024
+
+    def build():
+        torch.manual_seed(5)
+        model = Llama(cfg, init="normal").to(torch.bfloat16).cuda()
+        return DataParallelBucket(model)
+
+    g = torch.Generator(device="cuda").manual_seed(6)
+    batches = [torch.randint(0, cfg.vocab_size, (B, S), device="cuda", generator=g) for _ in range(3)]
+
+    def accumulate(w, context=None):
+        import contextlib
+        w.reset()
+        for i, ids in enumerate(batches):
+            w.require_backward_grad_sync = i == len(batches) - 1
+            with context() if context else contextlib.nullcontext():
+                loss = w(input_ids=ids, target_ids=ids, loss_scale=0.5)
+            loss.backward()
+            # what the pass freed is taken and overwritten at once
+            junk = [torch.full((n,), float("nan"), device="cuda") for n in (1 << 18, 1 << 20, 1 << 22)]
+            del junk, loss
+        return w.bucket_manager.flat
+
+    def close(x, y):
+        # (dQ, the norm weights' and the embedding's gradients add in any order; a rounding of bf16 moved by that moves what follows)
+        assert torch.isfinite(x).all() and float((x - y).norm()) <= 4e-3 * float(y.norm())
+
+    w = build()
+    accumulate(w)
+    handles = [layer.register_forward_pre_hook(lambda *a: None) for layer in w.module.decoder_layers]
+    want = accumulate(w).clone()
+    for h in handles:
+        h.remove()
+    close(accumulate(w), want)
+    close(accumulate(w, torch.autograd.graph.save_on_cpu), want)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        close(accumulate(w), want)
+    torch.cuda.current_stream().wait_stream(side)
+
+    models, errors = [build(), build()], []
+
+    def work(m):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                accumulate(m)
+                torch.cuda.current_stream().synchronize()
+        except Exception as e:                               # noqa: BLE001
+            errors.append(e)
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=(m,)) for m in models]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    for m in models:
+        close(m.bucket_manager.flat, want)
+
+    graph, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        w.require_backward_grad_sync = False
+        w(input_ids=batches[0], target_ids=batches[0], loss_scale=0.5).backward()
+    torch.cuda.current_stream().wait_stream(s)
+    ids = batches[0].clone()
+    with torch.cuda.graph(graph):
+        w(input_ids=ids, target_ids=ids, loss_scale=0.5).backward()
+    w.reset()
+    for b in batches:
+        ids.copy_(b)
+        graph.replay()
+    close(w.bucket_manager.flat, want)
