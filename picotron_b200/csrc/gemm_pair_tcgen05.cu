@@ -57,7 +57,7 @@ namespace gemm_pair {
 constexpr int BM = 128;        // rows of A per CTA (256 per pair)
 constexpr int BK = 64;
 constexpr int UMMA_K = 16;
-constexpr int STAGES = 6;
+constexpr int MAX_STAGES = 8;
 constexpr int A_BYTES = BM * BK * 2;        // 16 KiB
 constexpr int NUM_THREADS = 192;
 constexpr int TMEM_COLS = 512;
@@ -66,13 +66,15 @@ constexpr unsigned KERNEL_ID = 2;
 enum OutMode { OUT_BF16 = 0, OUT_F32_ACC = 1, OUT_F32 = 2 };
 enum Epilogue { EPI_NONE = 0, EPI_SWIGLU = 1, EPI_ROPE64 = 2, EPI_ROPE128 = 3, EPI_ADD = 4, EPI_SWIGLU_BWD = 5, EPI_CE = 6 };
 // operand stages and staging buffers per epilogue warp of each variant (see the smem budget in launch())
-__host__ __device__ constexpr int stages_of(int epi) { return epi == EPI_SWIGLU_BWD ? 5 : 6; }
+// (128-column tiles: as many as fit. They are what GEMMs of few rows run with, whose k-blocks take the latency of a load from HBM divided by the
+// stages. With that and B's prefetch to L2 below the forward pass of the 135M shape on 256 tokens went from 1,368 to 1,298 us.)
+__host__ __device__ constexpr int stages_of(int epi, int bn) { return (bn == 128 ? 8 : 6) - (epi == EPI_SWIGLU_BWD ? (bn == 128 ? 2 : 1) : 0); }
 __host__ __device__ constexpr int staging_bufs_of(int epi) { return epi == EPI_SWIGLU_BWD ? 4 : 2; }
 // a stage holds BM x BK of A and bn / 2 x BK of B; four epilogue warps stage [32 rows][128 B] per buffer
 // (MN-major operands come in boxes of 64 columns: 192-column tiles fetch 128 columns per CTA and use 96)
 __host__ __device__ constexpr int b_bytes_of(int bn) { return (bn / 2 + 63) / 64 * 64 * BK * 2; }
 __host__ __device__ constexpr int smem_bytes_of(int epi, int bn) {
-  return stages_of(epi) * (A_BYTES + b_bytes_of(bn)) + 4 * staging_bufs_of(epi) * 4096 + 1024;
+  return stages_of(epi, bn) * (A_BYTES + b_bytes_of(bn)) + 4 * staging_bufs_of(epi) * 4096 + 1024;
 }
 
 struct EpiArgs {
@@ -97,8 +99,8 @@ struct EpiArgs {
 };
 
 struct Barriers {
-  uint64_t full[STAGES];
-  uint64_t empty[STAGES];
+  uint64_t full[MAX_STAGES];
+  uint64_t empty[MAX_STAGES];
   uint64_t tmem_full[2];
   uint64_t tmem_empty[2];
   uint64_t epi_load[4][2];    // per epilogue warp and set of buffers: the TMA loads of the second operand (ADD / SWIGLU_BWD)
@@ -123,6 +125,10 @@ __device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* m, const vo
                    reinterpret_cast<uint64_t>(m)),
                "r"(smem_u32(smem_src)), "r"(x), "r"(y)
                : "memory");
+}
+// ask for a tile to be brought into L2
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* m, int x, int y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y) : "memory");
 }
 // byte offset of 16-byte unit u of row r in a [rows][128 B] tile stored with the 128-byte swizzle
 __device__ __forceinline__ uint32_t sw128_unit(int r, int u) { return (uint32_t)(r * 128 + ((u ^ (r & 7)) << 4)); }
@@ -159,7 +165,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   constexpr int BN_HALF = BN / 2;                 // columns of B per CTA
   constexpr int B_BYTES = b_bytes_of(BN), STAGE_BYTES = A_BYTES + B_BYTES;
   constexpr int LOAD_BYTES = A_BYTES + (B_MN ? B_BYTES : BN_HALF * BK * 2);      // what the loads of a stage bring
-  constexpr int STAGES = stages_of(EPI);          // shadows the namespace constant: the variants differ in their smem split
+  constexpr int STAGES = stages_of(EPI, BN);
   pdl_launch_dependents();
   extern __shared__ uint8_t smem_raw[];
   __shared__ Barriers bars;
@@ -245,6 +251,16 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         const int col0 = first_col(n_blk), kb0 = part * kbs;
         early = min(STAGES, min(num_kb - kb0, kbs));
         for (int i = 0; i < early; ++i) load_b(i, kb0 + i, col0);
+        // one tile a pair: the rest of its B (of 2,048 rows at most) at least comes to L2
+        if (num_tiles <= num_clusters)
+          for (int kb = kb0 + early; kb < min(num_kb, min(kb0 + kbs, kb0 + 32)); ++kb) {
+            if (!B_MN) {
+              tma_prefetch_2d(&tma_b, kb * BK, col0);
+            } else {
+#pragma unroll
+              for (int c = 0; c < B_BYTES / (BK * 128); ++c) tma_prefetch_2d(&tma_b, col0 + c * 64, kb * BK);
+            }
+          }
       }
       pdl_wait();                    // what the predecessor wrote is needed from here on
       for (int t = cluster_id; t < num_tiles && ok; t += num_clusters) {
