@@ -29,6 +29,10 @@ void pt_gemm_set_group_m(int g);
 void pt_gemm_set_tile_n(int n);
 int pt_gemm_tile_columns(int M, int n_cols, int K, int f32, int b_mn, int has_192);
 int pt_gemm_split_parts(int M, int N, int K, int kind, int* tile_n);
+int pt_gemm_parts(int M, int N, int K, int kind, int add, int* tile_n);
+void pt_gemm_set_cluster(int n);
+int pt_gemm_bf16_cluster(const void* A, const void* B, void* D, int M, int N, int K, long long lda, long long ldb, long long ldd, int b_mn, const void* res,
+                          long long ldr, void* status, cudaStream_t stream);
 long long pt_gemm_split_elems(int M, int N, int K, int kind, int parts);
 void pt_gemm_set_split_k(int on);
 int pt_gemm_bf16_split(const void* A, const void* B, void* D, float* ws, int M, int N, int K, long long lda, long long ldb,
@@ -227,7 +231,13 @@ bool gemm_split_into(const void* a, const void* b, void* d, int64_t M, int64_t N
       (((uintptr_t)a | (uintptr_t)b | (uintptr_t)d | (uintptr_t)res) & 15))
     return false;
   int tile_n = 256;
-  const int parts = pt_gemm_split_parts((int)M, (int)N, (int)K, kind, &tile_n);
+  const int parts = pt_gemm_parts((int)M, (int)N, (int)K, kind, res != nullptr, &tile_n);
+  if (parts < 0) {
+    const int rc = pt_gemm_bf16_cluster(a, b, d, (int)M, (int)N, (int)K, lda, ldb, ldd, kind == 0, res, ldr, pt_status_word(), stream());
+    if (rc == -5) return false;
+    TORCH_CHECK(rc == 0, "gemm (cluster) failed with code ", rc);
+    return true;
+  }
   if (parts <= 1) return false;
   auto ws = torch::empty({pt_gemm_split_elems((int)M, (int)N, (int)K, kind, parts)}, on.dtype(at::kFloat));
   const int rc = pt_gemm_bf16_split(a, b, d, ws.data_ptr<float>(), (int)M, (int)N, (int)K, lda, ldb, ldd, kind, parts, tile_n, res, ldr,
@@ -1329,6 +1339,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
          "calling thread)");
   m.def("set_gemm_split_parts", [](int64_t n) { pt_gemm_set_split_k(n > 1 ? (int)n : 1); },
         "GEMMs that may be split over K are always cut into n parts by this thread (tests, measurements); 0 or 1: the rule.");
+  m.def("set_gemm_cluster", [](int64_t n) { pt_gemm_set_cluster((int)n); },
+        "GEMMs X W^T (+ residual) and dY W share K between the pairs of a cluster: 0 by the rule, 1 never, 2 wherever it can be (this thread).");
   m.def("gemm_plan", [](const std::string& kind, int64_t M, int64_t N, int64_t K) {
           const int splits = kind == "dgrad" ? 0 : kind == "wgrad" ? 1 : kind == "fwd" || kind == "add" ? 2 : -1;
           TORCH_CHECK(splits >= 0 || kind == "rope" || kind == "swiglu" || kind == "swiglu_bwd", "gemm_plan: ", kind);

@@ -818,6 +818,232 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   }
 }
 
+// GEMM whose K is shared by the two CTA pairs of one cluster: each sums its half of K for a 256 x 128 tile in tensor memory, sends the 64 columns
+// that are the other's through distributed shared memory (fp32, in the place of the operand stages), adds what it is sent to its own 64 and
+// stores these (with the residual). One tile per cluster.
+// What it is for: few output tiles, where a tile's k-blocks, one after the other, are all that the time consists of. The same split through an
+// fp32 workspace costs two launches more (clearing, summing) and two passes over the slices. Measured whole or through a workspace / this way (us,
+// operands not in L2): with residual 256 x 960 x 2560: 17.4 / 14.4; 512 x 2048 x 8192: 29.7 / 26.7; input gradient 256 x 2048 x 3072: 19.5 / 16.4;
+// 384 x 2048 x 6144: 27.7 / 22.4. Clusters of four pairs and tiles of 256 columns were slower at all but one of 240 shapes (512 x 2048 x 8192: 45.1, 34.7).
+struct ClusterArgs {
+  int kb_per_part, num_m, early;
+};
+struct ClusterBarriers {
+  uint64_t full[MAX_STAGES];
+  uint64_t empty[MAX_STAGES];
+  uint64_t tmem_full;
+  uint64_t epi_load[4];
+  uint32_t tmem_base;
+  int abort_flag;
+};
+constexpr int CLUSTER_BN = 128, CLUSTER_PARTS = 2;
+
+template <bool B_MN, bool ADD>
+__global__ void __launch_bounds__(NUM_THREADS, 1)
+gemm_cluster_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b, const __grid_constant__ CUtensorMap tma_d,
+                    const __grid_constant__ CUtensorMap tma_h, int M, int N, int K, KernelStatus* status, ClusterArgs ca) {
+  constexpr int BN = CLUSTER_BN, BN_HALF = BN / 2, B_BYTES = b_bytes_of(BN), STAGE_BYTES = A_BYTES + B_BYTES, STAGES = stages_of(EPI_NONE, BN);
+  constexpr int LOAD_BYTES = A_BYTES + (B_MN ? B_BYTES : BN_HALF * BK * 2);
+  pdl_launch_dependents();
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ ClusterBarriers bars;
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem_a = smem;
+  uint8_t* smem_b = smem + STAGES * A_BYTES;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const uint32_t crank = cluster_ctarank(), pair = crank >> 1, rank = crank & 1, leader = crank & ~1u;
+  const int tile = (int)(blockIdx.x / (2 * CLUSTER_PARTS)), m_blk = tile % ca.num_m, n_blk = tile / ca.num_m;
+  const int num_kb = (K + BK - 1) / BK, kb0 = (int)pair * ca.kb_per_part, kbs = min(num_kb - kb0, ca.kb_per_part);
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(&bars.full[s], 1);
+      mbar_init(&bars.empty[s], 1);
+    }
+    mbar_init(&bars.tmem_full, 1);
+    for (int q = 0; q < 4; ++q) mbar_init(&bars.epi_load[q], 1);
+    bars.abort_flag = 0;
+    fence_barrier_init();
+    fence_proxy_async_smem();
+    tma_prefetch_desc(&tma_a);
+    tma_prefetch_desc(&tma_b);
+    tma_prefetch_desc(&tma_d);
+    if (ADD) tma_prefetch_desc(&tma_h);
+  }
+  if (warp == 1) {
+    tmem_alloc_pair(&bars.tmem_base, BN);
+    tmem_relinquish_pair();
+  }
+  tcgen05_fence_before();
+  __syncthreads();
+  cluster_arrive();
+  cluster_wait();
+  tcgen05_fence_after();
+  const uint32_t tmem_base = bars.tmem_base;
+  volatile int* abort_flag = &bars.abort_flag;
+  const int quarter = warp & 3;
+  const int row0 = m_blk * 2 * BM + (int)rank * BM + quarter * 32;
+  const uint32_t t_row = tmem_base + (uint32_t(quarter * 32) << 16);
+  uint8_t* const stg = smem + STAGES * STAGE_BYTES + quarter * 4096;
+  const int own0 = n_blk * BN + (int)pair * 64, other0 = n_blk * BN + (int)(pair ^ 1) * 64;      // columns this pair stores; those it sends
+  bool ok = true;
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ TMA producer (B ahead of the predecessor as in gemm_pair_kernel)
+    if (elect_one()) {
+      const int arow0 = m_blk * 2 * BM + (int)rank * BM, col0 = n_blk * BN + (int)rank * BN_HALF;
+      auto load_b = [&](int st, int kb) {
+        const uint32_t full_leader = mapa_u32(smem_u32(&bars.full[st]), leader);
+        if (rank == 0) mbar_expect_tx(&bars.full[st], 2 * LOAD_BYTES);
+        uint8_t* sb = smem_b + st * B_BYTES;
+        if (!B_MN) {
+          tma_load_2d_pair(sb, &tma_b, full_leader, kb * BK, col0);
+        } else {
+#pragma unroll
+          for (int c = 0; c < B_BYTES / (BK * 128); ++c)
+            tma_load_2d_pair(sb + c * (BK * 128), &tma_b, full_leader, col0 + c * 64, kb * BK);
+        }
+      };
+      const int early = ca.early ? min(STAGES, kbs) : 0;
+      for (int i = 0; i < early; ++i) load_b(i, kb0 + i);
+      pdl_wait();
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int i = 0; i < kbs; ++i) {
+        if (!mbar_wait(&bars.empty[stage], phase ^ 1, abort_flag)) {
+          report_error(status, KERNEL_ID, 11);
+          break;
+        }
+        if (i >= early) load_b(stage, kb0 + i);
+        tma_load_2d_pair(smem_a + stage * A_BYTES, &tma_a, mapa_u32(smem_u32(&bars.full[stage]), leader), (kb0 + i) * BK, arow0);
+        if (++stage == STAGES) {
+          stage = 0;
+          phase ^= 1;
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer (leader CTA of each pair)
+    if (rank == 0 && elect_one()) {
+      constexpr uint32_t idesc = make_idesc_bf16(2 * BM, BN, false, B_MN);
+      const uint64_t a_base = make_smem_desc_sw128(smem_u32(smem_a), 16, 1024);
+      const uint64_t b_base = make_smem_desc_sw128(smem_u32(smem_b), B_MN ? BK * 128 : 16, 1024);
+      int stage = 0;
+      uint32_t phase = 0;
+      bool fine = true;
+      for (int i = 0; i < kbs; ++i) {
+        if (!mbar_wait(&bars.full[stage], phase, abort_flag)) {
+          report_error(status, KERNEL_ID, 13);
+          fine = false;
+          break;
+        }
+        tcgen05_fence_after();
+        const uint64_t a_st = smem_desc_advance(a_base, stage * A_BYTES), b_st = smem_desc_advance(b_base, stage * B_BYTES);
+#pragma unroll
+        for (int k = 0; k < BK / UMMA_K; ++k)
+          umma_bf16_pair(tmem_base, smem_desc_advance(a_st, k * UMMA_K * 2), smem_desc_advance(b_st, k * UMMA_K * (B_MN ? 128 : 2)), idesc,
+                         (i > 0 || k > 0) ? 1u : 0u);
+        const uint32_t e = smem_u32(&bars.empty[stage]);
+        umma_commit_pair(mapa_u32(e, leader));
+        umma_commit_pair(mapa_u32(e, leader + 1));
+        if (++stage == STAGES) {
+          stage = 0;
+          phase ^= 1;
+        }
+      }
+      if (fine) {
+        const uint32_t f = smem_u32(&bars.tmem_full);
+        umma_commit_pair(mapa_u32(f, leader));
+        umma_commit_pair(mapa_u32(f, leader + 1));
+      }
+    }
+  } else {
+    pdl_wait();
+    if (ADD && own0 < N && row0 < M && elect_one()) {
+      mbar_expect_tx(&bars.epi_load[quarter], 4096);
+      tma_load_2d(stg, &tma_h, &bars.epi_load[quarter], own0, row0);
+    }
+    if (!mbar_wait(&bars.tmem_full, 0, abort_flag)) {
+      if (lane == 0) report_error(status, KERNEL_ID, 14);
+      ok = false;
+    }
+    tcgen05_fence_after();
+  }
+  // All MMAs of the cluster are done: the stages may take the sums.
+  __syncwarp();
+  cluster_arrive();
+  cluster_wait();
+  if (warp >= 2 && ok && other0 < N) {
+    uint32_t v[64];
+    tmem_ld_32x32b_x32_at(t_row + (pair ^ 1) * 64, v, 0);
+    tmem_ld_32x32b_x32_at(t_row + (pair ^ 1) * 64 + 32, v, 32);
+    tmem_ld_wait();
+    // [16 quads of columns][128 rows][4 floats]
+    const uint32_t to = mapa_u32(smem_u32(smem), (pair ^ 1) * 2 + rank) + (quarter * 32 + lane) * 16;
+#pragma unroll
+    for (int u = 0; u < 16; ++u)
+      asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(to + u * 2048), "r"(v[4 * u]), "r"(v[4 * u + 1]), "r"(v[4 * u + 2]),
+                   "r"(v[4 * u + 3])
+                   : "memory");
+  }
+  uint32_t v[64];
+  if (warp >= 2 && ok) {                       // its own columns, while the others' are on the way
+    tmem_ld_32x32b_x32_at(t_row + pair * 64, v, 0);
+    tmem_ld_32x32b_x32_at(t_row + pair * 64 + 32, v, 32);
+    tmem_ld_wait();
+  }
+  __syncwarp();
+  cluster_arrive();
+  cluster_wait();
+  if (ADD && warp >= 2 && ok && own0 < N && row0 < M && !mbar_wait(&bars.epi_load[quarter], 0, abort_flag)) {
+    if (lane == 0) report_error(status, KERNEL_ID, 15);
+    ok = false;
+  }
+  if (warp >= 2 && ok && own0 < N && row0 < M) {
+    const float4* sent = reinterpret_cast<const float4*>(smem) + quarter * 32 + lane;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      uint4* const at = reinterpret_cast<uint4*>(stg + sw128_unit(lane, u));
+      const uint4 r = ADD ? *at : make_uint4(0, 0, 0, 0);
+      const uint32_t res[4] = {r.x, r.y, r.z, r.w};
+      const float4 lo = sent[2 * u * 128], hi = sent[(2 * u + 1) * 128];
+      const float add[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+      uint32_t w[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        float a = __uint_as_float(v[8 * u + 2 * e]) + add[2 * e], b = __uint_as_float(v[8 * u + 2 * e + 1]) + add[2 * e + 1];
+        if (ADD) {
+          const float2 h = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&res[e]));
+          a += h.x;
+          b += h.y;
+        }
+        w[e] = pack_bf16(a, b);
+      }
+      *at = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (elect_one()) {
+      tma_store_2d(&tma_d, stg, own0, row0);
+      tma_store_commit();
+      tma_store_wait<0>();
+    }
+  }
+
+  tcgen05_fence_before();
+  __syncthreads();
+  if (*abort_flag) {
+    for (int i = 0; i < 2000; ++i) __nanosleep(1000);
+    __syncthreads();
+  }
+  cluster_arrive();
+  cluster_wait();
+  if (warp == 1) {
+    tcgen05_fence_after();
+    tmem_dealloc_pair(tmem_base, BN);
+  }
+}
+
 static int g_group_m = 8;   // rows of 256-row tiles per group; measured on the model's shapes: 8 and 16 beat 4 by ~1 %, 1 is worst
 
 // K-split GEMMs keep their parts in slices of an fp32 workspace: cleared before where two parts add to a slice, summed after in the
@@ -1031,14 +1257,99 @@ extern "C" int pt_gemm_tile_columns(int M, int n_cols, int K, int f32, int b_mn,
   return pt::gemm_pair::tile_columns(M, n_cols, K, f32 != 0, b_mn != 0, has_192 != 0);
 }
 
+// Thread's switch for K shared within clusters: 0 by the rule, 1 never, 2 wherever it can be.
+static thread_local int g_cluster = 0;
+extern "C" void pt_gemm_set_cluster(int n) { g_cluster = n == 1 || n == 2 ? n : 0; }
+
+namespace pt {
+namespace gemm_pair {
+template <bool B_MN, bool ADD>
+static int clusters_that_fit() {
+  static PerDevice fit;
+  return fit.get(current_device(), [] {
+    auto kern = gemm_cluster_kernel<B_MN, ADD>;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes_of(EPI_NONE, CLUSTER_BN)) != cudaSuccess) return -3;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * CLUSTER_PARTS, 1, 1);
+    cfg.blockDim = dim3(NUM_THREADS, 1, 1);
+    cfg.dynamicSmemBytes = smem_bytes_of(EPI_NONE, CLUSTER_BN);
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 2 * CLUSTER_PARTS;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
+      cudaGetLastError();
+      return -5;
+    }
+    return n;
+  });
+}
+template <typename F>
+static int with_cluster_kernel(bool b_mn, bool add, F f) {
+  return b_mn ? f(std::true_type{}, std::false_type{}) : add ? f(std::false_type{}, std::true_type{}) : f(std::false_type{}, std::false_type{});
+}
+}  // namespace gemm_pair
+}  // namespace pt
+
+// Whether K is shared within clusters: where one wave of them holds all tiles and gemm_us, with 0.8 us for the exchange, promises 5 % less than
+// `others_us`, what the GEMM takes whole or through a workspace, from K = 1536 on, with a residual (which comes in while the tensor cores work) from
+// 896. Below, the exchange costs what half of K takes: input gradient 1024 x 576 x 960: 12.3 us whole and this way; with residual 256 x 576 x 576 12.4
+// and 12.4, 256 x 960 x 960 14.3 and 12.3. Input gradients with K above 8192 stay with the workspace, whose parts can be many: 64 x 576 x 49152
+// has 5 tiles for 74 pairs, here 10 of them would work; what clusters gain is 4 to 7 % by then (512 x 2048 x 16384: 44.0 / 41.0). Of 240 shapes
+// (32 to 4,096 tokens; output projections and input gradients of the widths of a 20M to a 7B model) 108 go this way, 11 % faster.
+static bool shares_k_in_clusters(int M, int N, int K, bool b_mn, bool add, double others_us) {
+  using namespace pt::gemm_pair;
+  if (g_cluster == 1 || (g_tile_n && g_cluster != 2)) return false;
+  const GemmShape g(M, N, K);
+  const int kb_part = (g.kb + CLUSTER_PARTS - 1) / CLUSTER_PARTS;
+  if (g.kb < CLUSTER_PARTS) return false;
+  if (g_cluster != 2 && (K < (add ? 896 : 1536) || (b_mn && K > 8192))) return false;
+  if (g_cluster != 2 && gemm_us(g, CLUSTER_BN, 1, CLUSTER_PARTS, kb_part, false) + 0.8 >= 0.95 * others_us) return false;
+  const int fit = with_cluster_kernel(b_mn, add, [](auto b, auto a) { return clusters_that_fit<b(), a()>(); });
+  return fit > 0 && (g.tiles(CLUSTER_BN) <= fit || g_cluster == 2);
+}
+
+// D = A B (b_mn) or A B^T (+ res, bf16 [M, N], row stride ldr % 8 == 0, or nullptr) with K shared by the pairs of a cluster; N % 8 == 0, K > 64.
+extern "C" int pt_gemm_bf16_cluster(const void* A, const void* B, void* D, int M, int N, int K, long long lda, long long ldb, long long ldd, int b_mn,
+                                    const void* res, long long ldr, void* status, cudaStream_t stream) {
+  using namespace pt;
+  using namespace pt::gemm_pair;
+  CUtensorMap ma, mb, md, mh;
+  int rc;
+  if ((rc = make_bf16_map_2d(&ma, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda, BK, BM))) return rc * 10 - 1;
+  if ((rc = b_mn ? make_bf16_map_2d(&mb, B, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, 64, BK)
+                 : make_bf16_map_2d(&mb, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, BK, CLUSTER_BN / 2)))
+    return rc * 10 - 2;
+  if ((rc = make_bf16_map_2d(&md, D, (uint64_t)N, (uint64_t)M, (uint64_t)ldd, 64, 32))) return rc * 10 - 3;
+  mh = md;
+  if (res != nullptr && (rc = make_bf16_map_2d(&mh, res, (uint64_t)N, (uint64_t)M, (uint64_t)ldr, 64, 32))) return rc * 10 - 4;
+  ClusterArgs ca;
+  ca.kb_per_part = ((K + BK - 1) / BK + CLUSTER_PARTS - 1) / CLUSTER_PARTS;
+  ca.num_m = (M + 2 * BM - 1) / (2 * BM);
+  ca.early = pt_chain_early();
+  const int grid = ca.num_m * ((N + CLUSTER_BN - 1) / CLUSTER_BN) * 2 * CLUSTER_PARTS;
+  return with_cluster_kernel(b_mn != 0, res != nullptr, [&](auto b, auto a) {
+    if (clusters_that_fit<b(), a()>() <= 0) return -5;
+    const cudaError_t err = launch_pdl_cluster(gemm_cluster_kernel<b(), a()>, dim3(grid), dim3(NUM_THREADS), smem_bytes_of(EPI_NONE, CLUSTER_BN), stream,
+                                               2 * CLUSTER_PARTS, ma, mb, md, mh, M, N, K, reinterpret_cast<KernelStatus*>(status), ca);
+    pt_count_launches(1);
+    return err == cudaSuccess && cudaGetLastError() == cudaSuccess ? 0 : -4;
+  });
+}
+
 // How many parts K is split into (1: not at all) and the columns of a tile then, by gemm_us and gain_asked; adding the weight gradient to what is
 // there costs 0.08 us a megabyte more in the GEMM's epilogue than in the summing kernel; an input gradient clears its slices first. A
 // split has to give 3 %, or 15 % (2048 x 2048 x 128256 on 64 whole tiles: 724 us, in parts 760), and a forward GEMM 2 us more: its second
 // launch costs the host 3.5, and passes of small forward GEMMs are bound by the host (256 x 576 x 1536 is 8.7 us whole and 7.6 in five
 // parts; the forward pass of the 135M shape on 256 tokens, with 30 of them, took 1,590 us with whole ones and 1,740 with parts).
-extern "C" int pt_gemm_split_parts(int M, int N, int K, int kind, int* tile_n) {
+// (`us`: what the choice is expected to take, the host's extra included)
+static int split_parts(int M, int N, int K, int kind, int* tile_n, double* us) {
   using namespace pt::gemm_pair;
   *tile_n = g_tile_n ? g_tile_n : 256;
+  *us = 0;
   const bool wgrad = kind == SPLIT_WGRAD, b_mn = kind != SPLIT_FWD;
   if (M <= 0 || N <= 0 || K <= 0 || !g_split_k || (!wgrad && N % 8)) return 1;
   const GemmShape g(M, N, K);
@@ -1047,6 +1358,7 @@ extern "C" int pt_gemm_split_parts(int M, int N, int K, int kind, int* tile_n) {
   // (where whole tiles fill more than half of the pairs, what is left to gain is less than what parts at different K cost in L2 reuse)
   const bool few = 2 * g.tiles(256) <= num_pairs();
   const double whole = whole_us(g, tile_columns(M, N, K, wgrad, b_mn, true), wgrad, b_mn) + (wgrad ? 0.08 * g.mbytes32() : 0.0);
+  *us = whole;
   double best = 1e30, best_us = 0;
   int best_parts = 1, best_bn = 256;
   for (const int asked : {2, 3, 4, 5, 6, 8, 10, 12, 16, 20, 24, 32}) {
@@ -1066,7 +1378,20 @@ extern "C" int pt_gemm_split_parts(int M, int N, int K, int kind, int* tile_n) {
   const double split = best_us + (kind == SPLIT_DGRAD ? 2.0 : 0.0);
   if (split >= (few ? 0.97 : 0.85) * whole - (kind == SPLIT_FWD ? 2.0 : 0.0)) return 1;
   *tile_n = best_bn;
+  *us = split + (kind == SPLIT_FWD ? 2.0 : 0.0);
   return best_parts;
+}
+extern "C" int pt_gemm_split_parts(int M, int N, int K, int kind, int* tile_n) {
+  double us;
+  return split_parts(M, N, K, kind, tile_n, &us);
+}
+// The same, or -1: K shared within clusters (pt_gemm_bf16_cluster).
+extern "C" int pt_gemm_parts(int M, int N, int K, int kind, int add, int* tile_n) {
+  using namespace pt::gemm_pair;
+  double us;
+  const int parts = split_parts(M, N, K, kind, tile_n, &us);
+  if (kind == SPLIT_WGRAD || M <= 0 || N <= 0 || K <= 0 || N % 8 || !g_split_k || g_split_k > 1) return parts;
+  return shares_k_in_clusters(M, N, K, kind == SPLIT_DGRAD, add != 0, us) ? -1 : parts;
 }
 
 // Floats of workspace for pt_gemm_bf16_split with `parts` parts.

@@ -156,6 +156,40 @@ def test_gemm_tile_widths_and_parts_of_every_layout(tile_n, parts, M, N, K):
     assert _rel(acc.double() - 0.5, xt.double().t() @ wt.double()) < 1e-5
 
 
+@pytest.mark.parametrize("M,N,K", [(8, 8, 72), (264, 520, 448), (600, 584, 1000), (256, 64, 512), (1000, 136, 640), (225, 200, 1480), (512, 2048, 8192)])
+def test_gemm_with_k_shared_in_clusters(C, M, N, K):
+    """Two CTA pairs per tile, each half of K: tiles beyond the matrix, second halves of a tile with no column or eight, an odd number of
+    k-blocks, a last one of 8 rows; output and residual are rows of wider tensors, whose other columns stay as they were."""
+    C.set_gemm_pair(True)
+    C.set_gemm_tma_epilogue(True)
+    x, w, wt, wide = bf(M, K, seed=1), bf(N, K, seed=2), bf(K, N, seed=3), bf(M, N + 16, seed=4)
+    res = wide[:, 8:8 + N]
+    runs = []
+    try:
+        C.set_gemm_cluster(2)
+        for _ in range(3):
+            big = torch.full((M, N + 16), 3.0, device="cuda", dtype=torch.bfloat16)
+            n0 = C.launch_count()
+            C.gemm(x, wt, False, True, big[:, 8:8 + N], False)
+            runs.append([C.gemm(x, w, False, False), C.gemm_add(x, w, res), big])
+            assert C.launch_count() - n0 == 3
+        C.set_gemm_cluster(1)
+        C.set_gemm_split_dgrad(False)
+        whole = [C.gemm(x, w, False, False), C.gemm_add(x, w, res), C.gemm(x, wt, False, True)]
+    finally:
+        C.set_gemm_cluster(0)
+        C.set_gemm_split_dgrad(True)
+    _status_ok(C)
+    for run in runs[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(run, runs[0]))
+    got = runs[0][:2] + [runs[0][2][:, 8:8 + N]]
+    assert bool((runs[0][2][:, :8] == 3).all()) and bool((runs[0][2][:, 8 + N:] == 3).all())
+    y = x.double() @ w.double().t()
+    for g, one, want in zip(got, whole, [y, y + res.double(), x.double() @ wt.double()]):
+        # one bf16 rounding of the result (2^-9 of each value at most); the sums' order changes it for those at the edge of a rounding only
+        assert _rel(g.double(), want) < 2.5e-3 and _rel(g.double(), want) < 1.01 * _rel(one.double(), want) + 1e-5
+
+
 def test_gemm_over_nothing_is_zero(C):
     """The weight gradient of an empty batch: zeros, or what the destination holds where it is added to."""
     dy, x = bf(0, 72), bf(0, 136)
