@@ -1350,7 +1350,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                                                        splits >= 0 || kind == "swiglu_bwd");
           return std::pair<int64_t, int64_t>(tile_n, parts);
         }, "(columns of a tile, parts of K) that the rule gives a GEMM with output [M, N]: kind fwd, add, dgrad, wgrad, rope, swiglu (N = 2I) or\n"
-           "swiglu_bwd (N = I).");
+           "swiglu_bwd (N = I). Where K is shared within clusters instead (set_gemm_cluster), what it would be without.");
   m.def("set_gemm_tile_n", [](int64_t n) { pt_gemm_set_tile_n((int)n); },
         "columns of the GEMM output tiles: 128, 192 (where the epilogue has it), 256, or 0 for the choice by shape (for the calling thread). "
          "With a given width K is not split, unless set_gemm_split_parts says so.");

@@ -1344,7 +1344,8 @@ extern "C" int pt_gemm_bf16_cluster(const void* A, const void* B, void* D, int M
 // there costs 0.08 us a megabyte more in the GEMM's epilogue than in the summing kernel; an input gradient clears its slices first. A
 // split has to give 3 %, or 15 % (2048 x 2048 x 128256 on 64 whole tiles: 724 us, in parts 760), and a forward GEMM 2 us more: its second
 // launch costs the host 3.5, and passes of small forward GEMMs are bound by the host (256 x 576 x 1536 is 8.7 us whole and 7.6 in five
-// parts; the forward pass of the 135M shape on 256 tokens, with 30 of them, took 1,590 us with whole ones and 1,740 with parts).
+// parts; the forward pass of the 135M shape on 256 tokens, with 30 of them, took 1,590 us with whole ones and 1,740 with parts; these share K
+// within clusters by now, pt_gemm_parts).
 // (`us`: what the choice is expected to take, the host's extra included)
 static int split_parts(int M, int N, int K, int kind, int* tile_n, double* us) {
   using namespace pt::gemm_pair;
