@@ -1061,7 +1061,9 @@ Tensor decoder_stack_bwd(const Tensor& dout, const std::vector<Tensor>& xs, cons
   const auto on = dout.options();
   // Two streams where a layer keeps the device busier than the host (8 us a layer for the second): at least 12 GFLOP. Measured, us a pass, one / two:
   // 16 layers of the 135M shape, 3 x 601 tokens 3,307 / 3,099, 8 x 1024 7,957 / 7,669; 5 layers of the 1.7B shape, 2 x 4 x 128 4,679 / 4,416, 15
-  // layers, 4 x 1024 27,443 / 26,777; 4 of the 7B shape 21,094 / 21,083; 2 layers of width 512, 512 tokens 795 / 817.
+  // layers, 4 x 1024 27,443 / 26,777; 4 of the 7B shape 20,582 / 19,865; 3 of the 8B shape, 8192 tokens 52,643 / 52,411 and 53,161 / 53,033; 4 of the 1B
+  // shape, 32768 tokens 164,779 / 166,354 and 164,911 / 162,793 (no difference beyond what the power cap does from run to run); 2 layers of width 512,
+  // 512 tokens 795 / 817.
   const double gflop = 4e-9 * n.T() * (double)(n.H * (n.Q() + n.O() + 3 * n.I));
   SideStream* const side = gflop >= 12 ? side_stream() : nullptr;
   const cudaStream_t st = stream();
