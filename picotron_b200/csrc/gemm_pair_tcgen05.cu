@@ -448,9 +448,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                 const float2 g = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w0[e]));
                 const float2 up = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w1[e]));
                 const uint64_t g2 = pair_of(g.x, g.y), one = pair_of(1.f, 1.f), sg = sigmoid2(g2);
-                const uint64_t das = mul2(pair_of(__uint_as_float(v[8 * u + 2 * e]), __uint_as_float(v[8 * u + 2 * e + 1])), sg);
+                const uint64_t da = pair_of(__uint_as_float(v[8 * u + 2 * e]), __uint_as_float(v[8 * u + 2 * e + 1]));
                 const uint64_t slope = fma2(g2, fma2(sg, pair_of(-1.f, -1.f), one), one);              // 1 + g (1 - s)
-                const uint64_t dg = mul2(mul2(das, pair_of(up.x, up.y)), slope), du = mul2(das, g2);
+                // (da s in common would save a product, 0 to 1.5 %, 4096 x 2560 x 960 40.7 -> 40.0 us, but where s is next to the smallest
+                // normal number it flushes to zero what `up` or the gate would have brought back)
+                const uint64_t dg = mul2(mul2(da, pair_of(up.x, up.y)), mul2(sg, slope)), du = mul2(mul2(da, g2), sg);
                 w0[e] = pack_bf16(lo_of(dg), hi_of(dg));
                 w1[e] = pack_bf16(lo_of(du), hi_of(du));
               }

@@ -379,6 +379,27 @@ def test_dgrad_gemm_with_swiglu_backward_epilogue(T, I, H):
     assert C.gemm_dgrad_swiglu_bwd(dy, bf(H, 72, seed=54), bf(T, 144, seed=55)) is None      # I % 64 != 0: not covered
 
 
+@pytest.mark.parametrize("up,da", [(64.0, 2.0 ** -7), (2.0 ** -7, 64.0), (1.0, 2.0 ** -9)])
+def test_gemm_with_swiglu_backward_epilogue_of_very_negative_gates(up, da):
+    """Gates whose sigmoid is next to the smallest normal number, and the same ones positive: what `up`, the gate and the gradient make of
+    it is a normal number again and no zero. Rows of one 1 make the GEMM's result the weight itself."""
+    from picotron_b200.ops import _ext
+    C = _ext.load()
+    C.set_gemm_pair(True)
+    C.set_gemm_tma_epilogue(True)
+    T, I = 256, 64
+    g = torch.linspace(-87.0, 87.0, T * I, device="cuda").view(T, I).to(torch.bfloat16)
+    gu = torch.cat([g, torch.full_like(g, up)], 1).contiguous()
+    got = C.gemm_dgrad_swiglu_bwd(torch.eye(T, device="cuda", dtype=torch.bfloat16), torch.full((T, I), da, device="cuda", dtype=torch.bfloat16), gu)
+    _status_ok(C)
+    g = g.double()
+    s = torch.sigmoid(g)
+    want = torch.cat([da * up * s * (1 + g * (1 - s)), da * g * s], 1)
+    # bf16's rounding, and that of the exponential's argument (126 at most: 2^-18 of it, times ln 2) with a few more of 2^-24; what is below
+    # the smallest normal number may be zero
+    assert bool(((got.double() - want).abs() <= (2.0 ** -8) * want.abs() + 2.0 ** -126).all())
+
+
 @pytest.mark.parametrize("B,S,hq,hkv,d,K", [(2, 128, 4, 2, 64, 256), (1, 200, 3, 1, 64, 192), (2, 128, 4, 2, 128, 256),
                                             (4, 1024, 32, 32, 64, 512), (1, 96, 5, 5, 128, 128)])
 def test_gemm_with_rope_epilogue(B, S, hq, hkv, d, K):
