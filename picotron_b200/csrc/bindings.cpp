@@ -872,9 +872,8 @@ struct LayerActivations {
 };
 
 // A second stream beside the current one. It goes on (`go`) from where the current one was at the last `mark`; `done` notes how far it has got and
-// `join` makes the current stream wait for that (two notes, so that one may be a layer old). One per thread and device (a stream that two threads
-// use could be drawn into the graph capture of either), made at the first use and given back with the thread. The allocator keeps
-// memory that is allocated on it apart.
+// `join` makes the current stream wait for that (two notes, so that one may be a layer old). The allocator keeps memory that is allocated on it
+// apart.
 struct SideStream {
   c10::cuda::CUDAStream stream;
   cudaEvent_t marked, noted[2];
@@ -889,23 +888,40 @@ struct SideStream {
     pt_next_launch_waits();
   }
 };
-// That of the current device, or nullptr where none can be made.
-SideStream* side_stream() {
+// The one beside `current` on its device (the current one), or nullptr where there is none. A thread has up to four a device, for the streams that it used last,
+// made at the first use and given back with the thread. (Autograd runs the backward passes of all threads on one thread a device: one side stream
+// for all of them would put the weight gradients of one caller behind those of another.) One that is part of a graph capture other than the current
+// stream's is left alone: to make it wait for work outside of its capture is an error and ends that capture.
+SideStream* side_stream(cudaStream_t current) {
   struct Streams {
-    std::vector<std::unique_ptr<SideStream>> of;
+    struct Slot {
+      cudaStream_t beside = nullptr;
+      uint64_t used = 0;
+      std::unique_ptr<SideStream> side;
+    } slots[4];
     ~Streams() {
-      for (auto& s : of)
-        if (s) {                                     // (errors: the process may be past its CUDA context)
+      for (auto& slot : slots)
+        if (SideStream* s = slot.side.get()) {       // (errors: the process may be past its CUDA context)
           for (cudaEvent_t e : {s->marked, s->noted[0], s->noted[1]}) cudaEventDestroy(e);
           cudaStreamDestroy(s->stream);
         }
     }
   };
-  static thread_local Streams streams;
+  static thread_local std::vector<std::unique_ptr<Streams>> of;
+  static thread_local uint64_t uses = 0;
   const int device = c10::cuda::current_device();
-  if ((size_t)device >= streams.of.size()) streams.of.resize(device + 1);
-  auto& s = streams.of[device];
-  if (!s) {
+  if ((size_t)device >= of.size()) of.resize(device + 1);
+  if (!of[device]) of[device] = std::make_unique<Streams>();
+  auto* const slots = of[device]->slots;
+  auto* slot = &slots[0];
+  for (auto* s = slots; s != slots + 4; ++s) {
+    if (s->side && s->beside == current) {
+      slot = s;
+      break;
+    }
+    if (s->used < slot->used) slot = s;              // (never used: 0)
+  }
+  if (!slot->side) {
     cudaStream_t raw = nullptr;
     cudaEvent_t e[3] = {};
     bool made = cudaStreamCreateWithFlags(&raw, cudaStreamNonBlocking) == cudaSuccess;
@@ -917,9 +933,18 @@ SideStream* side_stream() {
       cudaGetLastError();
       return nullptr;
     }
-    s.reset(new SideStream{c10::cuda::getStreamFromExternal(raw, (c10::DeviceIndex)device), e[0], {e[1], e[2]}});
+    slot->side.reset(new SideStream{c10::cuda::getStreamFromExternal(raw, (c10::DeviceIndex)device), e[0], {e[1], e[2]}});
   }
-  return s.get();
+  cudaStreamCaptureStatus here = cudaStreamCaptureStatusNone, there = here;
+  unsigned long long here_id = 0, there_id = 0;
+  if (cudaStreamGetCaptureInfo(current, &here, &here_id) != cudaSuccess || cudaStreamGetCaptureInfo(slot->side->stream, &there, &there_id) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  if (there != cudaStreamCaptureStatusNone && (there != here || there_id != here_id)) return nullptr;
+  slot->beside = current;
+  slot->used = ++uses;
+  return slot->side.get();
 }
 
 // Where a layer's weight gradients are added (fp32).
@@ -1065,8 +1090,8 @@ Tensor decoder_stack_bwd(const Tensor& dout, const std::vector<Tensor>& xs, cons
   // shape, 32768 tokens 164,779 / 166,354 and 164,911 / 162,793 (no difference beyond what the power cap does from run to run); 2 layers of width 512,
   // 512 tokens 795 / 817.
   const double gflop = 4e-9 * n.T() * (double)(n.H * (n.Q() + n.O() + 3 * n.I));
-  SideStream* const side = gflop >= 12 ? side_stream() : nullptr;
   const cudaStream_t st = stream();
+  SideStream* const side = gflop >= 12 ? side_stream(st) : nullptr;
   // The second stream may be a layer behind, so layers take two scratch areas in turn (up to 1 GB for both) and a layer's incoming gradient is kept
   // for one layer more; a larger one is used again as soon as the second stream is done with it.
   const int64_t bytes = LayerScratch(n, side != nullptr).total;

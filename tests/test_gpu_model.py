@@ -330,3 +330,63 @@ def test_weight_gradients_on_a_second_stream(layers, inter):
         ids.copy_(b)
         graph.replay()
     close(w.bucket_manager.flat, want)
+
+
+def _side_stream_model():
+    """Layers whose weight gradients run on a second stream (12 GFLOP and more), a batch, and the gradients layer by layer."""
+    torch.manual_seed(7)
+    cfg = ModelConfig(hidden_size=512, intermediate_size=1024, num_hidden_layers=3, num_attention_heads=8, num_key_value_heads=4,
+                      vocab_size=512, max_position_embeddings=1024)
+    w = DataParallelBucket(Llama(cfg, init="normal").to(torch.bfloat16).cuda())
+    w.require_backward_grad_sync = False
+    ids = torch.randint(0, cfg.vocab_size, (2, 1024), device="cuda")
+    handles = [layer.register_forward_pre_hook(lambda *a: None) for layer in w.module.decoder_layers]
+    w(input_ids=ids, target_ids=ids).backward()
+    for h in handles:
+        h.remove()
+    want = w.bucket_manager.flat.clone()
+    w.reset()
+    return w, ids, want
+
+
+@pytest.mark.parametrize("streams", [1, 6])
+def test_eager_backward_while_another_thread_captures_one(streams):
+    """Autograd runs the backward passes of both threads on one thread of its own: the captured one's second stream has to stay out of the eager
+    ones, on one stream and on more than a thread keeps second streams for."""
+    import threading
+    captured, eager = _side_stream_model(), [_side_stream_model() for _ in range(streams)]
+    s, graph, errors = torch.cuda.Stream(), torch.cuda.CUDAGraph(), []
+    others = [torch.cuda.Stream() for _ in eager]
+
+    def one_pass(w, ids):
+        w(input_ids=ids, target_ids=ids).backward()
+
+    def work():
+        try:
+            for _ in range(2):
+                for (w, ids, _), stream in zip(eager, others):
+                    with torch.cuda.stream(stream):
+                        w.reset()
+                        one_pass(w, ids)
+        except Exception as e:                               # noqa: BLE001
+            errors.append(e)
+
+    for stream in [s] + others:
+        stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        one_pass(*captured[:2])
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=s, capture_error_mode="thread_local"):
+        one_pass(*captured[:2])
+        thread = threading.Thread(target=work)
+        thread.start()
+        thread.join()
+        one_pass(*captured[:2])                              # (the capture goes on)
+    assert not errors, errors
+    captured[0].reset()
+    graph.replay()
+    torch.cuda.synchronize()
+    for (w, _, want), passes in zip([captured] + eager, [2] + [1] * streams):
+        got = w.bucket_manager.flat
+        # (dQ, the norm weights' and the embedding's gradients add in any order; a rounding of bf16 moved by that moves what follows)
+        assert torch.isfinite(got).all() and float((got - passes * want).norm()) <= 4e-3 * passes * float(want.norm())
