@@ -27,6 +27,7 @@ from typing import List, Optional, Sequence
 import torch
 import torch.distributed as dist
 import torch.nn as nn
+from torch.autograd import forward_ad
 
 from .. import ops
 from .. import process_group_manager as pgm
@@ -585,7 +586,7 @@ _GLOBAL_HOOKS = [getattr(nn.modules.module, name) for name in ("_global_forward_
 
 def run_layers(layers, x: torch.Tensor) -> torch.Tensor:
     """``x`` through the decoder layers: in one native call where they are plain layers of one shape on one GPU that nobody observes
-    (hooks, NVTX ranges, tracing, checked mode), else layer by layer."""
+    (hooks, NVTX ranges, tracing, checked mode, function transforms, forward-mode derivatives), else layer by layer."""
     y = _run_stack(layers, x)
     if y is None:
         for layer in layers:
@@ -597,7 +598,7 @@ def run_layers(layers, x: torch.Tensor) -> torch.Tensor:
 def _run_stack(layers, x):
     if not ops.runs_layer_natively(x) or nvtx_enabled() or x.dim() != 3 or x.numel() == 0 or len(layers) == 0 or any(_GLOBAL_HOOKS):
         return None
-    if torch.jit.is_tracing() or torch.compiler.is_compiling():
+    if torch.jit.is_tracing() or torch.compiler.is_compiling() or torch._C._are_functorch_transforms_active():
         return None
     g = pgm.get()
     if g.tp_world_size > 1 or g.cp_dp_world_size > 1 or tpc.sequence_parallel_group() is not None:
@@ -616,6 +617,8 @@ def _run_stack(layers, x):
         dims = here
         params += ps
         tables += layer.rope(x.device, first)
+    if forward_ad._current_level >= 0 and any(forward_ad.unpack_dual(t).tangent is not None for t in (x, *params)):
+        return None                                  # (the layers' own nodes refuse what has no forward-mode derivative)
     if torch.is_grad_enabled() and (x.requires_grad or any(p.requires_grad for p in params)):
         # (without gradient buckets the layers' own nodes give back their activations as the backward pass goes)
         if any(getattr(p, "main_grad", None) is None for p in params):

@@ -230,3 +230,49 @@ def test_rope_scaling_matches_the_hugging_face_frequencies_and_defaults_to_plain
               vocab_size=32, max_position_embeddings=64, rope_theta=base)
     a, b = Llama(ModelConfig(**kw)), Llama(ModelConfig(**kw, rope_scaling=scaling))
     assert not torch.equal(a.decoder_layers[0].cos, b.decoder_layers[0].cos)
+
+
+@pytest.fixture
+def stack_calls(monkeypatch):
+    """A model whose layers take the native call for all of them, a stand-in that notes its calls and returns its input; the layers one by one run
+    as they do on the CPU. ``(model, calls)``."""
+    from picotron_b200 import ops
+    from picotron_b200.models import llama as M
+    torch.manual_seed(0)
+    calls, real = [], M._run_stack
+
+    def stand_in(x, params, tables, eps, B, S, hq, hkv, d, scale, save):
+        calls.append(save)
+        return [x.clone()] + [x.new_zeros(1) for _ in range(len(tables) // 2 * 3 if save else 0)]
+
+    def run_stack(layers, x):
+        with monkeypatch.context() as m:
+            m.setattr(ops, "runs_layer_natively", lambda t: True)
+            return real(layers, x)
+
+    monkeypatch.setattr(ops, "decoder_stack_fwd", stand_in)
+    monkeypatch.setattr(M, "_run_stack", run_stack)
+    return Llama(tiny_cfg()), calls
+
+
+def test_forward_mode_derivatives_are_refused_not_dropped(stack_calls):
+    """A tangent on a layer's weight or input: there is no forward-mode rule, and the layers say so."""
+    from torch.autograd import forward_ad
+    model, calls = stack_calls
+    model.requires_grad_(False)
+    ids = torch.randint(0, 97, (2, 16))
+    model(ids)
+    assert calls == [False]
+    name, w = "decoder_layers.1.mlp.down_proj.weight", model.decoder_layers[1].mlp.down_proj.weight
+    with forward_ad.dual_level():
+        model(ids)                                              # nothing carries a tangent
+        assert calls == [False] * 2
+        with pytest.raises(NotImplementedError, match="jvp"):
+            torch.func.functional_call(model, {name: forward_ad.make_dual(w.detach(), torch.ones_like(w))}, (ids,))
+        x = forward_ad.make_dual(torch.randn(1, 4, 64), torch.ones(1, 4, 64))
+        with pytest.raises(NotImplementedError, match="jvp"):
+            from picotron_b200.models.llama import run_layers
+            run_layers(model.decoder_layers, x)
+    with pytest.raises(RuntimeError, match="functorch|vmap|setup_context"):
+        torch.func.vmap(lambda v: torch.func.functional_call(model, {name: v}, (ids,)))(torch.stack([w, w]))
+    assert calls == [False] * 2
