@@ -586,7 +586,7 @@ _GLOBAL_HOOKS = [getattr(nn.modules.module, name) for name in ("_global_forward_
 
 def run_layers(layers, x: torch.Tensor) -> torch.Tensor:
     """``x`` through the decoder layers: in one native call where they are plain layers of one shape on one GPU that nobody observes
-    (hooks, NVTX ranges, tracing, checked mode, function transforms, forward-mode derivatives), else layer by layer."""
+    (hooks, replaced methods, NVTX ranges, tracing, checked mode, function transforms, forward-mode derivatives), else layer by layer."""
     y = _run_stack(layers, x)
     if y is None:
         for layer in layers:
@@ -600,14 +600,17 @@ def _run_stack(layers, x):
         return None
     if torch.jit.is_tracing() or torch.compiler.is_compiling() or torch._C._are_functorch_transforms_active():
         return None
+    if any(getattr(DecoderLayer, name) is not f for name, f in _LAYER_CALLS.items()):
+        return None
     g = pgm.get()
     if g.tp_world_size > 1 or g.cp_dp_world_size > 1 or tpc.sequence_parallel_group() is not None:
         return None
     first = layers[0]
     tables, params, dims = [], [], None
     for layer in layers:
-        if type(layer) is not DecoderLayer or "forward" in layer.__dict__ or layer._forward_hooks or layer._forward_pre_hooks or \
-                layer._backward_hooks or layer._backward_pre_hooks:
+        own = layer.__dict__
+        if type(layer) is not DecoderLayer or "forward" in own or "_call_impl" in own or "rope" in own or layer._compiled_call_impl is not None or \
+                layer._forward_hooks or layer._forward_pre_hooks or layer._backward_hooks or layer._backward_pre_hooks:
             return None
         ps = layer_parameters(layer)
         att = layer._modules["attention"]
@@ -724,6 +727,10 @@ class DecoderLayer(nn.Module):
                 x, self.input_layernorm.weight, self.post_attention_layernorm.weight,
                 a.q_proj.weight, a.k_proj.weight, a.v_proj.weight, a.out_proj.weight,
                 m.gate_proj.weight, m.up_proj.weight, m.down_proj.weight, self)
+
+
+# What a call of a layer runs: replaced on the class (instrumentation, a wrapper that recomputes), it is called layer by layer.
+_LAYER_CALLS = {name: getattr(DecoderLayer, name) for name in ("forward", "__call__", "_call_impl", "rope")}
 
 
 # ----------------------------------------------------------------------------------------------

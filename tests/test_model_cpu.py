@@ -276,3 +276,35 @@ def test_forward_mode_derivatives_are_refused_not_dropped(stack_calls):
     with pytest.raises(RuntimeError, match="functorch|vmap|setup_context"):
         torch.func.vmap(lambda v: torch.func.functional_call(model, {name: v}, (ids,)))(torch.stack([w, w]))
     assert calls == [False] * 2
+
+
+@pytest.mark.parametrize("where", ["class forward", "class call", "module call", "layer forward", "layer call", "compiled"])
+def test_replaced_layer_methods_are_called_layer_by_layer(stack_calls, monkeypatch, where):
+    from picotron_b200.models.llama import DecoderLayer
+    model, calls = stack_calls
+    ids, seen = torch.randint(0, 97, (2, 16)), []
+    with torch.no_grad():
+        want = model(ids)                                       # (the stand-in: the layers are passed by)
+        assert calls == [False]
+        owner = {"class": DecoderLayer, "module": torch.nn.Module, "layer": model.decoder_layers[1], "compiled": model.decoder_layers[1]}[where.split()[0]]
+        name = {"forward": "forward", "call": "__call__", "compiled": "_compiled_call_impl"}[where.split()[-1]]
+        if where == "layer call":
+            name = "_call_impl"
+        plain = DecoderLayer._call_impl if name in ("_call_impl", "_compiled_call_impl") else getattr(DecoderLayer, name)
+
+        def counted(*args, **kw):
+            if owner is model.decoder_layers[1]:
+                args = (owner, *args)
+            if isinstance(args[0], DecoderLayer):
+                seen.append(args[0].layer_idx)
+            return plain(*args, **kw)
+
+        with monkeypatch.context() as m:
+            m.setattr(owner, name, counted)
+            got = model(ids)
+    assert calls == [False] and seen == ([1] if owner is model.decoder_layers[1] else [0, 1])
+    assert not torch.equal(got, want)
+    model.decoder_layers[1].__dict__.pop(name, None)            # (what putting an instance's attribute back leaves there)
+    with torch.no_grad():
+        model(ids)
+    assert calls == [False] * 2                                 # in one call again
