@@ -586,7 +586,8 @@ _GLOBAL_HOOKS = [getattr(nn.modules.module, name) for name in ("_global_forward_
 
 def run_layers(layers, x: torch.Tensor) -> torch.Tensor:
     """``x`` through the decoder layers: in one native call where they are plain layers of one shape on one GPU that nobody observes
-    (hooks, replaced methods, NVTX ranges, tracing, checked mode, function transforms, forward-mode derivatives), else layer by layer."""
+    (hooks on modules or saved tensors, replaced methods, NVTX ranges, tracing, checked mode, function transforms, forward-mode
+    derivatives), else layer by layer."""
     y = _run_stack(layers, x)
     if y is None:
         for layer in layers:
@@ -623,8 +624,9 @@ def _run_stack(layers, x):
     if forward_ad._current_level >= 0 and any(forward_ad.unpack_dual(t).tangent is not None for t in (x, *params)):
         return None                                  # (the layers' own nodes refuse what has no forward-mode derivative)
     if torch.is_grad_enabled() and (x.requires_grad or any(p.requires_grad for p in params)):
-        # (without gradient buckets the layers' own nodes give back their activations as the backward pass goes)
-        if any(getattr(p, "main_grad", None) is None for p in params):
+        # (without gradient buckets the layers' own nodes give back their activations as the backward pass goes; with saved-tensor hooks, which
+        # offload or recompute, they hand them over and ask for them back one layer after the other)
+        if any(getattr(p, "main_grad", None) is None for p in params) or torch._C._autograd._top_saved_tensors_default_hooks(True) is not None:
             return None
         try:
             return DecoderStackFn.apply(x, tuple(layers), dims, tables, *params)

@@ -1,4 +1,7 @@
 """The fused model on the GPU (bf16, CUDA kernels) against the same model on CPU (fp32, PyTorch restatements)."""
+import contextlib
+import threading
+
 import pytest
 import torch
 
@@ -136,8 +139,8 @@ def test_checked_mode_sees_a_loss_that_is_not_finite_without_a_gradient():
 @pytest.mark.parametrize("layers,hq,hkv,d,inter,B,S", [(1, 2, 1, 64, 192, 1, 1), (3, 3, 1, 64, 320, 2, 97), (2, 2, 2, 128, 200, 1, 130)])
 def test_layers_in_one_native_call_equal_the_layers_one_by_one(layers, hq, hkv, d, inter, B, S):
     """The same launches: outputs, losses and logits equal to the bit, gradients up to the order of atomic additions; a hook on a layer is still
-    called (and its layers run one by one); weights that do not lie side by side, saved-tensor hooks are no matter;
-    another layer's norm weight swapped for the call is used."""
+    called, saved-tensor hooks get the tensors of one layer after the other (the layers run one by one then); weights that do not lie
+    side by side are no matter; another layer's norm weight swapped for the call is used."""
     from picotron_b200.models import llama as M
     torch.manual_seed(2)
     cfg = ModelConfig(hidden_size=hq * d, intermediate_size=inter, num_hidden_layers=layers, num_attention_heads=hq,
@@ -173,20 +176,20 @@ def test_layers_in_one_native_call_equal_the_layers_one_by_one(layers, hq, hkv, 
         model.embedding.weight.requires_grad_(layers != 2)      # once with an input that needs no gradient
         wrapped = DataParallelBucket(model)
 
-        def grads(hooked):
+        def grads(hooked, offload=False):
             wrapped.reset()
             stacks.clear()
             calls = []
             handle = model.decoder_layers[0].register_forward_hook(lambda *a: calls.append(1)) if hooked else None
-            with torch.autograd.graph.save_on_cpu():
+            with torch.autograd.graph.save_on_cpu() if offload else contextlib.nullcontext():
                 loss = wrapped(ids, target_ids=ids)
             loss.backward()
             if hooked:
                 handle.remove()
-            assert stacks == [not hooked] and len(calls) == hooked
+            assert stacks == [not hooked and not offload] and len(calls) == hooked
             return [loss.detach().clone()] + [p.main_grad.clone() for p in model.parameters() if p.requires_grad]
 
-        many, each = grads(False), grads(True)
+        many, each, offloaded = grads(False), grads(True), grads(False, True)
         handles = [layer.register_forward_pre_hook(lambda *a: None) for layer in model.decoder_layers]
         stacks.clear()
         single, single_swapped = passes(), passes(**{"final_norm.weight": model.final_norm.weight * 2,
@@ -199,8 +202,8 @@ def test_layers_in_one_native_call_equal_the_layers_one_by_one(layers, hq, hkv, 
     for x, y in zip(together + swapped, single + single_swapped):
         assert torch.equal(x, y)
     assert not torch.equal(together[0], swapped[0])
-    assert torch.equal(many[0], each[0])
-    for x, y in zip(many[1:], each[1:]):
+    assert torch.equal(many[0], each[0]) and torch.equal(offloaded[0], each[0])
+    for x, y in zip(many[1:] + offloaded[1:], each[1:] + each[1:]):
         # (dQ of more than two key blocks and the norm and embedding gradients add in any order: fp32 sums, rounded to bf16 once)
         assert float((x - y).norm()) <= 4e-3 * float(y.norm()) + 1e-12
 
@@ -249,9 +252,8 @@ def test_weights_changed_just_before_a_pass_are_those_it_uses(layers, T):
 @pytest.mark.parametrize("layers,inter", [(1, 1024), (2, 1024), (5, 1000)])
 def test_weight_gradients_on_a_second_stream(layers, inter):
     """Layers large enough that their weight gradients run beside their input gradients (12 GFLOP and more): the gradients of several micro-batches
-    equal those layer by layer, on the default stream, on another one, from two threads at once, with the saved tensors fetched from the
-    host, and from a captured graph that is replayed; memory that is freed right after the pass is not written by it any more."""
-    import threading
+    equal those layer by layer, on the default stream, on another one, from two threads at once, under saved-tensor hooks (layer by layer again),
+    and from a captured graph that is replayed; memory that is freed right after the pass is not written by it any more."""
     torch.manual_seed(4)
     cfg = ModelConfig(hidden_size=512, intermediate_size=inter, num_hidden_layers=layers, num_attention_heads=8, num_key_value_heads=4,
                       vocab_size=512, max_position_embeddings=1024)
@@ -266,7 +268,6 @@ def test_weight_gradients_on_a_second_stream(layers, inter):
     batches = [torch.randint(0, cfg.vocab_size, (B, S), device="cuda", generator=g) for _ in range(3)]
 
     def accumulate(w, context=None):
-        import contextlib
         w.reset()
         for i, ids in enumerate(batches):
             w.require_backward_grad_sync = i == len(batches) - 1
@@ -353,7 +354,6 @@ def _side_stream_model():
 def test_eager_backward_while_another_thread_captures_one(streams):
     """Autograd runs the backward passes of both threads on one thread of its own: the captured one's second stream has to stay out of the eager
     ones, on one stream and on more than a thread keeps second streams for."""
-    import threading
     captured, eager = _side_stream_model(), [_side_stream_model() for _ in range(streams)]
     s, graph, errors = torch.cuda.Stream(), torch.cuda.CUDAGraph(), []
     others = [torch.cuda.Stream() for _ in eager]

@@ -308,3 +308,19 @@ def test_replaced_layer_methods_are_called_layer_by_layer(stack_calls, monkeypat
     with torch.no_grad():
         model(ids)
     assert calls == [False] * 2                                 # in one call again
+
+
+def test_saved_tensor_hooks_see_one_layer_at_a_time(stack_calls):
+    """What offloads saved tensors keeps the activations of one layer on the device, not those of all."""
+    model, calls = stack_calls
+    wrapped, ids = DataParallelBucket(model), torch.randint(0, 97, (2, 16))
+    wrapped(ids, target_ids=ids)
+    assert calls == [True]
+    packed = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(t.shape) or t, lambda t: t):
+        loss = wrapped(ids, target_ids=ids)
+    assert calls == [True] and len(packed) > 2 * 11             # (eleven of every layer's own node)
+    loss.backward()
+    with torch.no_grad(), torch.autograd.graph.save_on_cpu():
+        model(ids)                                              # nothing is saved
+    assert calls == [True, False]
