@@ -131,10 +131,13 @@ def plan_memory(model_config, tp: int = 1, cp: int = 1, pp: int = 1, dp: int = 1
     d = h // mc.num_attention_heads
     qkv_cols = (mc.num_attention_heads + 2 * mc.num_key_value_heads) // tp * d
     layer_bwd = tokens * (2 * i_loc + 2 * h + qkv_cols) * dtype_bytes + tokens * (mc.num_attention_heads // tp) * d * 4
-    if tp == 1 and cp * dp == 1:
-        # (the native call for all layers: the attention's gradients beside dgu, two areas in turn up to 512 MiB each)
-        layer_bwd += tokens * h * dtype_bytes
-        layer_bwd *= 2 if layer_bwd <= 512 << 20 else 1
+    if tp == cp == dp == pp == 1:
+        # the native call for all layers: a layer's dgu, the attention's gradients and fp32 deltas beside it, dh and dx_mid; two such areas in turn up
+        # to 512 MiB each; the gradients into and out of a layer, and with two areas the one before; K-split workspaces of both streams, a
+        # wave of 256 x 256 fp32 tiles each
+        area = layer_bwd + tokens * (h * dtype_bytes + mc.num_attention_heads * 4)
+        two = area <= 512 << 20
+        layer_bwd = (2 if two else 1) * area + (3 if two else 2) * tokens * h * dtype_bytes + 2 * 74 * 4 * 256 ** 2
     head = min(ce_chunk_tokens, tokens) * (v // tp) * dtype_bytes if stage == pp - 1 else 0
     b["transients"] = max(layer_bwd, head)
 

@@ -96,6 +96,22 @@ def test_plan_of_the_benchmark_configurations_fits_a_b200_and_names_the_large_te
     assert c.fits() and c.bytes["comm_workspaces"] > (64 << 20)
 
 
+def test_plan_of_a_layers_backward_with_and_without_the_native_call_for_all_layers():
+    """One GPU: two scratch areas in turn and the gradients between layers; a pipeline stage, whose layers run one by one: the tensors of one layer."""
+    from picotron_b200.config import preset_model_config
+    from picotron_b200.utils.memory import plan_memory
+    mc = preset_model_config("HuggingFaceTB/SmolLM-1.7B")
+    T, H, I, Q = 4096, 2048, 8192, 6144                          # noqa: E741
+    one = T * (2 * I + 2 * H + Q) * 2 + T * H * 4               # dgu, dh, dx_mid, dqkv; fp32 dQ
+    stage = plan_memory(mc, pp=2, stage=0, micro_batch_size=4, seq_length=1024)
+    assert stage.bytes["transients"] == one
+    all_layers = plan_memory(mc, micro_batch_size=4, seq_length=1024)
+    area = one + T * (H * 2 + 32 * 4)                           # and the attention's incoming gradient and deltas
+    assert 0 <= all_layers.bytes["transients"] - 2 * area - 3 * T * H * 2 < 48 << 20
+    large = plan_memory(mc, micro_batch_size=16, seq_length=1024)                # beyond 512 MiB: one area
+    assert 0 <= large.bytes["transients"] - 4 * area - 2 * 4 * T * H * 2 < 48 << 20
+
+
 def test_train_dry_run_describes_the_stages_and_rejects_an_impossible_grid(tmp_path):
     import json
     import os
