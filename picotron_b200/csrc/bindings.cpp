@@ -1091,12 +1091,22 @@ Tensor decoder_stack_bwd(const Tensor& dout, const std::vector<Tensor>& xs, cons
   // 512 tokens 795 / 817.
   const double gflop = 4e-9 * n.T() * (double)(n.H * (n.Q() + n.O() + 3 * n.I));
   const cudaStream_t st = stream();
-  SideStream* const side = gflop >= 12 ? side_stream(st) : nullptr;
+  SideStream* side = gflop >= 12 ? side_stream(st) : nullptr;
   // The second stream may be a layer behind, so layers take two scratch areas in turn (up to 1 GB for both) and a layer's incoming gradient is kept
-  // for one layer more; a larger one is used again as soon as the second stream is done with it.
-  const int64_t bytes = LayerScratch(n, side != nullptr).total;
-  const bool late = side != nullptr && layers > 1 && bytes <= (512 << 20);
-  Tensor scratch = torch::empty({late ? 2 * bytes : bytes}, on.dtype(at::kByte)), grad = dout, kept[2];
+  // for one layer more; a larger one is used again as soon as the second stream is done with it. One stream needs the least: where the device is
+  // too full for more, it has to do.
+  int64_t bytes = LayerScratch(n, side != nullptr).total;
+  bool late = side != nullptr && layers > 1 && bytes <= (512 << 20);
+  Tensor scratch, grad = dout, kept[2];
+  try {
+    scratch = torch::empty({late ? 2 * bytes : bytes}, on.dtype(at::kByte));
+  } catch (const c10::OutOfMemoryError&) {
+    if (side == nullptr) throw;
+    side = nullptr;
+    late = false;
+    bytes = LayerScratch(n, false).total;
+    scratch = torch::empty({bytes}, on.dtype(at::kByte));
+  }
   struct Joined {                                                        // whatever happens, memory is not given back before it is done with
     SideStream* side;
     cudaStream_t st;
@@ -1118,8 +1128,8 @@ Tensor decoder_stack_bwd(const Tensor& dout, const std::vector<Tensor>& xs, cons
                        dx.data_ptr(), scale, on, side);
     if (side != nullptr) {
       side->done((int)i);
-      if (!late) side->join(st, (int)i);
-      kept[i & 1] = grad;
+      if (late) kept[i & 1] = grad;
+      else side->join(st, (int)i);
     }
     grad = dx;
   }

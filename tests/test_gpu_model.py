@@ -390,3 +390,44 @@ def test_eager_backward_while_another_thread_captures_one(streams):
         got = w.bucket_manager.flat
         # (dQ, the norm weights' and the embedding's gradients add in any order; a rounding of bf16 moved by that moves what follows)
         assert torch.isfinite(got).all() and float((got - passes * want).norm()) <= 4e-3 * passes * float(want.norm())
+
+
+@pytest.mark.parametrize("full", [False, True])
+def test_memory_of_the_layers_backward(full):
+    """What the backward pass takes beside what was there is within its plan; on a device too full for two streams' scratch it runs on one and
+    takes what one stream takes."""
+    from picotron_b200.utils.memory import plan_memory
+    cfg = ModelConfig(hidden_size=512, intermediate_size=1024, num_hidden_layers=3, num_attention_heads=8, num_key_value_heads=4,
+                      vocab_size=512, max_position_embeddings=1024)
+    B, S = 16, 1024
+    torch.manual_seed(8)
+    w = DataParallelBucket(Llama(cfg, init="normal").to(torch.bfloat16).cuda())
+    w.require_backward_grad_sync = False
+    ids = torch.randint(0, cfg.vocab_size, (B, S), device="cuda")
+    w(input_ids=ids, target_ids=ids).backward()
+    want = w.bucket_manager.flat.clone()
+    w.reset()
+    loss = w(input_ids=ids, target_ids=ids)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    T, H = B * S, 512
+    scratch_one = T * (max(4 * 1024, 2 * H + 2 * 1024 + 4 * H + 4 * 8) + 4 * H)
+    scratch_two = 2 * T * (4 * 1024 + 2 * H + 2 * 1024 + 4 * H + 4 * 8 + 4 * H)
+    others = 6 * T * H * 2 + (40 << 20)                         # gradients between layers and of the head; K-split workspaces
+    total = torch.cuda.get_device_properties(0).total_memory
+    assert scratch_one + others < scratch_two
+    try:
+        if full:
+            torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + scratch_one + others) / total)
+        loss.backward()
+        torch.cuda.synchronize()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    taken = torch.cuda.max_memory_allocated() - before
+    planned = plan_memory(cfg, micro_batch_size=B, seq_length=S, fused_comm=False).bytes["transients"]
+    assert taken < scratch_one + others if full else scratch_two < taken <= planned, (taken, planned)
+    got = w.bucket_manager.flat
+    # (dQ, the norm weights' and the embedding's gradients add in any order; a rounding of bf16 moved by that moves what follows)
+    assert float((got - want).norm()) <= 4e-3 * float(want.norm())
