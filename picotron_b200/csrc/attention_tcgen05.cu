@@ -1259,13 +1259,37 @@ static int launch_fwd(const CUtensorMap& mq, const KVSegs& segs, const CUtensorM
 // least, as far as the parts' sums fit beside each other (3 parts for d = 64, 2 for d = 128). 3 x 601, 9 / 3 heads are 45 key blocks of up to
 // 15 steps: 36.9 us, in three parts 29.9; 2 x 256, 8 / 4 heads, 16 of up to 4: 16.4, in two 17.8. Beyond one wave the CTAs' starts and ends and the
 // clusters' (of CTAs that fill an SM) waiting for neighbouring SMs cost more than evenness gives: 8 x 1024, 9 / 3 heads 57 us, in three 98.
-static int bwd_head_parts(const BwdParams& p, int d, long long ctas, int sms) {
+// `largest`: the largest cluster that can be had.
+static int bwd_head_parts(const BwdParams& p, int d, long long ctas, int sms, int largest) {
   const long long group = p.hq / p.hkv, steps = (p.Sq + 127) / 128 * group;
-  for (int parts = d == 64 ? 3 : 2; parts > 1; --parts)
+  for (int parts = std::min(d == 64 ? 3 : 2, largest); parts > 1; --parts)
     if (group % parts == 0 && ctas * parts <= sms && steps - steps / parts >= 4) return parts;
   return 1;
 }
+static long long key_blocks(const BwdParams& p) { return (long long)((p.Sk + 127) / 128) * p.n_segs * p.hkv * p.B; }
+static thread_local int g_largest_cluster = 3;       // (the thread's switch, for tests and measurements)
 
+// Whether clusters of `size` CTAs of `kern` can be placed on the device: each takes an SM for itself, and an SM partition (MIG, MPS) may not have
+// as many side by side.
+template <int D, typename Kern>
+static bool bwd_clusters_fit(Kern kern, int size) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)size);
+  cfg.blockDim = dim3(BwdWarps<bwd_parts<D>()>::THREADS);
+  cfg.dynamicSmemBytes = BwdCfg<D>::SMEM;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)size;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess) return n > 0;
+  cudaGetLastError();
+  return false;
+}
+
+// (SPLIT: p.parts CTAs of a cluster share a key block; -5, nothing launched, where such clusters cannot be had)
 template <int D, bool OUT_F32, bool PROF = false, bool SPLIT = false>
 static int launch_bwd(const CUtensorMap& mq, const KVSegs& segs, const CUtensorMap& mdo, const CUtensorMap& mdq, const CUtensorMap& mdk,
                       const CUtensorMap& mdv, const float* lse, const float* delta, void* dk, void* dv, BwdParams p, KernelStatus* st,
@@ -1277,7 +1301,7 @@ static int launch_bwd(const CUtensorMap& mq, const KVSegs& segs, const CUtensorM
     if constexpr (bwd_parts<D>() == 4) return attn_bwd_parts4_kernel<D, OUT_F32, PROF, SPLIT>;
     else return attn_bwd_kernel<D, OUT_F32, PROF, SPLIT>;
   }();
-  static PerDevice configured;
+  static PerDevice configured, clusters;
   const int sms = configured.get(current_device(), [&] {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdCfg<D>::SMEM) != cudaSuccess) return -3;
     cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
@@ -1290,14 +1314,19 @@ static int launch_bwd(const CUtensorMap& mq, const KVSegs& segs, const CUtensorM
     return n;
   });
   if (sms <= 0) return sms;
-  const long long ctas = (long long)((p.Sk + 127) / 128) * p.n_segs * p.hkv * p.B;
-  if constexpr (!SPLIT) {
-    p.parts = bwd_head_parts(p, D, ctas, sms);
-    if (p.parts > 1) return launch_bwd<D, OUT_F32, PROF, true>(mq, segs, mdo, mdq, mdk, mdv, lse, delta, dk, dv, p, st, stream);
+  if constexpr (SPLIT) {
+    const int largest = clusters.get(current_device(), [&] { return bwd_clusters_fit<D>(kern, 3) ? 3 : bwd_clusters_fit<D>(kern, 2) ? 2 : 1; });
+    if (p.parts > largest) return -5;                 // (nothing launched)
+  } else {
+    const long long ctas = key_blocks(p);
+    for (int largest = g_largest_cluster; (p.parts = bwd_head_parts(p, D, ctas, sms, largest)) > 1; largest = p.parts - 1) {
+      const int rc = launch_bwd<D, OUT_F32, PROF, true>(mq, segs, mdo, mdq, mdk, mdv, lse, delta, dk, dv, p, st, stream);
+      if (rc != -5) return rc;
+    }
   }
   static_assert((D == 64 ? 2 : 1) * BWD_SUM_BYTES<D> <= (BwdCfg<D>::QSTAGES + BwdCfg<D>::OSTAGES) * BwdCfg<D>::TILE_BYTES + BwdCfg<D>::DS_BYTES,
                 "the parts' sums take the place of the rings and dS");
-  const cudaError_t err = launch_pdl_cluster(kern, dim3((unsigned)(ctas * p.parts)), dim3(Warps::THREADS), BwdCfg<D>::SMEM, stream, p.parts, mq, segs,
+  const cudaError_t err = launch_pdl_cluster(kern, dim3((unsigned)(key_blocks(p) * p.parts)), dim3(Warps::THREADS), BwdCfg<D>::SMEM, stream, p.parts, mq, segs,
                                              mdo, mdq, mdk, mdv, lse, delta, dk, dv, p, st);
   pt_count_launches(1);
   return err == cudaSuccess && cudaGetLastError() == cudaSuccess ? 0 : -4;
@@ -1305,6 +1334,9 @@ static int launch_bwd(const CUtensorMap& mq, const KVSegs& segs, const CUtensorM
 
 }  // namespace attn
 }  // namespace pt
+
+// Largest cluster of CTAs that share a key block's query heads in the backward: 3 by default, 1: none (for the calling thread).
+extern "C" void pt_attention_set_clusters(int largest) { pt::attn::g_largest_cluster = largest; }
 
 // q [B,Sq,hq,d] bf16 with token stride q_row; K/V in `n_segs` segments: k_ptrs[i]/v_ptrs[i] are [B,Sk,hkv,d] bf16 with
 // token strides k_row/v_row (elements, multiples of 8) and may be peer-mapped pointers into other GPUs' memory.

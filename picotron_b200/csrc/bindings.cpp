@@ -91,6 +91,7 @@ int pt_embedding_gather_peers(const long long* ids, void* const* shard_ptrs, int
 int pt_gather_peer(void* dst, const void* const* src_ptrs, int n_src, long long bytes_each, cudaStream_t st);
 int pt_reduce_dkv_symm(void* const* buf_ptrs, long long offset_elems, int me, int world, long long tokens, int width,
                        void* dk, void* dv, long long dk_row, long long dv_row, cudaStream_t st);
+void pt_attention_set_clusters(int largest);
 int pt_attention_fwd_segs(const void* q, const void* const* k_ptrs, const void* const* v_ptrs, int n_segs, void* o,
                           float* lse, int B, int Sq, int Sk, int hq, int hkv, int d, long long q_row, long long k_row,
                           long long v_row, int causal, float scale, cudaStream_t st);
@@ -1400,6 +1401,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         }, py::arg("counters") = py::none(),
         "Phase profiling of the attention kernels: later forward/backward launches add their per-phase SM-cycle counts to "
         "`counters` (layout in csrc/attention_tcgen05.cu); None switches it off. The caller keeps the tensor alive.");
+  m.def("attention_set_clusters", [](int64_t largest) { pt_attention_set_clusters((int)largest); },
+        "Largest cluster of CTAs that share a key block's query heads in the attention backward: 3 by default, 1: none (this thread).");
   m.def("attention_fwd_segs", &attention_fwd_segs);
   m.def("attention_bwd_segs", &attention_bwd_segs);
   m.def("gemm_allreduce", &gemm_allreduce,

@@ -163,6 +163,27 @@ def test_attention_backward_of_few_key_blocks_with_long_groups(C, d, Sq, Sk, gro
         assert err <= 1e-2 * float(w.float().norm()) + 2e-3 * w.numel() ** 0.5, f"{name}: {err} of {float(w.float().norm())}"
 
 
+@pytest.mark.parametrize("d,group", [(64, 6), (128, 4)])
+@pytest.mark.parametrize("largest", [1, 2])
+def test_attention_backward_where_large_clusters_cannot_be_had(C, d, group, largest):
+    """Key blocks whose query heads two or three CTAs would share, on a device that places smaller clusters only, or none: the next smaller number
+    of CTAs, which gives the same gradients."""
+    q, k, v, do = rnd(1, 400, 2 * group, d, seed=1), rnd(1, 400, 2, d, seed=2), rnd(1, 400, 2, d, seed=3), rnd(1, 400, 2 * group, d, seed=4)
+    scale = 1.0 / math.sqrt(d)
+    o_ref, lse_ref = ref.attention_fwd(q, k, v, True, scale)
+    want = ref.attention_bwd(do, q, k, v, o_ref, lse_ref, True, scale)
+    try:
+        C.attention_set_clusters(largest)
+        got = C.attention_bwd(do, q, k, v, o_ref, lse_ref, True, scale)
+    finally:
+        C.attention_set_clusters(3)
+    torch.cuda.synchronize()
+    assert C.kernel_status() == 0
+    for name, g, w in zip(("dq", "dk", "dv"), got, want):          # (bounds as above)
+        err = float((g.float() - w.float()).norm())
+        assert err <= 1e-2 * float(w.float().norm()) + 2e-3 * w.numel() ** 0.5, f"{name}: {err} of {float(w.float().norm())}"
+
+
 @pytest.mark.parametrize("B,S,hq,hkv,d", [(2, 256, 4, 2, 64), (1, 300, 4, 4, 64), (2, 256, 2, 1, 128), (3, 128, 2, 2, 64)])
 def test_attention_backward_with_inverse_rope_on_dq_dk(C, B, S, hq, hkv, d):
     """dq / dk un-rotated inside the backward (dq in the fp32->bf16 conversion, dk in the epilogue) vs the RoPE kernel."""
