@@ -28,7 +28,6 @@ void pt_attention_set_profile(unsigned long long* counters);
 void pt_gemm_set_group_m(int g);
 void pt_gemm_set_tile_n(int n);
 int pt_gemm_tile_columns(int M, int n_cols, int K, int f32, int b_mn, int has_192);
-int pt_gemm_split_parts(int M, int N, int K, int kind, int* tile_n);
 int pt_gemm_parts(int M, int N, int K, int kind, int add, int* tile_n);
 void pt_gemm_set_cluster(int n);
 int pt_gemm_bf16_cluster(const void* A, const void* B, void* D, int M, int N, int K, long long lda, long long ldb, long long ldd, int b_mn, const void* res,
@@ -224,7 +223,7 @@ Tensor swiglu_bwd(const Tensor& gu, const Tensor& da) {
   return dgu;
 }
 
-// A GEMM with few output tiles, K in parts (pt_gemm_split_parts) through a workspace from the caching allocator; kind 0: D = A B,
+// A GEMM with few output tiles, K in parts (pt_gemm_parts) through a workspace from the caching allocator; kind 0: D = A B,
 // 1: D += A^T B (fp32), 2: D = A B^T (+ res). False (nothing launched) where it would not pay or the operands do not allow it.
 bool gemm_split_into(const void* a, const void* b, void* d, int64_t M, int64_t N, int64_t K, long long lda, long long ldb, long long ldd,
                      int kind, const void* res, long long ldr, const at::TensorOptions& on) {
@@ -1383,12 +1382,13 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           const int splits = kind == "dgrad" ? 0 : kind == "wgrad" ? 1 : kind == "fwd" || kind == "add" ? 2 : -1;
           TORCH_CHECK(splits >= 0 || kind == "rope" || kind == "swiglu" || kind == "swiglu_bwd", "gemm_plan: ", kind);
           int tile_n = 256;
-          const int parts = splits >= 0 ? pt_gemm_split_parts((int)M, (int)N, (int)K, splits, &tile_n) : 1;
+          const int parts = splits >= 0 ? pt_gemm_parts((int)M, (int)N, (int)K, splits, kind == "add", &tile_n) : 1;
+          if (parts < 0) return std::pair<int64_t, int64_t>(128, -2);
           if (parts <= 1) tile_n = pt_gemm_tile_columns((int)M, (int)N, (int)K, splits == 1, splits == 0 || splits == 1 || kind == "swiglu_bwd",
                                                        splits >= 0 || kind == "swiglu_bwd");
           return std::pair<int64_t, int64_t>(tile_n, parts);
         }, "(columns of a tile, parts of K) that the rule gives a GEMM with output [M, N]: kind fwd, add, dgrad, wgrad, rope, swiglu (N = 2I) or\n"
-           "swiglu_bwd (N = I). Where K is shared within clusters instead (set_gemm_cluster), what it would be without.");
+           "swiglu_bwd (N = I). (128, -2): K is shared by the two pairs of a cluster.");
   m.def("set_gemm_tile_n", [](int64_t n) { pt_gemm_set_tile_n((int)n); },
         "columns of the GEMM output tiles: 128, 192 (where the epilogue has it), 256, or 0 for the choice by shape (for the calling thread). "
          "With a given width K is not split, unless set_gemm_split_parts says so.");

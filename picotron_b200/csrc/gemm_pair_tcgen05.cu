@@ -1105,7 +1105,7 @@ static int num_pairs() {
 }
 
 // Switches for tests and measurements, of the calling thread only: other threads' launches keep the rules.
-static thread_local int g_split_k = 1;   // 0: never, 1: by pt_gemm_split_parts' rule, n > 1: always n parts
+static thread_local int g_split_k = 1;   // 0: never, 1: by split_parts' rule, n > 1: always n parts
 static thread_local int g_tile_n = 0;    // 0: by the rule below, 128 / 192 / 256: as given (tests, measurements)
 
 // Microseconds of a GEMM as far as they depend on the width of its tiles and on the parts K is split into: waves of units over the
@@ -1384,11 +1384,7 @@ static int split_parts(int M, int N, int K, int kind, int* tile_n, double* us) {
   *us = split + (kind == SPLIT_FWD ? 2.0 : 0.0);
   return best_parts;
 }
-extern "C" int pt_gemm_split_parts(int M, int N, int K, int kind, int* tile_n) {
-  double us;
-  return split_parts(M, N, K, kind, tile_n, &us);
-}
-// The same, or -1: K shared within clusters (pt_gemm_bf16_cluster).
+// The choice, or -1: K shared within clusters (pt_gemm_bf16_cluster).
 extern "C" int pt_gemm_parts(int M, int N, int K, int kind, int add, int* tile_n) {
   using namespace pt::gemm_pair;
   double us;

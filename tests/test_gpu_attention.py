@@ -163,6 +163,40 @@ def test_attention_backward_of_few_key_blocks_with_long_groups(C, d, Sq, Sk, gro
         assert err <= 1e-2 * float(w.float().norm()) + 2e-3 * w.numel() ** 0.5, f"{name}: {err} of {float(w.float().norm())}"
 
 
+@pytest.mark.parametrize("largest", [3, 1])
+@pytest.mark.parametrize("d,group,S,n,causal", [(64, 6, 300, 3, True), (64, 4, 260, 2, False), (128, 4, 200, 3, True), (128, 2, 520, 1, True)])
+def test_attention_of_several_key_segments_with_long_groups(C, d, group, S, n, causal, largest):
+    """Context parallelism's shape on local memory: keys and values in segments (the causal mask runs through the last one), fp32 dK and dV
+    per segment; the query heads of a key block are shared by the CTAs of a cluster, or not."""
+    B, hkv = 1, 2
+    hq, scale = hkv * group, 1.0 / math.sqrt(d)
+    q, do = rnd(B, S, hq, d, seed=1), rnd(B, S, hq, d, seed=2)
+    ks, vs = [rnd(B, S, hkv, d, seed=3 + i) for i in range(n)], [rnd(B, S, hkv, d, seed=30 + i) for i in range(n)]
+    Q, K, V = (t.float().transpose(1, 2).requires_grad_() for t in (q, torch.cat(ks, 1), torch.cat(vs, 1)))
+    s = Q @ K.repeat_interleave(group, 1).transpose(-1, -2) * scale
+    if causal:
+        s = s.masked_fill(torch.ones(S, n * S, device="cuda", dtype=torch.bool).triu((n - 1) * S + 1), -math.inf)
+    o_ref = s.softmax(-1) @ V.repeat_interleave(group, 1)
+    o_ref.backward(do.float().transpose(1, 2))
+    kp, vp = [t.data_ptr() for t in ks], [t.data_ptr() for t in vs]
+    per = B * S * hkv * d
+    part = torch.full((n, 2, B, S, hkv, d), float("nan"), device="cuda")
+    try:
+        C.attention_set_clusters(largest)
+        o, lse = C.attention_fwd_segs(q, kp, vp, S, hkv, hkv * d, causal, scale)
+        dq = C.attention_bwd_segs(do, q, kp, vp, S, hkv, hkv * d, o, lse, None, part.data_ptr(), 2 * per, causal, scale)
+    finally:
+        C.attention_set_clusters(3)
+    torch.cuda.synchronize()
+    assert C.kernel_status() == 0
+    torch.testing.assert_close(o.float(), o_ref.transpose(1, 2), rtol=2e-2, atol=2e-2)
+    back = lambda t: t.transpose(1, 2)                              # noqa: E731
+    dk, dv = torch.cat(list(part[:, 0]), 1), torch.cat(list(part[:, 1]), 1)
+    for name, g, w in (("dq", dq, back(Q.grad)), ("dk", dk, back(K.grad)), ("dv", dv, back(V.grad))):          # (bounds as above)
+        err = float((g.float() - w).norm())
+        assert err <= 1e-2 * float(w.norm()) + 2e-3 * w.numel() ** 0.5, f"{name}: {err} of {float(w.norm())}"
+
+
 @pytest.mark.parametrize("d,group", [(64, 6), (128, 4)])
 @pytest.mark.parametrize("largest", [1, 2])
 def test_attention_backward_where_large_clusters_cannot_be_had(C, d, group, largest):

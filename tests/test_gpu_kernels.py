@@ -190,6 +190,33 @@ def test_gemm_with_k_shared_in_clusters(C, M, N, K):
         assert _rel(g.double(), want) < 2.5e-3 and _rel(g.double(), want) < 1.01 * _rel(one.double(), want) + 1e-5
 
 
+@pytest.mark.parametrize("kind,M,N,K,shared", [("fwd", 256, 576, 1536, True), ("add", 256, 960, 1024, True), ("dgrad", 384, 2048, 6144, True),
+                                               ("fwd", 512, 2048, 8192, True), ("dgrad", 256, 2048, 3072, True), ("fwd", 256, 576, 1472, False),
+                                               ("add", 256, 960, 832, False), ("dgrad", 256, 576, 1472, False), ("dgrad", 512, 2048, 8256, False),
+                                               ("fwd", 1024, 2048, 2048, False), ("add", 4096, 2048, 8192, False)])
+def test_gemm_shares_k_in_clusters_by_rule(kind, M, N, K, shared):
+    """Shapes on both sides of the rule: few tiles and a long K share it, a short one, more tiles than clusters, and an input gradient over more
+    than 8192 do not; what runs by the rule is what runs when the switch says so, and its plan tells."""
+    from picotron_b200.ops import _ext
+    C = _ext.load()
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the rule counts SMs")
+    C.set_gemm_pair(True)
+    C.set_gemm_tma_epilogue(True)
+    x, w, wt, res = bf(M, K, seed=1), bf(N, K, seed=2), bf(K, N, seed=3), bf(M, N, seed=4)
+    call = {"fwd": lambda: C.gemm(x, w, False, False), "add": lambda: C.gemm_add(x, w, res), "dgrad": lambda: C.gemm(x, wt, False, True)}[kind]
+    assert (C.gemm_plan(kind, M, N, K) == (128, -2)) == shared
+    by_rule = call()
+    try:
+        C.set_gemm_cluster(2 if shared else 1)
+        assert torch.equal(by_rule, call())
+        C.set_gemm_cluster(1 if shared else 2)
+        assert not torch.equal(by_rule, call())               # (the other order of the sums moves a few roundings)
+    finally:
+        C.set_gemm_cluster(0)
+    _status_ok(C)
+
+
 def test_gemm_over_nothing_is_zero(C):
     """The weight gradient of an empty batch: zeros, or what the destination holds where it is added to."""
     dy, x = bf(0, 72), bf(0, 136)
@@ -202,7 +229,7 @@ def test_gemm_over_nothing_is_zero(C):
     assert C.gemm(x, bf(200, 136), False, False).shape == (0, 200)
 
 
-# us by (columns of a tile, parts), operands not in L2
+# us by (columns of a tile, parts; -2: shared within clusters), operands not in L2
 MEASURED_PLANS = [
     ("swiglu_bwd", 1024, 11008, 4096, {(128, 1): 101.0, (192, 1): 98.2, (256, 1): 86.1}),
     ("swiglu_bwd", 768, 14336, 4096, {(128, 1): 102.4, (256, 1): 88.1}),
@@ -212,7 +239,9 @@ MEASURED_PLANS = [
     ("dgrad", 1024, 2048, 16384, {(128, 1): 65.8, (256, 2): 60.4}),
     ("dgrad", 512, 4096, 12288, {(128, 1): 57.3, (256, 2): 52.9}),
     ("wgrad", 2048, 512, 8192, {(128, 2): 29.6, (256, 4): 27.6, (192, 3): 27.6}),
-    ("fwd", 128, 4096, 4096, {(128, 2): 23.5, (128, 1): 26.2}),
+    ("fwd", 128, 4096, 4096, {(128, -2): 18.8, (128, 2): 21.5, (128, 1): 22.9}),
+    ("add", 512, 2048, 8192, {(128, -2): 26.7, (256, 4): 29.7, (128, 1): 34.9}),
+    ("dgrad", 384, 2048, 6144, {(128, -2): 20.8, (256, 4): 25.6, (128, 2): 24.7}),
     ("dgrad", 4096, 576, 3072, {(256, 1): 20.7, (128, 1): 19.8, (192, 1): 17.2}),
     ("wgrad", 49152, 576, 2048, {(256, 1): 110.0, (128, 1): 118.0, (192, 1): 102.0}),
     ("fwd", 256, 576, 576, {(256, 1): 7.1, (128, 1): 5.3}),

@@ -208,12 +208,17 @@ def test_layers_in_one_native_call_equal_the_layers_one_by_one(layers, hq, hkv, 
         assert float((x - y).norm()) <= 4e-3 * float(y.norm()) + 1e-12
 
 
-@pytest.mark.parametrize("layers,T", [(1, 64), (4, 64), (4, 700)])
-def test_weights_changed_just_before_a_pass_are_those_it_uses(layers, T):
+@pytest.mark.parametrize("layers,T,H,I", [(1, 64, 192, 384), (4, 64, 192, 384), (4, 700, 192, 384), (2, 64, 1536, 1600)])
+def test_weights_changed_just_before_a_pass_are_those_it_uses(layers, T, H, I):     # noqa: E741
     """The layers' GEMMs fetch weights and saved activations ahead of the kernel before them; what an optimizer step or a copy wrote right before
-    the pass has to be seen, and a backward pass reads its own forward's activations: every pass equals the same one layer by layer."""
+    the pass has to be seen, and a backward pass reads its own forward's activations: every pass equals the same one layer by layer. (Width
+    1536: output and down projections and input gradients share K in clusters.)"""
+    from picotron_b200.ops import _ext
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        for kind, n, k in (("fwd", H, H), ("add", H, I), ("dgrad", H, H), ("dgrad", H, 2 * I)):
+            assert (_ext.load().gemm_plan(kind, T, n, k) == (128, -2)) == (H == 1536)
     torch.manual_seed(3)
-    cfg = ModelConfig(hidden_size=192, intermediate_size=384, num_hidden_layers=layers, num_attention_heads=3, num_key_value_heads=1,
+    cfg = ModelConfig(hidden_size=H, intermediate_size=I, num_hidden_layers=layers, num_attention_heads=H // 64, num_key_value_heads=H // 192,
                       vocab_size=256, max_position_embeddings=T)
     model = Llama(cfg, init="normal").to(torch.bfloat16).cuda()
     wrapped = DataParallelBucket(model)
@@ -249,15 +254,16 @@ def test_weights_changed_just_before_a_pass_are_those_it_uses(layers, T):
         assert float((x.float() - y.float()).norm()) <= 3e-2 * float(y.float().norm()) + 1e-12
 
 
-@pytest.mark.parametrize("layers,inter", [(1, 1024), (2, 1024), (5, 1000)])
-def test_weight_gradients_on_a_second_stream(layers, inter):
+@pytest.mark.parametrize("layers,inter,B", [(1, 1024, 2), (2, 1024, 2), (5, 1000, 2), (3, 1024, 48)])
+def test_weight_gradients_on_a_second_stream(layers, inter, B):
     """Layers large enough that their weight gradients run beside their input gradients (12 GFLOP and more): the gradients of several micro-batches
     equal those layer by layer, on the default stream, on another one, from two threads at once, under saved-tensor hooks (layer by layer again),
-    and from a captured graph that is replayed; memory that is freed right after the pass is not written by it any more."""
+    and from a captured graph that is replayed; memory that is freed right after the pass is not written by it any more. (48 x 1024 tokens: scratch beyond
+    512 MiB, one area for all layers.)"""
     torch.manual_seed(4)
     cfg = ModelConfig(hidden_size=512, intermediate_size=inter, num_hidden_layers=layers, num_attention_heads=8, num_key_value_heads=4,
                       vocab_size=512, max_position_embeddings=1024)
-    B, S = 2, 1024
+    S = 1024
 
     def build():
         torch.manual_seed(5)
