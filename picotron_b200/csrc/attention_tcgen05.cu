@@ -161,7 +161,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     tma_prefetch_desc(&tm_q);
     tma_prefetch_desc(&segs.k[0]);
     tma_prefetch_desc(&segs.v[0]);
-      tma_prefetch_desc(&tm_o);
+    tma_prefetch_desc(&tm_o);
     // The first loads leave before the other warps are let go: they travel under the tensor-memory allocation and the first barrier.
     pdl_wait();
     mbar_expect_tx(&bars.q_full, Cfg::Q_BYTES);
@@ -697,7 +697,7 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tm_q, const KVS
     tma_prefetch_desc(&segs.v[seg]);
     tma_prefetch_desc(&tm_do);
     tma_prefetch_desc(&tm_dq);
-      if (tm_out) {
+    if (tm_out) {
       tma_prefetch_desc(&tm_dk);
       tma_prefetch_desc(&tm_dv);
     }
@@ -1038,152 +1038,152 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tm_q, const KVS
       atomicAdd(&p.prof[5], (unsigned long long)(clock64() - pstart));
       atomicAdd(&p.prof[6], work.part == 0 ? 1ull : 0ull);
     }
-    {
-    if constexpr (SPLIT) {
-      // The other CTAs' sums come to the first one's shared memory, in the place of the operand rings and dS, when everybody's MMAs are done.
-      if (ok && !mbar_wait(&bars.acc_full, 0, abort_flag)) {
-        if (lane == 0) report_error(status, KID_BWD, 10);
-        ok = false;
+    {  // names of its own: what the end needs is read anew
+      if constexpr (SPLIT) {
+        // The other CTAs' sums come to the first one's shared memory, in the place of the operand rings and dS, when everybody's MMAs are done.
+        if (ok && !mbar_wait(&bars.acc_full, 0, abort_flag)) {
+          if (lane == 0) report_error(status, KID_BWD, 10);
+          ok = false;
+        }
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+        tcgen05_fence_after();
+        if (ok && cluster_ctarank() > 0) bwd_send_sums<D, PARTS>(tmem_base, mapa_u32(smem_u32(sQ), 0) + (cluster_ctarank() - 1) * BWD_SUM_BYTES<D>);
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
       }
-      __syncwarp();
-      cluster_arrive();
-      cluster_wait();
-      tcgen05_fence_after();
-      if (ok && cluster_ctarank() > 0) bwd_send_sums<D, PARTS>(tmem_base, mapa_u32(smem_u32(sQ), 0) + (cluster_ctarank() - 1) * BWD_SUM_BYTES<D>);
-      __syncwarp();
-      cluster_arrive();
-      cluster_wait();
-    }
-    // dK, dV of this key block (thread t <-> key k0 + t); fp32 when they are partials of a multi-rank reduction
-    // (The block and thread are read anew: what is kept from before the loop over the steps takes registers there, and with the stores below
-    // its compute warps executed 8 % more instructions, 14.0 -> 14.6 ms at 32,768 tokens.)
-    unsigned cta, thread;
-    asm volatile("mov.u32 %0, %%ctaid.x;" : "=r"(cta));
-    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(thread));
-    const BwdWork work = bwd_work<SPLIT>(p, Cfg::BM, Cfg::BN, cta);
-    const int kv_head = work.kv_head, b = work.b, k0 = work.k0, seg = work.seg, total_steps = work.steps;
-    constexpr int SUBS = PARTS / 2;
-    const int lane = thread & 31, quarter = (thread >> 5) & 3, part = thread >> 7, which = part / SUBS, sub = part % SUBS, key = k0 + (int)(thread & 127);
-    const uint32_t t_lane = tmem_base + (uint32_t(quarter * 32) << 16);
-    const bool tm_out = !OUT_F32 && p.tma_out;
-    const long long seg_off = (long long)seg * p.seg_stride;
-    if (SPLIT && work.part > 0) {            // (its sums are with the first)
-    } else if (total_steps == 0) {
-      if (key < p.Sk && sub == 0) {
-        {
-          const long long rs_ = which == 0 ? p.dv_row : p.dk_row;
-          const long long off = seg_off + ((long long)b * p.Sk + key) * rs_ + (long long)kv_head * D;
-          if (OUT_F32) {
-            float* orow = reinterpret_cast<float*>(which == 0 ? dV_ : dK_) + off;
-            for (int u = 0; u < D / 4; ++u) reinterpret_cast<float4*>(orow)[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-          } else {
-            bf16* orow = reinterpret_cast<bf16*>(which == 0 ? dV_ : dK_) + off;
-            for (int u = 0; u < D / 8; ++u) reinterpret_cast<uint4*>(orow)[u] = make_uint4(0, 0, 0, 0);
-          }
-        }
-      }
-    } else if (ok && (SPLIT || (which == 0 ? mbar_wait(&bars.p_free, (total_steps - 1) & 1, abort_flag) : mbar_wait(&bars.acc_full, 0, abort_flag)))) {
-      // dV is complete with its last MMA, half a step before dK. Rows of 16 columns (32 bytes) of each warp's 32 keys go to TMA through the
-      // place of V, which the last dP was the last to read, and of K: stored by every thread for itself they were 16-byte pieces of 32 rows an
-      // instruction, and the end of a CTA took 3,600 (d = 64) and 7,600 cycles (d = 128) of the 20,900 and 34,000 that one of 4 x 1024,
-      // 32 heads lives.
-      tcgen05_fence_after();
-      const long long rs_ = which == 0 ? p.dv_row : p.dk_row;
-      const long long off = seg_off + ((long long)b * p.Sk + (key < p.Sk ? key : 0)) * rs_ + (long long)kv_head * D;
-      uint8_t* const stg = (which == 0 ? sV : sK) + (sub * 4 + quarter) * (D / SUBS * 64);
-      int pieces = 0;
-      // 4 x N columns of this row from `col` on, of the other CTAs, in their order
-      auto add_parts = [&](int col, uint32_t* r, int quads) {
-        for (int o = 1; SPLIT && o < p.parts; ++o) {
-          const float4* const q = reinterpret_cast<const float4*>(sQ + (o - 1) * BWD_SUM_BYTES<D>) + (which * (D / 4) + col / 4) * 128 + (thread & 127);
-#pragma unroll
-          for (int u = 0; u < 8; ++u)
-            if (u < quads) {
-              const float4 v = q[u * 128];
-              r[4 * u] = __float_as_uint(__uint_as_float(r[4 * u]) + v.x);
-              r[4 * u + 1] = __float_as_uint(__uint_as_float(r[4 * u + 1]) + v.y);
-              r[4 * u + 2] = __float_as_uint(__uint_as_float(r[4 * u + 2]) + v.z);
-              r[4 * u + 3] = __float_as_uint(__uint_as_float(r[4 * u + 3]) + v.w);
-            }
-        }
-      };
-      auto put16 = [&](int col, const uint32_t* r) {        // 16 columns of this thread's row from `col` on
-        const uint4 lo = make_uint4(pack_bf16(__uint_as_float(r[0]), __uint_as_float(r[1])), pack_bf16(__uint_as_float(r[2]), __uint_as_float(r[3])),
-                                    pack_bf16(__uint_as_float(r[4]), __uint_as_float(r[5])), pack_bf16(__uint_as_float(r[6]), __uint_as_float(r[7])));
-        const uint4 hi = make_uint4(pack_bf16(__uint_as_float(r[8]), __uint_as_float(r[9])), pack_bf16(__uint_as_float(r[10]), __uint_as_float(r[11])),
-                                    pack_bf16(__uint_as_float(r[12]), __uint_as_float(r[13])), pack_bf16(__uint_as_float(r[14]), __uint_as_float(r[15])));
-        if (tm_out) {
-          uint4* const q = reinterpret_cast<uint4*>(stg + pieces * 1024 + lane * 32);
-          q[0] = lo;
-          q[1] = hi;
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (elect_one()) {
-            const int row0 = k0 + quarter * 32;
-            if (row0 < p.Sk) tma_store_4d(which == 0 ? &tm_dv : &tm_dk, stg + pieces * 1024, col, kv_head, row0, b);
-            tma_store_commit();
-          }
-          ++pieces;
-        } else if (key < p.Sk) {
-          uint4* const q = reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(which == 0 ? dV_ : dK_) + off + col);
-          q[0] = lo;
-          q[1] = hi;
-        }
-      };
-      if (!OUT_F32 && which == 1 && p.cosT != nullptr) {
-        // dK with the inverse rotation: pairs j <-> j + D/2, 16 columns of each half of the row at a time
-        const int pos = (key < p.Sk ? key : 0) % p.rope_seq;
-        const float* cos_row = p.cosT + (long long)pos * (D / 2);
-        const float* sin_row = p.sinT + (long long)pos * (D / 2);
-#pragma unroll 1
-        for (int c = sub; c < D / 32; c += SUBS) {
-          uint32_t lo[16], hi[16];
-          tmem_ld_32x32b_x16(t_lane + Cfg::DK_COL + c * 16, lo);
-          tmem_ld_32x32b_x16(t_lane + Cfg::DK_COL + D / 2 + c * 16, hi);
-          tmem_ld_wait();
-          add_parts(c * 16, lo, 4);
-          add_parts(D / 2 + c * 16, hi, 4);
-#pragma unroll
-          for (int j = 0; j < 16; j += 4) {
-            const float4 cs = __ldg(reinterpret_cast<const float4*>(cos_row + c * 16 + j));
-            const float4 sn = __ldg(reinterpret_cast<const float4*>(sin_row + c * 16 + j));
-            const float csv[4] = {cs.x, cs.y, cs.z, cs.w}, snv[4] = {sn.x, sn.y, sn.z, sn.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const float a = __uint_as_float(lo[j + i]), b_ = __uint_as_float(hi[j + i]);
-              lo[j + i] = __float_as_uint(a * csv[i] + b_ * snv[i]);
-              hi[j + i] = __float_as_uint(b_ * csv[i] - a * snv[i]);
+      // dK, dV of this key block (thread t <-> key k0 + t); fp32 when they are partials of a multi-rank reduction
+      // (The block and thread are read anew: what is kept from before the loop over the steps takes registers there, and with the stores below
+      // its compute warps executed 8 % more instructions, 14.0 -> 14.6 ms at 32,768 tokens.)
+      unsigned cta, thread;
+      asm volatile("mov.u32 %0, %%ctaid.x;" : "=r"(cta));
+      asm volatile("mov.u32 %0, %%tid.x;" : "=r"(thread));
+      const BwdWork work = bwd_work<SPLIT>(p, Cfg::BM, Cfg::BN, cta);
+      const int kv_head = work.kv_head, b = work.b, k0 = work.k0, seg = work.seg, total_steps = work.steps;
+      constexpr int SUBS = PARTS / 2;
+      const int lane = thread & 31, quarter = (thread >> 5) & 3, part = thread >> 7, which = part / SUBS, sub = part % SUBS, key = k0 + (int)(thread & 127);
+      const uint32_t t_lane = tmem_base + (uint32_t(quarter * 32) << 16);
+      const bool tm_out = !OUT_F32 && p.tma_out;
+      const long long seg_off = (long long)seg * p.seg_stride;
+      if (SPLIT && work.part > 0) {            // (its sums are with the first)
+      } else if (total_steps == 0) {
+        if (key < p.Sk && sub == 0) {
+          {
+            const long long rs_ = which == 0 ? p.dv_row : p.dk_row;
+            const long long off = seg_off + ((long long)b * p.Sk + key) * rs_ + (long long)kv_head * D;
+            if (OUT_F32) {
+              float* orow = reinterpret_cast<float*>(which == 0 ? dV_ : dK_) + off;
+              for (int u = 0; u < D / 4; ++u) reinterpret_cast<float4*>(orow)[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            } else {
+              bf16* orow = reinterpret_cast<bf16*>(which == 0 ? dV_ : dK_) + off;
+              for (int u = 0; u < D / 8; ++u) reinterpret_cast<uint4*>(orow)[u] = make_uint4(0, 0, 0, 0);
             }
           }
-          put16(c * 16, lo);
-          put16(D / 2 + c * 16, hi);
         }
-      } else {
-        const int col_base = which == 0 ? Cfg::DV_COL : Cfg::DK_COL;
-#pragma unroll 1
-        for (int c = sub; c < D / 32; c += SUBS) {
-          uint32_t r[32];
-          tmem_ld_32x32b_x32(t_lane + col_base + c * 32, r);
-          tmem_ld_wait();
-          add_parts(c * 32, r, 8);
-          if (OUT_F32) {
-            if (key < p.Sk) {
-              float* orow = reinterpret_cast<float*>(which == 0 ? dV_ : dK_) + off + c * 32;
-#pragma unroll
-              for (int u = 0; u < 8; ++u)
-                reinterpret_cast<float4*>(orow)[u] = make_float4(__uint_as_float(r[4 * u]), __uint_as_float(r[4 * u + 1]),
-                                                                 __uint_as_float(r[4 * u + 2]), __uint_as_float(r[4 * u + 3]));
+      } else if (ok && (SPLIT || (which == 0 ? mbar_wait(&bars.p_free, (total_steps - 1) & 1, abort_flag) : mbar_wait(&bars.acc_full, 0, abort_flag)))) {
+        // dV is complete with its last MMA, half a step before dK. Rows of 16 columns (32 bytes) of each warp's 32 keys go to TMA through the
+        // place of V, which the last dP was the last to read, and of K: stored by every thread for itself they were 16-byte pieces of 32 rows an
+        // instruction, and the end of a CTA took 3,600 (d = 64) and 7,600 cycles (d = 128) of the 20,900 and 34,000 that one of 4 x 1024,
+        // 32 heads lives.
+        tcgen05_fence_after();
+        const long long rs_ = which == 0 ? p.dv_row : p.dk_row;
+        const long long off = seg_off + ((long long)b * p.Sk + (key < p.Sk ? key : 0)) * rs_ + (long long)kv_head * D;
+        uint8_t* const stg = (which == 0 ? sV : sK) + (sub * 4 + quarter) * (D / SUBS * 64);
+        int pieces = 0;
+        // 4 x N columns of this row from `col` on, of the other CTAs, in their order
+        auto add_parts = [&](int col, uint32_t* r, int quads) {
+          for (int o = 1; SPLIT && o < p.parts; ++o) {
+            const float4* const q = reinterpret_cast<const float4*>(sQ + (o - 1) * BWD_SUM_BYTES<D>) + (which * (D / 4) + col / 4) * 128 + (thread & 127);
+  #pragma unroll
+            for (int u = 0; u < 8; ++u)
+              if (u < quads) {
+                const float4 v = q[u * 128];
+                r[4 * u] = __float_as_uint(__uint_as_float(r[4 * u]) + v.x);
+                r[4 * u + 1] = __float_as_uint(__uint_as_float(r[4 * u + 1]) + v.y);
+                r[4 * u + 2] = __float_as_uint(__uint_as_float(r[4 * u + 2]) + v.z);
+                r[4 * u + 3] = __float_as_uint(__uint_as_float(r[4 * u + 3]) + v.w);
+              }
+          }
+        };
+        auto put16 = [&](int col, const uint32_t* r) {        // 16 columns of this thread's row from `col` on
+          const uint4 lo = make_uint4(pack_bf16(__uint_as_float(r[0]), __uint_as_float(r[1])), pack_bf16(__uint_as_float(r[2]), __uint_as_float(r[3])),
+                                      pack_bf16(__uint_as_float(r[4]), __uint_as_float(r[5])), pack_bf16(__uint_as_float(r[6]), __uint_as_float(r[7])));
+          const uint4 hi = make_uint4(pack_bf16(__uint_as_float(r[8]), __uint_as_float(r[9])), pack_bf16(__uint_as_float(r[10]), __uint_as_float(r[11])),
+                                      pack_bf16(__uint_as_float(r[12]), __uint_as_float(r[13])), pack_bf16(__uint_as_float(r[14]), __uint_as_float(r[15])));
+          if (tm_out) {
+            uint4* const q = reinterpret_cast<uint4*>(stg + pieces * 1024 + lane * 32);
+            q[0] = lo;
+            q[1] = hi;
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (elect_one()) {
+              const int row0 = k0 + quarter * 32;
+              if (row0 < p.Sk) tma_store_4d(which == 0 ? &tm_dv : &tm_dk, stg + pieces * 1024, col, kv_head, row0, b);
+              tma_store_commit();
             }
-          } else {
-            put16(c * 32, r);
-            put16(c * 32 + 16, r + 16);
+            ++pieces;
+          } else if (key < p.Sk) {
+            uint4* const q = reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(which == 0 ? dV_ : dK_) + off + col);
+            q[0] = lo;
+            q[1] = hi;
+          }
+        };
+        if (!OUT_F32 && which == 1 && p.cosT != nullptr) {
+          // dK with the inverse rotation: pairs j <-> j + D/2, 16 columns of each half of the row at a time
+          const int pos = (key < p.Sk ? key : 0) % p.rope_seq;
+          const float* cos_row = p.cosT + (long long)pos * (D / 2);
+          const float* sin_row = p.sinT + (long long)pos * (D / 2);
+  #pragma unroll 1
+          for (int c = sub; c < D / 32; c += SUBS) {
+            uint32_t lo[16], hi[16];
+            tmem_ld_32x32b_x16(t_lane + Cfg::DK_COL + c * 16, lo);
+            tmem_ld_32x32b_x16(t_lane + Cfg::DK_COL + D / 2 + c * 16, hi);
+            tmem_ld_wait();
+            add_parts(c * 16, lo, 4);
+            add_parts(D / 2 + c * 16, hi, 4);
+  #pragma unroll
+            for (int j = 0; j < 16; j += 4) {
+              const float4 cs = __ldg(reinterpret_cast<const float4*>(cos_row + c * 16 + j));
+              const float4 sn = __ldg(reinterpret_cast<const float4*>(sin_row + c * 16 + j));
+              const float csv[4] = {cs.x, cs.y, cs.z, cs.w}, snv[4] = {sn.x, sn.y, sn.z, sn.w};
+  #pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const float a = __uint_as_float(lo[j + i]), b_ = __uint_as_float(hi[j + i]);
+                lo[j + i] = __float_as_uint(a * csv[i] + b_ * snv[i]);
+                hi[j + i] = __float_as_uint(b_ * csv[i] - a * snv[i]);
+              }
+            }
+            put16(c * 16, lo);
+            put16(D / 2 + c * 16, hi);
+          }
+        } else {
+          const int col_base = which == 0 ? Cfg::DV_COL : Cfg::DK_COL;
+  #pragma unroll 1
+          for (int c = sub; c < D / 32; c += SUBS) {
+            uint32_t r[32];
+            tmem_ld_32x32b_x32(t_lane + col_base + c * 32, r);
+            tmem_ld_wait();
+            add_parts(c * 32, r, 8);
+            if (OUT_F32) {
+              if (key < p.Sk) {
+                float* orow = reinterpret_cast<float*>(which == 0 ? dV_ : dK_) + off + c * 32;
+  #pragma unroll
+                for (int u = 0; u < 8; ++u)
+                  reinterpret_cast<float4*>(orow)[u] = make_float4(__uint_as_float(r[4 * u]), __uint_as_float(r[4 * u + 1]),
+                                                                   __uint_as_float(r[4 * u + 2]), __uint_as_float(r[4 * u + 3]));
+              }
+            } else {
+              put16(c * 32, r);
+              put16(c * 32 + 16, r + 16);
+            }
           }
         }
+        if (tm_out && elect_one()) tma_store_wait<0>();
+      } else if (ok && lane == 0) {
+        report_error(status, KID_BWD, 10);
       }
-      if (tm_out && elect_one()) tma_store_wait<0>();
-    } else if (ok && lane == 0) {
-      report_error(status, KID_BWD, 10);
-    }
     }
   }
   if constexpr (SPLIT) {

@@ -1084,11 +1084,12 @@ Tensor decoder_stack_bwd(const Tensor& dout, const std::vector<Tensor>& xs, cons
   }
   c10::cuda::CUDAGuard guard(dout.device());
   const auto on = dout.options();
-  // Two streams where a layer keeps the device busier than the host (8 us a layer for the second): at least 12 GFLOP. Measured, us a pass, one / two:
-  // 16 layers of the 135M shape, 3 x 601 tokens 3,307 / 3,099, 8 x 1024 7,957 / 7,669; 5 layers of the 1.7B shape, 2 x 4 x 128 4,679 / 4,416, 15
-  // layers, 4 x 1024 27,443 / 26,777; 4 of the 7B shape 20,582 / 19,865; 3 of the 8B shape, 8192 tokens 52,643 / 52,411 and 53,161 / 53,033; 4 of the 1B
-  // shape, 32768 tokens 164,779 / 166,354 and 164,911 / 162,793 (no difference beyond what the power cap does from run to run); 2 layers of width 512,
-  // 512 tokens 795 / 817.
+  // Two streams where a layer keeps the device busier than the host (8 us a layer for the second): at least 12 GFLOP. Passes in turn, 12 to 24 pairs,
+  // us one / two and the middle half of the gains: 16 layers of the 135M shape, 3 x 601 tokens 3,323 / 3,129 (6.1 to 6.3 %), 8 x 1024 8,044 / 7,939
+  // (1.0 to 1.7); 16 of the 360M shape, 4 x 1024 7,972 / 7,671 (3.3 to 4.5); 5 layers of the 1.7B shape, 2 x 4 x 128 4,620 / 4,503 (2.2 to 3.1), 15
+  // layers, 4 x 1024 27,493 / 26,929 (1.4 to 2.7; on another box 0.1 to 2.0); 4 of the 7B shape, 1 x 1024 6,693 / 6,522 (1.4 to 3.0), 4 x 1024 21,323 /
+  // 21,005 (0.8 to 2.3); no difference beyond what the power cap does from run to run at 3 of the 8B shape, 8192 tokens 55,321 / 55,412 (-1.0 to 0.6)
+  // and 4 of the 1B shape, 32768 tokens 173,197 / 172,975 (-1.4 to 2.0). 2 layers of width 512, 512 tokens lose: 795 / 817.
   const double gflop = 4e-9 * n.T() * (double)(n.H * (n.Q() + n.O() + 3 * n.I));
   const cudaStream_t st = stream();
   SideStream* side = gflop >= 12 ? side_stream(st) : nullptr;

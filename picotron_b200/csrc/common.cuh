@@ -52,6 +52,10 @@ constexpr long long kWaitCycles = 4000000000LL;  // ~2 s at 2 GHz: far above any
 // earlier kernel wrote AND stores to buffers an earlier kernel may still read); (2) since every kernel in the chain waits
 // for its predecessor's completion before touching memory, completion is transitive; (3) kernels that wait on other GPUs
 // are launched normally (pdl = false). Without the launch attribute both instructions are no-ops.
+// One exception to (1): between pt_chain_begin and pt_chain_end the GEMMs load their B operand, and the SwiGLU backward its second
+// one, before pdl_wait(). Two things make that safe: the chain's first launch, and the first after a join of streams, has no
+// programmatic edge, so that everything before it is complete when any kernel of the chain starts; and no kernel of the chain
+// writes such an operand (weights, the forward's activations).
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
