@@ -1255,79 +1255,109 @@ static int launch_fwd(const CUtensorMap& mq, const KVSegs& segs, const CUtensorM
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 
-// CTAs that share the query heads of a key block (`ctas` of them): where all parts still have an SM each and the longest CTA gets four steps shorter at
-// least, as far as the parts' sums fit beside each other (3 parts for d = 64, 2 for d = 128). 3 x 601, 9 / 3 heads are 45 key blocks of up to
-// 15 steps: 36.9 us, in three parts 29.9; 2 x 256, 8 / 4 heads, 16 of up to 4: 16.4, in two 17.8. Beyond one wave the CTAs' starts and ends and the
-// clusters' (of CTAs that fill an SM) waiting for neighbouring SMs cost more than evenness gives: 8 x 1024, 9 / 3 heads 57 us, in three 98.
-// `largest`: the largest cluster that can be had.
-static int bwd_head_parts(const BwdParams& p, int d, long long ctas, int sms, int largest) {
-  const long long group = p.hq / p.hkv, steps = (p.Sq + 127) / 128 * group;
-  for (int parts = std::min(d == 64 ? 3 : 2, largest); parts > 1; --parts)
-    if (group % parts == 0 && ctas * parts <= sms && steps - steps / parts >= 4) return parts;
-  return 1;
-}
 static long long key_blocks(const BwdParams& p) { return (long long)((p.Sk + 127) / 128) * p.n_segs * p.hkv * p.B; }
+
+// Steps until the last key block is done, `slots` of them at a time in the order of bwd_work (never longer than those before) with `parts` CTAs
+// each; a CTA that has to wait for another costs the six steps of its start and end, too. -1: three waves.
+static long long bwd_span(const BwdParams& p, int parts, long long slots) {
+  const long long bps = (p.Sk + 127) / 128, num_qb = (p.Sq + 127) / 128, heads = (long long)p.hkv * p.B, n = key_blocks(p);
+  auto steps = [&](long long i) {
+    const long long of_last = i / heads - (p.n_segs - 1) * bps;          // (causal: number in the last segment, whose blocks get shorter)
+    return (p.causal && of_last > 0 ? std::max(num_qb - of_last, 0LL) : num_qb) * (p.hq / p.hkv / parts);
+  };
+  if (n > 2 * slots) return -1;
+  long long span = steps(0);
+  for (long long j = 0; j + slots < n; ++j) span = std::max(span, steps(slots - 1 - j) + 6 + steps(slots + j));
+  return span;
+}
+
+// CTAs of a cluster that share the query heads of a key block, as far as their sums fit beside each other (3 for d = 64, 2 for d = 128) and all parts
+// could have an SM each: those that save the most steps beyond what sharing costs, four, or five for three CTAs from a third of the SMs on.
+// clusters(n): how many clusters of n CTAs the device holds at a time. Of three CTAs that is 45 here, but from 41 on some came late in every
+// few launches (16 steps: 40 clusters 77 us, 42 87, 44 112, 48 117), so a ninth less is counted on; pairs are as many as said (74: 89 us, 75: 117).
+// Of 678 shapes (9 head layouts, 64 to 2,048 tokens, causal or not, at most 160 CTAs) none is more than 2 % slower than with whole blocks, and the sum
+// is 0.3 % above that of the fastest: 3 x 601, 9 / 3 heads 34.5 us, in three parts 28.7; 8 x 256 (48 blocks, two waves) stays at 21.0, in three
+// 29.1; 4 x 256 (24 blocks of 6 steps) at 18.7, in three 19.9; 8 x 384, 12 / 2 heads 40.4, in two 32.3, in three 34.6. Without room for all parts:
+// 8 x 1024, 9 / 3 heads 57 us, in three 98.
+template <class Clusters>
+static int bwd_head_parts(const BwdParams& p, int d, int sms, int largest, Clusters clusters) {
+  const long long group = p.hq / p.hkv, ctas = key_blocks(p), whole = bwd_span(p, 1, sms);
+  long long most = -1;
+  int best = 1;
+  for (int parts = std::min(d == 64 ? 3 : 2, largest); parts > 1; --parts) {
+    const long long cost = parts == 3 && 3 * 3 * ctas > sms ? 5 : 4;
+    if (group % parts || ctas * parts > sms || whole - bwd_span(p, parts, ctas) - cost <= most) continue;       // (not even if all are there at once)
+    const int at_once = clusters(parts), slots = parts == 3 ? at_once - at_once / 9 : at_once;
+    const long long span = slots > 0 ? bwd_span(p, parts, slots) : -1;
+    if (span < 0 || whole - span - cost <= most) continue;
+    most = whole - span - cost;
+    best = parts;
+  }
+  return best;
+}
 static thread_local int g_largest_cluster = 3;       // (the thread's switch, for tests and measurements)
 
-// Whether clusters of `size` CTAs of `kern` can be placed on the device: each takes an SM for itself, and an SM partition (MIG, MPS) may not have
-// as many side by side.
-template <int D, typename Kern>
-static bool bwd_clusters_fit(Kern kern, int size) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)size);
-  cfg.blockDim = dim3(BwdWarps<bwd_parts<D>()>::THREADS);
-  cfg.dynamicSmemBytes = BwdCfg<D>::SMEM;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = (unsigned)size;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess) return n > 0;
-  cudaGetLastError();
-  return false;
+template <int D, bool OUT_F32, bool PROF, bool SPLIT>
+static auto bwd_kernel() {
+  if constexpr (bwd_parts<D>() == 4) return attn_bwd_parts4_kernel<D, OUT_F32, PROF, SPLIT>;
+  else return attn_bwd_kernel<D, OUT_F32, PROF, SPLIT>;
 }
-
-// (SPLIT: p.parts CTAs of a cluster share a key block; -5, nothing launched, where such clusters cannot be had)
-template <int D, bool OUT_F32, bool PROF = false, bool SPLIT = false>
-static int launch_bwd(const CUtensorMap& mq, const KVSegs& segs, const CUtensorMap& mdo, const CUtensorMap& mdq, const CUtensorMap& mdk,
-                      const CUtensorMap& mdv, const float* lse, const float* delta, void* dk, void* dv, BwdParams p, KernelStatus* st,
-                      cudaStream_t stream) {
-  if (!PROF && p.prof != nullptr)
-    return launch_bwd<D, OUT_F32, true>(mq, segs, mdo, mdq, mdk, mdv, lse, delta, dk, dv, p, st, stream);
+// Sets the kernel up for the device; SMs, or with SPLIT the clusters of `size` CTAs that it holds at a time (an SM partition may have none), or an error
+// code below zero.
+template <int D, bool OUT_F32, bool PROF, bool SPLIT>
+static int bwd_slots(int size) {
   using Warps = BwdWarps<bwd_parts<D>()>;
-  auto kern = [] {
-    if constexpr (bwd_parts<D>() == 4) return attn_bwd_parts4_kernel<D, OUT_F32, PROF, SPLIT>;
-    else return attn_bwd_kernel<D, OUT_F32, PROF, SPLIT>;
-  }();
-  static PerDevice configured, clusters;
-  const int sms = configured.get(current_device(), [&] {
+  static PerDevice slots[2];                         // (one more, so that none is a number, too)
+  const int n = slots[size > 2].get(current_device(), [&] {
+    auto kern = bwd_kernel<D, OUT_F32, PROF, SPLIT>();
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdCfg<D>::SMEM) != cudaSuccess) return -3;
     cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     // the warpgroups share out Warps::REGS registers per thread; with fewer at launch setmaxnreg.inc would wait forever (the build
     // fails for another count, build.py: FIXED_REGISTERS)
     cudaFuncAttributes fa;
     if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess || fa.numRegs != Warps::REGS) return -6;
-    int dev = 0, n = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -3;
-    return n;
-  });
-  if (sms <= 0) return sms;
-  if constexpr (SPLIT) {
-    const int largest = clusters.get(current_device(), [&] { return bwd_clusters_fit<D>(kern, 3) ? 3 : bwd_clusters_fit<D>(kern, 2) ? 2 : 1; });
-    if (p.parts > largest) return -5;                 // (nothing launched)
-  } else {
-    const long long ctas = key_blocks(p);
-    for (int largest = g_largest_cluster; (p.parts = bwd_head_parts(p, D, ctas, sms, largest)) > 1; largest = p.parts - 1) {
-      const int rc = launch_bwd<D, OUT_F32, PROF, true>(mq, segs, mdo, mdq, mdk, mdv, lse, delta, dk, dv, p, st, stream);
-      if (rc != -5) return rc;
+    int n = 0;
+    if (!SPLIT) {
+      int dev = 0;
+      if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -3;
+      return n + 1;
     }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)size);
+    cfg.blockDim = dim3(Warps::THREADS);
+    cfg.dynamicSmemBytes = BwdCfg<D>::SMEM;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)size;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    return n + 1;
+  });
+  return n > 0 ? n - 1 : n;
+}
+
+template <int D, bool OUT_F32, bool PROF = false, bool SPLIT = false>
+static int launch_bwd(const CUtensorMap& mq, const KVSegs& segs, const CUtensorMap& mdo, const CUtensorMap& mdq, const CUtensorMap& mdk,
+                      const CUtensorMap& mdv, const float* lse, const float* delta, void* dk, void* dv, BwdParams p, KernelStatus* st,
+                      cudaStream_t stream) {
+  if (!PROF && p.prof != nullptr)
+    return launch_bwd<D, OUT_F32, true>(mq, segs, mdo, mdq, mdk, mdv, lse, delta, dk, dv, p, st, stream);
+  if constexpr (!SPLIT) {
+    const int sms = bwd_slots<D, OUT_F32, PROF, false>(1);
+    if (sms <= 0) return sms;
+    p.parts = bwd_head_parts(p, D, sms, g_largest_cluster, bwd_slots<D, OUT_F32, PROF, true>);
+    if (p.parts > 1) return launch_bwd<D, OUT_F32, PROF, true>(mq, segs, mdo, mdq, mdk, mdv, lse, delta, dk, dv, p, st, stream);
   }
   static_assert((D == 64 ? 2 : 1) * BWD_SUM_BYTES<D> <= (BwdCfg<D>::QSTAGES + BwdCfg<D>::OSTAGES) * BwdCfg<D>::TILE_BYTES + BwdCfg<D>::DS_BYTES,
                 "the parts' sums take the place of the rings and dS");
-  const cudaError_t err = launch_pdl_cluster(kern, dim3((unsigned)(key_blocks(p) * p.parts)), dim3(Warps::THREADS), BwdCfg<D>::SMEM, stream, p.parts, mq, segs,
-                                             mdo, mdq, mdk, mdv, lse, delta, dk, dv, p, st);
+  const cudaError_t err = launch_pdl_cluster(bwd_kernel<D, OUT_F32, PROF, SPLIT>(), dim3((unsigned)(key_blocks(p) * p.parts)),
+                                             dim3(BwdWarps<bwd_parts<D>()>::THREADS), BwdCfg<D>::SMEM, stream, p.parts, mq, segs, mdo, mdq, mdk, mdv,
+                                             lse, delta, dk, dv, p, st);
   pt_count_launches(1);
   return err == cudaSuccess && cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
@@ -1337,6 +1367,12 @@ static int launch_bwd(const CUtensorMap& mq, const KVSegs& segs, const CUtensorM
 
 // Largest cluster of CTAs that share a key block's query heads in the backward: 3 by default, 1: none (for the calling thread).
 extern "C" void pt_attention_set_clusters(int largest) { pt::attn::g_largest_cluster = largest; }
+// What the rule says for a device with `sms` SMs that holds two / three CTAs a cluster pairs / triples times.
+extern "C" int pt_attention_bwd_parts(int B, int Sq, int Sk, int hq, int hkv, int d, int causal, int n_segs, int sms, int pairs, int triples) {
+  pt::attn::BwdParams p{};
+  p.B = B, p.Sq = Sq, p.Sk = Sk, p.hq = hq, p.hkv = hkv, p.causal = causal, p.n_segs = n_segs;
+  return pt::attn::bwd_head_parts(p, d, sms, 3, [&](int size) { return size == 3 ? triples : pairs; });
+}
 
 // q [B,Sq,hq,d] bf16 with token stride q_row; K/V in `n_segs` segments: k_ptrs[i]/v_ptrs[i] are [B,Sk,hkv,d] bf16 with
 // token strides k_row/v_row (elements, multiples of 8) and may be peer-mapped pointers into other GPUs' memory.

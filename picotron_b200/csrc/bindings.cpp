@@ -91,6 +91,7 @@ int pt_gather_peer(void* dst, const void* const* src_ptrs, int n_src, long long 
 int pt_reduce_dkv_symm(void* const* buf_ptrs, long long offset_elems, int me, int world, long long tokens, int width,
                        void* dk, void* dv, long long dk_row, long long dv_row, cudaStream_t st);
 void pt_attention_set_clusters(int largest);
+int pt_attention_bwd_parts(int B, int Sq, int Sk, int hq, int hkv, int d, int causal, int n_segs, int sms, int pairs, int triples);
 int pt_attention_fwd_segs(const void* q, const void* const* k_ptrs, const void* const* v_ptrs, int n_segs, void* o,
                           float* lse, int B, int Sq, int Sk, int hq, int hkv, int d, long long q_row, long long k_row,
                           long long v_row, int causal, float scale, cudaStream_t st);
@@ -1404,6 +1405,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         "`counters` (layout in csrc/attention_tcgen05.cu); None switches it off. The caller keeps the tensor alive.");
   m.def("attention_set_clusters", [](int64_t largest) { pt_attention_set_clusters((int)largest); },
         "Largest cluster of CTAs that share a key block's query heads in the attention backward: 3 by default, 1: none (this thread).");
+  m.def("attention_bwd_parts", [](int64_t B, int64_t Sq, int64_t Sk, int64_t hq, int64_t hkv, int64_t d, bool causal, int64_t n_segs, int64_t sms,
+                                  int64_t pairs, int64_t triples) {
+    return pt_attention_bwd_parts((int)B, (int)Sq, (int)Sk, (int)hq, (int)hkv, (int)d, causal, (int)n_segs, (int)sms, (int)pairs, (int)triples);
+  }, "CTAs that share a key block's query heads in the attention backward of a device with `sms` SMs and room for `pairs` clusters of two\n"
+     "or `triples` clusters of three CTAs.");
   m.def("attention_fwd_segs", &attention_fwd_segs);
   m.def("attention_bwd_segs", &attention_bwd_segs);
   m.def("gemm_allreduce", &gemm_allreduce,

@@ -163,6 +163,35 @@ def test_attention_backward_of_few_key_blocks_with_long_groups(C, d, Sq, Sk, gro
         assert err <= 1e-2 * float(w.float().norm()) + 2e-3 * w.numel() ** 0.5, f"{name}: {err} of {float(w.float().norm())}"
 
 
+# us by CTAs that share a key block's query heads, on a device with 148 SMs that says it holds 74 clusters of two or 45 of three
+MEASURED_PARTS = [
+    # B, S, query heads, key/value heads, d, causal
+    (3, 601, 9, 3, 64, True, {1: 34.5, 3: 28.7}),
+    (3, 601, 9, 3, 64, False, {1: 34.8, 3: 38.1}),           # 45 blocks of one length: two waves
+    (8, 256, 9, 3, 64, True, {1: 21.0, 3: 29.1}),
+    (8, 200, 9, 3, 64, False, {1: 20.2, 3: 30.5}),
+    (3, 384, 15, 5, 64, True, {1: 25.6, 3: 28.7}),
+    (3, 384, 15, 5, 64, False, {1: 25.8, 3: 33.3}),
+    (4, 256, 9, 3, 64, False, {1: 18.7, 3: 19.9}),
+    (8, 64, 6, 1, 64, True, {1: 16.9, 2: 16.4, 3: 15.6}),
+    (8, 384, 12, 2, 64, True, {1: 40.4, 2: 32.3, 3: 34.6}),
+    (3, 1024, 12, 2, 64, True, {1: 85.5, 2: 55.8, 3: 44.0}),
+    (3, 1024, 12, 2, 64, False, {1: 88.3, 2: 57.3, 3: 76.5}),
+    (4, 256, 32, 8, 64, True, {1: 25.1, 2: 24.1}),
+    (8, 128, 32, 8, 64, True, {1: 19.2, 2: 20.7}),
+    (1, 1024, 32, 8, 128, False, {1: 92.2, 2: 61.9}),
+    (2, 601, 32, 8, 128, False, {1: 64.9, 2: 81.7}),
+]
+
+
+@pytest.mark.parametrize("B,S,hq,hkv,d,causal,us", MEASURED_PARTS)
+def test_attention_backward_shares_key_blocks_where_it_is_faster(C, B, S, hq, hkv, d, causal, us):
+    parts = C.attention_bwd_parts(B, S, S, hq, hkv, d, causal, 1, 148, 74, 45)
+    assert parts in us and us[parts] <= 1.03 * min(us.values()), parts
+    assert C.attention_bwd_parts(B, S, S, hq, hkv, d, causal, 1, 148, 0, 0) == 1          # a device that holds no clusters
+    assert C.attention_bwd_parts(B, S, S, hq, hkv, d, causal, 1, 148, 74, 0) < 3
+
+
 @pytest.mark.parametrize("largest", [3, 1])
 @pytest.mark.parametrize("d,group,S,n,causal", [(64, 6, 300, 3, True), (64, 4, 260, 2, False), (128, 4, 200, 3, True), (128, 2, 520, 1, True)])
 def test_attention_of_several_key_segments_with_long_groups(C, d, group, S, n, causal, largest):
