@@ -67,14 +67,18 @@ enum OutMode { OUT_BF16 = 0, OUT_F32_ACC = 1, OUT_F32 = 2 };
 enum Epilogue { EPI_NONE = 0, EPI_SWIGLU = 1, EPI_ROPE64 = 2, EPI_ROPE128 = 3, EPI_ADD = 4, EPI_SWIGLU_BWD = 5, EPI_CE = 6 };
 // operand stages and staging buffers per epilogue warp of each variant (see the smem budget in launch())
 // (128-column tiles: as many as fit. They are what GEMMs of few rows run with, whose k-blocks take the latency of a load from HBM divided by the
-// stages. With that and B's prefetch to L2 below the forward pass of the 135M shape on 256 tokens went from 1,368 to 1,298 us.)
-__host__ __device__ constexpr int stages_of(int epi, int bn) { return (bn == 128 ? 8 : 6) - (epi == EPI_SWIGLU_BWD ? (bn == 128 ? 2 : 1) : 0); }
+// stages. With that and B's prefetch to L2 below the forward pass of the 135M shape on 256 tokens went from 1,368 to 1,298 us. One stage less with fp32
+// results: behind most of them comes the kernel that sums the parts of K, whose CTAs find no shared memory beside eight stages and so cannot
+// wait next to the GEMM's: 512 x 1024 x 2048 in four parts 10.9 us with eight, 10.2 with seven; the pass takes 1,278 us with seven for all.)
+__host__ __device__ constexpr int stages_of(int epi, int bn, bool f32 = false) {
+  return bn != 128 ? 6 - (epi == EPI_SWIGLU_BWD) : epi == EPI_SWIGLU_BWD ? 6 : f32 ? 7 : 8;
+}
 __host__ __device__ constexpr int staging_bufs_of(int epi) { return epi == EPI_SWIGLU_BWD ? 4 : 2; }
 // a stage holds BM x BK of A and bn / 2 x BK of B; four epilogue warps stage [32 rows][128 B] per buffer
 // (MN-major operands come in boxes of 64 columns: 192-column tiles fetch 128 columns per CTA and use 96)
 __host__ __device__ constexpr int b_bytes_of(int bn) { return (bn / 2 + 63) / 64 * 64 * BK * 2; }
-__host__ __device__ constexpr int smem_bytes_of(int epi, int bn) {
-  return stages_of(epi, bn) * (A_BYTES + b_bytes_of(bn)) + 4 * staging_bufs_of(epi) * 4096 + 1024;
+__host__ __device__ constexpr int smem_bytes_of(int epi, int bn, bool f32 = false) {
+  return stages_of(epi, bn, f32) * (A_BYTES + b_bytes_of(bn)) + 4 * staging_bufs_of(epi) * 4096 + 1024;
 }
 
 struct EpiArgs {
@@ -165,7 +169,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   constexpr int BN_HALF = BN / 2;                 // columns of B per CTA
   constexpr int B_BYTES = b_bytes_of(BN), STAGE_BYTES = A_BYTES + B_BYTES;
   constexpr int LOAD_BYTES = A_BYTES + (B_MN ? B_BYTES : BN_HALF * BK * 2);      // what the loads of a stage bring
-  constexpr int STAGES = stages_of(EPI, BN);
+  constexpr int STAGES = stages_of(EPI, BN, OUT_MODE != OUT_BF16);
   pdl_launch_dependents();
   extern __shared__ uint8_t smem_raw[];
   __shared__ Barriers bars;
@@ -1184,11 +1188,11 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMa
   auto kern = gemm_pair_kernel<A_MN, B_MN, OUT_MODE, EPI_TMA, EPI, BN>;
   static PerDevice clusters_that_fit;
   const int max_clusters = clusters_that_fit.get(current_device(), [&] {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes_of(EPI, BN)) != cudaSuccess) return -3;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes_of(EPI, BN, OUT_MODE != OUT_BF16)) != cudaSuccess) return -3;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2, 1, 1);
     cfg.blockDim = dim3(NUM_THREADS, 1, 1);
-    cfg.dynamicSmemBytes = smem_bytes_of(EPI, BN);
+    cfg.dynamicSmemBytes = smem_bytes_of(EPI, BN, OUT_MODE != OUT_BF16);
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
     attr.val.clusterDim.x = 2;
@@ -1212,7 +1216,7 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMa
   if (ea.kb_per_part <= 0) ea.kb_per_part = num_kb;
   const int units = tiles * ((num_kb + ea.kb_per_part - 1) / ea.kb_per_part);
   const int clusters = units < max_clusters ? units : max_clusters;
-  const cudaError_t err = launch_pdl(kern, dim3(2 * clusters), dim3(NUM_THREADS), smem_bytes_of(EPI, BN), stream, ma, mb, md,
+  const cudaError_t err = launch_pdl(kern, dim3(2 * clusters), dim3(NUM_THREADS), smem_bytes_of(EPI, BN, OUT_MODE != OUT_BF16), stream, ma, mb, md,
                                      mh ? *mh : md, D, M, N, K, ldd, status, ea);
   pt_count_launches(1);
   return (err == cudaSuccess && cudaGetLastError() == cudaSuccess) ? 0 : -4;
